@@ -29,6 +29,7 @@
 
 #include "prof.h"
 #include "solver.h"
+#include "umma.cuh"
 
 namespace ibem {
 namespace {
@@ -40,7 +41,6 @@ constexpr int STAGE_BYTES = 2 * A_TILE + 2 * B_TILE;  // 48 KB
 constexpr int GROUP_M = 16;                         // tile order: groups of 16 row tiles, columns inner
 constexpr int TMEM_COLS = 256;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
-constexpr long long kWaitLimit = 1LL << 22;
 constexpr int64_t kMaxKChunk = 8192;  // K is processed in chunks to bound the split workspace
 
 // ---------------------------------------------------------------- split kernels
@@ -78,70 +78,7 @@ __global__ void k_split_b(int64_t k, int64_t n, const float* __restrict__ B, int
   }
 }
 
-// ---------------------------------------------------------------- PTX helpers
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(done)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-// bounded wait; false (and the error flag raised) on time-out or when another thread failed
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* err, long long limit = kWaitLimit) {
-  for (long long it = 0; it < limit; ++it) {
-    if (mbar_test(bar, parity)) return true;
-    if ((it & 255) == 255 && *reinterpret_cast<volatile int*>(err) != 0) return false;
-  }
-  atomicExch(err, 1);
-  return false;
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
-      : "memory");
-}
-// UMMA shared-memory descriptor: K-major, 64-byte swizzle (rows of BK = 32 BF16), 8-row
-// groups 512 B apart
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);  // start address (16-byte units)
-  d |= (uint64_t)1 << 16;                     // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(512 >> 4) << 32;            // stride byte offset: 8 rows x 64 B
-  d |= (uint64_t)1 << 46;                     // descriptor version for tcgen05
-  d |= (uint64_t)4 << 61;                     // SWIZZLE_64B
-  return d;
-}
-// instruction descriptor: kind::f16, D = F32, A = B = BF16, both K-major, M = 128, N = 256
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-                            ((uint32_t)(BM >> 4) << 24);
-
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t acc) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(acc)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+constexpr uint32_t kIdesc = umma_idesc(BN);
 
 #define IBEM_TMEM_LD32(taddr, r)                                                                              \
   asm volatile(                                                                                              \
@@ -229,9 +166,9 @@ __global__ void __launch_bounds__(128, 1) k_umma_bf16x3(const __grid_constant__ 
 #pragma unroll
       for (int kk = 0; kk < BK / 16; ++kk) {
         const uint32_t off = kk * 32;  // 16 BF16 = 32 bytes along K inside the 64-byte row
-        umma(tmem, umma_desc(ahi + off), umma_desc(bhi + off), (kb | kk) != 0);
-        umma(tmem, umma_desc(ahi + off), umma_desc(blo + off), 1u);
-        umma(tmem, umma_desc(alo + off), umma_desc(bhi + off), 1u);
+        umma(tmem, umma_desc(ahi + off), umma_desc(bhi + off), kIdesc, (kb | kk) != 0);
+        umma(tmem, umma_desc(ahi + off), umma_desc(blo + off), kIdesc, 1u);
+        umma(tmem, umma_desc(alo + off), umma_desc(bhi + off), kIdesc, 1u);
       }
       umma_commit(empty0 + 8 * s);  // stage s free once these MMAs have read it
       ++done;

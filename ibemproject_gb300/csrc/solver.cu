@@ -132,8 +132,12 @@ struct GridSync {
 // Each wait is one polling thread, bounded by kSpinLimit; a wait that gives up sets the
 // sticky gs->err and the CTA returns.  Flags hold the tag of the launch (unique and
 // increasing within a factorisation), so they are never cleared between launches.
-// Pivots: largest |a| to 14 bits, ties to the smallest row, so the result is deterministic.
-constexpr int kCaluMinRows = 256;   // fewest rows a CTA takes before fewer CTAs are used
+// Pivots: largest |a| to 14 bits (FP64: 11), ties to the smallest row, so the result is deterministic.
+// Fewest rows a CTA takes before fewer CTAs are used: FP32 256 (latency-bound: fewer CTAs, a
+// smaller tree), FP64 128 (FP64-pipe-bound: its own rows, the rows of the tree's eliminations and
+// those of the final solve all count).  Both divide kNoAllocMaxN / 4.
+template <typename T>
+constexpr int kCaluMinRows = sizeof(T) == 8 ? 128 : 256;
 
 __device__ __forceinline__ int ld_acquire_s32(const int* p) {
   int v;
@@ -160,7 +164,25 @@ struct CaluBufs {
 constexpr int kCaluMaxCta = 256;
 constexpr int kMetaLen = 4 * kLeaf + 1;
 
-constexpr int kPanelRmax = 4;  // rows per thread at most (1024 rows per elimination)
+// Register layout of an elimination: Lay<T>::Q lanes share a row, lane q of them holding the
+// columns c = Q cc + q; Lay<T>::SL rows are held at a time, R times over.  FP32: a thread per
+// row.  FP64: four lanes per row, because the FP64 pipe does half a lane per clock and SM
+// quarter: the elimination is bound by it, so its columns are spread over all four quarters
+// and the columns already eliminated are left out (static column bounds, loop unrolled),
+// where the FP32 one rotates its row and updates all 31.  Panel of N = 7,200: 306 us with a
+// thread per row, 256 rows to a CTA and the full-width update; 190 us in this layout with 128.
+template <typename T>
+struct Lay {
+  static constexpr int Q = 1;
+};
+template <>
+struct Lay<double> {
+  static constexpr int Q = 4;
+};
+template <typename T>
+constexpr int kPanelRows = kPanelThreads / Lay<T>::Q;   // rows per register set
+template <typename T>
+constexpr int kPanelRmax = 1024 / kPanelRows<T>;        // 1024 rows per elimination at most
 
 // Partial-pivoting elimination of the rows held in registers: thread t holds rows
 // q = t + kPanelThreads i (i < R) in a[i][*]; live[i] marks rows that exist and are not yet
@@ -240,6 +262,76 @@ __device__ __forceinline__ void calu_elim(T (&a)[R][kLeaf], bool (&live)[R], int
   __syncthreads();
 }
 
+// The same for FP64 in the four-lane layout: thread t holds of row q = t / 4 + 64 i the columns
+// 4 cc + t % 4 in a[i][cc], unrotated.  The search key takes the top 22 bits of the FP64 |a|
+// (11 exponent and 11 mantissa bits).  s_pr: the pivot row; s_rp: its reciprocal, made by the
+// one thread that holds the pivot.
+template <int R>
+__device__ __forceinline__ void calu_elim(double (&a)[R][8], bool (&live)[R], int k, double* s_top, double* s_pr,
+                                          int* s_sel, unsigned* s_key) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q = tid & 3, slot = tid >> 2;
+  constexpr int nw = kPanelThreads / 32;
+  double* s_rp = s_pr + kLeaf;
+  bool out = false;
+#pragma unroll
+  for (int jc = 0; jc < 8; ++jc) {
+#pragma unroll 1
+    for (int jq = 0; jq < 4; ++jq) {
+      const int j = 4 * jc + jq;
+      if (j >= k || out) break;   // uniform
+      unsigned key = 0;
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+        if (live[i] && q == jq)
+          key = max(key, (((((unsigned)__double2hiint(a[i][jc]) & 0x7fffffffu) >> 9) + 1u) << 10) |
+                             (unsigned)(1023 - (slot + 64 * i)));
+      key = __reduce_max_sync(0xffffffffu, key);
+      if (lane == 0) s_key[warp] = key;
+      __syncthreads();
+#pragma unroll
+      for (int w = 0; w < nw; ++w) key = max(key, s_key[w]);
+      if (key == 0) {  // uniform: no rows left for this and later pivots
+        if (tid == 0)
+          for (int jj = j; jj < k; ++jj) s_sel[jj] = -1;
+        out = true;
+        break;
+      }
+      const int bq = 1023 - (int)(key & 1023u);
+      if (slot == (bq & 63)) {   // the four lanes of the pivot row publish it
+        const int oi = bq >> 6;
+#pragma unroll
+        for (int cc = 0; cc < 8; ++cc) {
+          double v = a[0][cc];
+#pragma unroll
+          for (int i = 1; i < R; ++i) v = oi == i ? a[i][cc] : v;
+          s_pr[4 * cc + q] = v;
+          s_top[j * kLdS + 4 * cc + q] = v;
+          if (cc == jc && q == jq) *s_rp = v != 0.0 ? calu_rcp(v) : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < R; ++i) live[i] = live[i] && oi != i;
+        if (q == 0) s_sel[j] = bq;
+      }
+      __syncthreads();
+      const double rp = *s_rp;
+      double pr[8];
+#pragma unroll
+      for (int cc = jc; cc < 8; ++cc) pr[cc] = s_pr[4 * cc + q];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const double l = __shfl_sync(0xffffffffu, a[i][jc], (lane & ~3) | jq) * rp;
+        if (live[i]) {
+          if (q > jq) a[i][jc] -= l * pr[jc];
+          else if (q == jq) a[i][jc] = l;
+#pragma unroll
+          for (int cc = jc + 1; cc < 8; ++cc) a[i][cc] -= l * pr[cc];
+        }
+      }
+    }
+  }
+  __syncthreads();
+}
+
 // one polling thread per flag: threads t < n wait for flags[t] == tag (bounded by limit polls)
 __device__ __forceinline__ void calu_wait(const int* flags, int n, int tag, GridSync* gs, int* s_fail,
                                           long long limit = kSpinLimit) {
@@ -276,18 +368,23 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_panel(T* __restrict__ P, i
   int* f1 = cb.flags + kCaluMaxCta;
   int* fb = cb.flags + 2 * kCaluMaxCta;
   if (tid == 0) s_fail = 0;
-  T a[R][kLeaf];
+  constexpr int Q = Lay<T>::Q, NC = kLeaf / Q, SL = kPanelRows<T>;
+  const int lq = tid % Q, slot = tid / Q;   // this thread's column class and row in a register set
+  T a[R][NC];
   bool live[R];
   // ---- 1. local elimination of this CTA's rows
 #pragma unroll
   for (int i = 0; i < R; ++i) {
-    const int q = tid + kPanelThreads * i;
+    const int q = slot + SL * i;
     live[i] = q < nr;
 #pragma unroll
-    for (int c = 0; c < kLeaf; ++c) a[i][c] = (live[i] && c < nb) ? P[(int64_t)c * lda + r0 + q] : (T)0;
+    for (int cc = 0; cc < NC; ++cc) {
+      const int c = Q * cc + lq;
+      a[i][cc] = (live[i] && c < nb) ? P[(int64_t)c * lda + r0 + q] : (T)0;
+    }
   }
   const int kl = min(nr, nb);
-  calu_elim<T, R>(a, live, kl, s_top, s_pr, s_sel, s_key);
+  calu_elim(a, live, kl, s_top, s_pr, s_sel, s_key);
   {
     T* cv = cb.cand + (size_t)cta * kLeaf * kLeaf;
     for (int idx = tid; idx < kLeaf * nb; idx += kPanelThreads) {
@@ -306,13 +403,16 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_panel(T* __restrict__ P, i
     if (s_fail) return;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-      const int q = tid + kPanelThreads * i;
-      const int slot = cta * kLeaf + q;  // member cta + q / kLeaf, candidate q % kLeaf
-      live[i] = q < gsz * kLeaf && __ldcg(cb.cidx + slot) >= 0;
+      const int q = slot + SL * i;
+      const int cs = cta * kLeaf + q;  // member cta + q / kLeaf, candidate q % kLeaf
+      live[i] = q < gsz * kLeaf && __ldcg(cb.cidx + cs) >= 0;
 #pragma unroll
-      for (int c = 0; c < kLeaf; ++c) a[i][c] = (live[i] && c < nb) ? __ldcg(cb.cand + (size_t)slot * kLeaf + c) : (T)0;
+      for (int cc = 0; cc < NC; ++cc) {
+        const int c = Q * cc + lq;
+        a[i][cc] = (live[i] && c < nb) ? __ldcg(cb.cand + (size_t)cs * kLeaf + c) : (T)0;
+      }
     }
-    calu_elim<T, R>(a, live, nb, s_top, s_pr, s_sel, s_key);
+    calu_elim(a, live, nb, s_top, s_pr, s_sel, s_key);
     T* lv = cb.lcand + (size_t)g * kLeaf * kLeaf;
     // the nb winners only: s_sel[j] for j >= nb is not set by this elimination (ragged
     // last panel, nb < kLeaf)
@@ -335,12 +435,15 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_panel(T* __restrict__ P, i
     if (s_fail) return;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-      const int q = tid + kPanelThreads * i;
+      const int q = slot + SL * i;
       live[i] = q < G * kLeaf && __ldcg(cb.lidx + q) >= 0;
 #pragma unroll
-      for (int c = 0; c < kLeaf; ++c) a[i][c] = (live[i] && c < nb) ? __ldcg(cb.lcand + (size_t)q * kLeaf + c) : (T)0;
+      for (int cc = 0; cc < NC; ++cc) {
+        const int c = Q * cc + lq;
+        a[i][cc] = (live[i] && c < nb) ? __ldcg(cb.lcand + (size_t)q * kLeaf + c) : (T)0;
+      }
     }
-    calu_elim<T, R>(a, live, nb, s_top, s_pr, s_sel, s_key);
+    calu_elim(a, live, nb, s_top, s_pr, s_sel, s_key);
     for (int idx = tid; idx < nb * nb; idx += kPanelThreads) {
       const int j = idx / nb, c = idx % nb;
       cb.top[j * kLeaf + c] = s_top[j * kLdS + c];
@@ -388,8 +491,11 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_panel(T* __restrict__ P, i
   calu_wait(fb, 1, tag, gs, &s_fail);
   if (s_fail) return;
   for (int idx = tid; idx < kLeaf * kLeaf; idx += kPanelThreads) {
-    const int i = idx / kLeaf, c = idx % kLeaf;  // s_pr[i][c] = U11[i][i + c], zero past the block
-    s_pr[idx] = (i < nb && i + c < nb) ? __ldcg(cb.top + i * kLeaf + i + c) : (T)0;
+    const int i = idx / kLeaf, c = idx % kLeaf;
+    if constexpr (Q == 1)   // s_pr[i][c] = U11[i][i + c], zero past the block
+      s_pr[idx] = (i < nb && i + c < nb) ? __ldcg(cb.top + i * kLeaf + i + c) : (T)0;
+    else                    // s_pr[i][c] = U11[i][c]
+      s_pr[idx] = (i < nb && c < nb && c >= i) ? __ldcg(cb.top + i * kLeaf + c) : (T)0;
   }
   if (tid < kMetaLen) s_meta[tid] = __ldcg(cb.meta + tid);
   if (tid < nb) {
@@ -398,6 +504,45 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_panel(T* __restrict__ P, i
   }
   __syncthreads();
   const int nd = s_meta[3 * kLeaf];
+  if constexpr (Q > 1) {
+    for (int base = 0; base < nr; base += SL) {   // uniform trip count: the lanes of a row exchange values
+      const int rr = base + slot, r = r0 + rr;
+      const bool in = rr < nr;
+      int src = -1;
+      if (in)
+        for (int t = 0; t < nd; ++t)
+          if (s_meta[kLeaf + t] == r) src = s_meta[2 * kLeaf + t];
+      T x[NC];
+#pragma unroll
+      for (int cc = 0; cc < NC; ++cc) {
+        const int c = Q * cc + lq;
+        x[cc] = (in && c < nb) ? (src < 0 ? P[(int64_t)c * lda + r] : __ldcg(cb.orig + src * kLeaf + c)) : (T)0;
+      }
+      // x U11 = original row, right-looking over the columns left
+#pragma unroll
+      for (int kc = 0; kc < NC; ++kc) {
+#pragma unroll 1
+        for (int kq = 0; kq < Q; ++kq) {
+          const int kk = Q * kc + kq;
+          if (kk >= nb) break;
+          const T xk = __shfl_sync(0xffffffffu, x[kc], ((tid & 31) & ~(Q - 1)) | kq) * s_rinv[kk];
+          const T* ur = s_pr + kk * kLeaf + lq;
+          if (lq > kq) x[kc] -= xk * ur[Q * kc];
+          else if (lq == kq) x[kc] = xk;
+#pragma unroll
+          for (int cc = kc + 1; cc < NC; ++cc) x[cc] -= xk * ur[Q * cc];
+        }
+      }
+      if (in) {
+#pragma unroll
+        for (int cc = 0; cc < NC; ++cc) {
+          const int c = Q * cc + lq;
+          if (c < nb) P[(int64_t)c * lda + r] = r < nb ? __ldcg(cb.top + r * kLeaf + c) : x[cc];
+        }
+      }
+    }
+    return;
+  } else {
   for (int rr = tid; rr < nr; rr += kPanelThreads) {
     const int r = r0 + rr;
     if (r < nb) {
@@ -429,6 +574,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_panel(T* __restrict__ P, i
       const int col = (c + nb) & (kLeaf - 1);
       if (col < nb) P[(int64_t)col * lda + r] = x[c];
     }
+  }
   }
 }
 
@@ -553,6 +699,39 @@ __global__ void __launch_bounds__(kTrsmCols) k_trsm_small_fixed(const T* __restr
 template <typename T, int NB>
 constexpr size_t trsm_fixed_smem() {
   return sizeof(T) * (NB * NB + NB * (kTrsmCols + 1));
+}
+
+// FP64 form of the same solve, n1 <= NB.  One thread per column runs its n1^2 / 2 multiply-adds
+// through one quarter of an SM's FP64 pipe (64 clocks per warp instruction): 8 lanes share a
+// column instead, rows 8 r + q to lane q, so that a launch of a few hundred columns still
+// spreads over all SMs.  16 columns per CTA.  n1 = 64, 3,600 columns: 150 us with a thread per
+// column and the columns in shared memory, 17 us here.
+constexpr int kTrsm64Cols = 16;
+template <int NB>
+__global__ void __launch_bounds__(8 * kTrsm64Cols) k_trsm_f64(const double* __restrict__ L, int64_t ldl, int n1,
+                                                  double* __restrict__ B, int64_t ldb, int64_t n2) {
+  __shared__ double sL[NB * NB];   // [i][k] = L(k, i) for k > i, else 0
+  const int q = threadIdx.x & 7, lane = threadIdx.x & 31;
+  const int64_t c = blockIdx.x * (int64_t)kTrsm64Cols + (threadIdx.x >> 3);
+  for (int idx = threadIdx.x; idx < NB * NB; idx += 8 * kTrsm64Cols) {
+    const int k = idx % NB, i = idx / NB;
+    sL[idx] = (k > i && k < n1) ? L[(int64_t)i * ldl + k] : 0.0;
+  }
+  double x[NB / 8];
+  double* b = B + c * ldb;
+#pragma unroll
+  for (int r = 0; r < NB / 8; ++r) x[r] = (c < n2 && 8 * r + q < n1) ? b[8 * r + q] : 0.0;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < NB; ++i) {
+    const double xi = __shfl_sync(0xffffffffu, x[i / 8], (lane & ~7) | (i & 7));
+    if (q > (i & 7)) x[i / 8] -= sL[i * NB + (i & ~7) + q] * xi;
+#pragma unroll
+    for (int r = i / 8 + 1; r < NB / 8; ++r) x[r] -= sL[i * NB + 8 * r + q] * xi;
+  }
+#pragma unroll
+  for (int r = 0; r < NB / 8; ++r)
+    if (c < n2 && 8 * r + q < n1) b[8 * r + q] = x[r];
 }
 
 // ---------------------------------------------------------------- SIMT GEMM  C -= A B
@@ -965,17 +1144,19 @@ size_t trsv_persist_smem() {
 
 template <typename T>
 cudaError_t set_solver_smem_attrs() {
-  cudaError_t e = cudaFuncSetAttribute((const void*)k_trsm_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(2 * 64 * 65 * sizeof(T)));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute((const void*)k_gemm_sub_smallk<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)gemm_smallk_smem<T>());
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute((const void*)k_trsm_small_fixed<T, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)trsm_fixed_smem<T, 32>());
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute((const void*)k_trsm_small_fixed<T, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)trsm_fixed_smem<T, 64>());
+  cudaError_t e = cudaFuncSetAttribute((const void*)k_gemm_sub_smallk<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)gemm_smallk_smem<T>());
+  if constexpr (sizeof(T) == sizeof(float)) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute((const void*)k_trsm_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)(2 * 64 * 65 * sizeof(T)));
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute((const void*)k_trsm_small_fixed<T, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)trsm_fixed_smem<T, 32>());
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute((const void*)k_trsm_small_fixed<T, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)trsm_fixed_smem<T, 64>());
+  }
   const int inv = (int)(sizeof(T) * (kTrsvB * (kTrsvB + 1) + kTrsvB));
   const int ps = (int)trsv_persist_smem<T>();
   if (e == cudaSuccess)
@@ -1020,7 +1201,7 @@ struct LuWork {
   int* tflags = nullptr;     // per-block release flags of the triangular solves
   int ttag = 0;              // tag of the last triangular-solve launch
   int trsv_grid = 0;         // co-resident CTAs of the persistent triangular solve
-  void* gemm_ws = nullptr;   // BF16 split workspace of the tensor-core GEMM (FP32 LU only)
+  void* gemm_ws = nullptr;   // BF16 split workspace of the tensor-core GEMM
   size_t gemm_ws_bytes = 0;
   int* gemm_err = nullptr;   // raised by the tensor-core GEMM's bounded waits
 };
@@ -1028,7 +1209,7 @@ struct LuWork {
 template <typename T>
 static ibem_status panel(T* A, int64_t lda, int64_t k0, int64_t m, int nb, LuWork<T>& w, cudaStream_t st) {
   // CTAs: at most one per SM, at least kCaluMinRows rows each; the tree's fan-in F ~ sqrt
-  int ncta = (int)std::max<int64_t>(1, std::min<int64_t>(w.ncta, (m + kCaluMinRows - 1) / kCaluMinRows));
+  int ncta = (int)std::max<int64_t>(1, std::min<int64_t>(w.ncta, (m + kCaluMinRows<T> - 1) / kCaluMinRows<T>));
   int rows_per = (int)((m + ncta - 1) / ncta);
   ncta = (int)((m + rows_per - 1) / rows_per);
   int F = 1;
@@ -1036,11 +1217,19 @@ static ibem_status panel(T* A, int64_t lda, int64_t k0, int64_t m, int nb, LuWor
   const int G = (ncta + F - 1) / F;
   // rows of the largest elimination (own rows, a group's or the root's candidates)
   const int rows = std::max(rows_per, std::max(F, G) * kLeaf);
-  if (rows > kPanelThreads * kPanelRmax || ncta > kCaluMaxCta)
-    return fail(IBEM_ERR_ARG, "panel too tall for the panel kernel");
-  const void* fn = rows <= kPanelThreads       ? (const void*)k_panel<T, 1>
-                   : rows <= 2 * kPanelThreads ? (const void*)k_panel<T, 2>
-                                               : (const void*)k_panel<T, 4>;
+  if (rows > 1024 || ncta > kCaluMaxCta) return fail(IBEM_ERR_ARG, "panel too tall for the panel kernel");
+  const int sets = (rows + kPanelRows<T> - 1) / kPanelRows<T>;   // register sets of rows
+  const void* fn = nullptr;
+  if constexpr (sizeof(T) == 8)
+    fn = sets <= 2   ? (const void*)k_panel<T, 2>
+         : sets <= 4 ? (const void*)k_panel<T, 4>
+         : sets <= 6 ? (const void*)k_panel<T, 6>
+         : sets <= 8 ? (const void*)k_panel<T, 8>
+                     : (const void*)k_panel<T, 16>;
+  else
+    fn = sets <= 1   ? (const void*)k_panel<T, 1>
+         : sets <= 2 ? (const void*)k_panel<T, 2>
+                     : (const void*)k_panel<T, 4>;
   T* P = A + k0 * lda + k0;
   int mm = (int)m;
   int* ip = w.ipiv_dev + k0;
@@ -1060,8 +1249,12 @@ static ibem_status gemm_sub(int64_t m, int64_t n, int64_t k, const T* A, int64_t
 template <>
 ibem_status gemm_sub<double>(int64_t m, int64_t n, int64_t k, const double* A, int64_t lda, const double* B,
                              int64_t ldb, double* C, int64_t ldc, LuWork<double>& w, cudaStream_t st) {
-  (void)w;
   if (m <= 0 || n <= 0 || k <= 0) return IBEM_OK;
+  // tensor cores from 32 in every dimension: a 64 x 64 SIMT tile takes 1.08 us per unit of k on
+  // the FP64 pipe (34 us at k = 32), a whole tensor-core call of that size 25 us (300 spheres,
+  // N = 7,200: all updates 246 ms on the FP64 pipe, 29 ms on the tensor cores)
+  if (w.gemm_ws && m >= 32 && n >= 32 && k >= 32)
+    return gemm_sub_f64_tc(m, n, k, A, lda, B, ldb, C, ldc, w.gemm_ws, w.gemm_ws_bytes, w.gemm_err, st);
   ProfScope ps(PROF_GEMM_SIMT, st, 2.0 * m * n * k);
   dim3 grid((unsigned)((m + 63) / 64), (unsigned)((n + 63) / 64));
   if (k <= kSmallK)
@@ -1098,10 +1291,14 @@ static ibem_status trsm(const T* L, int64_t ldl, int64_t n1, T* B, int64_t ldb, 
   if (n1 <= 0 || n2 <= 0) return IBEM_OK;
   if (n1 <= 64) {
     ProfScope ps(PROF_TRSM_SMALL, st);
-    if (n1 == 32)
+    if constexpr (sizeof(T) == sizeof(double)) {
+      const unsigned grid = (unsigned)((n2 + kTrsm64Cols - 1) / kTrsm64Cols);
+      if (n1 <= 32) ::ibem::count_launch(), k_trsm_f64<32><<<grid, 8 * kTrsm64Cols, 0, st>>>(L, ldl, (int)n1, B, ldb, n2);
+      else ::ibem::count_launch(), k_trsm_f64<64><<<grid, 8 * kTrsm64Cols, 0, st>>>(L, ldl, (int)n1, B, ldb, n2);
+    } else if (n1 == 32)
       ::ibem::count_launch(), k_trsm_small_fixed<T, 32><<<(unsigned)((n2 + kTrsmCols - 1) / kTrsmCols), kTrsmCols,
                                                           trsm_fixed_smem<T, 32>(), st>>>(L, ldl, B, ldb, n2);
-    else if (n1 == 64 && sizeof(T) == sizeof(float))
+    else if (n1 == 64)
       ::ibem::count_launch(), k_trsm_small_fixed<T, 64><<<(unsigned)((n2 + kTrsmCols - 1) / kTrsmCols), kTrsmCols,
                                                           trsm_fixed_smem<T, 64>(), st>>>(L, ldl, B, ldb, n2);
     else
@@ -1156,10 +1353,10 @@ static ibem_status lu_alloc(LuWork<T>& w, int64_t N) {
   IBEM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   IBEM_CUDA(set_solver_smem_attrs<T>());
   int per_sm = 0;
-  IBEM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_panel<T, kPanelRmax>, kPanelThreads, 0));
+  IBEM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_panel<T, kPanelRmax<T>>, kPanelThreads, 0));
   if (per_sm < 1) return fail(IBEM_ERR_CUDA, "panel kernel cannot be resident");
   w.ncta = std::min(nsm, kCaluMaxCta);  // at most one CTA per SM (co-resident for the cooperative launch)
-  if ((int64_t)w.ncta * kPanelThreads * kPanelRmax < N) return fail(IBEM_ERR_ARG, "matrix too large for the panel kernel");
+  if ((int64_t)w.ncta * 1024 < N) return fail(IBEM_ERR_ARG, "matrix too large for the panel kernel");
   IBEM_CUDA(cudaMalloc(&w.cb_mem, calu_bytes<T>(w.ncta)));
   IBEM_CUDA(cudaMemset(w.cb_mem, 0, calu_bytes<T>(w.ncta)));
   w.cb = calu_carve<T>(static_cast<unsigned char*>(w.cb_mem), w.ncta);
@@ -1186,6 +1383,15 @@ static ibem_status lu_alloc(LuWork<T>& w, int64_t N) {
     IBEM_CUDA(cudaMalloc(&w.gemm_ws, w.gemm_ws_bytes));
     IBEM_CUDA(cudaMalloc(&w.gemm_err, sizeof(int)));
     IBEM_CUDA(cudaMemset(w.gemm_err, 0, sizeof(int)));
+  } else {
+    w.gemm_ws_bytes = gemm_tc64_workspace_bytes(N, N / 2 + 2 * kLeaf);
+    if (cudaMalloc(&w.gemm_ws, w.gemm_ws_bytes) != cudaSuccess) {   // no room: the updates stay on the FP64 pipe
+      cudaGetLastError();
+      w.gemm_ws = nullptr;
+    } else {
+      IBEM_CUDA(cudaMalloc(&w.gemm_err, sizeof(int)));
+      IBEM_CUDA(cudaMemset(w.gemm_err, 0, sizeof(int)));
+    }
   }
   return IBEM_OK;
 }
@@ -1757,9 +1963,20 @@ ibem_status solve_dense(ibem_solver_form form, int64_t N, double* A, int64_t lda
       s = lu_apply<double>(W, N, N, w, ys, st);
       if (!s) s = sticky_err(w, st);
     }
-    cudaEventRecord(e2, st);
     if (!s) s = finish_norm();
     if (!s) s = scaled_backward_error(cx, A, lda, ys, bs, rvec, tmp, as_norm, R.backward_error);
+    if (!s && w.gemm_ws && std::isfinite(R.backward_error)) {
+      // One step of refinement.  The tensor-core updates round normwise (to the largest entry
+      // of a row and column), which costs the small entries of the solution digits that an
+      // FP64 residual gives back: 300 spheres (N = 7,200) against a 64-bit solution 9.3e-15
+      // with FP64 updates, 4.9e-14 with the tensor-core updates alone, 2.0e-15 with this step
+      // (1.2 ms of 86).
+      s = lu_apply<double>(W, N, N, w, rvec, st);
+      if (!s) s = sticky_err(w, st);
+      if (!s) ::ibem::count_launch(), k_axpby<<<nb, 256, 0, st>>>(N, 1.0, rvec, 1.0, ys);
+      if (!s) s = scaled_backward_error(cx, A, lda, ys, bs, rvec, tmp, as_norm, R.backward_error);
+    }
+    cudaEventRecord(e2, st);
     lu_free(w);
     cudaFree(W);
   } else if (form == IBEM_SOLVE_GMRES_BJ) {
@@ -1960,7 +2177,7 @@ constexpr size_t kNaW = 0;                                                      
 constexpr size_t kNaVec = align256(sizeof(double) * kNoAllocMaxN * kNoAllocMaxN);    // 6 N-vectors
 constexpr size_t kNaPerm = kNaVec + 6 * align256(sizeof(double) * kNoAllocMaxN);     // perm, ipiv
 constexpr size_t kNaCand = kNaPerm + 2 * align256(sizeof(int) * kNoAllocMaxN);
-constexpr int kNoAllocCaluCta = (int)((kNoAllocMaxN + kCaluMinRows - 1) / kCaluMinRows);  // panel CTAs at most
+constexpr int kNoAllocCaluCta = (int)((kNoAllocMaxN + 255) / 256);  // panel CTAs at most
 constexpr size_t kNaGs = kNaCand + calu_bytes<double>(kNoAllocCaluCta);                    // panel buffers
 constexpr size_t kNaInfo = kNaGs + align256(sizeof(GridSync));
 constexpr size_t kNaPart = kNaInfo + align256(sizeof(int));
@@ -2024,7 +2241,7 @@ static ibem_status noalloc_setup(int dev, unsigned char** base, int* ncta, int* 
     IBEM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     IBEM_CUDA(set_solver_smem_attrs<double>());
     int per_sm = 0;
-    IBEM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_panel<double, kPanelRmax>, kPanelThreads, 0));
+    IBEM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_panel<double, kPanelRmax<double>>, kPanelThreads, 0));
     if (per_sm < 1) return fail(IBEM_ERR_CUDA, "solve_noalloc: panel kernel cannot be resident");
     int per_tr = 0;
     IBEM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_tr, k_trsv_persist<double, true, true>, kTrsvThreads,

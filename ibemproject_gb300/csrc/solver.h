@@ -17,6 +17,13 @@ ibem_status gemm_sub_f32_tc(int64_t m, int64_t n, int64_t k, const float* A, int
                             cudaStream_t st);
 size_t gemm_tc_workspace_bytes(int64_t max_m, int64_t max_n);
 
+// The same with FP64 storage and at least FP64 accuracy (gemm_tc64.cu), any sizes; `ws` of at
+// least gemm_tc64_workspace_bytes(max m, max n) bytes.
+ibem_status gemm_sub_f64_tc(int64_t m, int64_t n, int64_t k, const double* A, int64_t lda, const double* B,
+                            int64_t ldb, double* C, int64_t ldc, void* ws, size_t ws_bytes, int* err,
+                            cudaStream_t st);
+size_t gemm_tc64_workspace_bytes(int64_t max_m, int64_t max_n);
+
 // block: diagonal block size of the IBEM_SOLVE_GMRES_BJ form (1..80; unknowns per particle);
 // ws32: optional FP32 workspace of that form, ((N + 3) / 4 * 4) x N floats (allocated and
 // freed inside when null).
