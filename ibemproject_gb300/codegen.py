@@ -37,6 +37,8 @@ import os
 import re
 from collections import OrderedDict
 
+from . import codegen_mf60
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 
 # radial functions: name -> (kind, data)
@@ -772,6 +774,7 @@ def generate(out_dir: str | None = None) -> dict:
                 parts.append(gen_bem_stress_function(f"bem_stress_o{o}_w{wn}_n{n}", o, W, [n]))
     parts.append(gen_bem_stress_function("bem_stress_post", 0, (), [0, 1, 2]))
     files["gen_bem.cuh"] = "\n\n".join(parts) + "\n"
+    files["gen_mf60.cuh"] = codegen_mf60.generate_source()
     for fn, src in files.items():
         path = os.path.join(out_dir, fn)
         old = open(path).read() if os.path.exists(path) else None

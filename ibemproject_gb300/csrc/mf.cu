@@ -896,6 +896,10 @@ ibem_status mf_batch_init(MfBatch& b, const ibem_e3d_batch& in, cudaStream_t st,
   ::ibem::count_launch(), k_mf_prep<<<nblk(b.num), 256, 0, st>>>(b.nu, b.num, b.cen, b.rad, b.seg_of, b.matd, b.gh, b.gl,
                                                                  b.dr, b.dc);
   IBEM_LAUNCH_CHECK("mf prep");
+  if (b.nu == 60) {
+    IBEM_CUDA(alloc_async((void**)&b.self60, sizeof(double) * 3600 * in.nseg, st));
+    if (ibem_status q = mf60_self(b, b.self60, st)) return q;
+  }
   // the host vectors above must outlive the copies
   IBEM_CUDA(cudaStreamSynchronize(st));
   return IBEM_OK;
@@ -910,6 +914,7 @@ void mf_batch_free(MfBatch& b) {
   free_async(b.matd, st);
   free_async(b.matf, st);
   free_async(b.mats, st);
+  free_async(b.self60, st);
   free_async(b.dr, st);
   free_async(b.dc, st);
   free_async(b.tiles, st);
@@ -1069,7 +1074,7 @@ ibem_status mf_tune(MfBatch& b, cudaStream_t st) {
   float best_ms = 1e30f;
   for (int ts = 0; ts < 3 && !s; ++ts)
     for (int h : slice_candidates(b.ntiles_s[ts], b.max_seg, sms)) {
-      if (b.nu == 60 && ts != 1) break;   // the layout-60 products have 128-target tiles only
+      if (b.nu == 60 && ts != 0) break;   // the layout-60 products have 64-target tiles only
       for (int pers = 0; pers < (b.nu == 60 ? 1 : 2) && !s; ++pers) {
         if ((s = mf_set_f32_shape(b, ts, h, pers, st))) break;
         float ms = 0.f;
@@ -1084,7 +1089,7 @@ ibem_status mf_tune(MfBatch& b, cudaStream_t st) {
       if (s) break;
     }
   best_ms = 1e30f;
-  for (int h : slice_candidates(b.ntiles, b.max_seg, sms)) {
+  for (int h : slice_candidates(b.nu == 60 ? b.ntiles_s[0] : b.ntiles, b.max_seg, sms)) {
     if (s) break;
     b.hsplit_wide = h;
     float ms = 0.f;
@@ -1121,8 +1126,8 @@ void launch_f32(const MfBatch& b, const float* x, float* y, cudaStream_t st, con
 
 ibem_status mf_apply_f32(const MfBatch& b, const float* x, float* y, cudaStream_t st, const int* mask, int mask_on) {
   ProfScope ps(PROF_MF_F32, st, 0.0);
-  IBEM_CUDA(cudaMemsetAsync(y, 0, sizeof(float) * b.N, st));
   if (b.nu == 60) return mf60_apply_f32(b, x, y, st, mask, mask_on);
+  IBEM_CUDA(cudaMemsetAsync(y, 0, sizeof(float) * b.N, st));
   if (b.tshape == 0) launch_f32<64>(b, x, y, st, mask, mask_on);
   else if (b.tshape == 2) launch_f32<256>(b, x, y, st, mask, mask_on);
   else launch_f32<128>(b, x, y, st, mask, mask_on);
@@ -1132,8 +1137,8 @@ ibem_status mf_apply_f32(const MfBatch& b, const float* x, float* y, cudaStream_
 
 ibem_status mf_apply_f64(const MfBatch& b, const double* x, double* y, cudaStream_t st, const int* mask, int mask_on) {
   ProfScope ps(PROF_MF_F64, st, 0.0);
-  IBEM_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * b.N, st));
   if (b.nu == 60) return mf60_apply_f64(b, x, y, st, mask, mask_on);
+  IBEM_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * b.N, st));
   // near sources in FP64, far sources (beyond kMfFarRadii of their radius from the box of
   // the warp's targets) in double-float: their contributions are at most kMfFarRadii^-3 of a
   // touching one, so the double-float rounding (~2^-44 per operation, times 4^-3) is ~1e-15
@@ -1158,8 +1163,8 @@ ibem_status mf_apply_f64(const MfBatch& b, const double* x, double* y, cudaStrea
 
 ibem_status mf_apply_f64_all(const MfBatch& b, const double* x, double* y, cudaStream_t st) {
   ProfScope ps(PROF_MF_F64, st, 0.0);
-  IBEM_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * b.N, st));
   if (b.nu == 60) return mf60_apply_f64(b, x, y, st, nullptr, 1);
+  IBEM_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * b.N, st));
   ::ibem::count_launch(), k_mf_apply_f64<<<dim3(b.ntiles, b.hsplit_wide), kMfThreads, 0, st>>>(
       b.tiles, b.seg_begin, nullptr, 1, b.cen, b.rad, b.mats, x, y, b.perm, 0);
   IBEM_LAUNCH_CHECK("mf apply f64 (all pairs)");
@@ -1168,8 +1173,8 @@ ibem_status mf_apply_f64_all(const MfBatch& b, const double* x, double* y, cudaS
 
 ibem_status mf_apply_df(const MfBatch& b, const double* x, double* y, cudaStream_t st, const int* mask, int mask_on) {
   ProfScope ps(PROF_MF_DF, st, 0.0);
-  IBEM_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * b.N, st));
   if (b.nu == 60) return mf60_apply_f64(b, x, y, st, mask, mask_on);   // no double-float form of layout 60
+  IBEM_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * b.N, st));
   ::ibem::count_launch(), k_mf_apply_df<kMfThreads><<<dim3(b.ntiles, b.hsplit_wide), kMfThreads, 0, st>>>(
       b.tiles, b.seg_begin, mask, mask_on, b.cen, b.rad, b.mats, x, y, b.perm, 0);
   IBEM_LAUNCH_CHECK("mf apply df");

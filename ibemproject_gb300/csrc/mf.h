@@ -27,6 +27,8 @@ namespace ibem {
 constexpr int kMfNu = 24;   // unknowns per particle of the matrix-free path
 constexpr int kKnn = 16;    // neighbours per particle of the learned preconditioner
 
+constexpr int kMf60Targets = 64;   // targets per CTA of the layout-60 products (tiles_s[0])
+
 struct MfTile {
   int seg, s0, ns, pad;     // one CTA's target particles s0 .. s0 + ns - 1 of segment seg
 };
@@ -58,6 +60,7 @@ struct MfBatch {
   SphMat* matd = nullptr;     // per segment, physical units
   SphMatF* matf = nullptr;    // per segment, divided by mu0
   SphMat* mats = nullptr;     // per segment, FP64, divided by mu0 (scaled system)
+  double* self60 = nullptr;   // layout 60: own block of each realisation's particles, column-major (scaled system)
   double* dr = nullptr;       // N: row scaling
   double* dc = nullptr;       // N: column scaling
   MfTile* tiles = nullptr;
@@ -75,12 +78,13 @@ struct MfBatch {
   int nwork = 0, persist_ctas = 0;
 };
 
-// layout-60 products (mf60.cu): FP32 and FP64 (the double-float entry points fall back to
-// FP64 there), the realisations' block-Jacobi inverses (Pseg: nseg x 60 x 60) and their
+// layout-60 products (mf60.cu; y is overwritten): FP32 and FP64 (the double-float entry points
+// fall back to FP64 there), the realisations' block-Jacobi inverses (Pseg: nseg x 60 x 60) and their
 // application
 ibem_status mf60_apply_f32(const MfBatch& b, const float* x, float* y, cudaStream_t st, const int* mask, int mask_on);
 ibem_status mf60_apply_f64(const MfBatch& b, const double* x, double* y, cudaStream_t st, const int* mask,
                            int mask_on);
+ibem_status mf60_self(const MfBatch& b, double* S, cudaStream_t st);   // fills b.self60 (nseg x 60 x 60)
 ibem_status mf60_block_jacobi(const MfBatch& b, float* Pseg, cudaStream_t st);
 ibem_status mf60_precond_apply(const MfBatch& b, const float* Pseg, const float* v, float* z, const int* kdev,
                                int64_t vstride, cudaStream_t st);

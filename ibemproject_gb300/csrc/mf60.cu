@@ -1,20 +1,25 @@
-// Matrix-free products of the layout-60 sphere systems (eigenstrain orders 0, 1 and 2):
-// the pair blocks that ibem_e3d_pair_blocks(layout 60) assembles (integratorElastic3D.cpp:
+// Matrix-free products of the layout-60 sphere systems (eigenstrain orders 0, 1 and 2): the
+// pair blocks that ibem_e3d_pair_blocks(layout 60) assembles (integratorElastic3D.cpp:
 // 341-682: ...EquivalentInclusion, ...FirstOrderInclusion, ...SecondOrderInclusion) are
-// evaluated inside the product from the generated straight-line code (gen_sphere60*.cuh),
-// so a batch of quadratic realisations is solved without storing its matrices.
+// applied inside the product (mf60_contract.cuh: in the frame of the pair's offset, where a
+// block has 520 entries instead of 3,600), so a batch of quadratic realisations is solved
+// without storing its matrices.
 //
 // Scaled system As = Dr A Dc with Dr = a_s^order / mu0 (rows of target s), Dc = a_h^-order
 // (columns of source h): in coordinates x' = (c_s - c_h) / a_h and with the moduli divided by
-// mu0 a block is the unit-sphere block times (a_s / a_h)^(row order).  The kernels stage the
-// sources' coefficients already multiplied by a_h^-(row order) and multiply the sums by
-// a_s^(row order) once, then add the self term C0 / mu0.
+// mu0 a block is the unit-sphere block times (a_s / a_h)^(row order).  The kernels scale a
+// source's powers of 1/r by a_h^-(row order) and the sums by a_s^(row order) once.
 //
-// One thread per target particle, 128 consecutive targets of one realisation per CTA, source
-// slices over gridDim.y; one kernel per row order (6, 18 and 36 rows) and group of columns
-// (the generated sub-blocks, the largest split into groups of 6 columns), so that its sums
-// and the straight-line code's values stay in registers: FP32 (the GMRES operator) and FP64
-// (the refinement residuals).
+// One thread per target particle, 64 consecutive targets of one realisation per CTA, source
+// slices over gridDim.y, partial sums added atomically to the target's own block times its
+// coefficients (k_self_apply60, which also clears the sums).  A target whose centre lies
+// inside a source (overlapping spheres) takes that pair from the generated dense block.
+//
+// Bound by the FP32 (FP64) multiply-adds.  FP32: one kernel for all 60 rows, which rotates a
+// source's coefficients once.  FP64: one kernel per row order, because 60 sums and 60 rotated
+// coefficients do not fit 255 registers; the rotation of the coefficients is repeated.
+// Measured, 12 realisations of 50 to 300 spheres (437,000 pairs): FP32 product 1.13 -> 0.14 ms,
+// FP64 product 45.2 -> 5.0 ms, against the generated blocks in 18 and 7 kernels.
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -22,14 +27,15 @@
 #include "gen_sphere60.cuh"
 #include "gen_sphere60_f32.cuh"
 #include "mf.h"
+#include "mf60_contract.cuh"
 #include "prof.h"
 
 namespace ibem {
 namespace {
 
 constexpr int kNu = 60;
-constexpr int kT = 128;      // targets per CTA
-constexpr int kChunk = 16;   // sources staged per chunk
+constexpr int kT = kMf60Targets;   // targets per CTA
+constexpr int kChunk = 16;         // sources staged per chunk
 
 template <int RO>
 struct Rows;
@@ -46,91 +52,94 @@ struct Rows<2> {
   static constexpr int off = 24, n = 36;
 };
 
-__device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
-__device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
-
-// acc[r - off] += v * xs[c] for the rows of order RO (the generated functions of one row
-// order emit only those rows; the self function emits all of them, the others are skipped)
-template <class T, int RO>
+// acc[r] += v * xs[c]
+template <class T>
 struct RowSink {
   T* acc;
-  const T* __restrict__ xs;
-  __device__ __forceinline__ void operator()(int r, int c, T v) const {
-    if (r >= Rows<RO>::off && r < Rows<RO>::off + Rows<RO>::n) acc[r - Rows<RO>::off] = fma_t(v, xs[c], acc[r - Rows<RO>::off]);
-  }
+  const T* xs;
+  __device__ __forceinline__ void operator()(int r, int c, T v) const { acc[r] += v * xs[c]; }
 };
 
-template <class T>
-__device__ __forceinline__ T powi(T v, int n) {
-  return n == 0 ? T(1) : (n == 1 ? v : v * v);
-}
-
-// The generated FP32 sub-blocks one launch evaluates: row order RO, group F (RO 0: F -1,
-// all columns; RO 1: F 0 the order-0 and order-1 columns, F 1..6 the order-2 columns of pair
-// F - 1; RO 2: F 0 the order-0 columns, F 1..3 the order-1 columns of pairs 2(F-1),
-// 2(F-1)+1, F 4..9 the order-2 columns of pair F - 4).  The launch with F <= 0 adds the
-// self term.  (FP64: whole column orders, F = CO; splitting them repeats the shared
-// intermediates on the FP64 pipe, which costs more than the spills it saves.)
-template <class T, int RO, int F, class Sink, class M>
-__device__ __forceinline__ void blk(T x0, T x1, T x2, const M& mc, Sink& sk) {
-  const T one = T(1);
-  if constexpr (std::is_same<T, double>::value) {
-    if constexpr (RO == 0) {
-      sph_block60_c0_r0(x0, x1, x2, one, mc, sk);
-      sph_block60_c1_r0(x0, x1, x2, one, mc, sk);
-      sph_block60_c2_r0(x0, x1, x2, one, mc, sk);
-    } else if constexpr (RO == 1) {
-      if constexpr (F == 0) sph_block60_c0_r1(x0, x1, x2, one, mc, sk);
-      else if constexpr (F == 1) sph_block60_c1_r1(x0, x1, x2, one, mc, sk);
-      else sph_block60_c2_r1(x0, x1, x2, one, mc, sk);
-    } else {
-      if constexpr (F == 0) sph_block60_c0_r2(x0, x1, x2, one, mc, sk);
-      else if constexpr (F == 1) sph_block60_c1_r2(x0, x1, x2, one, mc, sk);
-      else sph_block60_c2_r2(x0, x1, x2, one, mc, sk);
-    }
-    return;
-  } else {
-#define IBEM_B(NM) sph_block60f##NM(x0, x1, x2, one, mc, sk)
-#define IBEM_BM(NM) sph_block60fm##NM(x0, x1, x2, one, mc, sk)
-  if constexpr (RO == 0) {
-    IBEM_BM(_c0_r0);
-    IBEM_BM(_c1_r0);
-    IBEM_BM(_c2_r0);
-  } else if constexpr (RO == 1) {
-    if constexpr (F == 0) {
-      IBEM_BM(_c0_r1);
-      IBEM_BM(_c1_r1);
-    } else if constexpr (F == 1) IBEM_B(_c2g0_r1);
-    else if constexpr (F == 2) IBEM_B(_c2g1_r1);
-    else if constexpr (F == 3) IBEM_B(_c2g2_r1);
-    else if constexpr (F == 4) IBEM_B(_c2g3_r1);
-    else if constexpr (F == 5) IBEM_B(_c2g4_r1);
-    else IBEM_B(_c2g5_r1);
-  } else {
-    if constexpr (F == 0) IBEM_BM(_c0_r2);
-    else if constexpr (F == 1) IBEM_B(_c1g0_r2);
-    else if constexpr (F == 2) IBEM_B(_c1g1_r2);
-    else if constexpr (F == 3) IBEM_B(_c1g2_r2);
-    else if constexpr (F == 4) IBEM_B(_c2g0_r2);
-    else if constexpr (F == 5) IBEM_B(_c2g1_r2);
-    else if constexpr (F == 6) IBEM_B(_c2g2_r2);
-    else if constexpr (F == 7) IBEM_B(_c2g3_r2);
-    else if constexpr (F == 8) IBEM_B(_c2g4_r2);
-    else IBEM_B(_c2g5_r2);
-  }
+// A pair whose target centre lies inside the source, from the generated blocks (dense): rare
+// (overlapping spheres), so out of line and straight into y.  as, ia: radius of the target,
+// 1 / radius of the source; xs: the source's coefficients.
+__device__ __noinline__ void pair_inside(float x0, float x1, float x2, float as, float ia, const SphMatF& mc,
+                                         const float* xs, float* y) {
+  float acc[kNu];
+  for (int r = 0; r < kNu; ++r) acc[r] = 0.f;
+  RowSink<float> sk{acc, xs};
+#define IBEM_B(NM) sph_block60f##NM(x0, x1, x2, 1.0f, mc, sk)
+  IBEM_B(m_c0_r0); IBEM_B(m_c1_r0); IBEM_B(m_c2_r0); IBEM_B(m_c0_r1); IBEM_B(m_c1_r1); IBEM_B(m_c0_r2);
+  IBEM_B(_c2g0_r1); IBEM_B(_c2g1_r1); IBEM_B(_c2g2_r1); IBEM_B(_c2g3_r1); IBEM_B(_c2g4_r1); IBEM_B(_c2g5_r1);
+  IBEM_B(_c1g0_r2); IBEM_B(_c1g1_r2); IBEM_B(_c1g2_r2);
+  IBEM_B(_c2g0_r2); IBEM_B(_c2g1_r2); IBEM_B(_c2g2_r2); IBEM_B(_c2g3_r2); IBEM_B(_c2g4_r2); IBEM_B(_c2g5_r2);
 #undef IBEM_B
-#undef IBEM_BM
+  for (int r = 0; r < kNu; ++r) atomicAdd(y + r, acc[r] * (r < 6 ? 1.f : r < 24 ? as * ia : as * ia * as * ia));
+}
+// the nine FP64 sub-blocks (column order, row order) of the unit sphere
+template <class Sink>
+__device__ __forceinline__ void blocks60(int which, double x0, double x1, double x2, const SphMat& mc, Sink& sk) {
+  switch (which) {
+#define IBEM_B(I, NM) case I: sph_block60_##NM(x0, x1, x2, 1.0, mc, sk); break
+    IBEM_B(0, c2_r2); IBEM_B(1, c2_r1); IBEM_B(2, c1_r2); IBEM_B(3, c2_r0); IBEM_B(4, c0_r2);
+    IBEM_B(5, c1_r1); IBEM_B(6, c1_r0); IBEM_B(7, c0_r1); IBEM_B(8, c0_r0);
+#undef IBEM_B
   }
 }
+__device__ __noinline__ void pair_inside(double x0, double x1, double x2, double as, double ia, const SphMat& mc,
+                                         const double* xs, double* y) {
+  double acc[kNu];
+  for (int r = 0; r < kNu; ++r) acc[r] = 0.0;
+  RowSink<double> sk{acc, xs};
+  for (int i = 0; i < 9; ++i) blocks60(i, x0, x1, x2, mc, sk);
+  for (int r = 0; r < kNu; ++r) atomicAdd(y + r, acc[r] * (r < 6 ? 1.0 : r < 24 ? as * ia : as * ia * as * ia));
+}
 
-template <int RO, int F>
+// Own block of a realisation's particles (unit sphere at x = 0 plus C0, moduli / mu0; the same
+// for all of them in the scaled system): S[seg][column][row].  One CTA per realisation, the
+// nine sub-blocks by one thread of a warp each.
+__global__ void __launch_bounds__(288) k_self60(const SphMat* __restrict__ mats, double* __restrict__ S) {
+  __shared__ double M[kNu * kNu];
+  for (int i = threadIdx.x; i < kNu * kNu; i += blockDim.x) M[i] = 0.0;
+  __syncthreads();
+  const SphMat mc = mats[blockIdx.x];
+  struct Put {
+    double* M;
+    __device__ void operator()(int r, int c, double v) const { M[c * kNu + r] += v; }
+  } put{M};
+  if (threadIdx.x % 32 == 0) blocks60(threadIdx.x / 32, 0.0, 0.0, 0.0, mc, put);
+  __syncthreads();
+  if (threadIdx.x == 0) sph_self60(mc, put);
+  __syncthreads();
+  for (int i = threadIdx.x; i < kNu * kNu; i += blockDim.x) S[(int64_t)blockIdx.x * kNu * kNu + i] = M[i];
+}
+
+// y = own block times the particle's coefficients, or 0 for a realisation masked out
+template <class T>
+__global__ void __launch_bounds__(240) k_self_apply60(int64_t n, const int* __restrict__ seg_of,
+                                                      const int* __restrict__ mask, int mask_on,
+                                                      const double* __restrict__ S, const T* __restrict__ x,
+                                                      T* __restrict__ y) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const int64_t p = t / kNu;
+  const int r = (int)(t % kNu), seg = seg_of[p];
+  T s = T(0);
+  if (!mask || mask[seg] == mask_on) {
+    const double* m = S + (int64_t)seg * kNu * kNu + r;
+    const T* v = x + p * kNu;
+#pragma unroll 10
+    for (int c = 0; c < kNu; ++c) s += (T)m[c * kNu] * v[c];
+  }
+  y[t] = s;
+}
+
 __global__ void __launch_bounds__(kT)
     k_mf60_f32(const MfTile* __restrict__ tiles, const int* __restrict__ seg_begin, const int* __restrict__ mask,
                int mask_on, const float4* __restrict__ gh, const float4* __restrict__ gl,
                const SphMatF* __restrict__ mats, const float* __restrict__ x, float* __restrict__ y) {
-  constexpr int NR = Rows<RO>::n;
   __shared__ float4 sgh[kChunk], sgl[kChunk];
-  __shared__ float sx[kChunk * kNu];
+  __shared__ __align__(16) float sx[kChunk * kNu];
   const MfTile t = tiles[blockIdx.x];
   if (mask && mask[t.seg] != mask_on) return;
   const int hb0 = seg_begin[t.seg], he0 = seg_begin[t.seg + 1];
@@ -139,12 +148,12 @@ __global__ void __launch_bounds__(kT)
   if (hb >= he) return;
   const int s = t.s0 + threadIdx.x;
   const bool act = threadIdx.x < t.ns;
-  const SphMatF mc = mats[t.seg];
+  const float kmu = mats[t.seg].kmu, klam = mats[t.seg].klam, nu = 0.5f * mats[t.seg].tn2;
   const float4 ph = act ? gh[s] : make_float4(0.f, 0.f, 0.f, 1.f);
   const float4 pl = act ? gl[s] : make_float4(0.f, 0.f, 0.f, 1.f);
-  float acc[NR];
+  float acc[kNu];
 #pragma unroll
-  for (int r = 0; r < NR; ++r) acc[r] = 0.f;
+  for (int r = 0; r < kNu; ++r) acc[r] = 0.f;
   for (int h0 = hb; h0 < he; h0 += kChunk) {
     const int nh = min(kChunk, he - h0);
     __syncthreads();
@@ -152,8 +161,7 @@ __global__ void __launch_bounds__(kT)
       sgh[i] = gh[h0 + i];
       sgl[i] = gl[h0 + i];
     }
-    for (int i = threadIdx.x; i < nh * kNu; i += kT)
-      sx[i] = x[(int64_t)kNu * h0 + i] * powi(gl[h0 + i / kNu].w, RO);   // times a_h^-RO
+    for (int i = threadIdx.x; i < nh * kNu; i += kT) sx[i] = x[(int64_t)kNu * h0 + i] * mf60_weight(i % kNu);
     __syncthreads();
     if (!act) continue;
 #pragma unroll 1
@@ -163,31 +171,38 @@ __global__ void __launch_bounds__(kT)
       const float x0 = ((ph.x - qh.x) + (pl.x - ql.x)) * ia;
       const float x1 = ((ph.y - qh.y) + (pl.y - ql.y)) * ia;
       const float x2 = ((ph.z - qh.z) + (pl.z - ql.z)) * ia;
-      RowSink<float, RO> sk{acc, sx + kNu * hh};
-      blk<float, RO, F>(x0, x1, x2, mc, sk);
+      const float r2 = x0 * x0 + x1 * x1 + x2 * x2;
+      if (!(r2 > 1.f)) {
+        if (h0 + hh != s) pair_inside(x0, x1, x2, ph.w, ia, mats[t.seg], x + (int64_t)kNu * (h0 + hh), y + (int64_t)kNu * s);
+        continue;
+      }
+      const float ir = rsqrtf(r2);
+      Mf60Frame<float> f;
+      mf60_frame(x0 * ir, x1 * ir, x2 * ir, f);
+      float A0[6], A1[6][3], A2[6][6];
+      mf60_source(f, sx + kNu * hh, A0, A1, A2);
+      mf60_rows<0>(f, A0, A1, A2, ir, 1.f, nu, acc);
+      mf60_rows<1>(f, A0, A1, A2, ir, ia, nu, acc + 6);
+      mf60_rows<2>(f, A0, A1, A2, ir, ia * ia, nu, acc + 24);
     }
   }
   if (!act) return;
-  const float f = powi(ph.w, RO);   // a_s^RO
+  mf60_map<0>(kmu, klam, acc);
+  mf60_map<1>(kmu, klam, acc + 6);
+  mf60_map<2>(kmu, klam, acc + 24);
+  float* o = y + (int64_t)kNu * s;
 #pragma unroll
-  for (int r = 0; r < NR; ++r) acc[r] *= f;
-  if (F <= 0 && s >= hb && s < he) {   // the slice holding the target adds its self term (C0 / mu0)
-    RowSink<float, RO> sk{acc, x + (int64_t)kNu * s};
-    sph_self60f(mc, sk);
-  }
-  float* o = y + (int64_t)kNu * s + Rows<RO>::off;
-#pragma unroll
-  for (int r = 0; r < NR; ++r) atomicAdd(o + r, acc[r]);
+  for (int r = 0; r < kNu; ++r) atomicAdd(o + r, acc[r] * (r < 6 ? 1.f : r < 24 ? ph.w : ph.w * ph.w));
 }
 
-template <int RO, int F>
+template <int RO>
 __global__ void __launch_bounds__(kT)
     k_mf60_f64(const MfTile* __restrict__ tiles, const int* __restrict__ seg_begin, const int* __restrict__ mask,
                int mask_on, const double* __restrict__ cen, const double* __restrict__ rad,
                const SphMat* __restrict__ mats, const double* __restrict__ x, double* __restrict__ y) {
   constexpr int NR = Rows<RO>::n;
   __shared__ double sc[kChunk * 4];
-  __shared__ double sx[kChunk * kNu];
+  __shared__ __align__(16) double sx[kChunk * kNu];
   const MfTile t = tiles[blockIdx.x];
   if (mask && mask[t.seg] != mask_on) return;
   const int hb0 = seg_begin[t.seg], he0 = seg_begin[t.seg + 1];
@@ -196,7 +211,7 @@ __global__ void __launch_bounds__(kT)
   if (hb >= he) return;
   const int s = t.s0 + threadIdx.x;
   const bool act = threadIdx.x < t.ns;
-  const SphMat mc = mats[t.seg];
+  const double kmu = mats[t.seg].kmu, klam = mats[t.seg].klam, nu = 0.5 * mats[t.seg].tn2;
   double p0 = 0.0, p1 = 0.0, p2 = 0.0, as = 1.0;
   if (act) {
     p0 = cen[3 * (int64_t)s];
@@ -216,37 +231,40 @@ __global__ void __launch_bounds__(kT)
       sc[4 * i + 2] = cen[3 * (int64_t)(h0 + i) + 2];
       sc[4 * i + 3] = 1.0 / rad[h0 + i];
     }
-    for (int i = threadIdx.x; i < nh * kNu; i += kT)
-      sx[i] = x[(int64_t)kNu * h0 + i] * powi(1.0 / rad[h0 + i / kNu], RO);
+    for (int i = threadIdx.x; i < nh * kNu; i += kT) sx[i] = x[(int64_t)kNu * h0 + i] * (double)mf60_weight(i % kNu);
     __syncthreads();
     if (!act) continue;
 #pragma unroll 1
     for (int hh = 0; hh < nh; ++hh) {
       const double ia = sc[4 * hh + 3];
       const double x0 = (p0 - sc[4 * hh]) * ia, x1 = (p1 - sc[4 * hh + 1]) * ia, x2 = (p2 - sc[4 * hh + 2]) * ia;
-      RowSink<double, RO> sk{acc, sx + kNu * hh};
-      blk<double, RO, F>(x0, x1, x2, mc, sk);
+      const double r2 = x0 * x0 + x1 * x1 + x2 * x2;
+      if (!(r2 > 1.0)) {
+        if (RO == 0 && h0 + hh != s)
+          pair_inside(x0, x1, x2, as, ia, mats[t.seg], x + (int64_t)kNu * (h0 + hh), y + (int64_t)kNu * s);
+        continue;
+      }
+      const double ir = rsqrt(r2);
+      Mf60Frame<double> f;
+      mf60_frame(x0 * ir, x1 * ir, x2 * ir, f);
+      double A0[6], A1[6][3], A2[6][6];
+      mf60_source(f, sx + kNu * hh, A0, A1, A2);
+      mf60_rows<RO>(f, A0, A1, A2, ir, RO == 0 ? 1.0 : RO == 1 ? ia : ia * ia, nu, acc);
     }
   }
   if (!act) return;
-  const double f = powi(as, RO);
-#pragma unroll
-  for (int r = 0; r < NR; ++r) acc[r] *= f;
-  if (F <= 0 && s >= hb && s < he) {
-    RowSink<double, RO> sk{acc, x + (int64_t)kNu * s};
-    sph_self60(mc, sk);
-  }
+  mf60_map<RO>(kmu, klam, acc);
   double* o = y + (int64_t)kNu * s + Rows<RO>::off;
 #pragma unroll
-  for (int r = 0; r < NR; ++r) atomicAdd(o + r, acc[r]);
+  for (int r = 0; r < NR; ++r) atomicAdd(o + r, acc[r] * (RO == 0 ? 1.0 : RO == 1 ? as : as * as));
 }
 
-// Scaled diagonal block of a realisation (unit sphere at x = 0 plus C0, moduli / mu0) inverted
-// by Gauss-Jordan with partial pivoting in FP64: one CTA of 64 threads per realisation, the
-// 60 x 120 augmented matrix in dynamic shared memory (57.6 KB).
+// The own block of a realisation's particles inverted by Gauss-Jordan with partial pivoting in
+// FP64: one CTA of 64 threads per realisation, the 60 x 120 augmented matrix in dynamic shared
+// memory (57.6 KB).
 constexpr int kBjThreads = 64;
 constexpr size_t kBjSmem = sizeof(double) * kNu * (2 * kNu + 1);
-__global__ void __launch_bounds__(kBjThreads) k_block_jacobi60(const SphMat* __restrict__ mats, float* __restrict__ P) {
+__global__ void __launch_bounds__(kBjThreads) k_block_jacobi60(const double* __restrict__ S, float* __restrict__ P) {
   extern __shared__ double smem[];
   double (*M)[2 * kNu + 1] = reinterpret_cast<double (*)[2 * kNu + 1]>(smem);
   __shared__ int piv;
@@ -255,25 +273,7 @@ __global__ void __launch_bounds__(kBjThreads) k_block_jacobi60(const SphMat* __r
   const int t = threadIdx.x;
   for (int i = t; i < kNu * 2 * kNu; i += kBjThreads) {
     const int r = i / (2 * kNu), c = i % (2 * kNu);
-    M[r][c] = (c >= kNu && c - kNu == r) ? 1.0 : 0.0;
-  }
-  __syncthreads();
-  if (t == 0) {
-    SphMat mc = mats[p];
-    struct Put {
-      double (*M)[2 * kNu + 1];
-      __device__ void operator()(int r, int c, double v) const { M[r][c] += v; }
-    } put{M};
-    sph_block60_c0_r0(0.0, 0.0, 0.0, 1.0, mc, put);
-    sph_block60_c1_r0(0.0, 0.0, 0.0, 1.0, mc, put);
-    sph_block60_c2_r0(0.0, 0.0, 0.0, 1.0, mc, put);
-    sph_block60_c0_r1(0.0, 0.0, 0.0, 1.0, mc, put);
-    sph_block60_c1_r1(0.0, 0.0, 0.0, 1.0, mc, put);
-    sph_block60_c2_r1(0.0, 0.0, 0.0, 1.0, mc, put);
-    sph_block60_c0_r2(0.0, 0.0, 0.0, 1.0, mc, put);
-    sph_block60_c1_r2(0.0, 0.0, 0.0, 1.0, mc, put);
-    sph_block60_c2_r2(0.0, 0.0, 0.0, 1.0, mc, put);
-    sph_self60(mc, put);
+    M[r][c] = c < kNu ? S[(int64_t)p * kNu * kNu + c * kNu + r] : (c - kNu == r ? 1.0 : 0.0);
   }
   __syncthreads();
   for (int k = 0; k < kNu; ++k) {
@@ -328,48 +328,41 @@ __global__ void k_precond_apply60(int num, const int* __restrict__ seg_of, const
 
 }  // namespace
 
-// FP32: 18 launches (row order 0; row order 1 in 7 column groups; row order 2 in 10)
-#define IBEM_MF60_ALL(K, ...)                                                                            \
-  K(0, -1, __VA_ARGS__); K(1, 0, __VA_ARGS__); K(1, 1, __VA_ARGS__); K(1, 2, __VA_ARGS__); K(1, 3, __VA_ARGS__); \
-  K(1, 4, __VA_ARGS__); K(1, 5, __VA_ARGS__); K(1, 6, __VA_ARGS__); K(2, 0, __VA_ARGS__); K(2, 1, __VA_ARGS__); \
-  K(2, 2, __VA_ARGS__); K(2, 3, __VA_ARGS__); K(2, 4, __VA_ARGS__); K(2, 5, __VA_ARGS__); K(2, 6, __VA_ARGS__); \
-  K(2, 7, __VA_ARGS__); K(2, 8, __VA_ARGS__); K(2, 9, __VA_ARGS__)
+ibem_status mf60_self(const MfBatch& b, double* S, cudaStream_t st) {
+  ::ibem::count_launch(), k_self60<<<b.nseg, 288, 0, st>>>(b.mats, S);
+  IBEM_LAUNCH_CHECK("mf60 own blocks");
+  return IBEM_OK;
+}
 
 ibem_status mf60_apply_f32(const MfBatch& b, const float* x, float* y, cudaStream_t st, const int* mask,
                            int mask_on) {
-  const dim3 grid(b.ntiles_s[1], b.hsplit);
-#define IBEM_MF60_F32(RO, F, unused)                                                                           \
-  ::ibem::count_launch(), k_mf60_f32<RO, F><<<grid, kT, 0, st>>>(b.tiles_s[1], b.seg_begin, mask, mask_on, b.gh, \
-                                                                  b.gl, b.matf, x, y)
-  IBEM_MF60_ALL(IBEM_MF60_F32, 0);
-#undef IBEM_MF60_F32
+  ::ibem::count_launch(), k_self_apply60<float><<<(unsigned)((b.N + 239) / 240), 240, 0, st>>>(b.N, b.seg_of, mask, mask_on,
+                                                                                               b.self60, x, y);
+  ::ibem::count_launch(), k_mf60_f32<<<dim3(b.ntiles_s[0], b.hsplit), kT, 0, st>>>(b.tiles_s[0], b.seg_begin, mask, mask_on,
+                                                                                   b.gh, b.gl, b.matf, x, y);
   IBEM_LAUNCH_CHECK("mf60 apply f32");
   return IBEM_OK;
 }
 
-// FP64: 7 launches (row order 0; row orders 1 and 2 one column order at a time)
 ibem_status mf60_apply_f64(const MfBatch& b, const double* x, double* y, cudaStream_t st, const int* mask,
                            int mask_on) {
-  const dim3 grid(b.ntiles_s[1], b.hsplit_wide);
-#define IBEM_MF60_F64(RO, F)                                                                                     \
-  ::ibem::count_launch(), k_mf60_f64<RO, F><<<grid, kT, 0, st>>>(b.tiles_s[1], b.seg_begin, mask, mask_on, b.cen, \
-                                                                  b.rad, b.mats, x, y)
-  IBEM_MF60_F64(0, -1);
-  IBEM_MF60_F64(1, 0);
-  IBEM_MF60_F64(1, 1);
-  IBEM_MF60_F64(1, 2);
-  IBEM_MF60_F64(2, 0);
-  IBEM_MF60_F64(2, 1);
-  IBEM_MF60_F64(2, 2);
+  const dim3 grid(b.ntiles_s[0], b.hsplit_wide);
+  ::ibem::count_launch(), k_self_apply60<double><<<(unsigned)((b.N + 239) / 240), 240, 0, st>>>(b.N, b.seg_of, mask, mask_on,
+                                                                                                b.self60, x, y);
+#define IBEM_MF60_F64(RO)                                                                                         \
+  ::ibem::count_launch(), k_mf60_f64<RO><<<grid, kT, 0, st>>>(b.tiles_s[0], b.seg_begin, mask, mask_on, b.cen, b.rad, \
+                                                              b.mats, x, y)
+  IBEM_MF60_F64(2);
+  IBEM_MF60_F64(1);
+  IBEM_MF60_F64(0);
 #undef IBEM_MF60_F64
   IBEM_LAUNCH_CHECK("mf60 apply f64");
   return IBEM_OK;
 }
-#undef IBEM_MF60_ALL
 
 ibem_status mf60_block_jacobi(const MfBatch& b, float* Pseg, cudaStream_t st) {
   IBEM_CUDA(cudaFuncSetAttribute(k_block_jacobi60, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBjSmem));
-  ::ibem::count_launch(), k_block_jacobi60<<<b.nseg, kBjThreads, kBjSmem, st>>>(b.mats, Pseg);
+  ::ibem::count_launch(), k_block_jacobi60<<<b.nseg, kBjThreads, kBjSmem, st>>>(b.self60, Pseg);
   IBEM_LAUNCH_CHECK("mf60 block jacobi");
   return IBEM_OK;
 }
