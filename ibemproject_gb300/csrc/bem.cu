@@ -3,14 +3,12 @@
 //  bem_hg        classical Q4 BEM H and G with 8x8 Gauss-Legendre quadrature, the singular
 //                element split into two degenerate triangles, and the rigid-body diagonal
 //                (BEMBuilderElastic3D.cpp:1169-1509, BEMElasticHelper3D.cpp:29-321).
-//                One thread per (collocation node, element); the element's 12 traction
-//                columns are scattered into node columns with FP64 atomics (the reference
-//                accumulates them under `omp critical`, :1432-1454).
+//                One thread per (collocation node, element), a warp per singular pair; the
+//                element's 12 traction columns are summed per node in a fixed order (the
+//                reference accumulates them under `omp critical`, :1432-1454).
 //  bem_to_incl   stress and its 1st/2nd gradient at particle centres from unit boundary
 //                displacements/tractions (addFluxEquivalent{,FirstOrder,SecondOrder}BEM,
-//                :1511-1867).  One thread per (particle, element, derivative tuple W, dof),
-//                48 accumulators each; the generated kernel for (order, W, dof) is picked
-//                by blockIdx.z.
+//                :1511-1867), from moments of the derivatives of R over each element.
 //  bem_post      boundary part of the stress at sample points (post_stress_BEM,
 //                postProcessorElastic3D.cpp:224-365), contracted with U and T at every
 //                Gauss point: a per-call quadrature table (point, normal, weight x Jacobian,
@@ -19,8 +17,8 @@
 #include <algorithm>
 #include <cuda_runtime.h>
 
-#include "gen_bem.cuh"
 #include "bem_contract.cuh"
+#include "bem_moments.cuh"
 #include "ibem_internal.h"
 #include "prof.h"
 
@@ -113,65 +111,163 @@ struct KelvinC {
 // The traction part of this element is written to TG, laid out like G (column 12e + 3a + j,
 // row 3i + ii; zero for the singular corner); node_gather then sums the columns of the
 // elements that share a node in a fixed order, so H is the same bit for bit on every run.
+
+// UK / TK (BEMElasticHelper3D.cpp:269-321) at offset x from the collocation node, without the
+// quadrature weight: U symmetric (xx xy xz yy yz zz), T row-major 3 x 3
+__device__ __forceinline__ void kelvin_ut(double x0, double x1, double x2, const double* nv, const KelvinC& kc,
+                                          double (&U)[6], double (&T)[9]) {
+  const double ir = ibem::rsqrt_h3(x0 * x0 + x1 * x1 + x2 * x2);
+  const double dr[3] = {x0 * ir, x1 * ir, x2 * ir};
+  const double conr = kc.cu * ir, c0 = conr * kc.c1;
+  const double cth = nv[0] * dr[0] + nv[1] * dr[1] + nv[2] * dr[2];
+  const double cr = kc.ct * (ir * ir), c3 = cr * kc.c3, ct3 = -3.0 * cr * cth;
+  int q = 0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = i; j < 3; ++j, ++q) {
+      const double dd = dr[i] * dr[j];
+      U[q] = i == j ? conr * dd + c0 : conr * dd;
+      if (i == j) T[3 * i + i] = ct3 * dd - c3 * cth;
+      else {
+        const double as = c3 * (nv[j] * dr[i] - nv[i] * dr[j]);
+        T[3 * i + j] = ct3 * dd + as;
+        T[3 * j + i] = ct3 * dd - as;
+      }
+    }
+}
+
+// Pairs whose node is not a corner of the element: one thread per node, 128 nodes per CTA and
+// one element, whose 64 Gauss points (position, normal, shape functions x weight x Jacobian:
+// the part that does not depend on the node, with its square root and divisions) are formed
+// once per CTA in shared memory.  U is symmetric, so 15 sums of four shape functions are kept
+// instead of 72 entries formed one by one.  Bound by the FP64 pipe, about 135 operations per
+// (node, Gauss point); 294 elements, 296 nodes: 6.5 -> 1.6 ms, the singular pairs included.
 __global__ void __launch_bounds__(128) bem_hg_kernel(const double* __restrict__ nodes, int NN,
                                                      const int* __restrict__ conn, KelvinC kc,
                                                      double* __restrict__ TG, int64_t ldt,
                                                      double* __restrict__ G, int64_t ldg) {
+  __shared__ double sg[64][10];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int e = blockIdx.y;
-  if (i >= NN) return;
   Elem el;
   int sc[4];
-  if (!load_elem(nodes, NN, conn, e, el, sc)) return;
-  const double xP[3] = {nodes[3 * i], nodes[3 * i + 1], nodes[3 * i + 2]};
-  int l_pi = -1;
+  if (!load_elem(nodes, NN, conn, e, el, sc)) return;   // the same for the whole CTA
+  if (threadIdx.x < 64) {
+    const int mq = threadIdx.x / 8, kq = threadIdx.x % 8;
+    double N[4], gc[3], nv[3], jac;
+    q4_point(el.c, kGP[mq], kGP[kq], N, gc, nv, jac);
+    const double wj = kGW[mq] * kGW[kq] * jac;
+    double* g = sg[threadIdx.x];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      g[d] = gc[d];
+      g[3 + d] = nv[d];
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) g[6 + a] = N[a] * wj;
+  }
+  __syncthreads();
+  if (i >= NN) return;
 #pragma unroll
   for (int n = 0; n < 4; ++n)
-    if (sc[n] == i + 1) l_pi = n;
-  double dU[3][12], dT[3][12];
+    if (sc[n] == i + 1) return;   // bem_hg_singular
+  const double p0 = nodes[3 * i], p1 = nodes[3 * i + 1], p2 = nodes[3 * i + 2];
+  double aU[6][4], aT[9][4];
 #pragma unroll
-  for (int a = 0; a < 3; ++a)
+  for (int n = 0; n < 4; ++n) {
 #pragma unroll
-    for (int b = 0; b < 12; ++b) { dU[a][b] = 0.0; dT[a][b] = 0.0; }
-  const int ntri = l_pi < 0 ? 1 : 2;
-  for (int ntr = 0; ntr < ntri; ++ntr)
-    for (int mq = 0; mq < 8; ++mq)
-      for (int kq = 0; kq < 8; ++kq) {
-        const double W = kGW[mq] * kGW[kq];
-        double xi = kGP[mq], et = kGP[kq], jb = 1.0;
-        if (l_pi >= 0) tri_map(ntr, l_pi, kGP[mq], kGP[kq], xi, et, jb);
-        double N[4], gc[3], nv[3], jac;
-        q4_point(el.c, xi, et, N, gc, nv, jac);
-        jac *= jb;
-        const double dx0 = gc[0] - xP[0], dx1 = gc[1] - xP[1], dx2 = gc[2] - xP[2];
-        const double r = sqrt(dx0 * dx0 + dx1 * dx1 + dx2 * dx2);
-        const double dr[3] = {dx0 / r, dx1 / r, dx2 / r};
-        // UK / TK (BEMElasticHelper3D.cpp:269-321)
-        const double conr = kc.cu / r;
-        const double cth = nv[0] * dr[0] + nv[1] * dr[1] + nv[2] * dr[2];
-        const double cr = kc.ct / (r * r);
-        const double wj = jac * W;
+    for (int q = 0; q < 6; ++q) aU[q][n] = 0.0;
 #pragma unroll
-        for (int ii = 0; ii < 3; ++ii)
+    for (int q = 0; q < 9; ++q) aT[q][n] = 0.0;
+  }
+#pragma unroll 1
+  for (int q = 0; q < 64; ++q) {
+    const double* g = sg[q];
+    double U[6], T[9];
+    kelvin_ut(g[0] - p0, g[1] - p1, g[2] - p2, g + 3, kc, U, T);
 #pragma unroll
-          for (int jj = 0; jj < 3; ++jj) {
-            const double U = conr * ((ii == jj ? kc.c1 : 0.0) + dr[ii] * dr[jj]);
-            const double T = (ii == jj) ? -cr * (kc.c3 + 3 * dr[ii] * dr[ii]) * cth
-                                        : -cr * (3 * dr[ii] * dr[jj] * cth - kc.c3 * (nv[jj] * dr[ii] - nv[ii] * dr[jj]));
+    for (int n = 0; n < 4; ++n) {
+      const double w = g[6 + n];
 #pragma unroll
-            for (int n = 0; n < 4; ++n) {
-              dU[ii][3 * n + jj] += N[n] * U * wj;
-              if (l_pi < 0 || n != l_pi) dT[ii][3 * n + jj] += N[n] * T * wj;
-            }
-          }
-      }
-  // G columns of this element, and its traction columns for H (summed per node by node_gather)
+      for (int t = 0; t < 6; ++t) aU[t][n] += w * U[t];
+#pragma unroll
+      for (int t = 0; t < 9; ++t) aT[t][n] += w * T[t];
+    }
+  }
+  const int sym[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
 #pragma unroll
   for (int ii = 0; ii < 3; ++ii)
 #pragma unroll
     for (int k = 0; k < 12; ++k) {
-      G[(12 * (int64_t)e + k) * ldg + 3 * i + ii] = dU[ii][k];
-      TG[(12 * (int64_t)e + k) * ldt + 3 * i + ii] = (l_pi < 0 || k / 3 != l_pi) ? dT[ii][k] : 0.0;
+      G[(12 * (int64_t)e + k) * ldg + 3 * i + ii] = aU[sym[3 * ii + k % 3]][k / 3];
+      TG[(12 * (int64_t)e + k) * ldt + 3 * i + ii] = aT[3 * ii + k % 3][k / 3];
+    }
+}
+
+// Pairs whose node is a corner of the element: a warp per (element, corner), two triangles of 64
+// Gauss points, four points per lane, the 60 sums added over the warp by a butterfly (the same
+// order on every run).  An element that names a node twice keeps the last of its corners, as
+// the first form of this loop did.
+__global__ void __launch_bounds__(128) bem_hg_singular(const double* __restrict__ nodes, int NN,
+                                                       const int* __restrict__ conn, int NE, KelvinC kc,
+                                                       double* __restrict__ TG, int64_t ldt,
+                                                       double* __restrict__ G, int64_t ldg) {
+  const int id = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
+  if (id >= 4 * NE) return;
+  const int e = id / 4, l_pi = id % 4;
+  Elem el;
+  int sc[4];
+  if (!load_elem(nodes, NN, conn, e, el, sc)) return;
+  for (int n = l_pi + 1; n < 4; ++n)
+    if (sc[n] == sc[l_pi]) return;
+  const int i = sc[l_pi] - 1;
+  double aU[6][4], aT[9][4];
+#pragma unroll
+  for (int n = 0; n < 4; ++n) {
+#pragma unroll
+    for (int q = 0; q < 6; ++q) aU[q][n] = 0.0;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) aT[q][n] = 0.0;
+  }
+  for (int g = lane; g < 128; g += 32) {
+    const int mq = (g & 63) / 8, kq = g % 8;
+    double xi, et, jb;
+    tri_map(g / 64, l_pi, kGP[mq], kGP[kq], xi, et, jb);
+    double N[4], gc[3], nv[3], jac;
+    q4_point(el.c, xi, et, N, gc, nv, jac);
+    const double wj = jac * jb * (kGW[mq] * kGW[kq]);
+    double U[6], T[9];
+    kelvin_ut(gc[0] - el.c[3 * l_pi], gc[1] - el.c[3 * l_pi + 1], gc[2] - el.c[3 * l_pi + 2], nv, kc, U, T);
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      const double w = N[n] * wj;
+#pragma unroll
+      for (int t = 0; t < 6; ++t) aU[t][n] += w * U[t];
+      if (n != l_pi) {
+#pragma unroll
+        for (int t = 0; t < 9; ++t) aT[t][n] += w * T[t];
+      }
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < 4; ++n) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+      for (int t = 0; t < 6; ++t) aU[t][n] += __shfl_xor_sync(0xffffffffu, aU[t][n], off);
+#pragma unroll
+      for (int t = 0; t < 9; ++t) aT[t][n] += __shfl_xor_sync(0xffffffffu, aT[t][n], off);
+    }
+  }
+  if (lane != 0) return;
+  const int sym[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
+#pragma unroll
+  for (int ii = 0; ii < 3; ++ii)
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+      G[(12 * (int64_t)e + k) * ldg + 3 * i + ii] = aU[sym[3 * ii + k % 3]][k / 3];
+      TG[(12 * (int64_t)e + k) * ldt + 3 * i + ii] = k / 3 != l_pi ? aT[3 * ii + k % 3][k / 3] : 0.0;
     }
 }
 
@@ -276,99 +372,146 @@ __global__ void bem_diag_kernel(int NN, double* __restrict__ H, int64_t ldh) {
 }
 
 // ---- boundary -> inclusion rows ----
-typedef void (*StressFn)(double, double, double, double, double, double, const BemMat&, double,
-                         double, double*, double*);
-
-template <int ORDER>
-__device__ __forceinline__ void stress_dispatch(int f, double x0, double x1, double x2, double n0,
-                                                double n1, double n2, const BemMat& bm,
-                                                double* su, double* st) {
-  const double dl = bm.dlam, dm = bm.dmu;
-#define IBEM_S(fn) fn(x0, x1, x2, n0, n1, n2, bm, dl, dm, su, st)
-  if (ORDER == 0) {
-    switch (f) {
-      case 0: IBEM_S(bem_stress_o0_w_n0); break;
-      case 1: IBEM_S(bem_stress_o0_w_n1); break;
-      default: IBEM_S(bem_stress_o0_w_n2); break;
-    }
-  } else if (ORDER == 1) {
-    switch (f) {
-      case 0: IBEM_S(bem_stress_o1_w0_n0); break; case 1: IBEM_S(bem_stress_o1_w0_n1); break;
-      case 2: IBEM_S(bem_stress_o1_w0_n2); break; case 3: IBEM_S(bem_stress_o1_w1_n0); break;
-      case 4: IBEM_S(bem_stress_o1_w1_n1); break; case 5: IBEM_S(bem_stress_o1_w1_n2); break;
-      case 6: IBEM_S(bem_stress_o1_w2_n0); break; case 7: IBEM_S(bem_stress_o1_w2_n1); break;
-      default: IBEM_S(bem_stress_o1_w2_n2); break;
-    }
-  } else {
-    switch (f) {
-#define IBEM_C2(F, WS, N) case F: IBEM_S(bem_stress_o2_w##WS##_n##N); break;
-      IBEM_C2(0, 00, 0) IBEM_C2(1, 00, 1) IBEM_C2(2, 00, 2) IBEM_C2(3, 01, 0) IBEM_C2(4, 01, 1)
-      IBEM_C2(5, 01, 2) IBEM_C2(6, 02, 0) IBEM_C2(7, 02, 1) IBEM_C2(8, 02, 2) IBEM_C2(9, 10, 0)
-      IBEM_C2(10, 10, 1) IBEM_C2(11, 10, 2) IBEM_C2(12, 11, 0) IBEM_C2(13, 11, 1)
-      IBEM_C2(14, 11, 2) IBEM_C2(15, 12, 0) IBEM_C2(16, 12, 1) IBEM_C2(17, 12, 2)
-      IBEM_C2(18, 20, 0) IBEM_C2(19, 20, 1) IBEM_C2(20, 20, 2) IBEM_C2(21, 21, 0)
-      IBEM_C2(22, 21, 1) IBEM_C2(23, 21, 2) IBEM_C2(24, 22, 0) IBEM_C2(25, 22, 1)
-      default: IBEM_S(bem_stress_o2_w22_n2); break;
-#undef IBEM_C2
-    }
-  }
-#undef IBEM_S
-}
-
-// blockIdx.z = W index * 3 + dof.  Rows of the layout: order 0 -> t; order 1 -> 6 + 3t + w;
-// order 2 -> 24 + 9t + 3w + z (layout 78) or 24 + 6t + pairidx(w<=z) (layout 60).
+// One CTA per element and group of particles, two particles at a time:
+//  1. a thread per (particle, Gauss point): the derivatives of R of orders 3 .. 4 + MAXO;
+//  2. their moments over the element (bem_moments.cuh), a thread per (derivative, column);
+//  3. the rows of orders 0 .. MAXO from the moments, a thread per (row, dof, corner).
+// Rows of the layout: order 0 -> t; order 1 -> 6 + 3t + w; order 2 -> 24 + 9t + 3w + z (layout
+// 78, both orders of w and z) or 24 + 6t + pairidx(w <= z) (layout 60).
 // The displacement part (the H rows) is written per element into UG, laid out like G;
 // node_gather sums it per node in a fixed element order (no atomics on matrix entries).
-template <int ORDER>
-__global__ void __launch_bounds__(128) bem_incl_kernel(
-    const double* __restrict__ nodes, int NN, const int* __restrict__ conn, const double* __restrict__ cen,
-    int num, BemMat bm, int nu, int compact, double* __restrict__ UG, int64_t ldu,
-    double* __restrict__ G, int64_t ldg) {
-  const int K = blockIdx.x * blockDim.x + threadIdx.x;
-  const int e = blockIdx.y;
-  const int f = blockIdx.z;
-  if (K >= num) return;
-  const int wi = f / 3, n = f % 3;
-  const int w = ORDER == 2 ? wi / 3 : wi, z = wi % 3;
-  if (ORDER == 2 && compact && z < w) return;
+// Bound by the FP64 pipe: about 2,200 operations per (particle, Gauss point) for all three
+// orders (derivatives 700, moments 950, rows 500), 1,100 without order 2, where forming the
+// stress kernels of one derivative tuple at a time took 15,000.  21 particles, 294 elements, 24
+// unknowns: 12.0 -> 0.76 ms.
+constexpr int kInclK = 2;           // particles at a time
+constexpr int kInclGroup = 8;       // particles per CTA
+template <int MAXO>
+struct InclShape {
+  static constexpr int nd = MAXO == 2 ? 74 : 46;             // derivatives of orders 3 .. 4 + MAXO
+  static constexpr int mid = MAXO == 2 ? 36 : 15;            // of orders 4 .. 3 + MAXO
+  static constexpr int top = MAXO == 2 ? 28 : 21;            // of order 4 + MAXO
+  static constexpr int tasks = 10 + 4 * mid + 3 * top;       // moments: (derivative, column)
+  static constexpr int rows = MAXO == 2 ? 60 : 24;
+  static constexpr size_t smem = sizeof(double) * (kInclK * nd * 65 + kInclK * nd * 16 + 64 * 16 + 64 * 3);
+};
+struct InclMom {
+  const double* m;   // [derivative][column * 4 + corner], offset to the corner
+  __device__ __forceinline__ double operator()(int c, int i) const { return m[16 * i + 4 * c]; }
+};
+
+template <int MAXO>
+__global__ void __launch_bounds__(128) bem_incl_kernel(const double* __restrict__ nodes, int NN,
+                                                       const int* __restrict__ conn, const double* __restrict__ cen,
+                                                       int num, BemMat bm, int nu, double* __restrict__ UG, int64_t ldu,
+                                                       double* __restrict__ G, int64_t ldg) {
+  using S = InclShape<MAXO>;
+  extern __shared__ __align__(16) double incl_smem[];
+  double* sd = incl_smem;                          // [particle][derivative][65]: value at the Gauss points
+  double* sm = sd + kInclK * S::nd * 65;           // [particle][derivative][16]: moments
+  double* sw = sm + kInclK * S::nd * 16;           // [Gauss point][16]: N_j w J {1, n}
+  double* sp = sw + 64 * 16;                       // [Gauss point][3]
+  const int e = blockIdx.x;
   Elem el;
   int sc[4];
-  if (!load_elem(nodes, NN, conn, e, el, sc)) return;
-  const double P0 = cen[3 * K], P1 = cen[3 * K + 1], P2 = cen[3 * K + 2];
-  double au[6][4], at[6][4];
+  if (!load_elem(nodes, NN, conn, e, el, sc)) return;   // the same for the whole CTA
+  if (threadIdx.x < 64) {
+    const int mq = threadIdx.x / 8, kq = threadIdx.x % 8;
+    double N[4], gc[3], nv[3], jac;
+    q4_point(el.c, kGP[mq], kGP[kq], N, gc, nv, jac);
+    const double wj = kGW[mq] * kGW[kq] * jac;
 #pragma unroll
-  for (int t = 0; t < 6; ++t)
+    for (int j = 0; j < 4; ++j) {
+      const double w = N[j] * wj;
+      sw[16 * threadIdx.x + j] = w;
 #pragma unroll
-    for (int a = 0; a < 4; ++a) { au[t][a] = 0.0; at[t][a] = 0.0; }
-  for (int mq = 0; mq < 8; ++mq)
-    for (int kq = 0; kq < 8; ++kq) {
-      double N[4], gc[3], nv[3], jac;
-      q4_point(el.c, kGP[mq], kGP[kq], N, gc, nv, jac);
-      const double wj = kGW[mq] * kGW[kq] * jac;
-      double su[18], st[18];
-      stress_dispatch<ORDER>(f, gc[0] - P0, gc[1] - P1, gc[2] - P2, nv[0], nv[1], nv[2], bm, su, st);
+      for (int m = 0; m < 3; ++m) sw[16 * threadIdx.x + 4 + 4 * m + j] = w * nv[m];
+    }
 #pragma unroll
-      for (int t = 0; t < 6; ++t) {
-        const double vu = su[3 * t + n] * wj, vt = st[3 * t + n] * wj;
-#pragma unroll
-        for (int a = 0; a < 4; ++a) { au[t][a] += vu * N[a]; at[t][a] += vt * N[a]; }
+    for (int d = 0; d < 3; ++d) sp[3 * threadIdx.x + d] = gc[d];
+  }
+  __syncthreads();
+  const int kb = blockIdx.y * kInclGroup, ke = min(num, kb + kInclGroup);
+  for (int k0 = kb; k0 < ke; k0 += kInclK) {
+    const int nk = min(kInclK, ke - k0);
+    {
+      const int kk = threadIdx.x / 64, g = threadIdx.x % 64;
+      if (kk < nk) {
+        const double* c = cen + 3 * (int64_t)(k0 + kk);
+        const double x0 = sp[3 * g] - c[0], x1 = sp[3 * g + 1] - c[1], x2 = sp[3 * g + 2] - c[2];
+        double* d = sd + kk * S::nd * 65 + g;
+        ibem::bmo_derivatives<4 + MAXO>(x0, x1, x2, ibem::rsqrt_h3(x0 * x0 + x1 * x1 + x2 * x2),
+                                        [&](int i, double v) { d[65 * i] = v; });
       }
     }
-  const double fac = ORDER == 2 ? 0.5 : 1.0;
-  int cidx = 0;  // compact (w<=z) pair index
-  if (ORDER == 2 && compact) cidx = (w == 0) ? z : (w == 1 ? 2 + z : 5);
-#pragma unroll
-  for (int t = 0; t < 6; ++t) {
-    int r;
-    if (ORDER == 0) r = t;
-    else if (ORDER == 1) r = 6 + 3 * t + w;
-    else r = compact ? 24 + 6 * t + cidx : 24 + 9 * t + 3 * w + z;
-    const int64_t row = (int64_t)nu * K + r;
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      UG[(12 * (int64_t)e + 3 * a + n) * ldu + row] = -fac * au[t][a];   // summed per node by node_gather
-      G[(12 * (int64_t)e + 3 * a + n) * ldg + row] = fac * at[t][a];
+    __syncthreads();
+    for (int t = threadIdx.x; t < nk * S::tasks; t += 128) {
+      const int kk = t / S::tasks, i = t % S::tasks;
+      int a, c;   // column 0 for orders 3 .. 3 + MAXO, the normal's for 4 .. 4 + MAXO
+      if (i < 10) {
+        a = i;
+        c = 0;
+      } else if (i < 10 + 4 * S::mid) {
+        a = 10 + (i - 10) % S::mid;
+        c = (i - 10) / S::mid;
+      } else {
+        a = 10 + S::mid + (i - 10 - 4 * S::mid) % S::top;
+        c = 1 + (i - 10 - 4 * S::mid) / S::top;
+      }
+      const double* d = sd + (kk * S::nd + a) * 65;
+      const double* w = sw + 4 * c;
+      double m0 = 0.0, m1 = 0.0, m2 = 0.0, m3 = 0.0;
+#pragma unroll 8
+      for (int g = 0; g < 64; ++g) {
+        const double v = d[g];
+        const double2 w01 = *reinterpret_cast<const double2*>(w + 16 * g), w23 = *reinterpret_cast<const double2*>(w + 16 * g + 2);
+        m0 += v * w01.x;
+        m1 += v * w01.y;
+        m2 += v * w23.x;
+        m3 += v * w23.y;
+      }
+      double* o = sm + (kk * S::nd + a) * 16 + 4 * c;
+      o[0] = m0;
+      o[1] = m1;
+      o[2] = m2;
+      o[3] = m3;
     }
+    __syncthreads();
+    for (int t = threadIdx.x; t < nk * S::rows * 12; t += 128) {
+      const int r = t % S::rows, col = (t / S::rows) % 12, kk = t / (S::rows * 12), n = col % 3;
+      int o, tt, w = 0, z = 0, row = r;
+      if (r < 6) {
+        o = 0;
+        tt = r;
+      } else if (r < 24) {
+        o = 1;
+        tt = (r - 6) / 3;
+        w = (r - 6) % 3;
+      } else {
+        o = 2;
+        tt = (r - 24) / 6;
+        const int q = (r - 24) % 6;
+        w = q < 3 ? 0 : (q < 5 ? 1 : 2);
+        z = q < 3 ? q : (q < 5 ? q - 2 : 2);
+        if (nu == 78) row = 24 + 9 * tt + 3 * w + z;
+      }
+      const int k = tt < 3 ? 0 : (tt < 5 ? 1 : 2), l = tt < 3 ? tt : (tt < 5 ? tt - 2 : 2);
+      const ibem::BmoEntries<InclMom> en{InclMom{sm + kk * S::nd * 16 + col / 3}, bm.kA, bm.kB, bm.lam0, bm.mu0, bm.dlam,
+                                         bm.dmu};
+      const int cnt = o == 0 ? 0 : ibem::bmo_e(w) + (o == 2 ? ibem::bmo_e(z) : 0);
+      double st, su;
+      en.entry(k, l, o, cnt, n, st, su);
+      const double fac = o == 2 ? 0.5 : 1.0;
+      const int64_t at = (int64_t)nu * (k0 + kk), c = 12 * (int64_t)e + col;
+      UG[c * ldu + at + row] = -fac * su;   // summed per node by node_gather
+      G[c * ldg + at + row] = fac * st;
+      if (nu == 78 && o == 2 && w != z) {
+        const int64_t mirror = at + 24 + 9 * tt + 3 * z + w;
+        UG[c * ldu + mirror] = -fac * su;
+        G[c * ldg + mirror] = fac * st;
+      }
+    }
+    __syncthreads();   // sd and sm are refilled
   }
 }
 
@@ -379,7 +522,7 @@ __global__ void __launch_bounds__(128) bem_incl_kernel(
 // per-point kernel then only evaluates the Kelvin stress kernels and contracts them.
 constexpr int kPostQ = 64;        // 8 x 8 Gauss points per element
 constexpr int kPostRec = 13;      // x y z, nx ny nz, w*J, u(3), t(3)
-constexpr int kPostStage = 128;   // table records per shared-memory stage (13 KB)
+constexpr int kPostStage = 128;   // Gauss points per slice are a multiple of this
 
 __global__ void bem_post_table(const double* __restrict__ nodes, int NN, const int* __restrict__ conn, int NE,
                                const double* __restrict__ U, const double* __restrict__ T,
@@ -413,8 +556,6 @@ __global__ void bem_post_table(const double* __restrict__ nodes, int NN, const i
   r[6] = kGW[mq] * kGW[kq] * jac;
 }
 
-// sums over the staged Gauss points of the stress contracted with their boundary values
-// (bem_contract.cuh: ~115 FP64 operations per pair instead of forming the 2 x 18 Kelvin kernels)
 // Gauss points [q_begin, q_end) of slice blockIdx.y of gridDim.y (a multiple of kPostStage)
 __device__ __forceinline__ void post_slice(int64_t nq, int64_t& qb, int64_t& qe) {
   const int64_t per = ((nq + gridDim.y - 1) / gridDim.y + kPostStage - 1) / kPostStage * kPostStage;
@@ -422,36 +563,44 @@ __device__ __forceinline__ void post_slice(int64_t nq, int64_t& qb, int64_t& qe)
   qe = min(nq, qb + per);
 }
 
+// the sums' records of the Gauss points (one thread each)
+__global__ void k_post_rec(const double* __restrict__ tab, int64_t nq, BemPostCoef cf, BemPostRec* __restrict__ out) {
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (q < nq) out[q] = bem_post_rec(tab + q * kPostRec, cf);
+}
+
+// FP64 sums: one thread per sample point, the records of 64 Gauss points at a time in shared
+// memory.  Bound by the FP64 pipe: 59 operations per (point, Gauss point).  600 elements, 32^3
+// points: 238 -> 144 ms.
+constexpr int kPostStageRec = 64;
 __global__ void __launch_bounds__(128) bem_post_kernel(const double* __restrict__ pts, int nump,
-                                                       const double* __restrict__ tab, int64_t nq, BemPostCoef cf,
+                                                       const BemPostRec* __restrict__ rec, int64_t nq, BemPostCoef cf,
                                                        double* __restrict__ part) {
-  __shared__ double sq[kPostStage * kPostRec];
+  static_assert(sizeof(BemPostRec) == 12 * sizeof(double2), "BemPostRec is copied as 12 double2");
+  __shared__ __align__(16) BemPostRec sq[kPostStageRec];
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   const bool act = s < nump;
   double P0 = 0, P1 = 0, P2 = 0;
-  if (act) { P0 = pts[3 * s]; P1 = pts[3 * s + 1]; P2 = pts[3 * s + 2]; }
+  if (act) { P0 = pts[3 * (int64_t)s]; P1 = pts[3 * (int64_t)s + 1]; P2 = pts[3 * (int64_t)s + 2]; }
   double acc[6] = {0, 0, 0, 0, 0, 0};
   int64_t qb, qe;
-  post_slice(nq, qb, qe);
-  for (int64_t q0 = qb; q0 < qe; q0 += kPostStage) {
-    const int nqs = (int)min((int64_t)kPostStage, qe - q0);
+  post_slice(nq, qb, qe);   // slice boundaries are multiples of kPostStage, hence of kPostStageRec
+  for (int64_t q0 = qb; q0 < qe; q0 += kPostStageRec) {
+    const int nqs = (int)min((int64_t)kPostStageRec, qe - q0);
     __syncthreads();
-    for (int idx = threadIdx.x; idx < nqs * kPostRec; idx += blockDim.x) sq[idx] = tab[q0 * kPostRec + idx];
+    {
+      const double2* src = reinterpret_cast<const double2*>(rec + q0);
+      double2* dst = reinterpret_cast<double2*>(sq);
+      for (int i = threadIdx.x; i < nqs * 12; i += blockDim.x) dst[i] = src[i];
+    }
     __syncthreads();
     if (!act) continue;
-    for (int qq = 0; qq < nqs; ++qq) {
-      const double* r = sq + qq * kPostRec;
-      double sg[6];
-      bem_post_contracted(r[0] - P0, r[1] - P1, r[2] - P2, r[3], r[4], r[5], r[7], r[8], r[9], r[10], r[11], r[12], cf,
-                          sg);
-      const double wj = r[6];
-#pragma unroll
-      for (int t = 0; t < 6; ++t) acc[t] += wj * sg[t];
-    }
+#pragma unroll 2
+    for (int qq = 0; qq < nqs; ++qq) bem_post_add(P0, P1, P2, sq[qq], cf, acc);
   }
   if (act)
 #pragma unroll
-    for (int t = 0; t < 6; ++t) part[6 * ((int64_t)blockIdx.y * nump + s) + t] = acc[t];
+    for (int t = 0; t < 6; ++t) part[6 * ((int64_t)blockIdx.y * nump + s) + t] = bem_post_value(acc, t);
 }
 
 // stress = sum of the slices' partial sums, in slice order (the same result on every run)
@@ -555,7 +704,10 @@ ibem_status bem_hg(const double* nodes, int NN, const int* conn, int NE, const i
   kc.ct = 1.0 / (8 * IBEM_PI * (1 - m.nu0));
   kc.c3 = 1 - 2 * m.nu0;
   dim3 grid((NN + 127) / 128, NE);
-  if (NE > 0) ::ibem::count_launch(), bem_hg_kernel<<<grid, 128, 0, st>>>(nodes, NN, conn, kc, TG, ldt, Gb, ldg);
+  if (NE > 0) {
+    ::ibem::count_launch(), bem_hg_kernel<<<grid, 128, 0, st>>>(nodes, NN, conn, kc, TG, ldt, Gb, ldg);
+    ::ibem::count_launch(), bem_hg_singular<<<(unsigned)NE, 128, 0, st>>>(nodes, NN, conn, NE, kc, TG, ldt, Gb, ldg);
+  }
   ::ibem::count_launch(), k_node_gather<<<gather_grid(ldt, NN), 256, 0, st>>>(ldt, NN, start, slot, TG, ldt, Hb, ldh, 0);
   ::ibem::count_launch(), bem_diag_kernel<<<(3 * NN + 127) / 128, 128, 0, st>>>(NN, Hb, ldh);
   cudaFreeAsync(start, st);
@@ -571,7 +723,6 @@ ibem_status bem_to_incl(const double* nodes, int NN, const int* conn, int NE, co
   BemMat bm = bem_mat_init(m.E0, m.nu0, m.E1, m.nu1);
   double* Hb = H + hcol0 * ldh + row0;
   double* Gb = G + gcol0 * ldg + row0;
-  const int compact = layout == 60;
   if (NN <= 0 || NE <= 0 || num <= 0) return IBEM_OK;
   const int64_t rows = (int64_t)layout * num;
   double* UG = nullptr;
@@ -581,14 +732,23 @@ ibem_status bem_to_incl(const double* nodes, int NN, const int* conn, int NE, co
   int *start = nullptr, *slot = nullptr;
   ibem_status s = node_incidence(conn, NN, NE, &start, &slot, st);
   if (s) { cudaFreeAsync(UG, st); return s; }
-  dim3 g0((num + 127) / 128, NE, 3), g1((num + 127) / 128, NE, 9), g2((num + 127) / 128, NE, 27);
-  ::ibem::count_launch(), bem_incl_kernel<0><<<g0, 128, 0, st>>>(nodes, NN, conn, cen, num, bm, layout, compact, UG, rows, Gb, ldg);
-  ::ibem::count_launch(), bem_incl_kernel<1><<<g1, 128, 0, st>>>(nodes, NN, conn, cen, num, bm, layout, compact, UG, rows, Gb, ldg);
-  if (layout != 24)
-    ::ibem::count_launch(), bem_incl_kernel<2><<<g2, 128, 0, st>>>(nodes, NN, conn, cen, num, bm, layout, compact, UG, rows, Gb, ldg);
+  const dim3 grid((unsigned)NE, (unsigned)((num + kInclGroup - 1) / kInclGroup));
+  cudaError_t ce = cudaSuccess;
+  if (layout == 24) {
+    ce = cudaFuncSetAttribute((const void*)bem_incl_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)InclShape<1>::smem);
+    ::ibem::count_launch(), bem_incl_kernel<1><<<grid, 128, InclShape<1>::smem, st>>>(nodes, NN, conn, cen, num, bm, layout, UG,
+                                                                                     rows, Gb, ldg);
+  } else {
+    ce = cudaFuncSetAttribute((const void*)bem_incl_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)InclShape<2>::smem);
+    ::ibem::count_launch(), bem_incl_kernel<2><<<grid, 128, InclShape<2>::smem, st>>>(nodes, NN, conn, cen, num, bm, layout, UG,
+                                                                                     rows, Gb, ldg);
+  }
   ::ibem::count_launch(), k_node_gather<<<gather_grid(rows, NN), 256, 0, st>>>(rows, NN, start, slot, UG, rows, Hb, ldh, 1);
   cudaFreeAsync(start, st);
   cudaFreeAsync(UG, st);
+  if (ce != cudaSuccess) return cuda_fail(ce, "bem_to_incl");
   IBEM_LAUNCH_CHECK("bem_to_incl");
   return IBEM_OK;
 }
@@ -610,20 +770,23 @@ ibem_status bem_post(const double* pts, int nump, const double* nodes, int NN, c
   const int64_t chunks = (nq + kPostStage - 1) / kPostStage;
   const int nslice = (int)std::max<int64_t>(1, std::min<int64_t>((8 * (int64_t)nsm + gx - 1) / gx, chunks));
   const size_t tab_bytes = (sizeof(double) * kPostRec * (nq > 0 ? nq : 1) + 255) / 256 * 256;
-  const size_t df_bytes = mixed ? (sizeof(BemPostDF) * (nq > 0 ? nq : 1) + 255) / 256 * 256 : 0;
+  const size_t df_bytes = ((mixed ? sizeof(BemPostDF) : sizeof(BemPostRec)) * (nq > 0 ? nq : 1) + 255) / 256 * 256;
   const size_t part_bytes = sizeof(double) * 6 * (size_t)nslice * (size_t)nump;
   IBEM_CUDA(cudaMallocAsync((void**)&tab, tab_bytes + df_bytes + part_bytes, st));
-  BemPostDF* tdf = mixed ? reinterpret_cast<BemPostDF*>(reinterpret_cast<char*>(tab) + tab_bytes) : nullptr;
+  void* recs = reinterpret_cast<char*>(tab) + tab_bytes;   // the form's records of the Gauss points
   double* part = reinterpret_cast<double*>(reinterpret_cast<char*>(tab) + tab_bytes + df_bytes);
   const unsigned gq = (unsigned)((nq + 127) / 128);
   const dim3 grid((unsigned)gx, (unsigned)nslice);
   if (nq > 0)
     ::ibem::count_launch(), bem_post_table<<<gq, 128, 0, st>>>(nodes, NN, conn, NE, U, T, tab);
   if (mixed) {
+    BemPostDF* tdf = static_cast<BemPostDF*>(recs);
     if (nq > 0) ::ibem::count_launch(), k_post_df_table<<<gq, 128, 0, st>>>(tab, nq, cf, tdf);
     ::ibem::count_launch(), bem_post_kernel_df<<<grid, 128, 0, st>>>(pts, nump, tdf, nq, bem_post_coef_df(cf), part);
   } else {
-    ::ibem::count_launch(), bem_post_kernel<<<grid, 128, 0, st>>>(pts, nump, tab, nq, cf, part);
+    BemPostRec* trec = static_cast<BemPostRec*>(recs);
+    if (nq > 0) ::ibem::count_launch(), k_post_rec<<<gq, 128, 0, st>>>(tab, nq, cf, trec);
+    ::ibem::count_launch(), bem_post_kernel<<<grid, 128, 0, st>>>(pts, nump, trec, nq, cf, part);
   }
   ::ibem::count_launch(), k_post_reduce<<<(unsigned)((6 * (int64_t)nump + 255) / 256), 256, 0, st>>>(nump, nslice,
                                                                                                    part, stress);

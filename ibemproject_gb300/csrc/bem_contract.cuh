@@ -16,6 +16,7 @@
 // tests compare the two to 1e-13).
 // About 115 FP64 operations per (point, Gauss point) against ~700 for forming Dsu and Dst.
 #pragma once
+#include "fp64_math.cuh"
 #include "gen_sphere_common.cuh"
 
 struct BemPostCoef {
@@ -67,6 +68,68 @@ IBEM_HD IBEM_INLINE void bem_post_contracted(double x0, double x1, double x2, do
     if (k == l) v += a;
     s[q] = v;
   }
+}
+
+// The same contraction for the sums over the Gauss points, with all that belongs to the Gauss
+// point alone in its record (192 bytes: position, normal, u and t times the weight, ct2 t,
+// and cu4 (n u + u n), cu0 n.u, cu1 n.u halved where they fall on the diagonal) and the factor
+// 1/R^3 applied last.  b x x is folded into w (b/2 x), and the diagonal is summed halved, so
+// that it takes one multiply-add per component.  59 FP64 operations per (point, Gauss point),
+// five of them for 1/R, where the form above takes about 105.
+struct BemPostRec {
+  double y[3], n[3], u[3], t[3], T[3];
+  double P[6];       // cu4 (n_k u_l + n_l u_k), halved for k = l
+  double h0, h1;     // cu0 n.u / 2, cu1 n.u / 2
+  double pad;
+};
+
+// r: y, n, w, u, t of one Gauss point (y 0-2, n 3-5, w 6, u 7-9, t 10-12)
+IBEM_HD inline BemPostRec bem_post_rec(const double* r, const BemPostCoef& c) {
+  BemPostRec o;
+  for (int k = 0; k < 3; ++k) {
+    o.y[k] = r[k];
+    o.n[k] = r[3 + k];
+    o.u[k] = r[6] * r[7 + k];
+    o.t[k] = r[6] * r[10 + k];
+    o.T[k] = c.ct2 * o.t[k];
+  }
+  const double nu = o.n[0] * o.u[0] + o.n[1] * o.u[1] + o.n[2] * o.u[2];
+  o.h0 = 0.5 * c.cu0 * nu;
+  o.h1 = 0.5 * c.cu1 * nu;
+  const int pi[6] = {0, 0, 0, 1, 1, 2}, pj[6] = {0, 1, 2, 1, 2, 2};
+  for (int q = 0; q < 6; ++q) {
+    const int k = pi[q], l = pj[q];
+    o.P[q] = c.cu4 * (k == l ? o.n[k] * o.u[k] : o.n[k] * o.u[l] + o.n[l] * o.u[k]);
+  }
+  o.pad = 0.0;
+  return o;
+}
+
+// acc[6] += w sigma of one Gauss point, the diagonal components halved (bem_post_value)
+IBEM_HD IBEM_INLINE void bem_post_add(double p0, double p1, double p2, const BemPostRec& g, const BemPostCoef& c,
+                                      double (&acc)[6]) {
+  const double x[3] = {g.y[0] - p0, g.y[1] - p1, g.y[2] - p2};
+  const double ir = ibem::rsqrt_h3(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
+  const double i2 = ir * ir, i3 = i2 * ir;
+  const double xn = x[0] * g.n[0] + x[1] * g.n[1] + x[2] * g.n[2];
+  const double xu = x[0] * g.u[0] + x[1] * g.u[1] + x[2] * g.u[2];
+  const double xt = x[0] * g.t[0] + x[1] * g.t[1] + x[2] * g.t[2];
+  const double s = xn * xu * i2;
+  const double a = (0.5 * c.cu1) * s + ((0.5 * c.ct0) * xt + g.h0);
+  const double b = i2 * ((0.5 * c.cu3) * s + ((0.5 * c.ct1) * xt + g.h1));
+  const double k5 = c.cu5 * i2, d = k5 * xu, e = k5 * xn;
+  double w[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) w[k] = d * g.n[k] + (e * g.u[k] + (b * x[k] + g.T[k]));
+  acc[0] += i3 * (w[0] * x[0] + (g.P[0] + a));
+  acc[1] += i3 * (w[0] * x[1] + (w[1] * x[0] + g.P[1]));
+  acc[2] += i3 * (w[0] * x[2] + (w[2] * x[0] + g.P[2]));
+  acc[3] += i3 * (w[1] * x[1] + (g.P[3] + a));
+  acc[4] += i3 * (w[1] * x[2] + (w[2] * x[1] + g.P[4]));
+  acc[5] += i3 * (w[2] * x[2] + (g.P[5] + a));
+}
+IBEM_HD IBEM_INLINE double bem_post_value(const double* acc, int q) {
+  return q == 0 || q == 3 || q == 5 ? 2.0 * acc[q] : acc[q];
 }
 
 // ---------------------------------------------------------------------------------------
