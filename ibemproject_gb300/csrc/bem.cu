@@ -142,7 +142,7 @@ __device__ __forceinline__ void kelvin_ut(double x0, double x1, double x2, const
 // the part that does not depend on the node, with its square root and divisions) are formed
 // once per CTA in shared memory.  U is symmetric, so 15 sums of four shape functions are kept
 // instead of 72 entries formed one by one.  Bound by the FP64 pipe, about 135 operations per
-// (node, Gauss point); 294 elements, 296 nodes: 6.5 -> 1.6 ms, the singular pairs included.
+// (node, Gauss point); 600 elements, 602 nodes: 18.7 -> 5.1 ms, the singular pairs included.
 __global__ void __launch_bounds__(128) bem_hg_kernel(const double* __restrict__ nodes, int NN,
                                                      const int* __restrict__ conn, KelvinC kc,
                                                      double* __restrict__ TG, int64_t ldt,
@@ -382,8 +382,8 @@ __global__ void bem_diag_kernel(int NN, double* __restrict__ H, int64_t ldh) {
 // node_gather sums it per node in a fixed element order (no atomics on matrix entries).
 // Bound by the FP64 pipe: about 2,200 operations per (particle, Gauss point) for all three
 // orders (derivatives 700, moments 950, rows 500), 1,100 without order 2, where forming the
-// stress kernels of one derivative tuple at a time took 15,000.  21 particles, 294 elements, 24
-// unknowns: 12.0 -> 0.76 ms.
+// stress kernels of one derivative tuple at a time took 15,000.  64 particles, 600 elements, 78
+// unknowns: 106 -> 9.2 ms; 21 particles, 294 elements, 24 unknowns: 12.0 -> 0.76 ms.
 constexpr int kInclK = 2;           // particles at a time
 constexpr int kInclGroup = 8;       // particles per CTA
 template <int MAXO>
