@@ -41,14 +41,37 @@ __global__ void k_ell_rot(int num, const double* __restrict__ quat, double* __re
   if (h < num) ell::quat_to_rot(quat + 4 * (int64_t)h, Q + 9 * (int64_t)h);
 }
 
+// rotation matrices on symmetric tensors (kRotSize values) of every ellipsoid: one CTA each, the
+// rows of an order in parallel
+__global__ void __launch_bounds__(32) k_ell_rotmat(const double* __restrict__ Q, double* __restrict__ M) {
+  const double* q = Q + 9 * (int64_t)blockIdx.x;
+  double* m = M + (int64_t)ell::kRotSize * blockIdx.x;
+  for (int n = 2; n <= 5; ++n) {
+    if ((int)threadIdx.x < ell::ssize(n))
+      ell::rot_row(q, n, threadIdx.x, n == 2 ? q : m + ell::rot_off(n - 1), m + ell::rot_off(n) + threadIdx.x * ell::ssize(n));
+    __syncthreads();
+  }
+}
+
+__device__ __noinline__ void pair24_any(const double* d, const double* Q, const double* a, const SphMat& mc, bool self,
+                                        double* blk) {
+  ell::ell_block24_any<double>(d, Q, a, mc, self, blk);
+}
+
+// Close neighbours of very flat sources take the general path (pair24_any); all others
+// ell_block24_ext, with the source's matrices in shared memory.
 __global__ void __launch_bounds__(kEllPairThreads) k_ell_pair24(const double* __restrict__ cen,
                                                                 const double* __restrict__ axes,
-                                                                const double* __restrict__ Qall, int num, SphMat mc,
+                                                                const double* __restrict__ Qall,
+                                                                const double* __restrict__ Mall, int num, SphMat mc,
                                                                 double* __restrict__ A, int64_t lda) {
   __shared__ double stage[kEllPairThreads / 32][32 * 24];
+  __shared__ double sM[ell::kRotSize];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   const int h = blockIdx.y;
+  for (int i = threadIdx.x; i < ell::kRotSize; i += kEllPairThreads) sM[i] = Mall[(int64_t)ell::kRotSize * h + i];
+  __syncthreads();
   const int s0 = s - lane;
   if (s0 >= num) return;   // whole warp past the end
   const int nact = min(32, num - s0);
@@ -63,7 +86,8 @@ __global__ void __launch_bounds__(kEllPairThreads) k_ell_pair24(const double* __
     }
 #pragma unroll
     for (int i = 0; i < 9; ++i) Q[i] = Qall[9 * (int64_t)h + i];
-    ell::ell_block24<double>(d, Q, a, mc, s == h, blk);
+    if (!ell::ell_block24_ext<double>(d, Q, a, sM, mc, blk)) pair24_any(d, Q, a, mc, s == h, blk);
+    else if (s == h) ell::ell_self_add<double>(mc, blk);
   }
   double* base = A + 24 * (int64_t)h * lda + 24 * (int64_t)s0;
   for (int c = 0; c < 24; ++c) {
@@ -222,14 +246,16 @@ ibem_status ibem_e3d_ell_pair_blocks(const double* centers_dev, const double* ax
   if (lda < row0 + 24 * (int64_t)num) return fail(IBEM_ERR_ARG, "ell_pair_blocks: lda too small");
   if (num == 0) return IBEM_OK;
   cudaStream_t st = as_stream(stream);
-  double* Q = nullptr;
-  IBEM_CUDA(cudaMallocAsync((void**)&Q, sizeof(double) * 9 * (size_t)num, st));
+  double* Q = nullptr;   // rotations, then their matrices on symmetric tensors
+  IBEM_CUDA(cudaMallocAsync((void**)&Q, sizeof(double) * (9 + ell::kRotSize) * (size_t)num, st));
+  double* M = Q + 9 * (size_t)num;
   s = ell_rotations(quats_dev, num, Q, st);
   if (!s) {
     const SphMat mc = sph_mat_init(mat->E0, mat->nu0, mat->E1, mat->nu1);
     ProfScope ps(PROF_PAIR, st);
+    ::ibem::count_launch(), k_ell_rotmat<<<(unsigned)num, 32, 0, st>>>(Q, M);
     dim3 grid((unsigned)((num + kEllPairThreads - 1) / kEllPairThreads), (unsigned)num);
-    ::ibem::count_launch(), k_ell_pair24<<<grid, kEllPairThreads, 0, st>>>(centers_dev, axes_dev, Q, num, mc,
+    ::ibem::count_launch(), k_ell_pair24<<<grid, kEllPairThreads, 0, st>>>(centers_dev, axes_dev, Q, M, num, mc,
                                                                            A_dev + col0 * lda + row0, lda);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) s = cuda_fail(e, "ell_pair_blocks");

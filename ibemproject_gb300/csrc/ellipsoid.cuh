@@ -36,6 +36,7 @@
 #pragma once
 #include <math.h>
 
+#include "fp64_math.cuh"
 #include "gen_sphere_common.cuh"
 
 namespace ibem {
@@ -45,10 +46,17 @@ namespace ell {
 // The evaluator runs in double or float.  Scalar functions and the unit roundoff by type:
 IBEM_HD inline double vsqrt(double x) { return sqrt(x); }
 IBEM_HD inline float vsqrt(float x) { return sqrtf(x); }
+IBEM_HD inline double vrsqrt(double x) { return rsqrt_h3(x); }
+IBEM_HD inline float vrsqrt(float x) { return 1.0f / sqrtf(x); }
 IBEM_HD inline double vfabs(double x) { return fabs(x); }
 IBEM_HD inline float vfabs(float x) { return fabsf(x); }
 template <typename T>
 IBEM_HD inline T vfmax(T a, T b) { return a > b ? a : b; }
+template <typename T>
+IBEM_HD inline T vfmin3(const T* a) {
+  const T m = a[0] < a[1] ? a[0] : a[1];
+  return m < a[2] ? m : a[2];
+}
 template <typename T>
 struct NumTraits;
 template <>
@@ -710,6 +718,14 @@ IBEM_HD inline T Dsum(const EllDer<T, K>& D, T nu, int rho, int i, int j, int k,
 IBEM_HD constexpr int pair_i(int t) { return t < 3 ? 0 : (t < 5 ? 1 : 2); }
 IBEM_HD constexpr int pair_j(int t) { return t < 3 ? t : (t < 5 ? t - 2 : 2); }
 
+}  // namespace ell
+}  // namespace ibem
+
+#include "ellipsoid_ext.cuh"   // the short route
+
+namespace ibem {
+namespace ell {
+
 // One (s, h) block of the layout-24 equivalent-inclusion system for an ellipsoidal source
 // h (integratorElastic3D.cpp:341-567 with the sphere's potentials replaced): rows (s, ij[,r]),
 // columns (h, mn[,p]):
@@ -718,8 +734,9 @@ IBEM_HD constexpr int pair_j(int t) { return t < 3 ? t : (t < 5 ? t - 2 : 2); }
 // The evaluation runs in coordinates scaled by the source's longest semi-axis s, where every
 // quantity is O(1); the tensor is scale-free except for one factor s per column of order 1
 // and 1/s per row of order 1.
+// This is the general path (any target, inside or outside).
 template <typename T>
-IBEM_HD inline void ell_block24(const T d[3], const T Q[9], const T a[3], const SphMat& mc, bool self, T* out) {
+IBEM_HD inline void ell_block24_any(const T d[3], const T Q[9], const T a[3], const SphMat& mc, bool self, T* out) {
   const T sc = vfmax(a[0], vfmax(a[1], a[2])), isc = T(1) / sc;
   EllDer<T, 4> P;
   {
@@ -774,6 +791,23 @@ IBEM_HD inline void ell_block24(const T d[3], const T Q[9], const T a[3], const 
       out[rr * 24 + cc] = (m == n ? T(1) : T(2)) * v;
     }
   }
+}
+
+// all rotation matrices of a source (kRotSize values)
+template <typename T>
+IBEM_HD inline void rot_matrices(const T Q[9], T* M) {
+  for (int n = 2; n <= 5; ++n)
+    for (int row = 0; row < ssize(n); ++row)
+      rot_row(Q, n, row, n == 2 ? Q : M + rot_off(n - 1), M + rot_off(n) + row * ssize(n));
+}
+
+// the block by the shorter of the two routes
+template <typename T>
+IBEM_HD inline void ell_block24(const T d[3], const T Q[9], const T a[3], const SphMat& mc, bool self, T* out) {
+  T M[kRotSize];
+  rot_matrices(Q, M);
+  if (!ell_block24_ext(d, Q, a, M, mc, out)) ell_block24_any(d, Q, a, mc, self, out);
+  else if (self) ell_self_add(mc, out);
 }
 
 // Strain (6: xx xy xz yy yz zz) at c + d due to the layout-24 eigenstrain E of an
