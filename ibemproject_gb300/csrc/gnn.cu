@@ -66,8 +66,16 @@ struct Layout {
 // lower index.  One warp per particle: every lane keeps a sorted list of the best 16 of its
 // own share of the candidates (q = first + lane, + 32, ...), then 16 rounds of a warp-wide
 // minimum over the lanes' list heads pick the result in order.
+// Two passes over the candidates.  The first finds every lane's nearest one in FP32; the 16th
+// smallest of these 32 minima bounds the 16th neighbour's distance, so the second pass forms
+// the FP64 distance and inserts only the few candidates (about 22) within it.  Without that
+// bound some lane of the warp inserts at almost every step, 16 compare-and-swaps each.  The
+// FP32 offset from the centres' hi / lo parts is off by at most 2^-22 of itself per axis, its
+// square by less than 2e-6, and the lo parts leave out less than `slack`.  20,000 particles:
+// 16.0 -> 2.0 ms.
 __global__ void k_knn(int num, const int* __restrict__ seg_of, const int* __restrict__ seg_begin,
-                      const double* __restrict__ cen, int* __restrict__ nbr) {
+                      const double* __restrict__ cen, const float4* __restrict__ gh, const float4* __restrict__ gl,
+                      int* __restrict__ nbr) {
   const int p = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (p >= num) return;  // uniform per warp
@@ -81,8 +89,29 @@ __global__ void k_knn(int num, const int* __restrict__ seg_of, const int* __rest
     bd[j] = INFINITY;
     bi[j] = -1;
   }
+  const float4 ph = gh[p], pl = gl[p];
+  const float slack = (fabsf(ph.x) + fabsf(ph.y) + fabsf(ph.z)) * 0x1p-44f;   // what the hi / lo parts leave out
+  auto d2f = [&](int q) {
+    const float4 qh = gh[q], ql = gl[q];
+    const float fx = (qh.x - ph.x) + (ql.x - pl.x), fy = (qh.y - ph.y) + (ql.y - pl.y), fz = (qh.z - ph.z) + (ql.z - pl.z);
+    return fx * fx + fy * fy + fz * fz;
+  };
+  float near = INFINITY;
+#pragma unroll 4
+  for (int q = b0 + lane; q < b1; q += 32)
+    if (q != p) near = fminf(near, d2f(q));
+  int rank = 0;
+#pragma unroll
+  for (int l = 0; l < 32; ++l) {
+    const float o = __shfl_sync(0xffffffffu, near, l);
+    rank += o < near || (o == near && l < lane);
+  }
+  const unsigned at = __ballot_sync(0xffffffffu, rank == kKnn - 1);
+  const float bound = at ? __shfl_sync(0xffffffffu, near, __ffs(at) - 1) : INFINITY;
+  const float far = sqrtf(bound) + 2.f * slack, limit = far * far * 1.00001f;
+#pragma unroll 4
   for (int q = b0 + lane; q < b1; q += 32) {
-    if (q == p) continue;
+    if (q == p || d2f(q) > limit) continue;   // (false for NaN: the FP64 test decides)
     const double dx = cen[3 * (int64_t)q] - px, dy = cen[3 * (int64_t)q + 1] - py, dz = cen[3 * (int64_t)q + 2] - pz;
     const double d2 = dx * dx + dy * dy + dz * dz;
     if (!(d2 < bd[kKnn - 1])) continue;  // later q of this lane: an equal distance loses
@@ -815,7 +844,8 @@ int64_t gnn_param_count() { return Layout().total; }
 
 ibem_status gnn_knn(const MfBatch& b, int* nbr, cudaStream_t st) {
   ProfScope ps(PROF_KNN, st);
-  ::ibem::count_launch(), k_knn<<<nb((int64_t)b.num * 32, 128), 128, 0, st>>>(b.num, b.seg_of, b.seg_begin, b.cen, nbr);
+  ::ibem::count_launch(), k_knn<<<nb((int64_t)b.num * 32, 128), 128, 0, st>>>(b.num, b.seg_of, b.seg_begin, b.cen,
+                                                                                     b.gh, b.gl, nbr);
   IBEM_LAUNCH_CHECK("knn");
   return IBEM_OK;
 }
