@@ -662,7 +662,7 @@ namespace ibem {
 static ibem_status node_incidence(const int* conn, int NN, int NE, int** start, int** slot, cudaStream_t st) {
   int* buf = nullptr;
   const size_t n = (size_t)(NN + 1) + 2 * (size_t)NN + 4 * (size_t)NE;
-  IBEM_CUDA(cudaMallocAsync((void**)&buf, sizeof(int) * n, st));
+  IBEM_CUDA(pool_alloc((void**)&buf, sizeof(int) * n, st));
   int* s0 = buf;
   int* cnt = s0 + NN + 1;
   int* cur = cnt + NN;
@@ -692,11 +692,11 @@ ibem_status bem_hg(const double* nodes, int NN, const int* conn, int NE, const i
   const int64_t ldt = 3 * (int64_t)NN;
   double* TG = nullptr;
   const size_t tg_bytes = sizeof(double) * ldt * 12 * (size_t)(NE > 0 ? NE : 1);
-  IBEM_CUDA(cudaMallocAsync((void**)&TG, tg_bytes, st));
+  IBEM_CUDA(pool_alloc((void**)&TG, tg_bytes, st));
   IBEM_CUDA(cudaMemsetAsync(TG, 0, tg_bytes, st));   // an element with bad connectivity adds nothing
   int *start = nullptr, *slot = nullptr;
   ibem_status s = node_incidence(conn, NN, NE, &start, &slot, st);
-  if (s) { cudaFreeAsync(TG, st); return s; }
+  if (s) { pool_free(TG, st); return s; }
   const double mu = m.E0 / (2 * (1 + m.nu0));
   KelvinC kc;
   kc.cu = 1.0 / (16 * IBEM_PI * mu * (1 - m.nu0));
@@ -710,8 +710,8 @@ ibem_status bem_hg(const double* nodes, int NN, const int* conn, int NE, const i
   }
   ::ibem::count_launch(), k_node_gather<<<gather_grid(ldt, NN), 256, 0, st>>>(ldt, NN, start, slot, TG, ldt, Hb, ldh, 0);
   ::ibem::count_launch(), bem_diag_kernel<<<(3 * NN + 127) / 128, 128, 0, st>>>(NN, Hb, ldh);
-  cudaFreeAsync(start, st);
-  cudaFreeAsync(TG, st);
+  pool_free(start, st);
+  pool_free(TG, st);
   IBEM_LAUNCH_CHECK("bem_hg");
   return IBEM_OK;
 }
@@ -727,11 +727,11 @@ ibem_status bem_to_incl(const double* nodes, int NN, const int* conn, int NE, co
   const int64_t rows = (int64_t)layout * num;
   double* UG = nullptr;
   const size_t ug_bytes = sizeof(double) * rows * 12 * (size_t)NE;
-  IBEM_CUDA(cudaMallocAsync((void**)&UG, ug_bytes, st));
+  IBEM_CUDA(pool_alloc((void**)&UG, ug_bytes, st));
   IBEM_CUDA(cudaMemsetAsync(UG, 0, ug_bytes, st));   // an element with bad connectivity adds nothing
   int *start = nullptr, *slot = nullptr;
   ibem_status s = node_incidence(conn, NN, NE, &start, &slot, st);
-  if (s) { cudaFreeAsync(UG, st); return s; }
+  if (s) { pool_free(UG, st); return s; }
   const dim3 grid((unsigned)NE, (unsigned)((num + kInclGroup - 1) / kInclGroup));
   cudaError_t ce = cudaSuccess;
   if (layout == 24) {
@@ -746,8 +746,8 @@ ibem_status bem_to_incl(const double* nodes, int NN, const int* conn, int NE, co
                                                                                      rows, Gb, ldg);
   }
   ::ibem::count_launch(), k_node_gather<<<gather_grid(rows, NN), 256, 0, st>>>(rows, NN, start, slot, UG, rows, Hb, ldh, 1);
-  cudaFreeAsync(start, st);
-  cudaFreeAsync(UG, st);
+  pool_free(start, st);
+  pool_free(UG, st);
   if (ce != cudaSuccess) return cuda_fail(ce, "bem_to_incl");
   IBEM_LAUNCH_CHECK("bem_to_incl");
   return IBEM_OK;
@@ -772,7 +772,7 @@ ibem_status bem_post(const double* pts, int nump, const double* nodes, int NN, c
   const size_t tab_bytes = (sizeof(double) * kPostRec * (nq > 0 ? nq : 1) + 255) / 256 * 256;
   const size_t df_bytes = ((mixed ? sizeof(BemPostDF) : sizeof(BemPostRec)) * (nq > 0 ? nq : 1) + 255) / 256 * 256;
   const size_t part_bytes = sizeof(double) * 6 * (size_t)nslice * (size_t)nump;
-  IBEM_CUDA(cudaMallocAsync((void**)&tab, tab_bytes + df_bytes + part_bytes, st));
+  IBEM_CUDA(pool_alloc((void**)&tab, tab_bytes + df_bytes + part_bytes, st));
   void* recs = reinterpret_cast<char*>(tab) + tab_bytes;   // the form's records of the Gauss points
   double* part = reinterpret_cast<double*>(reinterpret_cast<char*>(tab) + tab_bytes + df_bytes);
   const unsigned gq = (unsigned)((nq + 127) / 128);
@@ -790,7 +790,7 @@ ibem_status bem_post(const double* pts, int nump, const double* nodes, int NN, c
   }
   ::ibem::count_launch(), k_post_reduce<<<(unsigned)((6 * (int64_t)nump + 255) / 256), 256, 0, st>>>(nump, nslice,
                                                                                                    part, stress);
-  cudaFreeAsync(tab, st);
+  pool_free(tab, st);
   IBEM_LAUNCH_CHECK("bem_post");
   return IBEM_OK;
 }

@@ -380,7 +380,7 @@ ibem_status ibem_e3d_field_grid(ibem_solver_form form, const double* lo, const d
   if (nump == 0) return IBEM_OK;
   cudaStream_t st = as_stream(stream);
   double* pts = nullptr;
-  IBEM_CUDA(cudaMallocAsync((void**)&pts, sizeof(double) * 3 * nump, st));
+  IBEM_CUDA(pool_alloc(&pts, sizeof(double) * 3 * nump, st));
   GridSpec g;
   for (int d = 0; d < 3; ++d) g.lo[d] = lo[d], g.span[d] = hi[d] - lo[d], g.n[d] = n[d];
   ::ibem::count_launch(), k_grid_points<<<(unsigned)((nump + 255) / 256), 256, 0, st>>>(nump, g, pts);
@@ -390,7 +390,7 @@ ibem_status ibem_e3d_field_grid(ibem_solver_form form, const double* lo, const d
   if (!s)
     s = ibem_e3d_field_form(form, pts, (int)nump, centers_dev, radius_dev, num, mat, layout, E_dev, nodes_dev, NN,
                             conn_dev, NE, U_dev, T_dev, sig_inf, stress_dev, stream);
-  cudaFreeAsync(pts, st);
+  pool_free(pts, st);
   return s;
 }
 

@@ -247,7 +247,7 @@ ibem_status ibem_e3d_ell_pair_blocks(const double* centers_dev, const double* ax
   if (num == 0) return IBEM_OK;
   cudaStream_t st = as_stream(stream);
   double* Q = nullptr;   // rotations, then their matrices on symmetric tensors
-  IBEM_CUDA(cudaMallocAsync((void**)&Q, sizeof(double) * (9 + ell::kRotSize) * (size_t)num, st));
+  IBEM_CUDA(pool_alloc((void**)&Q, sizeof(double) * (9 + ell::kRotSize) * (size_t)num, st));
   double* M = Q + 9 * (size_t)num;
   s = ell_rotations(quats_dev, num, Q, st);
   if (!s) {
@@ -260,7 +260,7 @@ ibem_status ibem_e3d_ell_pair_blocks(const double* centers_dev, const double* ax
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) s = cuda_fail(e, "ell_pair_blocks");
   }
-  cudaFreeAsync(Q, st);
+  pool_free(Q, st);
   return s;
 }
 
@@ -282,7 +282,7 @@ ibem_status ibem_e3d_ell_field(ibem_solver_form form, const double* points_dev, 
   IBEM_LAUNCH_CHECK("ell_field init");
   if (num == 0) return IBEM_OK;
   double* Q = nullptr;
-  IBEM_CUDA(cudaMallocAsync((void**)&Q, sizeof(double) * 9 * (size_t)num, st));
+  IBEM_CUDA(pool_alloc((void**)&Q, sizeof(double) * 9 * (size_t)num, st));
   s = ell_rotations(quats_dev, num, Q, st);
   if (!s) {
     const SphMat mc = sph_mat_init(mat->E0, mat->nu0, mat->E1, mat->nu1);
@@ -294,7 +294,7 @@ ibem_status ibem_e3d_ell_field(ibem_solver_form form, const double* points_dev, 
     const int gx = (nump + kEllFieldThreads - 1) / kEllFieldThreads;
     const int nsl = std::max(1, std::min((8 * nsm + gx - 1) / gx, (num + kEllChunk - 1) / kEllChunk));
     double* part = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&part, (sizeof(double) * 6 + sizeof(int)) * (size_t)nsl * nump, st);
+    cudaError_t e = pool_alloc((void**)&part, (sizeof(double) * 6 + sizeof(int)) * (size_t)nsl * nump, st);
     if (e == cudaSuccess) {
       int* inside = reinterpret_cast<int*>(part + 6 * (size_t)nsl * nump);
       ::ibem::count_launch(), k_ell_field24<<<dim3((unsigned)gx, (unsigned)nsl), kEllFieldThreads, 0, st>>>(
@@ -303,11 +303,11 @@ ibem_status ibem_e3d_ell_field(ibem_solver_form form, const double* points_dev, 
       ::ibem::count_launch(), k_ell_field_reduce<<<(unsigned)((nump + 255) / 256), 256, 0, st>>>(
           nump, nsl, part, inside, points_dev, centers_dev, E_dev, mc, stress_dev);
       e = cudaGetLastError();
-      cudaFreeAsync(part, st);
+      pool_free(part, st);
     }
     if (e != cudaSuccess) s = cuda_fail(e, "ell_field");
   }
-  cudaFreeAsync(Q, st);
+  pool_free(Q, st);
   return s;
 }
 
@@ -324,8 +324,8 @@ ibem_status ibem_e3d_run_host_ell(ibem_solver_form form, const ibem_material* ma
   double *A = nullptr, *g = nullptr;
   const size_t geo = (size_t)num * 10 + (size_t)nump * 9 + 2 * (size_t)N;
   ibem_status s = IBEM_OK;
-  cudaError_t e = cudaMalloc((void**)&A, sizeof(double) * (size_t)N * (size_t)N);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&g, sizeof(double) * geo);
+  cudaError_t e = pool_alloc(&A, sizeof(double) * (size_t)N * (size_t)N, st);
+  if (e == cudaSuccess) e = pool_alloc(&g, sizeof(double) * geo, st);
   if (e != cudaSuccess) s = cuda_fail(e, "run_host_ell: device memory");
   double *c = g, *a = g + 3 * (size_t)num, *q = g + 6 * (size_t)num, *p = g + 10 * (size_t)num;
   double *S = p + 3 * (size_t)nump, *b = S + 6 * (size_t)nump, *x = b + N;
@@ -349,8 +349,9 @@ ibem_status ibem_e3d_run_host_ell(ibem_solver_form form, const ibem_material* ma
     if (e != cudaSuccess) s = cuda_fail(e, "run_host_ell: download");
   }
   if (report) *report = rep;
-  cudaFree(A);
-  cudaFree(g);
+  if (s) cudaStreamSynchronize(st);   // after an error: nothing in flight uses them
+  pool_free(A, st);
+  pool_free(g, st);
   cudaStreamDestroy(st);
   return s;
 }

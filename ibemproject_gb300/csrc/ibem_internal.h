@@ -26,6 +26,21 @@ ibem_status cuda_fail(cudaError_t e, const char* where);
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// Stream-ordered device memory for the library's buffers and workspaces, from a pool of its own
+// (one per device, made on first use): allocation and release are queued on the stream, safe
+// from any thread and stream.  Between calls the pool keeps at most kPoolKeep bytes (what is
+// beyond goes back at the next synchronisation), because mapping and unmapping memory on
+// every call cost more than the small solves themselves (a training step: 0.4 of 1.3 ms; six
+// ellipsoid realisations on four threads: 19 of 34 ms in cudaMalloc alone); an allocation that
+// fails gives everything kept back and tries once more.
+constexpr size_t kPoolKeep = (size_t)1 << 30;
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st);
+void pool_free(void* p, cudaStream_t st);
+template <class T>
+cudaError_t pool_alloc(T** p, size_t bytes, cudaStream_t st) {
+  return pool_alloc(reinterpret_cast<void**>(p), bytes, st);
+}
+
 // Counts kernel launches of this library (read through ibem_kernel_launches); every
 // launch site is written `::ibem::count_launch(), kernel<<<...>>>(...)`.
 int count_launch();

@@ -34,14 +34,10 @@ struct MfTile {
 };
 
 // Stream-ordered scratch: allocations and frees of the solver's temporaries are queued on
-// the call's stream (cudaMallocAsync / cudaFreeAsync), so that no call synchronises the
-// device to release memory.
-inline cudaError_t alloc_async(void** p, size_t bytes, cudaStream_t st) {
-  return cudaMallocAsync(p, bytes > 0 ? bytes : 1, st);
-}
-inline void free_async(void* p, cudaStream_t st) {
-  if (p) cudaFreeAsync(p, st);
-}
+// the call's stream (the library's pool), so that no call synchronises the device to release
+// memory.
+inline cudaError_t alloc_async(void** p, size_t bytes, cudaStream_t st) { return pool_alloc(p, bytes, st); }
+inline void free_async(void* p, cudaStream_t st) { pool_free(p, st); }
 
 struct MfBatch {
   cudaStream_t st = nullptr;   // stream of the call that owns the batch's buffers

@@ -27,6 +27,55 @@ std::vector<Rec> g_recs;
 std::vector<cudaEvent_t> g_pool;
 }  // namespace
 
+// ---- stream-ordered device memory (ibem_internal.h) ----
+namespace {
+constexpr int kMaxDevices = 64;
+std::mutex g_mem_mu;
+cudaMemPool_t g_mem[kMaxDevices] = {};
+bool g_mem_tried[kMaxDevices] = {};
+
+// the device's pool, or nullptr: the default pool is used then
+cudaMemPool_t device_pool(int dev) {
+  if (dev < 0 || dev >= kMaxDevices) return nullptr;
+  std::lock_guard<std::mutex> l(g_mem_mu);
+  if (!g_mem_tried[dev]) {
+    g_mem_tried[dev] = true;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    uint64_t keep = kPoolKeep;
+    if (cudaMemPoolCreate(&pool, &props) == cudaSuccess &&
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+      g_mem[dev] = pool;
+    else
+      cudaGetLastError();
+  }
+  return g_mem[dev];
+}
+}  // namespace
+
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st) {
+  int dev = 0;
+  *p = nullptr;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (bytes == 0) bytes = 1;
+  const cudaMemPool_t pool = device_pool(dev);
+  e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMallocAsync(p, bytes, st);
+  if (e == cudaErrorMemoryAllocation && pool) {
+    cudaGetLastError();
+    cudaStreamSynchronize(st);   // what this stream released goes back too
+    cudaMemPoolTrimTo(pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+  }
+  return e;
+}
+void pool_free(void* p, cudaStream_t st) {
+  if (p) cudaFreeAsync(p, st);
+}
+
 bool prof_on() { return g_on.load(std::memory_order_relaxed); }
 
 cudaEvent_t prof_event() {

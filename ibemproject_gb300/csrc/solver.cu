@@ -1189,6 +1189,7 @@ __global__ void k_vmul(int64_t n, const double* __restrict__ a, const double* __
 // =====================================================================================
 template <typename T>
 struct LuWork {
+  cudaStream_t st = nullptr; // stream of the allocations
   CaluBufs<T> cb{};          // buffers of the panel kernel (one allocation at cb_mem)
   void* cb_mem = nullptr;
   int* ipiv_dev = nullptr;  // N entries (global, absolute row of each exchange)
@@ -1357,40 +1358,40 @@ static ibem_status lu_alloc(LuWork<T>& w, int64_t N) {
   if (per_sm < 1) return fail(IBEM_ERR_CUDA, "panel kernel cannot be resident");
   w.ncta = std::min(nsm, kCaluMaxCta);  // at most one CTA per SM (co-resident for the cooperative launch)
   if ((int64_t)w.ncta * 1024 < N) return fail(IBEM_ERR_ARG, "matrix too large for the panel kernel");
-  IBEM_CUDA(cudaMalloc(&w.cb_mem, calu_bytes<T>(w.ncta)));
-  IBEM_CUDA(cudaMemset(w.cb_mem, 0, calu_bytes<T>(w.ncta)));
+  IBEM_CUDA(pool_alloc(&w.cb_mem, calu_bytes<T>(w.ncta), w.st));
+  IBEM_CUDA(cudaMemsetAsync(w.cb_mem, 0, calu_bytes<T>(w.ncta), w.st));
   w.cb = calu_carve<T>(static_cast<unsigned char*>(w.cb_mem), w.ncta);
-  IBEM_CUDA(cudaMalloc(&w.ipiv_dev, sizeof(int) * (size_t)N));
-  IBEM_CUDA(cudaMalloc(&w.perm, sizeof(int) * (size_t)N));
-  IBEM_CUDA(cudaMalloc(&w.tmp, sizeof(double) * (size_t)N));
-  IBEM_CUDA(cudaMalloc(&w.info, sizeof(int)));
-  IBEM_CUDA(cudaMalloc(&w.gs, sizeof(GridSync)));
+  IBEM_CUDA(pool_alloc(&w.ipiv_dev, sizeof(int) * (size_t)N, w.st));
+  IBEM_CUDA(pool_alloc(&w.perm, sizeof(int) * (size_t)N, w.st));
+  IBEM_CUDA(pool_alloc(&w.tmp, sizeof(double) * (size_t)N, w.st));
+  IBEM_CUDA(pool_alloc(&w.info, sizeof(int), w.st));
+  IBEM_CUDA(pool_alloc(&w.gs, sizeof(GridSync), w.st));
   {
     const int64_t nblk = (N + kTrsvB - 1) / kTrsvB;
-    IBEM_CUDA(cudaMalloc(&w.dinv, sizeof(T) * 2 * (size_t)nblk * kTrsvB * kTrsvB));
-    IBEM_CUDA(cudaMalloc(&w.tflags, sizeof(int) * (size_t)nblk));
-    IBEM_CUDA(cudaMemset(w.tflags, 0, sizeof(int) * (size_t)nblk));
+    IBEM_CUDA(pool_alloc(&w.dinv, sizeof(T) * 2 * (size_t)nblk * kTrsvB * kTrsvB, w.st));
+    IBEM_CUDA(pool_alloc(&w.tflags, sizeof(int) * (size_t)nblk, w.st));
+    IBEM_CUDA(cudaMemsetAsync(w.tflags, 0, sizeof(int) * (size_t)nblk, w.st));
     int per = 0;
     IBEM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trsv_persist<T, true, true>, kTrsvThreads,
                                                             trsv_persist_smem<T>()));
     if (per < 1) return fail(IBEM_ERR_CUDA, "triangular-solve kernel cannot be resident");
     w.trsv_grid = per * nsm;
   }
-  IBEM_CUDA(cudaMemset(w.info, 0, sizeof(int)));
-  IBEM_CUDA(cudaMemset(w.gs, 0, sizeof(GridSync)));
+  IBEM_CUDA(cudaMemsetAsync(w.info, 0, sizeof(int), w.st));
+  IBEM_CUDA(cudaMemsetAsync(w.gs, 0, sizeof(GridSync), w.st));
   if (sizeof(T) == sizeof(float)) {
     w.gemm_ws_bytes = gemm_tc_workspace_bytes(N, N / 2 + 2 * kLeaf);
-    IBEM_CUDA(cudaMalloc(&w.gemm_ws, w.gemm_ws_bytes));
-    IBEM_CUDA(cudaMalloc(&w.gemm_err, sizeof(int)));
-    IBEM_CUDA(cudaMemset(w.gemm_err, 0, sizeof(int)));
+    IBEM_CUDA(pool_alloc(&w.gemm_ws, w.gemm_ws_bytes, w.st));
+    IBEM_CUDA(pool_alloc(&w.gemm_err, sizeof(int), w.st));
+    IBEM_CUDA(cudaMemsetAsync(w.gemm_err, 0, sizeof(int), w.st));
   } else {
     w.gemm_ws_bytes = gemm_tc64_workspace_bytes(N, N / 2 + 2 * kLeaf);
-    if (cudaMalloc(&w.gemm_ws, w.gemm_ws_bytes) != cudaSuccess) {   // no room: the updates stay on the FP64 pipe
+    if (pool_alloc(&w.gemm_ws, w.gemm_ws_bytes, w.st) != cudaSuccess) {   // no room: the updates stay on the FP64 pipe
       cudaGetLastError();
       w.gemm_ws = nullptr;
     } else {
-      IBEM_CUDA(cudaMalloc(&w.gemm_err, sizeof(int)));
-      IBEM_CUDA(cudaMemset(w.gemm_err, 0, sizeof(int)));
+      IBEM_CUDA(pool_alloc(&w.gemm_err, sizeof(int), w.st));
+      IBEM_CUDA(cudaMemsetAsync(w.gemm_err, 0, sizeof(int), w.st));
     }
   }
   return IBEM_OK;
@@ -1398,16 +1399,16 @@ static ibem_status lu_alloc(LuWork<T>& w, int64_t N) {
 
 template <typename T>
 static void lu_free(LuWork<T>& w) {
-  cudaFree(w.cb_mem);
-  cudaFree(w.ipiv_dev);
-  cudaFree(w.perm);
-  cudaFree(w.tmp);
-  cudaFree(w.info);
-  cudaFree(w.gs);
-  cudaFree(w.dinv);
-  cudaFree(w.tflags);
-  cudaFree(w.gemm_ws);
-  cudaFree(w.gemm_err);
+  pool_free(w.cb_mem, w.st);
+  pool_free(w.ipiv_dev, w.st);
+  pool_free(w.perm, w.st);
+  pool_free(w.tmp, w.st);
+  pool_free(w.info, w.st);
+  pool_free(w.gs, w.st);
+  pool_free(w.dinv, w.st);
+  pool_free(w.tflags, w.st);
+  pool_free(w.gemm_ws, w.st);
+  pool_free(w.gemm_err, w.st);
   w = LuWork<T>();
 }
 
@@ -1557,17 +1558,17 @@ struct SolveCtx {
   ibem_status alloc(int64_t n, cudaStream_t s) {
     N = n;
     st = s;
-    IBEM_CUDA(cudaMalloc(&r, sizeof(double) * N));
-    IBEM_CUDA(cudaMalloc(&c, sizeof(double) * N));
-    IBEM_CUDA(cudaMalloc(&rs, sizeof(double) * N));
-    IBEM_CUDA(cudaMalloc(&part, sizeof(double) * N * nparts));
+    IBEM_CUDA(pool_alloc(&r, sizeof(double) * N, st));
+    IBEM_CUDA(pool_alloc(&c, sizeof(double) * N, st));
+    IBEM_CUDA(pool_alloc(&rs, sizeof(double) * N, st));
+    IBEM_CUDA(pool_alloc(&part, sizeof(double) * N * nparts, st));
     return IBEM_OK;
   }
   ~SolveCtx() {
-    cudaFree(r);
-    cudaFree(c);
-    cudaFree(part);
-    cudaFree(rs);
+    pool_free(r, st);
+    pool_free(c, st);
+    pool_free(part, st);
+    pool_free(rs, st);
   }
 };
 
@@ -1795,7 +1796,8 @@ static ibem_status equilibrate(SolveCtx& cx, const double* A, int64_t lda) {
 template <typename T>
 static ibem_status factor(SolveCtx& cx, const double* A, int64_t lda, T*& W, LuWork<T>& w, int& info) {
   const int64_t N = cx.N;
-  IBEM_CUDA(cudaMalloc(&W, sizeof(T) * (size_t)N * N));
+  IBEM_CUDA(pool_alloc(&W, sizeof(T) * (size_t)N * N, cx.st));
+  w.st = cx.st;
   {
     ProfScope ps(PROF_EQUIL, cx.st);
     if (ibem_status q = equilibrate(cx, A, lda)) return q;
@@ -1929,10 +1931,10 @@ ibem_status solve_dense(ibem_solver_form form, int64_t N, double* A, int64_t lda
   // bs = R b, x = C ys: errors are measured row-relative, so the small boundary rows of
   // the iBEM matrix weigh as much as the inclusion rows.
   double *bs = nullptr, *ys = nullptr, *rvec = nullptr, *tmp = nullptr;
-  IBEM_CUDA(cudaMalloc(&bs, sizeof(double) * N));
-  IBEM_CUDA(cudaMalloc(&ys, sizeof(double) * N));
-  IBEM_CUDA(cudaMalloc(&rvec, sizeof(double) * N));
-  IBEM_CUDA(cudaMalloc(&tmp, sizeof(double) * N));
+  IBEM_CUDA(pool_alloc(&bs, sizeof(double) * N, st));
+  IBEM_CUDA(pool_alloc(&ys, sizeof(double) * N, st));
+  IBEM_CUDA(pool_alloc(&rvec, sizeof(double) * N, st));
+  IBEM_CUDA(pool_alloc(&tmp, sizeof(double) * N, st));
   cudaEvent_t e0, e1, e2;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -1978,7 +1980,7 @@ ibem_status solve_dense(ibem_solver_form form, int64_t N, double* A, int64_t lda
     }
     cudaEventRecord(e2, st);
     lu_free(w);
-    cudaFree(W);
+    pool_free(W, st);
   } else if (form == IBEM_SOLVE_GMRES_BJ) {
     // As32 = FP32 copy of the scaled matrix, P = FP32 inverses of its block x block diagonal
     // blocks; refinement: FP64 residual rs = bs - As ys, GMRES with As32 products (FP64
@@ -1990,15 +1992,15 @@ ibem_status solve_dense(ibem_solver_form form, int64_t N, double* A, int64_t lda
     float *W = nullptr, *P = nullptr, *zf = nullptr;
     double *V = nullptr, *Z = nullptr, *hd = nullptr;
     int* info_dev = nullptr;
-    cudaError_t ce = ws32 ? cudaSuccess : cudaMalloc(&W, sizeof(float) * (size_t)ldw * N);
+    cudaError_t ce = ws32 ? cudaSuccess : pool_alloc(&W, sizeof(float) * (size_t)ldw * N, st);
     float* const Wown = W;
     if (ws32) W = ws32;
-    if (ce == cudaSuccess) ce = cudaMalloc(&P, sizeof(float) * (size_t)nblk * block * block);
-    if (ce == cudaSuccess) ce = cudaMalloc(&zf, sizeof(float) * (size_t)N);
-    if (ce == cudaSuccess) ce = cudaMalloc(&V, sizeof(double) * (size_t)N * (m + 1));
-    if (ce == cudaSuccess) ce = cudaMalloc(&Z, sizeof(double) * (size_t)N * m);
-    if (ce == cudaSuccess) ce = cudaMalloc(&hd, sizeof(double) * (m + 1) * 2);
-    if (ce == cudaSuccess) ce = cudaMalloc(&info_dev, sizeof(int));
+    if (ce == cudaSuccess) ce = pool_alloc(&P, sizeof(float) * (size_t)nblk * block * block, st);
+    if (ce == cudaSuccess) ce = pool_alloc(&zf, sizeof(float) * (size_t)N, st);
+    if (ce == cudaSuccess) ce = pool_alloc(&V, sizeof(double) * (size_t)N * (m + 1), st);
+    if (ce == cudaSuccess) ce = pool_alloc(&Z, sizeof(double) * (size_t)N * m, st);
+    if (ce == cudaSuccess) ce = pool_alloc(&hd, sizeof(double) * (m + 1) * 2, st);
+    if (ce == cudaSuccess) ce = pool_alloc(&info_dev, sizeof(int), st);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(info_dev, 0, sizeof(int), st);
     if (ce != cudaSuccess) s = cuda_fail(ce, "block-Jacobi workspace");
     if (!s) {
@@ -2066,13 +2068,13 @@ ibem_status solve_dense(ibem_solver_form form, int64_t N, double* A, int64_t lda
     cudaEventRecord(e2, st);
     if (!s && R.backward_error > tol) s = fail(IBEM_ERR_NOCONV, "block-Jacobi GMRES did not reach the tolerance");
     R.iterations = iters;
-    cudaFree(Wown);
-    cudaFree(P);
-    cudaFree(zf);
-    cudaFree(V);
-    cudaFree(Z);
-    cudaFree(hd);
-    cudaFree(info_dev);
+    pool_free(Wown, st);
+    pool_free(P, st);
+    pool_free(zf, st);
+    pool_free(V, st);
+    pool_free(Z, st);
+    pool_free(hd, st);
+    pool_free(info_dev, st);
   } else {
     float* W = nullptr;
     LuWork<float> w;
@@ -2084,9 +2086,9 @@ ibem_status solve_dense(ibem_solver_form form, int64_t N, double* A, int64_t lda
     const int m = 30, max_outer = 20;
     double *V = nullptr, *Z = nullptr, *hd = nullptr;
     if (!s) {
-      cudaError_t ce = cudaMalloc(&V, sizeof(double) * (size_t)N * (m + 1));
-      if (ce == cudaSuccess) ce = cudaMalloc(&Z, sizeof(double) * (size_t)N * m);
-      if (ce == cudaSuccess) ce = cudaMalloc(&hd, sizeof(double) * (m + 1) * 2);
+      cudaError_t ce = pool_alloc(&V, sizeof(double) * (size_t)N * (m + 1), st);
+      if (ce == cudaSuccess) ce = pool_alloc(&Z, sizeof(double) * (size_t)N * m, st);
+      if (ce == cudaSuccess) ce = pool_alloc(&hd, sizeof(double) * (m + 1) * 2, st);
       if (ce != cudaSuccess) s = cuda_fail(ce, "gmres workspace");
     }
     if (!s) {
@@ -2124,11 +2126,11 @@ ibem_status solve_dense(ibem_solver_form form, int64_t N, double* A, int64_t lda
       if (!s && be > tol) s = fail(IBEM_ERR_NOCONV, "GMRES-IR did not reach the tolerance");
     }
     R.iterations = iters;
-    cudaFree(V);
-    cudaFree(Z);
-    cudaFree(hd);
+    pool_free(V, st);
+    pool_free(Z, st);
+    pool_free(hd, st);
     lu_free(w);
-    cudaFree(W);
+    pool_free(W, st);
   }
   // x = C ys; also when the tolerance was missed, so that the caller gets the iterate reached
   if (!s || s == IBEM_ERR_NOCONV) ::ibem::count_launch(), k_vmul<<<nb, 256, 0, st>>>(N, cx.c, ys, x);
@@ -2141,10 +2143,10 @@ ibem_status solve_dense(ibem_solver_form form, int64_t N, double* A, int64_t lda
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaEventDestroy(e2);
-  cudaFree(bs);
-  cudaFree(ys);
-  cudaFree(rvec);
-  cudaFree(tmp);
+  pool_free(bs, st);
+  pool_free(ys, st);
+  pool_free(rvec, st);
+  pool_free(tmp, st);
   if (rep) *rep = R;
   return s;
 }

@@ -258,7 +258,7 @@ ibem_status launch_field24_df(const SphLaunch& p, const double* pts, int nump, c
   const size_t nacc = up((size_t)nump * 6 * sizeof(dfloat));
   const size_t bytes = 256 + 4 * n4 + nsph + nmsk + nacc + sort_bytes;
   char* buf = nullptr;
-  IBEM_CUDA(cudaMallocAsync((void**)&buf, bytes, st));
+  IBEM_CUDA(pool_alloc((void**)&buf, bytes, st));
   unsigned long long* box = reinterpret_cast<unsigned long long*>(buf);
   char* q = buf + 256;
   unsigned* k0 = reinterpret_cast<unsigned*>(q);
@@ -292,7 +292,7 @@ ibem_status launch_field24_df(const SphLaunch& p, const double* pts, int nump, c
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) s = cuda_fail(e, "field24_df");
-  cudaFreeAsync(buf, st);
+  pool_free(buf, st);
   return s;
 }
 

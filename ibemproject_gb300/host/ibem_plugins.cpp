@@ -20,15 +20,15 @@ static void check_cuda(cudaError_t e, const char* where) {
 }
 
 template <typename T>
-void DeviceArray<T>::alloc(size_t count) {
+void DeviceArray<T>::alloc(size_t count, cudaStream_t stream) {
   reset();
   if (count == 0) return;
-  check_cuda(cudaMalloc(&p, count * sizeof(T)), "cudaMalloc");
+  check_cuda(ibem::pool_alloc(&p, count * sizeof(T), stream), "device memory");
   n = count;
 }
 template <typename T>
 void DeviceArray<T>::upload(const std::vector<T>& h, cudaStream_t st) {
-  alloc(h.size());
+  alloc(h.size(), st);
   if (!h.empty()) check_cuda(cudaMemcpyAsync(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, st), "upload");
 }
 template <typename T>
@@ -132,14 +132,14 @@ void configElastic3D_gb300::upload() {
   d_rad.upload(radius, stream);
   d_pts.upload(x_p, stream);
   const int64_t N = n_unknowns();
-  HMAT.alloc((size_t)N * N);
+  HMAT.alloc((size_t)N * N, stream);
   check_cuda(cudaMemsetAsync(HMAT.p, 0, sizeof(double) * (size_t)N * N, stream), "HMAT zero");
   if (NE > 0) {
-    GMAT.alloc((size_t)N * 12 * NE);
+    GMAT.alloc((size_t)N * 12 * NE, stream);
     check_cuda(cudaMemsetAsync(GMAT.p, 0, sizeof(double) * GMAT.n, stream), "GMAT zero");
   }
-  b.alloc(N);
-  X.alloc(N);
+  b.alloc(N, stream);
+  X.alloc(N, stream);
 }
 
 // ------------------------------------------------------------------ integrator
@@ -202,7 +202,7 @@ void BEMBuilderElastic3D_gb300::ApplyBC(Config& c_) {
         "ApplyBC plan");
   c.d_ucol.upload(c.ucol, c.stream);
   c.d_tcol.upload(c.tcol, c.stream);
-  c.A.alloc((size_t)N * N);
+  c.A.alloc((size_t)N * N, c.stream);
   check(ibem_e3d_apply_bc(c.NN, c.NE, N, c.d_ucol.p, c.d_tcol.p, c.d_bc.p, c.d_tbc.p, c.HMAT.p, N, c.GMAT.p, N, c.A.p,
                           N, c.b.p, c.stream),
         "ApplyBC");
@@ -215,12 +215,12 @@ void BEMBuilderElastic3D_gb300::ApplyBC(Config& c_) {
 void BEMBuilderElastic3D_gb300::getUTVector(Config& c_) {
   auto& c = as_e3d(c_);
   const int64_t N = c.n_unknowns();
-  c.U.alloc(N);
+  c.U.alloc(N, c.stream);
   if (c.NE == 0) {
     check_cuda(cudaMemcpyAsync(c.U.p, c.X.p, sizeof(double) * N, cudaMemcpyDeviceToDevice, c.stream), "getUTVector");
     return;
   }
-  c.T.alloc(12 * (size_t)c.NE);
+  c.T.alloc(12 * (size_t)c.NE, c.stream);
   check(ibem_e3d_get_ut(c.NN, c.NE, N, c.d_ucol.p, c.d_tcol.p, c.d_bc.p, c.d_tbc.p, c.X.p, c.U.p, c.T.p, c.stream),
         "getUTVector");
 }
@@ -236,7 +236,7 @@ void systemSolverElastic3D_gb300::solve(Config& c_) {
 void postProcessorElastic3D_gb300::getFlux(Config& c_) {
   auto& c = as_e3d(c_);
   const ibem_material m = c.material();
-  c.stress.alloc(6 * (size_t)c.nump);
+  c.stress.alloc(6 * (size_t)c.nump, c.stream);
   const double* E = c.U.p + 3 * (int64_t)c.NN;
   check(ibem_e3d_field_form(c.form, c.d_pts.p, c.nump, c.d_cen.p, c.d_rad.p, c.num, &m, c.layout, E, c.d_nodes.p,
                             c.NN, c.d_conn.p, c.NE, c.U.p, c.T.p, c.sig_inf.empty() ? nullptr : c.sig_inf.data(),

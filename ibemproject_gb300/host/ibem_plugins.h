@@ -34,7 +34,7 @@ struct ibem_error : std::runtime_error {
 };
 
 template <typename T>
-struct DeviceArray {
+struct DeviceArray {   // memory of the library's pool, allocated on the configuration's stream
   T* p = nullptr;
   size_t n = 0;
   DeviceArray() = default;
@@ -42,11 +42,14 @@ struct DeviceArray {
   DeviceArray& operator=(const DeviceArray&) = delete;
   ~DeviceArray() { reset(); }
   void reset() {
-    if (p) cudaFree(p);
+    if (p) {
+      cudaDeviceSynchronize();   // cudaFree waits for nothing when it gives pool memory back
+      cudaFree(p);
+    }
     p = nullptr;
     n = 0;
   }
-  void alloc(size_t count);
+  void alloc(size_t count, cudaStream_t st);
   void upload(const std::vector<T>& h, cudaStream_t st);
   void download(std::vector<T>& h, cudaStream_t st) const;
 };
