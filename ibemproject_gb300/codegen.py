@@ -655,13 +655,13 @@ IBEM_HD inline SphMat sph_mat_init(double E0, double nu0, double E1, double nu1)
 _F32_LIT = re.compile(r"(?<![\w.])(\d+\.\d*(?:[eE][+-]?\d+)?)(?![\w.])")
 
 F32_HEAD = """// GENERATED by ibemproject_gb300/codegen.py -- do not edit by hand.
-// FP32 variant of the layout-24 sphere blocks for the matrix-free solver, which calls
-// them in coordinates scaled by the source radius (a = 1), so that every intermediate is
-// O(1) in single precision.  Same derivation as gen_sphere24.cuh.
+// FP32 materials and own (C0) term of the matrix-free layout-24 products, which work in
+// coordinates scaled by the source radius (a = 1), so that every intermediate is O(1) in
+// single precision.  Same derivation as gen_sphere24.cuh.
 #pragma once
 #include "gen_sphere_common.cuh"
 
-// Dimensionless material constants of the FP32 blocks (sph_matf_init: SphMat / mu0).
+// Dimensionless material constants of the FP32 products (sph_matf_init: SphMat / mu0).
 struct SphMatF {
   float kmu, klam, tn1, tn2;  // as SphMat, contrast terms divided by mu0
   float lam0, mu0;            // C0 / mu0 (self term): lam0 / mu0 and 1
@@ -719,10 +719,6 @@ def generate(out_dir: str | None = None) -> dict:
     parts.append(gen_self_function("sph_self24", 24))
     files["gen_sphere24.cuh"] = "\n\n".join(parts) + "\n"
     fparts = [F32_HEAD]
-    for co in range(2):
-        for ro in range(2):
-            nm = f"sph_block24_c{co}_r{ro}"
-            fparts.append(to_f32(parts[1 + 2 * co + ro], nm, nm.replace("block24", "block24f")))
     fparts.append(to_f32(gen_self_function("sph_self24", 24), "sph_self24", "sph_self24f"))
     files["gen_sphere24_f32.cuh"] = "\n\n".join(fparts) + "\n"
     for lay in (78, 60):

@@ -1,11 +1,11 @@
 // GENERATED by ibemproject_gb300/codegen.py -- do not edit by hand.
-// FP32 variant of the layout-24 sphere blocks for the matrix-free solver, which calls
-// them in coordinates scaled by the source radius (a = 1), so that every intermediate is
-// O(1) in single precision.  Same derivation as gen_sphere24.cuh.
+// FP32 materials and own (C0) term of the matrix-free layout-24 products, which work in
+// coordinates scaled by the source radius (a = 1), so that every intermediate is O(1) in
+// single precision.  Same derivation as gen_sphere24.cuh.
 #pragma once
 #include "gen_sphere_common.cuh"
 
-// Dimensionless material constants of the FP32 blocks (sph_matf_init: SphMat / mu0).
+// Dimensionless material constants of the FP32 products (sph_matf_init: SphMat / mu0).
 struct SphMatF {
   float kmu, klam, tn1, tn2;  // as SphMat, contrast terms divided by mu0
   float lam0, mu0;            // C0 / mu0 (self term): lam0 / mu0 and 1
@@ -23,2825 +23,6 @@ IBEM_HD inline SphMatF sph_matf_init(const SphMat& m) {
   return f;
 }
 
-
-template <class Sink>
-IBEM_HD IBEM_INLINE void sph_block24f_c0_r0(const float x0, const float x1, const float x2,
-    const float a, const SphMatF& mc, Sink& sink) {
-  const float a2 = a * a; const float a4 = a2 * a2;
-  const float u = 0.5f * (x0 * x0 + x1 * x1 + x2 * x2);
-  const float lam = 2.0f * u - a2;
-  const float ext = lam > 0.0f ? 1.0f : 0.0f;
-  const float rho2 = lam > 0.0f ? a2 + lam : a2;
-  float Jv[5];
-  {
-    // J_m = 4 pi a^3 / ((2m+1) rho^(2m+1)),  rho^2 = a^2 + lambda
-    const float irho2 = 1.0f / rho2;
-    float pw = 4.0f * 3.14159265358979f * a * a2 / sqrtf(rho2);
-    for (int m = 0; m <= 4; ++m) { Jv[m] = pw / (2 * m + 1); pw *= irho2; }
-  }
-  const float kmu = mc.kmu, klam = mc.klam, tn1 = mc.tn1, tn2 = mc.tn2;
-  (void)kmu; (void)klam; (void)tn1; (void)tn2; (void)a4;
-  const float t0 = ext * (35.0f * Jv[3]);
-  const float t1 = -(t0);
-  const float t2 = ext * (63.0f * Jv[4]);
-  const float t3 = -(t2);
-  const float t4 = (1.0f) * t1 + (-a2) * t3;
-  const float t5 = x0 * x0;
-  const float t6 = t5 * x0;
-  const float t7 = t6 * x0;
-  const float t8 = ext * (-5.0f * Jv[2]);
-  const float t9 = -(t8);
-  const float t10 = ext * (-7.0f * Jv[3]);
-  const float t11 = -(t10);
-  const float t12 = (1.0f) * t9 + (-a2) * t11;
-  const float t13 = -(Jv[1]);
-  const float t14 = -(Jv[2]);
-  const float t15 = (1.0f) * t13 + (-a2) * t14;
-  const float t16 = t4 * t7 + 6.0f * t12 * t5 + 3.0f * t15;
-  const float t17 = t16;
-  const float t18 = t9 * t5 + t13;
-  const float t19 = t18;
-  const float t20 = t5 * x1;
-  const float t21 = t20 * x1;
-  const float t22 = x1 * x1;
-  const float t23 = t4 * t21 + t12 * t5 + t12 * t22 + t15;
-  const float t24 = t23;
-  const float t25 = t9 * t22 + t13;
-  const float t26 = t25;
-  const float t27 = t5 * x2;
-  const float t28 = t27 * x2;
-  const float t29 = x2 * x2;
-  const float t30 = t4 * t28 + t12 * t5 + t12 * t29 + t15;
-  const float t31 = t30;
-  const float t32 = t9 * t29 + t13;
-  const float t33 = t32;
-  const float t34 = (t17 - tn2 * t19 - tn1 * (t19 + t19 + t19 + t19));
-  const float t35 = (t17 - tn2 * t19 - tn1 * (t19 + t19 + t19 + t19)) + (t24 - tn2 * t26) + (t31 - tn2 * t33);
-  const float t36 = 1.0f * (kmu * t34 + klam * t35);
-  sink(0, 0, t36);
-  const float t37 = t6 * x1;
-  const float t38 = x0 * x1;
-  const float t39 = t4 * t37 + 3.0f * t12 * t38;
-  const float t40 = t39;
-  const float t41 = t9 * t38;
-  const float t42 = t41;
-  const float t43 = (t40 - tn2 * t42 - tn1 * (t42 + t42));
-  const float t44 = 1.0f * (kmu * t43);
-  sink(1, 0, t44);
-  const float t45 = t6 * x2;
-  const float t46 = x0 * x2;
-  const float t47 = t4 * t45 + 3.0f * t12 * t46;
-  const float t48 = t47;
-  const float t49 = t9 * t46;
-  const float t50 = t49;
-  const float t51 = (t48 - tn2 * t50 - tn1 * (t50 + t50));
-  const float t52 = 1.0f * (kmu * t51);
-  sink(2, 0, t52);
-  const float t53 = (t24 - tn2 * t26);
-  const float t54 = (t17 - tn2 * t19 - tn1 * (t19 + t19 + t19 + t19)) + (t24 - tn2 * t26) + (t31 - tn2 * t33);
-  const float t55 = 1.0f * (kmu * t53 + klam * t54);
-  sink(3, 0, t55);
-  const float t56 = t20 * x2;
-  const float t57 = x1 * x2;
-  const float t58 = t4 * t56 + t12 * t57;
-  const float t59 = t58;
-  const float t60 = t9 * t57;
-  const float t61 = t60;
-  const float t62 = (t59 - tn2 * t61);
-  const float t63 = 1.0f * (kmu * t62);
-  sink(4, 0, t63);
-  const float t64 = (t31 - tn2 * t33);
-  const float t65 = (t17 - tn2 * t19 - tn1 * (t19 + t19 + t19 + t19)) + (t24 - tn2 * t26) + (t31 - tn2 * t33);
-  const float t66 = 1.0f * (kmu * t64 + klam * t65);
-  sink(5, 0, t66);
-  const float t67 = t38 * x1;
-  const float t68 = t67 * x1;
-  const float t69 = t4 * t68 + 3.0f * t12 * t38;
-  const float t70 = t69;
-  const float t71 = t38 * x2;
-  const float t72 = t71 * x2;
-  const float t73 = t4 * t72 + t12 * t38;
-  const float t74 = t73;
-  const float t75 = (t40 - tn1 * (t42 + t42));
-  const float t76 = (t40 - tn1 * (t42 + t42)) + (t70 - tn1 * (t42 + t42)) + (t74);
-  const float t77 = 2.0f * (kmu * t75 + klam * t76);
-  sink(0, 1, t77);
-  const float t78 = (t24 - tn1 * (t19 + t26));
-  const float t79 = 2.0f * (kmu * t78);
-  sink(1, 1, t79);
-  const float t80 = (t59 - tn1 * (t61));
-  const float t81 = 2.0f * (kmu * t80);
-  sink(2, 1, t81);
-  const float t82 = (t70 - tn1 * (t42 + t42));
-  const float t83 = (t40 - tn1 * (t42 + t42)) + (t70 - tn1 * (t42 + t42)) + (t74);
-  const float t84 = 2.0f * (kmu * t82 + klam * t83);
-  sink(3, 1, t84);
-  const float t85 = t67 * x2;
-  const float t86 = t4 * t85 + t12 * t46;
-  const float t87 = t86;
-  const float t88 = (t87 - tn1 * (t50));
-  const float t89 = 2.0f * (kmu * t88);
-  sink(4, 1, t89);
-  const float t90 = (t74);
-  const float t91 = (t40 - tn1 * (t42 + t42)) + (t70 - tn1 * (t42 + t42)) + (t74);
-  const float t92 = 2.0f * (kmu * t90 + klam * t91);
-  sink(5, 1, t92);
-  const float t93 = t46 * x2;
-  const float t94 = t93 * x2;
-  const float t95 = t4 * t94 + 3.0f * t12 * t46;
-  const float t96 = t95;
-  const float t97 = (t48 - tn1 * (t50 + t50));
-  const float t98 = (t48 - tn1 * (t50 + t50)) + (t87) + (t96 - tn1 * (t50 + t50));
-  const float t99 = 2.0f * (kmu * t97 + klam * t98);
-  sink(0, 2, t99);
-  const float t100 = (t59 - tn1 * (t61));
-  const float t101 = 2.0f * (kmu * t100);
-  sink(1, 2, t101);
-  const float t102 = (t31 - tn1 * (t19 + t33));
-  const float t103 = 2.0f * (kmu * t102);
-  sink(2, 2, t103);
-  const float t104 = (t87);
-  const float t105 = (t48 - tn1 * (t50 + t50)) + (t87) + (t96 - tn1 * (t50 + t50));
-  const float t106 = 2.0f * (kmu * t104 + klam * t105);
-  sink(3, 2, t106);
-  const float t107 = (t74 - tn1 * (t42));
-  const float t108 = 2.0f * (kmu * t107);
-  sink(4, 2, t108);
-  const float t109 = (t96 - tn1 * (t50 + t50));
-  const float t110 = (t48 - tn1 * (t50 + t50)) + (t87) + (t96 - tn1 * (t50 + t50));
-  const float t111 = 2.0f * (kmu * t109 + klam * t110);
-  sink(5, 2, t111);
-  const float t112 = t22 * x1;
-  const float t113 = t112 * x1;
-  const float t114 = t4 * t113 + 6.0f * t12 * t22 + 3.0f * t15;
-  const float t115 = t114;
-  const float t116 = t22 * x2;
-  const float t117 = t116 * x2;
-  const float t118 = t4 * t117 + t12 * t22 + t12 * t29 + t15;
-  const float t119 = t118;
-  const float t120 = (t24 - tn2 * t19);
-  const float t121 = (t24 - tn2 * t19) + (t115 - tn2 * t26 - tn1 * (t26 + t26 + t26 + t26)) + (t119 - tn2 * t33);
-  const float t122 = 1.0f * (kmu * t120 + klam * t121);
-  sink(0, 3, t122);
-  const float t123 = (t70 - tn2 * t42 - tn1 * (t42 + t42));
-  const float t124 = 1.0f * (kmu * t123);
-  sink(1, 3, t124);
-  const float t125 = (t87 - tn2 * t50);
-  const float t126 = 1.0f * (kmu * t125);
-  sink(2, 3, t126);
-  const float t127 = (t115 - tn2 * t26 - tn1 * (t26 + t26 + t26 + t26));
-  const float t128 = (t24 - tn2 * t19) + (t115 - tn2 * t26 - tn1 * (t26 + t26 + t26 + t26)) + (t119 - tn2 * t33);
-  const float t129 = 1.0f * (kmu * t127 + klam * t128);
-  sink(3, 3, t129);
-  const float t130 = t112 * x2;
-  const float t131 = t4 * t130 + 3.0f * t12 * t57;
-  const float t132 = t131;
-  const float t133 = (t132 - tn2 * t61 - tn1 * (t61 + t61));
-  const float t134 = 1.0f * (kmu * t133);
-  sink(4, 3, t134);
-  const float t135 = (t119 - tn2 * t33);
-  const float t136 = (t24 - tn2 * t19) + (t115 - tn2 * t26 - tn1 * (t26 + t26 + t26 + t26)) + (t119 - tn2 * t33);
-  const float t137 = 1.0f * (kmu * t135 + klam * t136);
-  sink(5, 3, t137);
-  const float t138 = t57 * x2;
-  const float t139 = t138 * x2;
-  const float t140 = t4 * t139 + 3.0f * t12 * t57;
-  const float t141 = t140;
-  const float t142 = (t59);
-  const float t143 = (t59) + (t132 - tn1 * (t61 + t61)) + (t141 - tn1 * (t61 + t61));
-  const float t144 = 2.0f * (kmu * t142 + klam * t143);
-  sink(0, 4, t144);
-  const float t145 = (t87 - tn1 * (t50));
-  const float t146 = 2.0f * (kmu * t145);
-  sink(1, 4, t146);
-  const float t147 = (t74 - tn1 * (t42));
-  const float t148 = 2.0f * (kmu * t147);
-  sink(2, 4, t148);
-  const float t149 = (t132 - tn1 * (t61 + t61));
-  const float t150 = (t59) + (t132 - tn1 * (t61 + t61)) + (t141 - tn1 * (t61 + t61));
-  const float t151 = 2.0f * (kmu * t149 + klam * t150);
-  sink(3, 4, t151);
-  const float t152 = (t119 - tn1 * (t26 + t33));
-  const float t153 = 2.0f * (kmu * t152);
-  sink(4, 4, t153);
-  const float t154 = (t141 - tn1 * (t61 + t61));
-  const float t155 = (t59) + (t132 - tn1 * (t61 + t61)) + (t141 - tn1 * (t61 + t61));
-  const float t156 = 2.0f * (kmu * t154 + klam * t155);
-  sink(5, 4, t156);
-  const float t157 = t29 * x2;
-  const float t158 = t157 * x2;
-  const float t159 = t4 * t158 + 6.0f * t12 * t29 + 3.0f * t15;
-  const float t160 = t159;
-  const float t161 = (t31 - tn2 * t19);
-  const float t162 = (t31 - tn2 * t19) + (t119 - tn2 * t26) + (t160 - tn2 * t33 - tn1 * (t33 + t33 + t33 + t33));
-  const float t163 = 1.0f * (kmu * t161 + klam * t162);
-  sink(0, 5, t163);
-  const float t164 = (t74 - tn2 * t42);
-  const float t165 = 1.0f * (kmu * t164);
-  sink(1, 5, t165);
-  const float t166 = (t96 - tn2 * t50 - tn1 * (t50 + t50));
-  const float t167 = 1.0f * (kmu * t166);
-  sink(2, 5, t167);
-  const float t168 = (t119 - tn2 * t26);
-  const float t169 = (t31 - tn2 * t19) + (t119 - tn2 * t26) + (t160 - tn2 * t33 - tn1 * (t33 + t33 + t33 + t33));
-  const float t170 = 1.0f * (kmu * t168 + klam * t169);
-  sink(3, 5, t170);
-  const float t171 = (t141 - tn2 * t61 - tn1 * (t61 + t61));
-  const float t172 = 1.0f * (kmu * t171);
-  sink(4, 5, t172);
-  const float t173 = (t160 - tn2 * t33 - tn1 * (t33 + t33 + t33 + t33));
-  const float t174 = (t31 - tn2 * t19) + (t119 - tn2 * t26) + (t160 - tn2 * t33 - tn1 * (t33 + t33 + t33 + t33));
-  const float t175 = 1.0f * (kmu * t173 + klam * t174);
-  sink(5, 5, t175);
-}
-
-template <class Sink>
-IBEM_HD IBEM_INLINE void sph_block24f_c0_r1(const float x0, const float x1, const float x2,
-    const float a, const SphMatF& mc, Sink& sink) {
-  const float a2 = a * a; const float a4 = a2 * a2;
-  const float u = 0.5f * (x0 * x0 + x1 * x1 + x2 * x2);
-  const float lam = 2.0f * u - a2;
-  const float ext = lam > 0.0f ? 1.0f : 0.0f;
-  const float rho2 = lam > 0.0f ? a2 + lam : a2;
-  float Jv[6];
-  {
-    // J_m = 4 pi a^3 / ((2m+1) rho^(2m+1)),  rho^2 = a^2 + lambda
-    const float irho2 = 1.0f / rho2;
-    float pw = 4.0f * 3.14159265358979f * a * a2 / sqrtf(rho2);
-    for (int m = 0; m <= 5; ++m) { Jv[m] = pw / (2 * m + 1); pw *= irho2; }
-  }
-  const float kmu = mc.kmu, klam = mc.klam, tn1 = mc.tn1, tn2 = mc.tn2;
-  (void)kmu; (void)klam; (void)tn1; (void)tn2; (void)a4;
-  const float t0 = ext * (-315.0f * Jv[4]);
-  const float t1 = -(t0);
-  const float t2 = ext * (-693.0f * Jv[5]);
-  const float t3 = -(t2);
-  const float t4 = (1.0f) * t1 + (-a2) * t3;
-  const float t5 = x0 * x0;
-  const float t6 = t5 * x0;
-  const float t7 = t6 * x0;
-  const float t8 = t7 * x0;
-  const float t9 = ext * (35.0f * Jv[3]);
-  const float t10 = -(t9);
-  const float t11 = ext * (63.0f * Jv[4]);
-  const float t12 = -(t11);
-  const float t13 = (1.0f) * t10 + (-a2) * t12;
-  const float t14 = ext * (-5.0f * Jv[2]);
-  const float t15 = -(t14);
-  const float t16 = ext * (-7.0f * Jv[3]);
-  const float t17 = -(t16);
-  const float t18 = (1.0f) * t15 + (-a2) * t17;
-  const float t19 = t4 * t8 + 10.0f * t13 * t6 + 15.0f * t18 * x0;
-  const float t20 = t19;
-  const float t21 = t10 * t6 + 3.0f * t15 * x0;
-  const float t22 = t21;
-  const float t23 = t6 * x1;
-  const float t24 = t23 * x1;
-  const float t25 = x0 * x1;
-  const float t26 = t25 * x1;
-  const float t27 = t4 * t24 + t13 * t6 + 3.0f * t13 * t26 + 3.0f * t18 * x0;
-  const float t28 = t27;
-  const float t29 = t10 * t26 + t15 * x0;
-  const float t30 = t29;
-  const float t31 = t6 * x2;
-  const float t32 = t31 * x2;
-  const float t33 = x0 * x2;
-  const float t34 = t33 * x2;
-  const float t35 = t4 * t32 + t13 * t6 + 3.0f * t13 * t34 + 3.0f * t18 * x0;
-  const float t36 = t35;
-  const float t37 = t10 * t34 + t15 * x0;
-  const float t38 = t37;
-  const float t39 = (t20 - tn2 * t22 - tn1 * (t22 + t22 + t22 + t22));
-  const float t40 = (t20 - tn2 * t22 - tn1 * (t22 + t22 + t22 + t22)) + (t28 - tn2 * t30) + (t36 - tn2 * t38);
-  const float t41 = 1.0f * (kmu * t39 + klam * t40);
-  sink(6, 0, t41);
-  const float t42 = t7 * x1;
-  const float t43 = t5 * x1;
-  const float t44 = t4 * t42 + 6.0f * t13 * t43 + 3.0f * t18 * x1;
-  const float t45 = t44;
-  const float t46 = t10 * t43 + t15 * x1;
-  const float t47 = t46;
-  const float t48 = t43 * x1;
-  const float t49 = t48 * x1;
-  const float t50 = x1 * x1;
-  const float t51 = t50 * x1;
-  const float t52 = t4 * t49 + 3.0f * t13 * t43 + t13 * t51 + 3.0f * t18 * x1;
-  const float t53 = t52;
-  const float t54 = t10 * t51 + 3.0f * t15 * x1;
-  const float t55 = t54;
-  const float t56 = t43 * x2;
-  const float t57 = t56 * x2;
-  const float t58 = x1 * x2;
-  const float t59 = t58 * x2;
-  const float t60 = t4 * t57 + t13 * t43 + t13 * t59 + t18 * x1;
-  const float t61 = t60;
-  const float t62 = t10 * t59 + t15 * x1;
-  const float t63 = t62;
-  const float t64 = (t45 - tn2 * t47 - tn1 * (t47 + t47 + t47 + t47));
-  const float t65 = (t45 - tn2 * t47 - tn1 * (t47 + t47 + t47 + t47)) + (t53 - tn2 * t55) + (t61 - tn2 * t63);
-  const float t66 = 1.0f * (kmu * t64 + klam * t65);
-  sink(7, 0, t66);
-  const float t67 = t7 * x2;
-  const float t68 = t5 * x2;
-  const float t69 = t4 * t67 + 6.0f * t13 * t68 + 3.0f * t18 * x2;
-  const float t70 = t69;
-  const float t71 = t10 * t68 + t15 * x2;
-  const float t72 = t71;
-  const float t73 = t48 * x2;
-  const float t74 = t50 * x2;
-  const float t75 = t4 * t73 + t13 * t68 + t13 * t74 + t18 * x2;
-  const float t76 = t75;
-  const float t77 = t10 * t74 + t15 * x2;
-  const float t78 = t77;
-  const float t79 = t68 * x2;
-  const float t80 = t79 * x2;
-  const float t81 = x2 * x2;
-  const float t82 = t81 * x2;
-  const float t83 = t4 * t80 + 3.0f * t13 * t68 + t13 * t82 + 3.0f * t18 * x2;
-  const float t84 = t83;
-  const float t85 = t10 * t82 + 3.0f * t15 * x2;
-  const float t86 = t85;
-  const float t87 = (t70 - tn2 * t72 - tn1 * (t72 + t72 + t72 + t72));
-  const float t88 = (t70 - tn2 * t72 - tn1 * (t72 + t72 + t72 + t72)) + (t76 - tn2 * t78) + (t84 - tn2 * t86);
-  const float t89 = 1.0f * (kmu * t87 + klam * t88);
-  sink(8, 0, t89);
-  const float t90 = (t45 - tn2 * t47 - tn1 * (t47 + t47));
-  const float t91 = 1.0f * (kmu * t90);
-  sink(9, 0, t91);
-  const float t92 = (t28 - tn2 * t30 - tn1 * (t30 + t30));
-  const float t93 = 1.0f * (kmu * t92);
-  sink(10, 0, t93);
-  const float t94 = t23 * x2;
-  const float t95 = t25 * x2;
-  const float t96 = t4 * t94 + 3.0f * t13 * t95;
-  const float t97 = t96;
-  const float t98 = t10 * t95;
-  const float t99 = t98;
-  const float t100 = (t97 - tn2 * t99 - tn1 * (t99 + t99));
-  const float t101 = 1.0f * (kmu * t100);
-  sink(11, 0, t101);
-  const float t102 = (t70 - tn2 * t72 - tn1 * (t72 + t72));
-  const float t103 = 1.0f * (kmu * t102);
-  sink(12, 0, t103);
-  const float t104 = (t97 - tn2 * t99 - tn1 * (t99 + t99));
-  const float t105 = 1.0f * (kmu * t104);
-  sink(13, 0, t105);
-  const float t106 = (t36 - tn2 * t38 - tn1 * (t38 + t38));
-  const float t107 = 1.0f * (kmu * t106);
-  sink(14, 0, t107);
-  const float t108 = (t28 - tn2 * t30);
-  const float t109 = (t20 - tn2 * t22 - tn1 * (t22 + t22 + t22 + t22)) + (t28 - tn2 * t30) + (t36 - tn2 * t38);
-  const float t110 = 1.0f * (kmu * t108 + klam * t109);
-  sink(15, 0, t110);
-  const float t111 = (t53 - tn2 * t55);
-  const float t112 = (t45 - tn2 * t47 - tn1 * (t47 + t47 + t47 + t47)) + (t53 - tn2 * t55) + (t61 - tn2 * t63);
-  const float t113 = 1.0f * (kmu * t111 + klam * t112);
-  sink(16, 0, t113);
-  const float t114 = (t76 - tn2 * t78);
-  const float t115 = (t70 - tn2 * t72 - tn1 * (t72 + t72 + t72 + t72)) + (t76 - tn2 * t78) + (t84 - tn2 * t86);
-  const float t116 = 1.0f * (kmu * t114 + klam * t115);
-  sink(17, 0, t116);
-  const float t117 = (t97 - tn2 * t99);
-  const float t118 = 1.0f * (kmu * t117);
-  sink(18, 0, t118);
-  const float t119 = (t76 - tn2 * t78);
-  const float t120 = 1.0f * (kmu * t119);
-  sink(19, 0, t120);
-  const float t121 = (t61 - tn2 * t63);
-  const float t122 = 1.0f * (kmu * t121);
-  sink(20, 0, t122);
-  const float t123 = (t36 - tn2 * t38);
-  const float t124 = (t20 - tn2 * t22 - tn1 * (t22 + t22 + t22 + t22)) + (t28 - tn2 * t30) + (t36 - tn2 * t38);
-  const float t125 = 1.0f * (kmu * t123 + klam * t124);
-  sink(21, 0, t125);
-  const float t126 = (t61 - tn2 * t63);
-  const float t127 = (t45 - tn2 * t47 - tn1 * (t47 + t47 + t47 + t47)) + (t53 - tn2 * t55) + (t61 - tn2 * t63);
-  const float t128 = 1.0f * (kmu * t126 + klam * t127);
-  sink(22, 0, t128);
-  const float t129 = (t84 - tn2 * t86);
-  const float t130 = (t70 - tn2 * t72 - tn1 * (t72 + t72 + t72 + t72)) + (t76 - tn2 * t78) + (t84 - tn2 * t86);
-  const float t131 = 1.0f * (kmu * t129 + klam * t130);
-  sink(23, 0, t131);
-  const float t132 = (t45 - tn1 * (t47 + t47));
-  const float t133 = (t45 - tn1 * (t47 + t47)) + (t53 - tn1 * (t47 + t47)) + (t61);
-  const float t134 = 2.0f * (kmu * t132 + klam * t133);
-  sink(6, 1, t134);
-  const float t135 = t26 * x1;
-  const float t136 = t135 * x1;
-  const float t137 = t4 * t136 + 6.0f * t13 * t26 + 3.0f * t18 * x0;
-  const float t138 = t137;
-  const float t139 = t26 * x2;
-  const float t140 = t139 * x2;
-  const float t141 = t4 * t140 + t13 * t26 + t13 * t34 + t18 * x0;
-  const float t142 = t141;
-  const float t143 = (t28 - tn1 * (t30 + t30));
-  const float t144 = (t28 - tn1 * (t30 + t30)) + (t138 - tn1 * (t30 + t30)) + (t142);
-  const float t145 = 2.0f * (kmu * t143 + klam * t144);
-  sink(7, 1, t145);
-  const float t146 = t135 * x2;
-  const float t147 = t4 * t146 + 3.0f * t13 * t95;
-  const float t148 = t147;
-  const float t149 = t95 * x2;
-  const float t150 = t149 * x2;
-  const float t151 = t4 * t150 + 3.0f * t13 * t95;
-  const float t152 = t151;
-  const float t153 = (t97 - tn1 * (t99 + t99));
-  const float t154 = (t97 - tn1 * (t99 + t99)) + (t148 - tn1 * (t99 + t99)) + (t152);
-  const float t155 = 2.0f * (kmu * t153 + klam * t154);
-  sink(8, 1, t155);
-  const float t156 = (t28 - tn1 * (t22 + t30));
-  const float t157 = 2.0f * (kmu * t156);
-  sink(9, 1, t157);
-  const float t158 = (t53 - tn1 * (t47 + t55));
-  const float t159 = 2.0f * (kmu * t158);
-  sink(10, 1, t159);
-  const float t160 = (t76 - tn1 * (t72 + t78));
-  const float t161 = 2.0f * (kmu * t160);
-  sink(11, 1, t161);
-  const float t162 = (t97 - tn1 * (t99));
-  const float t163 = 2.0f * (kmu * t162);
-  sink(12, 1, t163);
-  const float t164 = (t76 - tn1 * (t78));
-  const float t165 = 2.0f * (kmu * t164);
-  sink(13, 1, t165);
-  const float t166 = (t61 - tn1 * (t63));
-  const float t167 = 2.0f * (kmu * t166);
-  sink(14, 1, t167);
-  const float t168 = (t53 - tn1 * (t47 + t47));
-  const float t169 = (t45 - tn1 * (t47 + t47)) + (t53 - tn1 * (t47 + t47)) + (t61);
-  const float t170 = 2.0f * (kmu * t168 + klam * t169);
-  sink(15, 1, t170);
-  const float t171 = (t138 - tn1 * (t30 + t30));
-  const float t172 = (t28 - tn1 * (t30 + t30)) + (t138 - tn1 * (t30 + t30)) + (t142);
-  const float t173 = 2.0f * (kmu * t171 + klam * t172);
-  sink(16, 1, t173);
-  const float t174 = (t148 - tn1 * (t99 + t99));
-  const float t175 = (t97 - tn1 * (t99 + t99)) + (t148 - tn1 * (t99 + t99)) + (t152);
-  const float t176 = 2.0f * (kmu * t174 + klam * t175);
-  sink(17, 1, t176);
-  const float t177 = (t76 - tn1 * (t72));
-  const float t178 = 2.0f * (kmu * t177);
-  sink(18, 1, t178);
-  const float t179 = (t148 - tn1 * (t99));
-  const float t180 = 2.0f * (kmu * t179);
-  sink(19, 1, t180);
-  const float t181 = (t142 - tn1 * (t38));
-  const float t182 = 2.0f * (kmu * t181);
-  sink(20, 1, t182);
-  const float t183 = (t61);
-  const float t184 = (t45 - tn1 * (t47 + t47)) + (t53 - tn1 * (t47 + t47)) + (t61);
-  const float t185 = 2.0f * (kmu * t183 + klam * t184);
-  sink(21, 1, t185);
-  const float t186 = (t142);
-  const float t187 = (t28 - tn1 * (t30 + t30)) + (t138 - tn1 * (t30 + t30)) + (t142);
-  const float t188 = 2.0f * (kmu * t186 + klam * t187);
-  sink(22, 1, t188);
-  const float t189 = (t152);
-  const float t190 = (t97 - tn1 * (t99 + t99)) + (t148 - tn1 * (t99 + t99)) + (t152);
-  const float t191 = 2.0f * (kmu * t189 + klam * t190);
-  sink(23, 1, t191);
-  const float t192 = (t70 - tn1 * (t72 + t72));
-  const float t193 = (t70 - tn1 * (t72 + t72)) + (t76) + (t84 - tn1 * (t72 + t72));
-  const float t194 = 2.0f * (kmu * t192 + klam * t193);
-  sink(6, 2, t194);
-  const float t195 = (t97 - tn1 * (t99 + t99));
-  const float t196 = (t97 - tn1 * (t99 + t99)) + (t148) + (t152 - tn1 * (t99 + t99));
-  const float t197 = 2.0f * (kmu * t195 + klam * t196);
-  sink(7, 2, t197);
-  const float t198 = t34 * x2;
-  const float t199 = t198 * x2;
-  const float t200 = t4 * t199 + 6.0f * t13 * t34 + 3.0f * t18 * x0;
-  const float t201 = t200;
-  const float t202 = (t36 - tn1 * (t38 + t38));
-  const float t203 = (t36 - tn1 * (t38 + t38)) + (t142) + (t201 - tn1 * (t38 + t38));
-  const float t204 = 2.0f * (kmu * t202 + klam * t203);
-  sink(8, 2, t204);
-  const float t205 = (t97 - tn1 * (t99));
-  const float t206 = 2.0f * (kmu * t205);
-  sink(9, 2, t206);
-  const float t207 = (t76 - tn1 * (t78));
-  const float t208 = 2.0f * (kmu * t207);
-  sink(10, 2, t208);
-  const float t209 = (t61 - tn1 * (t63));
-  const float t210 = 2.0f * (kmu * t209);
-  sink(11, 2, t210);
-  const float t211 = (t36 - tn1 * (t22 + t38));
-  const float t212 = 2.0f * (kmu * t211);
-  sink(12, 2, t212);
-  const float t213 = (t61 - tn1 * (t47 + t63));
-  const float t214 = 2.0f * (kmu * t213);
-  sink(13, 2, t214);
-  const float t215 = (t84 - tn1 * (t72 + t86));
-  const float t216 = 2.0f * (kmu * t215);
-  sink(14, 2, t216);
-  const float t217 = (t76);
-  const float t218 = (t70 - tn1 * (t72 + t72)) + (t76) + (t84 - tn1 * (t72 + t72));
-  const float t219 = 2.0f * (kmu * t217 + klam * t218);
-  sink(15, 2, t219);
-  const float t220 = (t148);
-  const float t221 = (t97 - tn1 * (t99 + t99)) + (t148) + (t152 - tn1 * (t99 + t99));
-  const float t222 = 2.0f * (kmu * t220 + klam * t221);
-  sink(16, 2, t222);
-  const float t223 = (t142);
-  const float t224 = (t36 - tn1 * (t38 + t38)) + (t142) + (t201 - tn1 * (t38 + t38));
-  const float t225 = 2.0f * (kmu * t223 + klam * t224);
-  sink(17, 2, t225);
-  const float t226 = (t61 - tn1 * (t47));
-  const float t227 = 2.0f * (kmu * t226);
-  sink(18, 2, t227);
-  const float t228 = (t142 - tn1 * (t30));
-  const float t229 = 2.0f * (kmu * t228);
-  sink(19, 2, t229);
-  const float t230 = (t152 - tn1 * (t99));
-  const float t231 = 2.0f * (kmu * t230);
-  sink(20, 2, t231);
-  const float t232 = (t84 - tn1 * (t72 + t72));
-  const float t233 = (t70 - tn1 * (t72 + t72)) + (t76) + (t84 - tn1 * (t72 + t72));
-  const float t234 = 2.0f * (kmu * t232 + klam * t233);
-  sink(21, 2, t234);
-  const float t235 = (t152 - tn1 * (t99 + t99));
-  const float t236 = (t97 - tn1 * (t99 + t99)) + (t148) + (t152 - tn1 * (t99 + t99));
-  const float t237 = 2.0f * (kmu * t235 + klam * t236);
-  sink(22, 2, t237);
-  const float t238 = (t201 - tn1 * (t38 + t38));
-  const float t239 = (t36 - tn1 * (t38 + t38)) + (t142) + (t201 - tn1 * (t38 + t38));
-  const float t240 = 2.0f * (kmu * t238 + klam * t239);
-  sink(23, 2, t240);
-  const float t241 = (t28 - tn2 * t22);
-  const float t242 = (t28 - tn2 * t22) + (t138 - tn2 * t30 - tn1 * (t30 + t30 + t30 + t30)) + (t142 - tn2 * t38);
-  const float t243 = 1.0f * (kmu * t241 + klam * t242);
-  sink(6, 3, t243);
-  const float t244 = t51 * x1;
-  const float t245 = t244 * x1;
-  const float t246 = t4 * t245 + 10.0f * t13 * t51 + 15.0f * t18 * x1;
-  const float t247 = t246;
-  const float t248 = t51 * x2;
-  const float t249 = t248 * x2;
-  const float t250 = t4 * t249 + t13 * t51 + 3.0f * t13 * t59 + 3.0f * t18 * x1;
-  const float t251 = t250;
-  const float t252 = (t53 - tn2 * t47);
-  const float t253 = (t53 - tn2 * t47) + (t247 - tn2 * t55 - tn1 * (t55 + t55 + t55 + t55)) + (t251 - tn2 * t63);
-  const float t254 = 1.0f * (kmu * t252 + klam * t253);
-  sink(7, 3, t254);
-  const float t255 = t244 * x2;
-  const float t256 = t4 * t255 + 6.0f * t13 * t74 + 3.0f * t18 * x2;
-  const float t257 = t256;
-  const float t258 = t74 * x2;
-  const float t259 = t258 * x2;
-  const float t260 = t4 * t259 + 3.0f * t13 * t74 + t13 * t82 + 3.0f * t18 * x2;
-  const float t261 = t260;
-  const float t262 = (t76 - tn2 * t72);
-  const float t263 = (t76 - tn2 * t72) + (t257 - tn2 * t78 - tn1 * (t78 + t78 + t78 + t78)) + (t261 - tn2 * t86);
-  const float t264 = 1.0f * (kmu * t262 + klam * t263);
-  sink(8, 3, t264);
-  const float t265 = (t53 - tn2 * t47 - tn1 * (t47 + t47));
-  const float t266 = 1.0f * (kmu * t265);
-  sink(9, 3, t266);
-  const float t267 = (t138 - tn2 * t30 - tn1 * (t30 + t30));
-  const float t268 = 1.0f * (kmu * t267);
-  sink(10, 3, t268);
-  const float t269 = (t148 - tn2 * t99 - tn1 * (t99 + t99));
-  const float t270 = 1.0f * (kmu * t269);
-  sink(11, 3, t270);
-  const float t271 = (t76 - tn2 * t72);
-  const float t272 = 1.0f * (kmu * t271);
-  sink(12, 3, t272);
-  const float t273 = (t148 - tn2 * t99);
-  const float t274 = 1.0f * (kmu * t273);
-  sink(13, 3, t274);
-  const float t275 = (t142 - tn2 * t38);
-  const float t276 = 1.0f * (kmu * t275);
-  sink(14, 3, t276);
-  const float t277 = (t138 - tn2 * t30 - tn1 * (t30 + t30 + t30 + t30));
-  const float t278 = (t28 - tn2 * t22) + (t138 - tn2 * t30 - tn1 * (t30 + t30 + t30 + t30)) + (t142 - tn2 * t38);
-  const float t279 = 1.0f * (kmu * t277 + klam * t278);
-  sink(15, 3, t279);
-  const float t280 = (t247 - tn2 * t55 - tn1 * (t55 + t55 + t55 + t55));
-  const float t281 = (t53 - tn2 * t47) + (t247 - tn2 * t55 - tn1 * (t55 + t55 + t55 + t55)) + (t251 - tn2 * t63);
-  const float t282 = 1.0f * (kmu * t280 + klam * t281);
-  sink(16, 3, t282);
-  const float t283 = (t257 - tn2 * t78 - tn1 * (t78 + t78 + t78 + t78));
-  const float t284 = (t76 - tn2 * t72) + (t257 - tn2 * t78 - tn1 * (t78 + t78 + t78 + t78)) + (t261 - tn2 * t86);
-  const float t285 = 1.0f * (kmu * t283 + klam * t284);
-  sink(17, 3, t285);
-  const float t286 = (t148 - tn2 * t99 - tn1 * (t99 + t99));
-  const float t287 = 1.0f * (kmu * t286);
-  sink(18, 3, t287);
-  const float t288 = (t257 - tn2 * t78 - tn1 * (t78 + t78));
-  const float t289 = 1.0f * (kmu * t288);
-  sink(19, 3, t289);
-  const float t290 = (t251 - tn2 * t63 - tn1 * (t63 + t63));
-  const float t291 = 1.0f * (kmu * t290);
-  sink(20, 3, t291);
-  const float t292 = (t142 - tn2 * t38);
-  const float t293 = (t28 - tn2 * t22) + (t138 - tn2 * t30 - tn1 * (t30 + t30 + t30 + t30)) + (t142 - tn2 * t38);
-  const float t294 = 1.0f * (kmu * t292 + klam * t293);
-  sink(21, 3, t294);
-  const float t295 = (t251 - tn2 * t63);
-  const float t296 = (t53 - tn2 * t47) + (t247 - tn2 * t55 - tn1 * (t55 + t55 + t55 + t55)) + (t251 - tn2 * t63);
-  const float t297 = 1.0f * (kmu * t295 + klam * t296);
-  sink(22, 3, t297);
-  const float t298 = (t261 - tn2 * t86);
-  const float t299 = (t76 - tn2 * t72) + (t257 - tn2 * t78 - tn1 * (t78 + t78 + t78 + t78)) + (t261 - tn2 * t86);
-  const float t300 = 1.0f * (kmu * t298 + klam * t299);
-  sink(23, 3, t300);
-  const float t301 = (t97);
-  const float t302 = (t97) + (t148 - tn1 * (t99 + t99)) + (t152 - tn1 * (t99 + t99));
-  const float t303 = 2.0f * (kmu * t301 + klam * t302);
-  sink(6, 4, t303);
-  const float t304 = (t76);
-  const float t305 = (t76) + (t257 - tn1 * (t78 + t78)) + (t261 - tn1 * (t78 + t78));
-  const float t306 = 2.0f * (kmu * t304 + klam * t305);
-  sink(7, 4, t306);
-  const float t307 = t59 * x2;
-  const float t308 = t307 * x2;
-  const float t309 = t4 * t308 + 6.0f * t13 * t59 + 3.0f * t18 * x1;
-  const float t310 = t309;
-  const float t311 = (t61);
-  const float t312 = (t61) + (t251 - tn1 * (t63 + t63)) + (t310 - tn1 * (t63 + t63));
-  const float t313 = 2.0f * (kmu * t311 + klam * t312);
-  sink(8, 4, t313);
-  const float t314 = (t76 - tn1 * (t72));
-  const float t315 = 2.0f * (kmu * t314);
-  sink(9, 4, t315);
-  const float t316 = (t148 - tn1 * (t99));
-  const float t317 = 2.0f * (kmu * t316);
-  sink(10, 4, t317);
-  const float t318 = (t142 - tn1 * (t38));
-  const float t319 = 2.0f * (kmu * t318);
-  sink(11, 4, t319);
-  const float t320 = (t61 - tn1 * (t47));
-  const float t321 = 2.0f * (kmu * t320);
-  sink(12, 4, t321);
-  const float t322 = (t142 - tn1 * (t30));
-  const float t323 = 2.0f * (kmu * t322);
-  sink(13, 4, t323);
-  const float t324 = (t152 - tn1 * (t99));
-  const float t325 = 2.0f * (kmu * t324);
-  sink(14, 4, t325);
-  const float t326 = (t148 - tn1 * (t99 + t99));
-  const float t327 = (t97) + (t148 - tn1 * (t99 + t99)) + (t152 - tn1 * (t99 + t99));
-  const float t328 = 2.0f * (kmu * t326 + klam * t327);
-  sink(15, 4, t328);
-  const float t329 = (t257 - tn1 * (t78 + t78));
-  const float t330 = (t76) + (t257 - tn1 * (t78 + t78)) + (t261 - tn1 * (t78 + t78));
-  const float t331 = 2.0f * (kmu * t329 + klam * t330);
-  sink(16, 4, t331);
-  const float t332 = (t251 - tn1 * (t63 + t63));
-  const float t333 = (t61) + (t251 - tn1 * (t63 + t63)) + (t310 - tn1 * (t63 + t63));
-  const float t334 = 2.0f * (kmu * t332 + klam * t333);
-  sink(17, 4, t334);
-  const float t335 = (t142 - tn1 * (t30 + t38));
-  const float t336 = 2.0f * (kmu * t335);
-  sink(18, 4, t336);
-  const float t337 = (t251 - tn1 * (t55 + t63));
-  const float t338 = 2.0f * (kmu * t337);
-  sink(19, 4, t338);
-  const float t339 = (t261 - tn1 * (t78 + t86));
-  const float t340 = 2.0f * (kmu * t339);
-  sink(20, 4, t340);
-  const float t341 = (t152 - tn1 * (t99 + t99));
-  const float t342 = (t97) + (t148 - tn1 * (t99 + t99)) + (t152 - tn1 * (t99 + t99));
-  const float t343 = 2.0f * (kmu * t341 + klam * t342);
-  sink(21, 4, t343);
-  const float t344 = (t261 - tn1 * (t78 + t78));
-  const float t345 = (t76) + (t257 - tn1 * (t78 + t78)) + (t261 - tn1 * (t78 + t78));
-  const float t346 = 2.0f * (kmu * t344 + klam * t345);
-  sink(22, 4, t346);
-  const float t347 = (t310 - tn1 * (t63 + t63));
-  const float t348 = (t61) + (t251 - tn1 * (t63 + t63)) + (t310 - tn1 * (t63 + t63));
-  const float t349 = 2.0f * (kmu * t347 + klam * t348);
-  sink(23, 4, t349);
-  const float t350 = (t36 - tn2 * t22);
-  const float t351 = (t36 - tn2 * t22) + (t142 - tn2 * t30) + (t201 - tn2 * t38 - tn1 * (t38 + t38 + t38 + t38));
-  const float t352 = 1.0f * (kmu * t350 + klam * t351);
-  sink(6, 5, t352);
-  const float t353 = (t61 - tn2 * t47);
-  const float t354 = (t61 - tn2 * t47) + (t251 - tn2 * t55) + (t310 - tn2 * t63 - tn1 * (t63 + t63 + t63 + t63));
-  const float t355 = 1.0f * (kmu * t353 + klam * t354);
-  sink(7, 5, t355);
-  const float t356 = t82 * x2;
-  const float t357 = t356 * x2;
-  const float t358 = t4 * t357 + 10.0f * t13 * t82 + 15.0f * t18 * x2;
-  const float t359 = t358;
-  const float t360 = (t84 - tn2 * t72);
-  const float t361 = (t84 - tn2 * t72) + (t261 - tn2 * t78) + (t359 - tn2 * t86 - tn1 * (t86 + t86 + t86 + t86));
-  const float t362 = 1.0f * (kmu * t360 + klam * t361);
-  sink(8, 5, t362);
-  const float t363 = (t61 - tn2 * t47);
-  const float t364 = 1.0f * (kmu * t363);
-  sink(9, 5, t364);
-  const float t365 = (t142 - tn2 * t30);
-  const float t366 = 1.0f * (kmu * t365);
-  sink(10, 5, t366);
-  const float t367 = (t152 - tn2 * t99);
-  const float t368 = 1.0f * (kmu * t367);
-  sink(11, 5, t368);
-  const float t369 = (t84 - tn2 * t72 - tn1 * (t72 + t72));
-  const float t370 = 1.0f * (kmu * t369);
-  sink(12, 5, t370);
-  const float t371 = (t152 - tn2 * t99 - tn1 * (t99 + t99));
-  const float t372 = 1.0f * (kmu * t371);
-  sink(13, 5, t372);
-  const float t373 = (t201 - tn2 * t38 - tn1 * (t38 + t38));
-  const float t374 = 1.0f * (kmu * t373);
-  sink(14, 5, t374);
-  const float t375 = (t142 - tn2 * t30);
-  const float t376 = (t36 - tn2 * t22) + (t142 - tn2 * t30) + (t201 - tn2 * t38 - tn1 * (t38 + t38 + t38 + t38));
-  const float t377 = 1.0f * (kmu * t375 + klam * t376);
-  sink(15, 5, t377);
-  const float t378 = (t251 - tn2 * t55);
-  const float t379 = (t61 - tn2 * t47) + (t251 - tn2 * t55) + (t310 - tn2 * t63 - tn1 * (t63 + t63 + t63 + t63));
-  const float t380 = 1.0f * (kmu * t378 + klam * t379);
-  sink(16, 5, t380);
-  const float t381 = (t261 - tn2 * t78);
-  const float t382 = (t84 - tn2 * t72) + (t261 - tn2 * t78) + (t359 - tn2 * t86 - tn1 * (t86 + t86 + t86 + t86));
-  const float t383 = 1.0f * (kmu * t381 + klam * t382);
-  sink(17, 5, t383);
-  const float t384 = (t152 - tn2 * t99 - tn1 * (t99 + t99));
-  const float t385 = 1.0f * (kmu * t384);
-  sink(18, 5, t385);
-  const float t386 = (t261 - tn2 * t78 - tn1 * (t78 + t78));
-  const float t387 = 1.0f * (kmu * t386);
-  sink(19, 5, t387);
-  const float t388 = (t310 - tn2 * t63 - tn1 * (t63 + t63));
-  const float t389 = 1.0f * (kmu * t388);
-  sink(20, 5, t389);
-  const float t390 = (t201 - tn2 * t38 - tn1 * (t38 + t38 + t38 + t38));
-  const float t391 = (t36 - tn2 * t22) + (t142 - tn2 * t30) + (t201 - tn2 * t38 - tn1 * (t38 + t38 + t38 + t38));
-  const float t392 = 1.0f * (kmu * t390 + klam * t391);
-  sink(21, 5, t392);
-  const float t393 = (t310 - tn2 * t63 - tn1 * (t63 + t63 + t63 + t63));
-  const float t394 = (t61 - tn2 * t47) + (t251 - tn2 * t55) + (t310 - tn2 * t63 - tn1 * (t63 + t63 + t63 + t63));
-  const float t395 = 1.0f * (kmu * t393 + klam * t394);
-  sink(22, 5, t395);
-  const float t396 = (t359 - tn2 * t86 - tn1 * (t86 + t86 + t86 + t86));
-  const float t397 = (t84 - tn2 * t72) + (t261 - tn2 * t78) + (t359 - tn2 * t86 - tn1 * (t86 + t86 + t86 + t86));
-  const float t398 = 1.0f * (kmu * t396 + klam * t397);
-  sink(23, 5, t398);
-}
-
-template <class Sink>
-IBEM_HD IBEM_INLINE void sph_block24f_c1_r0(const float x0, const float x1, const float x2,
-    const float a, const SphMatF& mc, Sink& sink) {
-  const float a2 = a * a; const float a4 = a2 * a2;
-  const float u = 0.5f * (x0 * x0 + x1 * x1 + x2 * x2);
-  const float lam = 2.0f * u - a2;
-  const float ext = lam > 0.0f ? 1.0f : 0.0f;
-  const float rho2 = lam > 0.0f ? a2 + lam : a2;
-  float Jv[6];
-  {
-    // J_m = 4 pi a^3 / ((2m+1) rho^(2m+1)),  rho^2 = a^2 + lambda
-    const float irho2 = 1.0f / rho2;
-    float pw = 4.0f * 3.14159265358979f * a * a2 / sqrtf(rho2);
-    for (int m = 0; m <= 5; ++m) { Jv[m] = pw / (2 * m + 1); pw *= irho2; }
-  }
-  const float kmu = mc.kmu, klam = mc.klam, tn1 = mc.tn1, tn2 = mc.tn2;
-  (void)kmu; (void)klam; (void)tn1; (void)tn2; (void)a4;
-  const float t0 = ext * (63.0f * Jv[4]);
-  const float t1 = -(t0);
-  const float t2 = ext * (99.0f * Jv[5]);
-  const float t3 = -(t2);
-  const float t4 = (1.0f) * t1 + (-a2) * t3;
-  const float t5 = x0 * x0;
-  const float t6 = t5 * x0;
-  const float t7 = t6 * x0;
-  const float t8 = ext * (-7.0f * Jv[3]);
-  const float t9 = -(t8);
-  const float t10 = ext * (-9.0f * Jv[4]);
-  const float t11 = -(t10);
-  const float t12 = (1.0f) * t9 + (-a2) * t11;
-  const float t13 = -(Jv[2]);
-  const float t14 = -(Jv[3]);
-  const float t15 = (1.0f) * t13 + (-a2) * t14;
-  const float t16 = t4 * t7 + 6.0f * t12 * t5 + 3.0f * t15;
-  const float t17 = t12 * t6 + 3.0f * t15 * x0;
-  const float t18 = x0 * t16 + 4.0f * t17;
-  const float t19 = a2 * t18;
-  const float t20 = t9 * t5 + t13;
-  const float t21 = t13 * x0;
-  const float t22 = x0 * t20 + 2.0f * t21;
-  const float t23 = a2 * t22;
-  const float t24 = t5 * x1;
-  const float t25 = t24 * x1;
-  const float t26 = x1 * x1;
-  const float t27 = t4 * t25 + t12 * t5 + t12 * t26 + t15;
-  const float t28 = x0 * x1;
-  const float t29 = t28 * x1;
-  const float t30 = t12 * t29 + t15 * x0;
-  const float t31 = x0 * t27 + 2.0f * t30;
-  const float t32 = a2 * t31;
-  const float t33 = t9 * t26 + t13;
-  const float t34 = x0 * t33;
-  const float t35 = a2 * t34;
-  const float t36 = t5 * x2;
-  const float t37 = t36 * x2;
-  const float t38 = x2 * x2;
-  const float t39 = t4 * t37 + t12 * t5 + t12 * t38 + t15;
-  const float t40 = x0 * x2;
-  const float t41 = t40 * x2;
-  const float t42 = t12 * t41 + t15 * x0;
-  const float t43 = x0 * t39 + 2.0f * t42;
-  const float t44 = a2 * t43;
-  const float t45 = t9 * t38 + t13;
-  const float t46 = x0 * t45;
-  const float t47 = a2 * t46;
-  const float t48 = (t19 - tn2 * t23 - tn1 * (t23 + t23 + t23 + t23));
-  const float t49 = (t19 - tn2 * t23 - tn1 * (t23 + t23 + t23 + t23)) + (t32 - tn2 * t35) + (t44 - tn2 * t47);
-  const float t50 = 1.0f * (kmu * t48 + klam * t49);
-  sink(0, 6, t50);
-  const float t51 = t6 * x1;
-  const float t52 = t4 * t51 + 3.0f * t12 * t28;
-  const float t53 = t12 * t24 + t15 * x1;
-  const float t54 = x0 * t52 + 3.0f * t53;
-  const float t55 = a2 * t54;
-  const float t56 = t9 * t28;
-  const float t57 = t13 * x1;
-  const float t58 = x0 * t56 + t57;
-  const float t59 = a2 * t58;
-  const float t60 = (t55 - tn2 * t59 - tn1 * (t59 + t59));
-  const float t61 = 1.0f * (kmu * t60);
-  sink(1, 6, t61);
-  const float t62 = t6 * x2;
-  const float t63 = t4 * t62 + 3.0f * t12 * t40;
-  const float t64 = t12 * t36 + t15 * x2;
-  const float t65 = x0 * t63 + 3.0f * t64;
-  const float t66 = a2 * t65;
-  const float t67 = t9 * t40;
-  const float t68 = t13 * x2;
-  const float t69 = x0 * t67 + t68;
-  const float t70 = a2 * t69;
-  const float t71 = (t66 - tn2 * t70 - tn1 * (t70 + t70));
-  const float t72 = 1.0f * (kmu * t71);
-  sink(2, 6, t72);
-  const float t73 = (t32 - tn2 * t35);
-  const float t74 = (t19 - tn2 * t23 - tn1 * (t23 + t23 + t23 + t23)) + (t32 - tn2 * t35) + (t44 - tn2 * t47);
-  const float t75 = 1.0f * (kmu * t73 + klam * t74);
-  sink(3, 6, t75);
-  const float t76 = t24 * x2;
-  const float t77 = x1 * x2;
-  const float t78 = t4 * t76 + t12 * t77;
-  const float t79 = t28 * x2;
-  const float t80 = t12 * t79;
-  const float t81 = x0 * t78 + 2.0f * t80;
-  const float t82 = a2 * t81;
-  const float t83 = t9 * t77;
-  const float t84 = x0 * t83;
-  const float t85 = a2 * t84;
-  const float t86 = (t82 - tn2 * t85);
-  const float t87 = 1.0f * (kmu * t86);
-  sink(4, 6, t87);
-  const float t88 = (t44 - tn2 * t47);
-  const float t89 = (t19 - tn2 * t23 - tn1 * (t23 + t23 + t23 + t23)) + (t32 - tn2 * t35) + (t44 - tn2 * t47);
-  const float t90 = 1.0f * (kmu * t88 + klam * t89);
-  sink(5, 6, t90);
-  const float t91 = x1 * t16;
-  const float t92 = a2 * t91;
-  const float t93 = x1 * t20;
-  const float t94 = a2 * t93;
-  const float t95 = x1 * t27 + 2.0f * t53;
-  const float t96 = a2 * t95;
-  const float t97 = x1 * t33 + 2.0f * t57;
-  const float t98 = a2 * t97;
-  const float t99 = x1 * t39;
-  const float t100 = a2 * t99;
-  const float t101 = x1 * t45;
-  const float t102 = a2 * t101;
-  const float t103 = (t92 - tn2 * t94 - tn1 * (t94 + t94 + t94 + t94));
-  const float t104 = (t92 - tn2 * t94 - tn1 * (t94 + t94 + t94 + t94)) + (t96 - tn2 * t98) + (t100 - tn2 * t102);
-  const float t105 = 1.0f * (kmu * t103 + klam * t104);
-  sink(0, 7, t105);
-  const float t106 = x1 * t52 + t17;
-  const float t107 = a2 * t106;
-  const float t108 = x1 * t56 + t21;
-  const float t109 = a2 * t108;
-  const float t110 = (t107 - tn2 * t109 - tn1 * (t109 + t109));
-  const float t111 = 1.0f * (kmu * t110);
-  sink(1, 7, t111);
-  const float t112 = x1 * t63;
-  const float t113 = a2 * t112;
-  const float t114 = x1 * t67;
-  const float t115 = a2 * t114;
-  const float t116 = (t113 - tn2 * t115 - tn1 * (t115 + t115));
-  const float t117 = 1.0f * (kmu * t116);
-  sink(2, 7, t117);
-  const float t118 = (t96 - tn2 * t98);
-  const float t119 = (t92 - tn2 * t94 - tn1 * (t94 + t94 + t94 + t94)) + (t96 - tn2 * t98) + (t100 - tn2 * t102);
-  const float t120 = 1.0f * (kmu * t118 + klam * t119);
-  sink(3, 7, t120);
-  const float t121 = x1 * t78 + t64;
-  const float t122 = a2 * t121;
-  const float t123 = x1 * t83 + t68;
-  const float t124 = a2 * t123;
-  const float t125 = (t122 - tn2 * t124);
-  const float t126 = 1.0f * (kmu * t125);
-  sink(4, 7, t126);
-  const float t127 = (t100 - tn2 * t102);
-  const float t128 = (t92 - tn2 * t94 - tn1 * (t94 + t94 + t94 + t94)) + (t96 - tn2 * t98) + (t100 - tn2 * t102);
-  const float t129 = 1.0f * (kmu * t127 + klam * t128);
-  sink(5, 7, t129);
-  const float t130 = x2 * t16;
-  const float t131 = a2 * t130;
-  const float t132 = x2 * t20;
-  const float t133 = a2 * t132;
-  const float t134 = x2 * t27;
-  const float t135 = a2 * t134;
-  const float t136 = x2 * t33;
-  const float t137 = a2 * t136;
-  const float t138 = x2 * t39 + 2.0f * t64;
-  const float t139 = a2 * t138;
-  const float t140 = x2 * t45 + 2.0f * t68;
-  const float t141 = a2 * t140;
-  const float t142 = (t131 - tn2 * t133 - tn1 * (t133 + t133 + t133 + t133));
-  const float t143 = (t131 - tn2 * t133 - tn1 * (t133 + t133 + t133 + t133)) + (t135 - tn2 * t137) + (t139 - tn2 * t141);
-  const float t144 = 1.0f * (kmu * t142 + klam * t143);
-  sink(0, 8, t144);
-  const float t145 = x2 * t52;
-  const float t146 = a2 * t145;
-  const float t147 = x2 * t56;
-  const float t148 = a2 * t147;
-  const float t149 = (t146 - tn2 * t148 - tn1 * (t148 + t148));
-  const float t150 = 1.0f * (kmu * t149);
-  sink(1, 8, t150);
-  const float t151 = x2 * t63 + t17;
-  const float t152 = a2 * t151;
-  const float t153 = x2 * t67 + t21;
-  const float t154 = a2 * t153;
-  const float t155 = (t152 - tn2 * t154 - tn1 * (t154 + t154));
-  const float t156 = 1.0f * (kmu * t155);
-  sink(2, 8, t156);
-  const float t157 = (t135 - tn2 * t137);
-  const float t158 = (t131 - tn2 * t133 - tn1 * (t133 + t133 + t133 + t133)) + (t135 - tn2 * t137) + (t139 - tn2 * t141);
-  const float t159 = 1.0f * (kmu * t157 + klam * t158);
-  sink(3, 8, t159);
-  const float t160 = x2 * t78 + t53;
-  const float t161 = a2 * t160;
-  const float t162 = x2 * t83 + t57;
-  const float t163 = a2 * t162;
-  const float t164 = (t161 - tn2 * t163);
-  const float t165 = 1.0f * (kmu * t164);
-  sink(4, 8, t165);
-  const float t166 = (t139 - tn2 * t141);
-  const float t167 = (t131 - tn2 * t133 - tn1 * (t133 + t133 + t133 + t133)) + (t135 - tn2 * t137) + (t139 - tn2 * t141);
-  const float t168 = 1.0f * (kmu * t166 + klam * t167);
-  sink(5, 8, t168);
-  const float t169 = t29 * x1;
-  const float t170 = t4 * t169 + 3.0f * t12 * t28;
-  const float t171 = t26 * x1;
-  const float t172 = t12 * t171 + 3.0f * t15 * x1;
-  const float t173 = x0 * t170 + t172;
-  const float t174 = a2 * t173;
-  const float t175 = t79 * x2;
-  const float t176 = t4 * t175 + t12 * t28;
-  const float t177 = t77 * x2;
-  const float t178 = t12 * t177 + t15 * x1;
-  const float t179 = x0 * t176 + t178;
-  const float t180 = a2 * t179;
-  const float t181 = (t55 - tn1 * (t59 + t59));
-  const float t182 = (t55 - tn1 * (t59 + t59)) + (t174 - tn1 * (t59 + t59)) + (t180);
-  const float t183 = 2.0f * (kmu * t181 + klam * t182);
-  sink(0, 9, t183);
-  const float t184 = (t32 - tn1 * (t23 + t35));
-  const float t185 = 2.0f * (kmu * t184);
-  sink(1, 9, t185);
-  const float t186 = (t82 - tn1 * (t85));
-  const float t187 = 2.0f * (kmu * t186);
-  sink(2, 9, t187);
-  const float t188 = (t174 - tn1 * (t59 + t59));
-  const float t189 = (t55 - tn1 * (t59 + t59)) + (t174 - tn1 * (t59 + t59)) + (t180);
-  const float t190 = 2.0f * (kmu * t188 + klam * t189);
-  sink(3, 9, t190);
-  const float t191 = t29 * x2;
-  const float t192 = t4 * t191 + t12 * t40;
-  const float t193 = t26 * x2;
-  const float t194 = t12 * t193 + t15 * x2;
-  const float t195 = x0 * t192 + t194;
-  const float t196 = a2 * t195;
-  const float t197 = (t196 - tn1 * (t70));
-  const float t198 = 2.0f * (kmu * t197);
-  sink(4, 9, t198);
-  const float t199 = (t180);
-  const float t200 = (t55 - tn1 * (t59 + t59)) + (t174 - tn1 * (t59 + t59)) + (t180);
-  const float t201 = 2.0f * (kmu * t199 + klam * t200);
-  sink(5, 9, t201);
-  const float t202 = x1 * t170 + 3.0f * t30;
-  const float t203 = a2 * t202;
-  const float t204 = x1 * t176 + t42;
-  const float t205 = a2 * t204;
-  const float t206 = (t107 - tn1 * (t109 + t109));
-  const float t207 = (t107 - tn1 * (t109 + t109)) + (t203 - tn1 * (t109 + t109)) + (t205);
-  const float t208 = 2.0f * (kmu * t206 + klam * t207);
-  sink(0, 10, t208);
-  const float t209 = (t96 - tn1 * (t94 + t98));
-  const float t210 = 2.0f * (kmu * t209);
-  sink(1, 10, t210);
-  const float t211 = (t122 - tn1 * (t124));
-  const float t212 = 2.0f * (kmu * t211);
-  sink(2, 10, t212);
-  const float t213 = (t203 - tn1 * (t109 + t109));
-  const float t214 = (t107 - tn1 * (t109 + t109)) + (t203 - tn1 * (t109 + t109)) + (t205);
-  const float t215 = 2.0f * (kmu * t213 + klam * t214);
-  sink(3, 10, t215);
-  const float t216 = x1 * t192 + 2.0f * t80;
-  const float t217 = a2 * t216;
-  const float t218 = (t217 - tn1 * (t115));
-  const float t219 = 2.0f * (kmu * t218);
-  sink(4, 10, t219);
-  const float t220 = (t205);
-  const float t221 = (t107 - tn1 * (t109 + t109)) + (t203 - tn1 * (t109 + t109)) + (t205);
-  const float t222 = 2.0f * (kmu * t220 + klam * t221);
-  sink(5, 10, t222);
-  const float t223 = x2 * t170;
-  const float t224 = a2 * t223;
-  const float t225 = x2 * t176 + 2.0f * t80;
-  const float t226 = a2 * t225;
-  const float t227 = (t146 - tn1 * (t148 + t148));
-  const float t228 = (t146 - tn1 * (t148 + t148)) + (t224 - tn1 * (t148 + t148)) + (t226);
-  const float t229 = 2.0f * (kmu * t227 + klam * t228);
-  sink(0, 11, t229);
-  const float t230 = (t135 - tn1 * (t133 + t137));
-  const float t231 = 2.0f * (kmu * t230);
-  sink(1, 11, t231);
-  const float t232 = (t161 - tn1 * (t163));
-  const float t233 = 2.0f * (kmu * t232);
-  sink(2, 11, t233);
-  const float t234 = (t224 - tn1 * (t148 + t148));
-  const float t235 = (t146 - tn1 * (t148 + t148)) + (t224 - tn1 * (t148 + t148)) + (t226);
-  const float t236 = 2.0f * (kmu * t234 + klam * t235);
-  sink(3, 11, t236);
-  const float t237 = x2 * t192 + t30;
-  const float t238 = a2 * t237;
-  const float t239 = (t238 - tn1 * (t154));
-  const float t240 = 2.0f * (kmu * t239);
-  sink(4, 11, t240);
-  const float t241 = (t226);
-  const float t242 = (t146 - tn1 * (t148 + t148)) + (t224 - tn1 * (t148 + t148)) + (t226);
-  const float t243 = 2.0f * (kmu * t241 + klam * t242);
-  sink(5, 11, t243);
-  const float t244 = t41 * x2;
-  const float t245 = t4 * t244 + 3.0f * t12 * t40;
-  const float t246 = t38 * x2;
-  const float t247 = t12 * t246 + 3.0f * t15 * x2;
-  const float t248 = x0 * t245 + t247;
-  const float t249 = a2 * t248;
-  const float t250 = (t66 - tn1 * (t70 + t70));
-  const float t251 = (t66 - tn1 * (t70 + t70)) + (t196) + (t249 - tn1 * (t70 + t70));
-  const float t252 = 2.0f * (kmu * t250 + klam * t251);
-  sink(0, 12, t252);
-  const float t253 = (t82 - tn1 * (t85));
-  const float t254 = 2.0f * (kmu * t253);
-  sink(1, 12, t254);
-  const float t255 = (t44 - tn1 * (t23 + t47));
-  const float t256 = 2.0f * (kmu * t255);
-  sink(2, 12, t256);
-  const float t257 = (t196);
-  const float t258 = (t66 - tn1 * (t70 + t70)) + (t196) + (t249 - tn1 * (t70 + t70));
-  const float t259 = 2.0f * (kmu * t257 + klam * t258);
-  sink(3, 12, t259);
-  const float t260 = (t180 - tn1 * (t59));
-  const float t261 = 2.0f * (kmu * t260);
-  sink(4, 12, t261);
-  const float t262 = (t249 - tn1 * (t70 + t70));
-  const float t263 = (t66 - tn1 * (t70 + t70)) + (t196) + (t249 - tn1 * (t70 + t70));
-  const float t264 = 2.0f * (kmu * t262 + klam * t263);
-  sink(5, 12, t264);
-  const float t265 = x1 * t245;
-  const float t266 = a2 * t265;
-  const float t267 = (t113 - tn1 * (t115 + t115));
-  const float t268 = (t113 - tn1 * (t115 + t115)) + (t217) + (t266 - tn1 * (t115 + t115));
-  const float t269 = 2.0f * (kmu * t267 + klam * t268);
-  sink(0, 13, t269);
-  const float t270 = (t122 - tn1 * (t124));
-  const float t271 = 2.0f * (kmu * t270);
-  sink(1, 13, t271);
-  const float t272 = (t100 - tn1 * (t94 + t102));
-  const float t273 = 2.0f * (kmu * t272);
-  sink(2, 13, t273);
-  const float t274 = (t217);
-  const float t275 = (t113 - tn1 * (t115 + t115)) + (t217) + (t266 - tn1 * (t115 + t115));
-  const float t276 = 2.0f * (kmu * t274 + klam * t275);
-  sink(3, 13, t276);
-  const float t277 = (t205 - tn1 * (t109));
-  const float t278 = 2.0f * (kmu * t277);
-  sink(4, 13, t278);
-  const float t279 = (t266 - tn1 * (t115 + t115));
-  const float t280 = (t113 - tn1 * (t115 + t115)) + (t217) + (t266 - tn1 * (t115 + t115));
-  const float t281 = 2.0f * (kmu * t279 + klam * t280);
-  sink(5, 13, t281);
-  const float t282 = x2 * t245 + 3.0f * t42;
-  const float t283 = a2 * t282;
-  const float t284 = (t152 - tn1 * (t154 + t154));
-  const float t285 = (t152 - tn1 * (t154 + t154)) + (t238) + (t283 - tn1 * (t154 + t154));
-  const float t286 = 2.0f * (kmu * t284 + klam * t285);
-  sink(0, 14, t286);
-  const float t287 = (t161 - tn1 * (t163));
-  const float t288 = 2.0f * (kmu * t287);
-  sink(1, 14, t288);
-  const float t289 = (t139 - tn1 * (t133 + t141));
-  const float t290 = 2.0f * (kmu * t289);
-  sink(2, 14, t290);
-  const float t291 = (t238);
-  const float t292 = (t152 - tn1 * (t154 + t154)) + (t238) + (t283 - tn1 * (t154 + t154));
-  const float t293 = 2.0f * (kmu * t291 + klam * t292);
-  sink(3, 14, t293);
-  const float t294 = (t226 - tn1 * (t148));
-  const float t295 = 2.0f * (kmu * t294);
-  sink(4, 14, t295);
-  const float t296 = (t283 - tn1 * (t154 + t154));
-  const float t297 = (t152 - tn1 * (t154 + t154)) + (t238) + (t283 - tn1 * (t154 + t154));
-  const float t298 = 2.0f * (kmu * t296 + klam * t297);
-  sink(5, 14, t298);
-  const float t299 = t171 * x1;
-  const float t300 = t4 * t299 + 6.0f * t12 * t26 + 3.0f * t15;
-  const float t301 = x0 * t300;
-  const float t302 = a2 * t301;
-  const float t303 = t193 * x2;
-  const float t304 = t4 * t303 + t12 * t26 + t12 * t38 + t15;
-  const float t305 = x0 * t304;
-  const float t306 = a2 * t305;
-  const float t307 = (t32 - tn2 * t23);
-  const float t308 = (t32 - tn2 * t23) + (t302 - tn2 * t35 - tn1 * (t35 + t35 + t35 + t35)) + (t306 - tn2 * t47);
-  const float t309 = 1.0f * (kmu * t307 + klam * t308);
-  sink(0, 15, t309);
-  const float t310 = (t174 - tn2 * t59 - tn1 * (t59 + t59));
-  const float t311 = 1.0f * (kmu * t310);
-  sink(1, 15, t311);
-  const float t312 = (t196 - tn2 * t70);
-  const float t313 = 1.0f * (kmu * t312);
-  sink(2, 15, t313);
-  const float t314 = (t302 - tn2 * t35 - tn1 * (t35 + t35 + t35 + t35));
-  const float t315 = (t32 - tn2 * t23) + (t302 - tn2 * t35 - tn1 * (t35 + t35 + t35 + t35)) + (t306 - tn2 * t47);
-  const float t316 = 1.0f * (kmu * t314 + klam * t315);
-  sink(3, 15, t316);
-  const float t317 = t171 * x2;
-  const float t318 = t4 * t317 + 3.0f * t12 * t77;
-  const float t319 = x0 * t318;
-  const float t320 = a2 * t319;
-  const float t321 = (t320 - tn2 * t85 - tn1 * (t85 + t85));
-  const float t322 = 1.0f * (kmu * t321);
-  sink(4, 15, t322);
-  const float t323 = (t306 - tn2 * t47);
-  const float t324 = (t32 - tn2 * t23) + (t302 - tn2 * t35 - tn1 * (t35 + t35 + t35 + t35)) + (t306 - tn2 * t47);
-  const float t325 = 1.0f * (kmu * t323 + klam * t324);
-  sink(5, 15, t325);
-  const float t326 = x1 * t300 + 4.0f * t172;
-  const float t327 = a2 * t326;
-  const float t328 = x1 * t304 + 2.0f * t178;
-  const float t329 = a2 * t328;
-  const float t330 = (t96 - tn2 * t94);
-  const float t331 = (t96 - tn2 * t94) + (t327 - tn2 * t98 - tn1 * (t98 + t98 + t98 + t98)) + (t329 - tn2 * t102);
-  const float t332 = 1.0f * (kmu * t330 + klam * t331);
-  sink(0, 16, t332);
-  const float t333 = (t203 - tn2 * t109 - tn1 * (t109 + t109));
-  const float t334 = 1.0f * (kmu * t333);
-  sink(1, 16, t334);
-  const float t335 = (t217 - tn2 * t115);
-  const float t336 = 1.0f * (kmu * t335);
-  sink(2, 16, t336);
-  const float t337 = (t327 - tn2 * t98 - tn1 * (t98 + t98 + t98 + t98));
-  const float t338 = (t96 - tn2 * t94) + (t327 - tn2 * t98 - tn1 * (t98 + t98 + t98 + t98)) + (t329 - tn2 * t102);
-  const float t339 = 1.0f * (kmu * t337 + klam * t338);
-  sink(3, 16, t339);
-  const float t340 = x1 * t318 + 3.0f * t194;
-  const float t341 = a2 * t340;
-  const float t342 = (t341 - tn2 * t124 - tn1 * (t124 + t124));
-  const float t343 = 1.0f * (kmu * t342);
-  sink(4, 16, t343);
-  const float t344 = (t329 - tn2 * t102);
-  const float t345 = (t96 - tn2 * t94) + (t327 - tn2 * t98 - tn1 * (t98 + t98 + t98 + t98)) + (t329 - tn2 * t102);
-  const float t346 = 1.0f * (kmu * t344 + klam * t345);
-  sink(5, 16, t346);
-  const float t347 = x2 * t300;
-  const float t348 = a2 * t347;
-  const float t349 = x2 * t304 + 2.0f * t194;
-  const float t350 = a2 * t349;
-  const float t351 = (t135 - tn2 * t133);
-  const float t352 = (t135 - tn2 * t133) + (t348 - tn2 * t137 - tn1 * (t137 + t137 + t137 + t137)) + (t350 - tn2 * t141);
-  const float t353 = 1.0f * (kmu * t351 + klam * t352);
-  sink(0, 17, t353);
-  const float t354 = (t224 - tn2 * t148 - tn1 * (t148 + t148));
-  const float t355 = 1.0f * (kmu * t354);
-  sink(1, 17, t355);
-  const float t356 = (t238 - tn2 * t154);
-  const float t357 = 1.0f * (kmu * t356);
-  sink(2, 17, t357);
-  const float t358 = (t348 - tn2 * t137 - tn1 * (t137 + t137 + t137 + t137));
-  const float t359 = (t135 - tn2 * t133) + (t348 - tn2 * t137 - tn1 * (t137 + t137 + t137 + t137)) + (t350 - tn2 * t141);
-  const float t360 = 1.0f * (kmu * t358 + klam * t359);
-  sink(3, 17, t360);
-  const float t361 = x2 * t318 + t172;
-  const float t362 = a2 * t361;
-  const float t363 = (t362 - tn2 * t163 - tn1 * (t163 + t163));
-  const float t364 = 1.0f * (kmu * t363);
-  sink(4, 17, t364);
-  const float t365 = (t350 - tn2 * t141);
-  const float t366 = (t135 - tn2 * t133) + (t348 - tn2 * t137 - tn1 * (t137 + t137 + t137 + t137)) + (t350 - tn2 * t141);
-  const float t367 = 1.0f * (kmu * t365 + klam * t366);
-  sink(5, 17, t367);
-  const float t368 = t177 * x2;
-  const float t369 = t4 * t368 + 3.0f * t12 * t77;
-  const float t370 = x0 * t369;
-  const float t371 = a2 * t370;
-  const float t372 = (t82);
-  const float t373 = (t82) + (t320 - tn1 * (t85 + t85)) + (t371 - tn1 * (t85 + t85));
-  const float t374 = 2.0f * (kmu * t372 + klam * t373);
-  sink(0, 18, t374);
-  const float t375 = (t196 - tn1 * (t70));
-  const float t376 = 2.0f * (kmu * t375);
-  sink(1, 18, t376);
-  const float t377 = (t180 - tn1 * (t59));
-  const float t378 = 2.0f * (kmu * t377);
-  sink(2, 18, t378);
-  const float t379 = (t320 - tn1 * (t85 + t85));
-  const float t380 = (t82) + (t320 - tn1 * (t85 + t85)) + (t371 - tn1 * (t85 + t85));
-  const float t381 = 2.0f * (kmu * t379 + klam * t380);
-  sink(3, 18, t381);
-  const float t382 = (t306 - tn1 * (t35 + t47));
-  const float t383 = 2.0f * (kmu * t382);
-  sink(4, 18, t383);
-  const float t384 = (t371 - tn1 * (t85 + t85));
-  const float t385 = (t82) + (t320 - tn1 * (t85 + t85)) + (t371 - tn1 * (t85 + t85));
-  const float t386 = 2.0f * (kmu * t384 + klam * t385);
-  sink(5, 18, t386);
-  const float t387 = x1 * t369 + t247;
-  const float t388 = a2 * t387;
-  const float t389 = (t122);
-  const float t390 = (t122) + (t341 - tn1 * (t124 + t124)) + (t388 - tn1 * (t124 + t124));
-  const float t391 = 2.0f * (kmu * t389 + klam * t390);
-  sink(0, 19, t391);
-  const float t392 = (t217 - tn1 * (t115));
-  const float t393 = 2.0f * (kmu * t392);
-  sink(1, 19, t393);
-  const float t394 = (t205 - tn1 * (t109));
-  const float t395 = 2.0f * (kmu * t394);
-  sink(2, 19, t395);
-  const float t396 = (t341 - tn1 * (t124 + t124));
-  const float t397 = (t122) + (t341 - tn1 * (t124 + t124)) + (t388 - tn1 * (t124 + t124));
-  const float t398 = 2.0f * (kmu * t396 + klam * t397);
-  sink(3, 19, t398);
-  const float t399 = (t329 - tn1 * (t98 + t102));
-  const float t400 = 2.0f * (kmu * t399);
-  sink(4, 19, t400);
-  const float t401 = (t388 - tn1 * (t124 + t124));
-  const float t402 = (t122) + (t341 - tn1 * (t124 + t124)) + (t388 - tn1 * (t124 + t124));
-  const float t403 = 2.0f * (kmu * t401 + klam * t402);
-  sink(5, 19, t403);
-  const float t404 = x2 * t369 + 3.0f * t178;
-  const float t405 = a2 * t404;
-  const float t406 = (t161);
-  const float t407 = (t161) + (t362 - tn1 * (t163 + t163)) + (t405 - tn1 * (t163 + t163));
-  const float t408 = 2.0f * (kmu * t406 + klam * t407);
-  sink(0, 20, t408);
-  const float t409 = (t238 - tn1 * (t154));
-  const float t410 = 2.0f * (kmu * t409);
-  sink(1, 20, t410);
-  const float t411 = (t226 - tn1 * (t148));
-  const float t412 = 2.0f * (kmu * t411);
-  sink(2, 20, t412);
-  const float t413 = (t362 - tn1 * (t163 + t163));
-  const float t414 = (t161) + (t362 - tn1 * (t163 + t163)) + (t405 - tn1 * (t163 + t163));
-  const float t415 = 2.0f * (kmu * t413 + klam * t414);
-  sink(3, 20, t415);
-  const float t416 = (t350 - tn1 * (t137 + t141));
-  const float t417 = 2.0f * (kmu * t416);
-  sink(4, 20, t417);
-  const float t418 = (t405 - tn1 * (t163 + t163));
-  const float t419 = (t161) + (t362 - tn1 * (t163 + t163)) + (t405 - tn1 * (t163 + t163));
-  const float t420 = 2.0f * (kmu * t418 + klam * t419);
-  sink(5, 20, t420);
-  const float t421 = t246 * x2;
-  const float t422 = t4 * t421 + 6.0f * t12 * t38 + 3.0f * t15;
-  const float t423 = x0 * t422;
-  const float t424 = a2 * t423;
-  const float t425 = (t44 - tn2 * t23);
-  const float t426 = (t44 - tn2 * t23) + (t306 - tn2 * t35) + (t424 - tn2 * t47 - tn1 * (t47 + t47 + t47 + t47));
-  const float t427 = 1.0f * (kmu * t425 + klam * t426);
-  sink(0, 21, t427);
-  const float t428 = (t180 - tn2 * t59);
-  const float t429 = 1.0f * (kmu * t428);
-  sink(1, 21, t429);
-  const float t430 = (t249 - tn2 * t70 - tn1 * (t70 + t70));
-  const float t431 = 1.0f * (kmu * t430);
-  sink(2, 21, t431);
-  const float t432 = (t306 - tn2 * t35);
-  const float t433 = (t44 - tn2 * t23) + (t306 - tn2 * t35) + (t424 - tn2 * t47 - tn1 * (t47 + t47 + t47 + t47));
-  const float t434 = 1.0f * (kmu * t432 + klam * t433);
-  sink(3, 21, t434);
-  const float t435 = (t371 - tn2 * t85 - tn1 * (t85 + t85));
-  const float t436 = 1.0f * (kmu * t435);
-  sink(4, 21, t436);
-  const float t437 = (t424 - tn2 * t47 - tn1 * (t47 + t47 + t47 + t47));
-  const float t438 = (t44 - tn2 * t23) + (t306 - tn2 * t35) + (t424 - tn2 * t47 - tn1 * (t47 + t47 + t47 + t47));
-  const float t439 = 1.0f * (kmu * t437 + klam * t438);
-  sink(5, 21, t439);
-  const float t440 = x1 * t422;
-  const float t441 = a2 * t440;
-  const float t442 = (t100 - tn2 * t94);
-  const float t443 = (t100 - tn2 * t94) + (t329 - tn2 * t98) + (t441 - tn2 * t102 - tn1 * (t102 + t102 + t102 + t102));
-  const float t444 = 1.0f * (kmu * t442 + klam * t443);
-  sink(0, 22, t444);
-  const float t445 = (t205 - tn2 * t109);
-  const float t446 = 1.0f * (kmu * t445);
-  sink(1, 22, t446);
-  const float t447 = (t266 - tn2 * t115 - tn1 * (t115 + t115));
-  const float t448 = 1.0f * (kmu * t447);
-  sink(2, 22, t448);
-  const float t449 = (t329 - tn2 * t98);
-  const float t450 = (t100 - tn2 * t94) + (t329 - tn2 * t98) + (t441 - tn2 * t102 - tn1 * (t102 + t102 + t102 + t102));
-  const float t451 = 1.0f * (kmu * t449 + klam * t450);
-  sink(3, 22, t451);
-  const float t452 = (t388 - tn2 * t124 - tn1 * (t124 + t124));
-  const float t453 = 1.0f * (kmu * t452);
-  sink(4, 22, t453);
-  const float t454 = (t441 - tn2 * t102 - tn1 * (t102 + t102 + t102 + t102));
-  const float t455 = (t100 - tn2 * t94) + (t329 - tn2 * t98) + (t441 - tn2 * t102 - tn1 * (t102 + t102 + t102 + t102));
-  const float t456 = 1.0f * (kmu * t454 + klam * t455);
-  sink(5, 22, t456);
-  const float t457 = x2 * t422 + 4.0f * t247;
-  const float t458 = a2 * t457;
-  const float t459 = (t139 - tn2 * t133);
-  const float t460 = (t139 - tn2 * t133) + (t350 - tn2 * t137) + (t458 - tn2 * t141 - tn1 * (t141 + t141 + t141 + t141));
-  const float t461 = 1.0f * (kmu * t459 + klam * t460);
-  sink(0, 23, t461);
-  const float t462 = (t226 - tn2 * t148);
-  const float t463 = 1.0f * (kmu * t462);
-  sink(1, 23, t463);
-  const float t464 = (t283 - tn2 * t154 - tn1 * (t154 + t154));
-  const float t465 = 1.0f * (kmu * t464);
-  sink(2, 23, t465);
-  const float t466 = (t350 - tn2 * t137);
-  const float t467 = (t139 - tn2 * t133) + (t350 - tn2 * t137) + (t458 - tn2 * t141 - tn1 * (t141 + t141 + t141 + t141));
-  const float t468 = 1.0f * (kmu * t466 + klam * t467);
-  sink(3, 23, t468);
-  const float t469 = (t405 - tn2 * t163 - tn1 * (t163 + t163));
-  const float t470 = 1.0f * (kmu * t469);
-  sink(4, 23, t470);
-  const float t471 = (t458 - tn2 * t141 - tn1 * (t141 + t141 + t141 + t141));
-  const float t472 = (t139 - tn2 * t133) + (t350 - tn2 * t137) + (t458 - tn2 * t141 - tn1 * (t141 + t141 + t141 + t141));
-  const float t473 = 1.0f * (kmu * t471 + klam * t472);
-  sink(5, 23, t473);
-}
-
-template <class Sink>
-IBEM_HD IBEM_INLINE void sph_block24f_c1_r1(const float x0, const float x1, const float x2,
-    const float a, const SphMatF& mc, Sink& sink) {
-  const float a2 = a * a; const float a4 = a2 * a2;
-  const float u = 0.5f * (x0 * x0 + x1 * x1 + x2 * x2);
-  const float lam = 2.0f * u - a2;
-  const float ext = lam > 0.0f ? 1.0f : 0.0f;
-  const float rho2 = lam > 0.0f ? a2 + lam : a2;
-  float Jv[7];
-  {
-    // J_m = 4 pi a^3 / ((2m+1) rho^(2m+1)),  rho^2 = a^2 + lambda
-    const float irho2 = 1.0f / rho2;
-    float pw = 4.0f * 3.14159265358979f * a * a2 / sqrtf(rho2);
-    for (int m = 0; m <= 6; ++m) { Jv[m] = pw / (2 * m + 1); pw *= irho2; }
-  }
-  const float kmu = mc.kmu, klam = mc.klam, tn1 = mc.tn1, tn2 = mc.tn2;
-  (void)kmu; (void)klam; (void)tn1; (void)tn2; (void)a4;
-  const float t0 = ext * (-693.0f * Jv[5]);
-  const float t1 = -(t0);
-  const float t2 = ext * (-1287.0f * Jv[6]);
-  const float t3 = -(t2);
-  const float t4 = (1.0f) * t1 + (-a2) * t3;
-  const float t5 = x0 * x0;
-  const float t6 = t5 * x0;
-  const float t7 = t6 * x0;
-  const float t8 = t7 * x0;
-  const float t9 = ext * (63.0f * Jv[4]);
-  const float t10 = -(t9);
-  const float t11 = ext * (99.0f * Jv[5]);
-  const float t12 = -(t11);
-  const float t13 = (1.0f) * t10 + (-a2) * t12;
-  const float t14 = ext * (-7.0f * Jv[3]);
-  const float t15 = -(t14);
-  const float t16 = ext * (-9.0f * Jv[4]);
-  const float t17 = -(t16);
-  const float t18 = (1.0f) * t15 + (-a2) * t17;
-  const float t19 = t4 * t8 + 10.0f * t13 * t6 + 15.0f * t18 * x0;
-  const float t20 = -(Jv[2]);
-  const float t21 = -(Jv[3]);
-  const float t22 = (1.0f) * t20 + (-a2) * t21;
-  const float t23 = t13 * t7 + 6.0f * t18 * t5 + 3.0f * t22;
-  const float t24 = x0 * t19 + 5.0f * t23;
-  const float t25 = a2 * t24;
-  const float t26 = t10 * t6 + 3.0f * t15 * x0;
-  const float t27 = t15 * t5 + t20;
-  const float t28 = x0 * t26 + 3.0f * t27;
-  const float t29 = a2 * t28;
-  const float t30 = t6 * x1;
-  const float t31 = t30 * x1;
-  const float t32 = x0 * x1;
-  const float t33 = t32 * x1;
-  const float t34 = t4 * t31 + t13 * t6 + 3.0f * t13 * t33 + 3.0f * t18 * x0;
-  const float t35 = t5 * x1;
-  const float t36 = t35 * x1;
-  const float t37 = x1 * x1;
-  const float t38 = t13 * t36 + t18 * t5 + t18 * t37 + t22;
-  const float t39 = x0 * t34 + 3.0f * t38;
-  const float t40 = a2 * t39;
-  const float t41 = t10 * t33 + t15 * x0;
-  const float t42 = t15 * t37 + t20;
-  const float t43 = x0 * t41 + t42;
-  const float t44 = a2 * t43;
-  const float t45 = t6 * x2;
-  const float t46 = t45 * x2;
-  const float t47 = x0 * x2;
-  const float t48 = t47 * x2;
-  const float t49 = t4 * t46 + t13 * t6 + 3.0f * t13 * t48 + 3.0f * t18 * x0;
-  const float t50 = t5 * x2;
-  const float t51 = t50 * x2;
-  const float t52 = x2 * x2;
-  const float t53 = t13 * t51 + t18 * t5 + t18 * t52 + t22;
-  const float t54 = x0 * t49 + 3.0f * t53;
-  const float t55 = a2 * t54;
-  const float t56 = t10 * t48 + t15 * x0;
-  const float t57 = t15 * t52 + t20;
-  const float t58 = x0 * t56 + t57;
-  const float t59 = a2 * t58;
-  const float t60 = (t25 - tn2 * t29 - tn1 * (t29 + t29 + t29 + t29));
-  const float t61 = (t25 - tn2 * t29 - tn1 * (t29 + t29 + t29 + t29)) + (t40 - tn2 * t44) + (t55 - tn2 * t59);
-  const float t62 = 1.0f * (kmu * t60 + klam * t61);
-  sink(6, 6, t62);
-  const float t63 = t7 * x1;
-  const float t64 = t4 * t63 + 6.0f * t13 * t35 + 3.0f * t18 * x1;
-  const float t65 = t13 * t30 + 3.0f * t18 * t32;
-  const float t66 = x0 * t64 + 4.0f * t65;
-  const float t67 = a2 * t66;
-  const float t68 = t10 * t35 + t15 * x1;
-  const float t69 = t15 * t32;
-  const float t70 = x0 * t68 + 2.0f * t69;
-  const float t71 = a2 * t70;
-  const float t72 = t36 * x1;
-  const float t73 = t37 * x1;
-  const float t74 = t4 * t72 + 3.0f * t13 * t35 + t13 * t73 + 3.0f * t18 * x1;
-  const float t75 = t33 * x1;
-  const float t76 = t13 * t75 + 3.0f * t18 * t32;
-  const float t77 = x0 * t74 + 2.0f * t76;
-  const float t78 = a2 * t77;
-  const float t79 = t10 * t73 + 3.0f * t15 * x1;
-  const float t80 = x0 * t79;
-  const float t81 = a2 * t80;
-  const float t82 = t35 * x2;
-  const float t83 = t82 * x2;
-  const float t84 = x1 * x2;
-  const float t85 = t84 * x2;
-  const float t86 = t4 * t83 + t13 * t35 + t13 * t85 + t18 * x1;
-  const float t87 = t32 * x2;
-  const float t88 = t87 * x2;
-  const float t89 = t13 * t88 + t18 * t32;
-  const float t90 = x0 * t86 + 2.0f * t89;
-  const float t91 = a2 * t90;
-  const float t92 = t10 * t85 + t15 * x1;
-  const float t93 = x0 * t92;
-  const float t94 = a2 * t93;
-  const float t95 = (t67 - tn2 * t71 - tn1 * (t71 + t71 + t71 + t71));
-  const float t96 = (t67 - tn2 * t71 - tn1 * (t71 + t71 + t71 + t71)) + (t78 - tn2 * t81) + (t91 - tn2 * t94);
-  const float t97 = 1.0f * (kmu * t95 + klam * t96);
-  sink(7, 6, t97);
-  const float t98 = t7 * x2;
-  const float t99 = t4 * t98 + 6.0f * t13 * t50 + 3.0f * t18 * x2;
-  const float t100 = t13 * t45 + 3.0f * t18 * t47;
-  const float t101 = x0 * t99 + 4.0f * t100;
-  const float t102 = a2 * t101;
-  const float t103 = t10 * t50 + t15 * x2;
-  const float t104 = t15 * t47;
-  const float t105 = x0 * t103 + 2.0f * t104;
-  const float t106 = a2 * t105;
-  const float t107 = t36 * x2;
-  const float t108 = t37 * x2;
-  const float t109 = t4 * t107 + t13 * t50 + t13 * t108 + t18 * x2;
-  const float t110 = t33 * x2;
-  const float t111 = t13 * t110 + t18 * t47;
-  const float t112 = x0 * t109 + 2.0f * t111;
-  const float t113 = a2 * t112;
-  const float t114 = t10 * t108 + t15 * x2;
-  const float t115 = x0 * t114;
-  const float t116 = a2 * t115;
-  const float t117 = t51 * x2;
-  const float t118 = t52 * x2;
-  const float t119 = t4 * t117 + 3.0f * t13 * t50 + t13 * t118 + 3.0f * t18 * x2;
-  const float t120 = t48 * x2;
-  const float t121 = t13 * t120 + 3.0f * t18 * t47;
-  const float t122 = x0 * t119 + 2.0f * t121;
-  const float t123 = a2 * t122;
-  const float t124 = t10 * t118 + 3.0f * t15 * x2;
-  const float t125 = x0 * t124;
-  const float t126 = a2 * t125;
-  const float t127 = (t102 - tn2 * t106 - tn1 * (t106 + t106 + t106 + t106));
-  const float t128 = (t102 - tn2 * t106 - tn1 * (t106 + t106 + t106 + t106)) + (t113 - tn2 * t116) + (t123 - tn2 * t126);
-  const float t129 = 1.0f * (kmu * t127 + klam * t128);
-  sink(8, 6, t129);
-  const float t130 = (t67 - tn2 * t71 - tn1 * (t71 + t71));
-  const float t131 = 1.0f * (kmu * t130);
-  sink(9, 6, t131);
-  const float t132 = (t40 - tn2 * t44 - tn1 * (t44 + t44));
-  const float t133 = 1.0f * (kmu * t132);
-  sink(10, 6, t133);
-  const float t134 = t30 * x2;
-  const float t135 = t4 * t134 + 3.0f * t13 * t87;
-  const float t136 = t13 * t82 + t18 * t84;
-  const float t137 = x0 * t135 + 3.0f * t136;
-  const float t138 = a2 * t137;
-  const float t139 = t10 * t87;
-  const float t140 = t15 * t84;
-  const float t141 = x0 * t139 + t140;
-  const float t142 = a2 * t141;
-  const float t143 = (t138 - tn2 * t142 - tn1 * (t142 + t142));
-  const float t144 = 1.0f * (kmu * t143);
-  sink(11, 6, t144);
-  const float t145 = (t102 - tn2 * t106 - tn1 * (t106 + t106));
-  const float t146 = 1.0f * (kmu * t145);
-  sink(12, 6, t146);
-  const float t147 = (t138 - tn2 * t142 - tn1 * (t142 + t142));
-  const float t148 = 1.0f * (kmu * t147);
-  sink(13, 6, t148);
-  const float t149 = (t55 - tn2 * t59 - tn1 * (t59 + t59));
-  const float t150 = 1.0f * (kmu * t149);
-  sink(14, 6, t150);
-  const float t151 = (t40 - tn2 * t44);
-  const float t152 = (t25 - tn2 * t29 - tn1 * (t29 + t29 + t29 + t29)) + (t40 - tn2 * t44) + (t55 - tn2 * t59);
-  const float t153 = 1.0f * (kmu * t151 + klam * t152);
-  sink(15, 6, t153);
-  const float t154 = (t78 - tn2 * t81);
-  const float t155 = (t67 - tn2 * t71 - tn1 * (t71 + t71 + t71 + t71)) + (t78 - tn2 * t81) + (t91 - tn2 * t94);
-  const float t156 = 1.0f * (kmu * t154 + klam * t155);
-  sink(16, 6, t156);
-  const float t157 = (t113 - tn2 * t116);
-  const float t158 = (t102 - tn2 * t106 - tn1 * (t106 + t106 + t106 + t106)) + (t113 - tn2 * t116) + (t123 - tn2 * t126);
-  const float t159 = 1.0f * (kmu * t157 + klam * t158);
-  sink(17, 6, t159);
-  const float t160 = (t138 - tn2 * t142);
-  const float t161 = 1.0f * (kmu * t160);
-  sink(18, 6, t161);
-  const float t162 = (t113 - tn2 * t116);
-  const float t163 = 1.0f * (kmu * t162);
-  sink(19, 6, t163);
-  const float t164 = (t91 - tn2 * t94);
-  const float t165 = 1.0f * (kmu * t164);
-  sink(20, 6, t165);
-  const float t166 = (t55 - tn2 * t59);
-  const float t167 = (t25 - tn2 * t29 - tn1 * (t29 + t29 + t29 + t29)) + (t40 - tn2 * t44) + (t55 - tn2 * t59);
-  const float t168 = 1.0f * (kmu * t166 + klam * t167);
-  sink(21, 6, t168);
-  const float t169 = (t91 - tn2 * t94);
-  const float t170 = (t67 - tn2 * t71 - tn1 * (t71 + t71 + t71 + t71)) + (t78 - tn2 * t81) + (t91 - tn2 * t94);
-  const float t171 = 1.0f * (kmu * t169 + klam * t170);
-  sink(22, 6, t171);
-  const float t172 = (t123 - tn2 * t126);
-  const float t173 = (t102 - tn2 * t106 - tn1 * (t106 + t106 + t106 + t106)) + (t113 - tn2 * t116) + (t123 - tn2 * t126);
-  const float t174 = 1.0f * (kmu * t172 + klam * t173);
-  sink(23, 6, t174);
-  const float t175 = x1 * t19;
-  const float t176 = a2 * t175;
-  const float t177 = x1 * t26;
-  const float t178 = a2 * t177;
-  const float t179 = x1 * t34 + 2.0f * t65;
-  const float t180 = a2 * t179;
-  const float t181 = x1 * t41 + 2.0f * t69;
-  const float t182 = a2 * t181;
-  const float t183 = x1 * t49;
-  const float t184 = a2 * t183;
-  const float t185 = x1 * t56;
-  const float t186 = a2 * t185;
-  const float t187 = (t176 - tn2 * t178 - tn1 * (t178 + t178 + t178 + t178));
-  const float t188 = (t176 - tn2 * t178 - tn1 * (t178 + t178 + t178 + t178)) + (t180 - tn2 * t182) + (t184 - tn2 * t186);
-  const float t189 = 1.0f * (kmu * t187 + klam * t188);
-  sink(6, 7, t189);
-  const float t190 = x1 * t64 + t23;
-  const float t191 = a2 * t190;
-  const float t192 = x1 * t68 + t27;
-  const float t193 = a2 * t192;
-  const float t194 = x1 * t74 + 3.0f * t38;
-  const float t195 = a2 * t194;
-  const float t196 = x1 * t79 + 3.0f * t42;
-  const float t197 = a2 * t196;
-  const float t198 = x1 * t86 + t53;
-  const float t199 = a2 * t198;
-  const float t200 = x1 * t92 + t57;
-  const float t201 = a2 * t200;
-  const float t202 = (t191 - tn2 * t193 - tn1 * (t193 + t193 + t193 + t193));
-  const float t203 = (t191 - tn2 * t193 - tn1 * (t193 + t193 + t193 + t193)) + (t195 - tn2 * t197) + (t199 - tn2 * t201);
-  const float t204 = 1.0f * (kmu * t202 + klam * t203);
-  sink(7, 7, t204);
-  const float t205 = x1 * t99;
-  const float t206 = a2 * t205;
-  const float t207 = x1 * t103;
-  const float t208 = a2 * t207;
-  const float t209 = x1 * t109 + 2.0f * t136;
-  const float t210 = a2 * t209;
-  const float t211 = x1 * t114 + 2.0f * t140;
-  const float t212 = a2 * t211;
-  const float t213 = x1 * t119;
-  const float t214 = a2 * t213;
-  const float t215 = x1 * t124;
-  const float t216 = a2 * t215;
-  const float t217 = (t206 - tn2 * t208 - tn1 * (t208 + t208 + t208 + t208));
-  const float t218 = (t206 - tn2 * t208 - tn1 * (t208 + t208 + t208 + t208)) + (t210 - tn2 * t212) + (t214 - tn2 * t216);
-  const float t219 = 1.0f * (kmu * t217 + klam * t218);
-  sink(8, 7, t219);
-  const float t220 = (t191 - tn2 * t193 - tn1 * (t193 + t193));
-  const float t221 = 1.0f * (kmu * t220);
-  sink(9, 7, t221);
-  const float t222 = (t180 - tn2 * t182 - tn1 * (t182 + t182));
-  const float t223 = 1.0f * (kmu * t222);
-  sink(10, 7, t223);
-  const float t224 = x1 * t135 + t100;
-  const float t225 = a2 * t224;
-  const float t226 = x1 * t139 + t104;
-  const float t227 = a2 * t226;
-  const float t228 = (t225 - tn2 * t227 - tn1 * (t227 + t227));
-  const float t229 = 1.0f * (kmu * t228);
-  sink(11, 7, t229);
-  const float t230 = (t206 - tn2 * t208 - tn1 * (t208 + t208));
-  const float t231 = 1.0f * (kmu * t230);
-  sink(12, 7, t231);
-  const float t232 = (t225 - tn2 * t227 - tn1 * (t227 + t227));
-  const float t233 = 1.0f * (kmu * t232);
-  sink(13, 7, t233);
-  const float t234 = (t184 - tn2 * t186 - tn1 * (t186 + t186));
-  const float t235 = 1.0f * (kmu * t234);
-  sink(14, 7, t235);
-  const float t236 = (t180 - tn2 * t182);
-  const float t237 = (t176 - tn2 * t178 - tn1 * (t178 + t178 + t178 + t178)) + (t180 - tn2 * t182) + (t184 - tn2 * t186);
-  const float t238 = 1.0f * (kmu * t236 + klam * t237);
-  sink(15, 7, t238);
-  const float t239 = (t195 - tn2 * t197);
-  const float t240 = (t191 - tn2 * t193 - tn1 * (t193 + t193 + t193 + t193)) + (t195 - tn2 * t197) + (t199 - tn2 * t201);
-  const float t241 = 1.0f * (kmu * t239 + klam * t240);
-  sink(16, 7, t241);
-  const float t242 = (t210 - tn2 * t212);
-  const float t243 = (t206 - tn2 * t208 - tn1 * (t208 + t208 + t208 + t208)) + (t210 - tn2 * t212) + (t214 - tn2 * t216);
-  const float t244 = 1.0f * (kmu * t242 + klam * t243);
-  sink(17, 7, t244);
-  const float t245 = (t225 - tn2 * t227);
-  const float t246 = 1.0f * (kmu * t245);
-  sink(18, 7, t246);
-  const float t247 = (t210 - tn2 * t212);
-  const float t248 = 1.0f * (kmu * t247);
-  sink(19, 7, t248);
-  const float t249 = (t199 - tn2 * t201);
-  const float t250 = 1.0f * (kmu * t249);
-  sink(20, 7, t250);
-  const float t251 = (t184 - tn2 * t186);
-  const float t252 = (t176 - tn2 * t178 - tn1 * (t178 + t178 + t178 + t178)) + (t180 - tn2 * t182) + (t184 - tn2 * t186);
-  const float t253 = 1.0f * (kmu * t251 + klam * t252);
-  sink(21, 7, t253);
-  const float t254 = (t199 - tn2 * t201);
-  const float t255 = (t191 - tn2 * t193 - tn1 * (t193 + t193 + t193 + t193)) + (t195 - tn2 * t197) + (t199 - tn2 * t201);
-  const float t256 = 1.0f * (kmu * t254 + klam * t255);
-  sink(22, 7, t256);
-  const float t257 = (t214 - tn2 * t216);
-  const float t258 = (t206 - tn2 * t208 - tn1 * (t208 + t208 + t208 + t208)) + (t210 - tn2 * t212) + (t214 - tn2 * t216);
-  const float t259 = 1.0f * (kmu * t257 + klam * t258);
-  sink(23, 7, t259);
-  const float t260 = x2 * t19;
-  const float t261 = a2 * t260;
-  const float t262 = x2 * t26;
-  const float t263 = a2 * t262;
-  const float t264 = x2 * t34;
-  const float t265 = a2 * t264;
-  const float t266 = x2 * t41;
-  const float t267 = a2 * t266;
-  const float t268 = x2 * t49 + 2.0f * t100;
-  const float t269 = a2 * t268;
-  const float t270 = x2 * t56 + 2.0f * t104;
-  const float t271 = a2 * t270;
-  const float t272 = (t261 - tn2 * t263 - tn1 * (t263 + t263 + t263 + t263));
-  const float t273 = (t261 - tn2 * t263 - tn1 * (t263 + t263 + t263 + t263)) + (t265 - tn2 * t267) + (t269 - tn2 * t271);
-  const float t274 = 1.0f * (kmu * t272 + klam * t273);
-  sink(6, 8, t274);
-  const float t275 = x2 * t64;
-  const float t276 = a2 * t275;
-  const float t277 = x2 * t68;
-  const float t278 = a2 * t277;
-  const float t279 = x2 * t74;
-  const float t280 = a2 * t279;
-  const float t281 = x2 * t79;
-  const float t282 = a2 * t281;
-  const float t283 = x2 * t86 + 2.0f * t136;
-  const float t284 = a2 * t283;
-  const float t285 = x2 * t92 + 2.0f * t140;
-  const float t286 = a2 * t285;
-  const float t287 = (t276 - tn2 * t278 - tn1 * (t278 + t278 + t278 + t278));
-  const float t288 = (t276 - tn2 * t278 - tn1 * (t278 + t278 + t278 + t278)) + (t280 - tn2 * t282) + (t284 - tn2 * t286);
-  const float t289 = 1.0f * (kmu * t287 + klam * t288);
-  sink(7, 8, t289);
-  const float t290 = x2 * t99 + t23;
-  const float t291 = a2 * t290;
-  const float t292 = x2 * t103 + t27;
-  const float t293 = a2 * t292;
-  const float t294 = x2 * t109 + t38;
-  const float t295 = a2 * t294;
-  const float t296 = x2 * t114 + t42;
-  const float t297 = a2 * t296;
-  const float t298 = x2 * t119 + 3.0f * t53;
-  const float t299 = a2 * t298;
-  const float t300 = x2 * t124 + 3.0f * t57;
-  const float t301 = a2 * t300;
-  const float t302 = (t291 - tn2 * t293 - tn1 * (t293 + t293 + t293 + t293));
-  const float t303 = (t291 - tn2 * t293 - tn1 * (t293 + t293 + t293 + t293)) + (t295 - tn2 * t297) + (t299 - tn2 * t301);
-  const float t304 = 1.0f * (kmu * t302 + klam * t303);
-  sink(8, 8, t304);
-  const float t305 = (t276 - tn2 * t278 - tn1 * (t278 + t278));
-  const float t306 = 1.0f * (kmu * t305);
-  sink(9, 8, t306);
-  const float t307 = (t265 - tn2 * t267 - tn1 * (t267 + t267));
-  const float t308 = 1.0f * (kmu * t307);
-  sink(10, 8, t308);
-  const float t309 = x2 * t135 + t65;
-  const float t310 = a2 * t309;
-  const float t311 = x2 * t139 + t69;
-  const float t312 = a2 * t311;
-  const float t313 = (t310 - tn2 * t312 - tn1 * (t312 + t312));
-  const float t314 = 1.0f * (kmu * t313);
-  sink(11, 8, t314);
-  const float t315 = (t291 - tn2 * t293 - tn1 * (t293 + t293));
-  const float t316 = 1.0f * (kmu * t315);
-  sink(12, 8, t316);
-  const float t317 = (t310 - tn2 * t312 - tn1 * (t312 + t312));
-  const float t318 = 1.0f * (kmu * t317);
-  sink(13, 8, t318);
-  const float t319 = (t269 - tn2 * t271 - tn1 * (t271 + t271));
-  const float t320 = 1.0f * (kmu * t319);
-  sink(14, 8, t320);
-  const float t321 = (t265 - tn2 * t267);
-  const float t322 = (t261 - tn2 * t263 - tn1 * (t263 + t263 + t263 + t263)) + (t265 - tn2 * t267) + (t269 - tn2 * t271);
-  const float t323 = 1.0f * (kmu * t321 + klam * t322);
-  sink(15, 8, t323);
-  const float t324 = (t280 - tn2 * t282);
-  const float t325 = (t276 - tn2 * t278 - tn1 * (t278 + t278 + t278 + t278)) + (t280 - tn2 * t282) + (t284 - tn2 * t286);
-  const float t326 = 1.0f * (kmu * t324 + klam * t325);
-  sink(16, 8, t326);
-  const float t327 = (t295 - tn2 * t297);
-  const float t328 = (t291 - tn2 * t293 - tn1 * (t293 + t293 + t293 + t293)) + (t295 - tn2 * t297) + (t299 - tn2 * t301);
-  const float t329 = 1.0f * (kmu * t327 + klam * t328);
-  sink(17, 8, t329);
-  const float t330 = (t310 - tn2 * t312);
-  const float t331 = 1.0f * (kmu * t330);
-  sink(18, 8, t331);
-  const float t332 = (t295 - tn2 * t297);
-  const float t333 = 1.0f * (kmu * t332);
-  sink(19, 8, t333);
-  const float t334 = (t284 - tn2 * t286);
-  const float t335 = 1.0f * (kmu * t334);
-  sink(20, 8, t335);
-  const float t336 = (t269 - tn2 * t271);
-  const float t337 = (t261 - tn2 * t263 - tn1 * (t263 + t263 + t263 + t263)) + (t265 - tn2 * t267) + (t269 - tn2 * t271);
-  const float t338 = 1.0f * (kmu * t336 + klam * t337);
-  sink(21, 8, t338);
-  const float t339 = (t284 - tn2 * t286);
-  const float t340 = (t276 - tn2 * t278 - tn1 * (t278 + t278 + t278 + t278)) + (t280 - tn2 * t282) + (t284 - tn2 * t286);
-  const float t341 = 1.0f * (kmu * t339 + klam * t340);
-  sink(22, 8, t341);
-  const float t342 = (t299 - tn2 * t301);
-  const float t343 = (t291 - tn2 * t293 - tn1 * (t293 + t293 + t293 + t293)) + (t295 - tn2 * t297) + (t299 - tn2 * t301);
-  const float t344 = 1.0f * (kmu * t342 + klam * t343);
-  sink(23, 8, t344);
-  const float t345 = (t67 - tn1 * (t71 + t71));
-  const float t346 = (t67 - tn1 * (t71 + t71)) + (t78 - tn1 * (t71 + t71)) + (t91);
-  const float t347 = 2.0f * (kmu * t345 + klam * t346);
-  sink(6, 9, t347);
-  const float t348 = t75 * x1;
-  const float t349 = t4 * t348 + 6.0f * t13 * t33 + 3.0f * t18 * x0;
-  const float t350 = t73 * x1;
-  const float t351 = t13 * t350 + 6.0f * t18 * t37 + 3.0f * t22;
-  const float t352 = x0 * t349 + t351;
-  const float t353 = a2 * t352;
-  const float t354 = t110 * x2;
-  const float t355 = t4 * t354 + t13 * t33 + t13 * t48 + t18 * x0;
-  const float t356 = t108 * x2;
-  const float t357 = t13 * t356 + t18 * t37 + t18 * t52 + t22;
-  const float t358 = x0 * t355 + t357;
-  const float t359 = a2 * t358;
-  const float t360 = (t40 - tn1 * (t44 + t44));
-  const float t361 = (t40 - tn1 * (t44 + t44)) + (t353 - tn1 * (t44 + t44)) + (t359);
-  const float t362 = 2.0f * (kmu * t360 + klam * t361);
-  sink(7, 9, t362);
-  const float t363 = t75 * x2;
-  const float t364 = t4 * t363 + 3.0f * t13 * t87;
-  const float t365 = t73 * x2;
-  const float t366 = t13 * t365 + 3.0f * t18 * t84;
-  const float t367 = x0 * t364 + t366;
-  const float t368 = a2 * t367;
-  const float t369 = t88 * x2;
-  const float t370 = t4 * t369 + 3.0f * t13 * t87;
-  const float t371 = t85 * x2;
-  const float t372 = t13 * t371 + 3.0f * t18 * t84;
-  const float t373 = x0 * t370 + t372;
-  const float t374 = a2 * t373;
-  const float t375 = (t138 - tn1 * (t142 + t142));
-  const float t376 = (t138 - tn1 * (t142 + t142)) + (t368 - tn1 * (t142 + t142)) + (t374);
-  const float t377 = 2.0f * (kmu * t375 + klam * t376);
-  sink(8, 9, t377);
-  const float t378 = (t40 - tn1 * (t29 + t44));
-  const float t379 = 2.0f * (kmu * t378);
-  sink(9, 9, t379);
-  const float t380 = (t78 - tn1 * (t71 + t81));
-  const float t381 = 2.0f * (kmu * t380);
-  sink(10, 9, t381);
-  const float t382 = (t113 - tn1 * (t106 + t116));
-  const float t383 = 2.0f * (kmu * t382);
-  sink(11, 9, t383);
-  const float t384 = (t138 - tn1 * (t142));
-  const float t385 = 2.0f * (kmu * t384);
-  sink(12, 9, t385);
-  const float t386 = (t113 - tn1 * (t116));
-  const float t387 = 2.0f * (kmu * t386);
-  sink(13, 9, t387);
-  const float t388 = (t91 - tn1 * (t94));
-  const float t389 = 2.0f * (kmu * t388);
-  sink(14, 9, t389);
-  const float t390 = (t78 - tn1 * (t71 + t71));
-  const float t391 = (t67 - tn1 * (t71 + t71)) + (t78 - tn1 * (t71 + t71)) + (t91);
-  const float t392 = 2.0f * (kmu * t390 + klam * t391);
-  sink(15, 9, t392);
-  const float t393 = (t353 - tn1 * (t44 + t44));
-  const float t394 = (t40 - tn1 * (t44 + t44)) + (t353 - tn1 * (t44 + t44)) + (t359);
-  const float t395 = 2.0f * (kmu * t393 + klam * t394);
-  sink(16, 9, t395);
-  const float t396 = (t368 - tn1 * (t142 + t142));
-  const float t397 = (t138 - tn1 * (t142 + t142)) + (t368 - tn1 * (t142 + t142)) + (t374);
-  const float t398 = 2.0f * (kmu * t396 + klam * t397);
-  sink(17, 9, t398);
-  const float t399 = (t113 - tn1 * (t106));
-  const float t400 = 2.0f * (kmu * t399);
-  sink(18, 9, t400);
-  const float t401 = (t368 - tn1 * (t142));
-  const float t402 = 2.0f * (kmu * t401);
-  sink(19, 9, t402);
-  const float t403 = (t359 - tn1 * (t59));
-  const float t404 = 2.0f * (kmu * t403);
-  sink(20, 9, t404);
-  const float t405 = (t91);
-  const float t406 = (t67 - tn1 * (t71 + t71)) + (t78 - tn1 * (t71 + t71)) + (t91);
-  const float t407 = 2.0f * (kmu * t405 + klam * t406);
-  sink(21, 9, t407);
-  const float t408 = (t359);
-  const float t409 = (t40 - tn1 * (t44 + t44)) + (t353 - tn1 * (t44 + t44)) + (t359);
-  const float t410 = 2.0f * (kmu * t408 + klam * t409);
-  sink(22, 9, t410);
-  const float t411 = (t374);
-  const float t412 = (t138 - tn1 * (t142 + t142)) + (t368 - tn1 * (t142 + t142)) + (t374);
-  const float t413 = 2.0f * (kmu * t411 + klam * t412);
-  sink(23, 9, t413);
-  const float t414 = (t191 - tn1 * (t193 + t193));
-  const float t415 = (t191 - tn1 * (t193 + t193)) + (t195 - tn1 * (t193 + t193)) + (t199);
-  const float t416 = 2.0f * (kmu * t414 + klam * t415);
-  sink(6, 10, t416);
-  const float t417 = x1 * t349 + 4.0f * t76;
-  const float t418 = a2 * t417;
-  const float t419 = x1 * t355 + 2.0f * t89;
-  const float t420 = a2 * t419;
-  const float t421 = (t180 - tn1 * (t182 + t182));
-  const float t422 = (t180 - tn1 * (t182 + t182)) + (t418 - tn1 * (t182 + t182)) + (t420);
-  const float t423 = 2.0f * (kmu * t421 + klam * t422);
-  sink(7, 10, t423);
-  const float t424 = x1 * t364 + 3.0f * t111;
-  const float t425 = a2 * t424;
-  const float t426 = x1 * t370 + t121;
-  const float t427 = a2 * t426;
-  const float t428 = (t225 - tn1 * (t227 + t227));
-  const float t429 = (t225 - tn1 * (t227 + t227)) + (t425 - tn1 * (t227 + t227)) + (t427);
-  const float t430 = 2.0f * (kmu * t428 + klam * t429);
-  sink(8, 10, t430);
-  const float t431 = (t180 - tn1 * (t178 + t182));
-  const float t432 = 2.0f * (kmu * t431);
-  sink(9, 10, t432);
-  const float t433 = (t195 - tn1 * (t193 + t197));
-  const float t434 = 2.0f * (kmu * t433);
-  sink(10, 10, t434);
-  const float t435 = (t210 - tn1 * (t208 + t212));
-  const float t436 = 2.0f * (kmu * t435);
-  sink(11, 10, t436);
-  const float t437 = (t225 - tn1 * (t227));
-  const float t438 = 2.0f * (kmu * t437);
-  sink(12, 10, t438);
-  const float t439 = (t210 - tn1 * (t212));
-  const float t440 = 2.0f * (kmu * t439);
-  sink(13, 10, t440);
-  const float t441 = (t199 - tn1 * (t201));
-  const float t442 = 2.0f * (kmu * t441);
-  sink(14, 10, t442);
-  const float t443 = (t195 - tn1 * (t193 + t193));
-  const float t444 = (t191 - tn1 * (t193 + t193)) + (t195 - tn1 * (t193 + t193)) + (t199);
-  const float t445 = 2.0f * (kmu * t443 + klam * t444);
-  sink(15, 10, t445);
-  const float t446 = (t418 - tn1 * (t182 + t182));
-  const float t447 = (t180 - tn1 * (t182 + t182)) + (t418 - tn1 * (t182 + t182)) + (t420);
-  const float t448 = 2.0f * (kmu * t446 + klam * t447);
-  sink(16, 10, t448);
-  const float t449 = (t425 - tn1 * (t227 + t227));
-  const float t450 = (t225 - tn1 * (t227 + t227)) + (t425 - tn1 * (t227 + t227)) + (t427);
-  const float t451 = 2.0f * (kmu * t449 + klam * t450);
-  sink(17, 10, t451);
-  const float t452 = (t210 - tn1 * (t208));
-  const float t453 = 2.0f * (kmu * t452);
-  sink(18, 10, t453);
-  const float t454 = (t425 - tn1 * (t227));
-  const float t455 = 2.0f * (kmu * t454);
-  sink(19, 10, t455);
-  const float t456 = (t420 - tn1 * (t186));
-  const float t457 = 2.0f * (kmu * t456);
-  sink(20, 10, t457);
-  const float t458 = (t199);
-  const float t459 = (t191 - tn1 * (t193 + t193)) + (t195 - tn1 * (t193 + t193)) + (t199);
-  const float t460 = 2.0f * (kmu * t458 + klam * t459);
-  sink(21, 10, t460);
-  const float t461 = (t420);
-  const float t462 = (t180 - tn1 * (t182 + t182)) + (t418 - tn1 * (t182 + t182)) + (t420);
-  const float t463 = 2.0f * (kmu * t461 + klam * t462);
-  sink(22, 10, t463);
-  const float t464 = (t427);
-  const float t465 = (t225 - tn1 * (t227 + t227)) + (t425 - tn1 * (t227 + t227)) + (t427);
-  const float t466 = 2.0f * (kmu * t464 + klam * t465);
-  sink(23, 10, t466);
-  const float t467 = (t276 - tn1 * (t278 + t278));
-  const float t468 = (t276 - tn1 * (t278 + t278)) + (t280 - tn1 * (t278 + t278)) + (t284);
-  const float t469 = 2.0f * (kmu * t467 + klam * t468);
-  sink(6, 11, t469);
-  const float t470 = x2 * t349;
-  const float t471 = a2 * t470;
-  const float t472 = x2 * t355 + 2.0f * t111;
-  const float t473 = a2 * t472;
-  const float t474 = (t265 - tn1 * (t267 + t267));
-  const float t475 = (t265 - tn1 * (t267 + t267)) + (t471 - tn1 * (t267 + t267)) + (t473);
-  const float t476 = 2.0f * (kmu * t474 + klam * t475);
-  sink(7, 11, t476);
-  const float t477 = x2 * t364 + t76;
-  const float t478 = a2 * t477;
-  const float t479 = x2 * t370 + 3.0f * t89;
-  const float t480 = a2 * t479;
-  const float t481 = (t310 - tn1 * (t312 + t312));
-  const float t482 = (t310 - tn1 * (t312 + t312)) + (t478 - tn1 * (t312 + t312)) + (t480);
-  const float t483 = 2.0f * (kmu * t481 + klam * t482);
-  sink(8, 11, t483);
-  const float t484 = (t265 - tn1 * (t263 + t267));
-  const float t485 = 2.0f * (kmu * t484);
-  sink(9, 11, t485);
-  const float t486 = (t280 - tn1 * (t278 + t282));
-  const float t487 = 2.0f * (kmu * t486);
-  sink(10, 11, t487);
-  const float t488 = (t295 - tn1 * (t293 + t297));
-  const float t489 = 2.0f * (kmu * t488);
-  sink(11, 11, t489);
-  const float t490 = (t310 - tn1 * (t312));
-  const float t491 = 2.0f * (kmu * t490);
-  sink(12, 11, t491);
-  const float t492 = (t295 - tn1 * (t297));
-  const float t493 = 2.0f * (kmu * t492);
-  sink(13, 11, t493);
-  const float t494 = (t284 - tn1 * (t286));
-  const float t495 = 2.0f * (kmu * t494);
-  sink(14, 11, t495);
-  const float t496 = (t280 - tn1 * (t278 + t278));
-  const float t497 = (t276 - tn1 * (t278 + t278)) + (t280 - tn1 * (t278 + t278)) + (t284);
-  const float t498 = 2.0f * (kmu * t496 + klam * t497);
-  sink(15, 11, t498);
-  const float t499 = (t471 - tn1 * (t267 + t267));
-  const float t500 = (t265 - tn1 * (t267 + t267)) + (t471 - tn1 * (t267 + t267)) + (t473);
-  const float t501 = 2.0f * (kmu * t499 + klam * t500);
-  sink(16, 11, t501);
-  const float t502 = (t478 - tn1 * (t312 + t312));
-  const float t503 = (t310 - tn1 * (t312 + t312)) + (t478 - tn1 * (t312 + t312)) + (t480);
-  const float t504 = 2.0f * (kmu * t502 + klam * t503);
-  sink(17, 11, t504);
-  const float t505 = (t295 - tn1 * (t293));
-  const float t506 = 2.0f * (kmu * t505);
-  sink(18, 11, t506);
-  const float t507 = (t478 - tn1 * (t312));
-  const float t508 = 2.0f * (kmu * t507);
-  sink(19, 11, t508);
-  const float t509 = (t473 - tn1 * (t271));
-  const float t510 = 2.0f * (kmu * t509);
-  sink(20, 11, t510);
-  const float t511 = (t284);
-  const float t512 = (t276 - tn1 * (t278 + t278)) + (t280 - tn1 * (t278 + t278)) + (t284);
-  const float t513 = 2.0f * (kmu * t511 + klam * t512);
-  sink(21, 11, t513);
-  const float t514 = (t473);
-  const float t515 = (t265 - tn1 * (t267 + t267)) + (t471 - tn1 * (t267 + t267)) + (t473);
-  const float t516 = 2.0f * (kmu * t514 + klam * t515);
-  sink(22, 11, t516);
-  const float t517 = (t480);
-  const float t518 = (t310 - tn1 * (t312 + t312)) + (t478 - tn1 * (t312 + t312)) + (t480);
-  const float t519 = 2.0f * (kmu * t517 + klam * t518);
-  sink(23, 11, t519);
-  const float t520 = (t102 - tn1 * (t106 + t106));
-  const float t521 = (t102 - tn1 * (t106 + t106)) + (t113) + (t123 - tn1 * (t106 + t106));
-  const float t522 = 2.0f * (kmu * t520 + klam * t521);
-  sink(6, 12, t522);
-  const float t523 = (t138 - tn1 * (t142 + t142));
-  const float t524 = (t138 - tn1 * (t142 + t142)) + (t368) + (t374 - tn1 * (t142 + t142));
-  const float t525 = 2.0f * (kmu * t523 + klam * t524);
-  sink(7, 12, t525);
-  const float t526 = t120 * x2;
-  const float t527 = t4 * t526 + 6.0f * t13 * t48 + 3.0f * t18 * x0;
-  const float t528 = t118 * x2;
-  const float t529 = t13 * t528 + 6.0f * t18 * t52 + 3.0f * t22;
-  const float t530 = x0 * t527 + t529;
-  const float t531 = a2 * t530;
-  const float t532 = (t55 - tn1 * (t59 + t59));
-  const float t533 = (t55 - tn1 * (t59 + t59)) + (t359) + (t531 - tn1 * (t59 + t59));
-  const float t534 = 2.0f * (kmu * t532 + klam * t533);
-  sink(8, 12, t534);
-  const float t535 = (t138 - tn1 * (t142));
-  const float t536 = 2.0f * (kmu * t535);
-  sink(9, 12, t536);
-  const float t537 = (t113 - tn1 * (t116));
-  const float t538 = 2.0f * (kmu * t537);
-  sink(10, 12, t538);
-  const float t539 = (t91 - tn1 * (t94));
-  const float t540 = 2.0f * (kmu * t539);
-  sink(11, 12, t540);
-  const float t541 = (t55 - tn1 * (t29 + t59));
-  const float t542 = 2.0f * (kmu * t541);
-  sink(12, 12, t542);
-  const float t543 = (t91 - tn1 * (t71 + t94));
-  const float t544 = 2.0f * (kmu * t543);
-  sink(13, 12, t544);
-  const float t545 = (t123 - tn1 * (t106 + t126));
-  const float t546 = 2.0f * (kmu * t545);
-  sink(14, 12, t546);
-  const float t547 = (t113);
-  const float t548 = (t102 - tn1 * (t106 + t106)) + (t113) + (t123 - tn1 * (t106 + t106));
-  const float t549 = 2.0f * (kmu * t547 + klam * t548);
-  sink(15, 12, t549);
-  const float t550 = (t368);
-  const float t551 = (t138 - tn1 * (t142 + t142)) + (t368) + (t374 - tn1 * (t142 + t142));
-  const float t552 = 2.0f * (kmu * t550 + klam * t551);
-  sink(16, 12, t552);
-  const float t553 = (t359);
-  const float t554 = (t55 - tn1 * (t59 + t59)) + (t359) + (t531 - tn1 * (t59 + t59));
-  const float t555 = 2.0f * (kmu * t553 + klam * t554);
-  sink(17, 12, t555);
-  const float t556 = (t91 - tn1 * (t71));
-  const float t557 = 2.0f * (kmu * t556);
-  sink(18, 12, t557);
-  const float t558 = (t359 - tn1 * (t44));
-  const float t559 = 2.0f * (kmu * t558);
-  sink(19, 12, t559);
-  const float t560 = (t374 - tn1 * (t142));
-  const float t561 = 2.0f * (kmu * t560);
-  sink(20, 12, t561);
-  const float t562 = (t123 - tn1 * (t106 + t106));
-  const float t563 = (t102 - tn1 * (t106 + t106)) + (t113) + (t123 - tn1 * (t106 + t106));
-  const float t564 = 2.0f * (kmu * t562 + klam * t563);
-  sink(21, 12, t564);
-  const float t565 = (t374 - tn1 * (t142 + t142));
-  const float t566 = (t138 - tn1 * (t142 + t142)) + (t368) + (t374 - tn1 * (t142 + t142));
-  const float t567 = 2.0f * (kmu * t565 + klam * t566);
-  sink(22, 12, t567);
-  const float t568 = (t531 - tn1 * (t59 + t59));
-  const float t569 = (t55 - tn1 * (t59 + t59)) + (t359) + (t531 - tn1 * (t59 + t59));
-  const float t570 = 2.0f * (kmu * t568 + klam * t569);
-  sink(23, 12, t570);
-  const float t571 = (t206 - tn1 * (t208 + t208));
-  const float t572 = (t206 - tn1 * (t208 + t208)) + (t210) + (t214 - tn1 * (t208 + t208));
-  const float t573 = 2.0f * (kmu * t571 + klam * t572);
-  sink(6, 13, t573);
-  const float t574 = (t225 - tn1 * (t227 + t227));
-  const float t575 = (t225 - tn1 * (t227 + t227)) + (t425) + (t427 - tn1 * (t227 + t227));
-  const float t576 = 2.0f * (kmu * t574 + klam * t575);
-  sink(7, 13, t576);
-  const float t577 = x1 * t527;
-  const float t578 = a2 * t577;
-  const float t579 = (t184 - tn1 * (t186 + t186));
-  const float t580 = (t184 - tn1 * (t186 + t186)) + (t420) + (t578 - tn1 * (t186 + t186));
-  const float t581 = 2.0f * (kmu * t579 + klam * t580);
-  sink(8, 13, t581);
-  const float t582 = (t225 - tn1 * (t227));
-  const float t583 = 2.0f * (kmu * t582);
-  sink(9, 13, t583);
-  const float t584 = (t210 - tn1 * (t212));
-  const float t585 = 2.0f * (kmu * t584);
-  sink(10, 13, t585);
-  const float t586 = (t199 - tn1 * (t201));
-  const float t587 = 2.0f * (kmu * t586);
-  sink(11, 13, t587);
-  const float t588 = (t184 - tn1 * (t178 + t186));
-  const float t589 = 2.0f * (kmu * t588);
-  sink(12, 13, t589);
-  const float t590 = (t199 - tn1 * (t193 + t201));
-  const float t591 = 2.0f * (kmu * t590);
-  sink(13, 13, t591);
-  const float t592 = (t214 - tn1 * (t208 + t216));
-  const float t593 = 2.0f * (kmu * t592);
-  sink(14, 13, t593);
-  const float t594 = (t210);
-  const float t595 = (t206 - tn1 * (t208 + t208)) + (t210) + (t214 - tn1 * (t208 + t208));
-  const float t596 = 2.0f * (kmu * t594 + klam * t595);
-  sink(15, 13, t596);
-  const float t597 = (t425);
-  const float t598 = (t225 - tn1 * (t227 + t227)) + (t425) + (t427 - tn1 * (t227 + t227));
-  const float t599 = 2.0f * (kmu * t597 + klam * t598);
-  sink(16, 13, t599);
-  const float t600 = (t420);
-  const float t601 = (t184 - tn1 * (t186 + t186)) + (t420) + (t578 - tn1 * (t186 + t186));
-  const float t602 = 2.0f * (kmu * t600 + klam * t601);
-  sink(17, 13, t602);
-  const float t603 = (t199 - tn1 * (t193));
-  const float t604 = 2.0f * (kmu * t603);
-  sink(18, 13, t604);
-  const float t605 = (t420 - tn1 * (t182));
-  const float t606 = 2.0f * (kmu * t605);
-  sink(19, 13, t606);
-  const float t607 = (t427 - tn1 * (t227));
-  const float t608 = 2.0f * (kmu * t607);
-  sink(20, 13, t608);
-  const float t609 = (t214 - tn1 * (t208 + t208));
-  const float t610 = (t206 - tn1 * (t208 + t208)) + (t210) + (t214 - tn1 * (t208 + t208));
-  const float t611 = 2.0f * (kmu * t609 + klam * t610);
-  sink(21, 13, t611);
-  const float t612 = (t427 - tn1 * (t227 + t227));
-  const float t613 = (t225 - tn1 * (t227 + t227)) + (t425) + (t427 - tn1 * (t227 + t227));
-  const float t614 = 2.0f * (kmu * t612 + klam * t613);
-  sink(22, 13, t614);
-  const float t615 = (t578 - tn1 * (t186 + t186));
-  const float t616 = (t184 - tn1 * (t186 + t186)) + (t420) + (t578 - tn1 * (t186 + t186));
-  const float t617 = 2.0f * (kmu * t615 + klam * t616);
-  sink(23, 13, t617);
-  const float t618 = (t291 - tn1 * (t293 + t293));
-  const float t619 = (t291 - tn1 * (t293 + t293)) + (t295) + (t299 - tn1 * (t293 + t293));
-  const float t620 = 2.0f * (kmu * t618 + klam * t619);
-  sink(6, 14, t620);
-  const float t621 = (t310 - tn1 * (t312 + t312));
-  const float t622 = (t310 - tn1 * (t312 + t312)) + (t478) + (t480 - tn1 * (t312 + t312));
-  const float t623 = 2.0f * (kmu * t621 + klam * t622);
-  sink(7, 14, t623);
-  const float t624 = x2 * t527 + 4.0f * t121;
-  const float t625 = a2 * t624;
-  const float t626 = (t269 - tn1 * (t271 + t271));
-  const float t627 = (t269 - tn1 * (t271 + t271)) + (t473) + (t625 - tn1 * (t271 + t271));
-  const float t628 = 2.0f * (kmu * t626 + klam * t627);
-  sink(8, 14, t628);
-  const float t629 = (t310 - tn1 * (t312));
-  const float t630 = 2.0f * (kmu * t629);
-  sink(9, 14, t630);
-  const float t631 = (t295 - tn1 * (t297));
-  const float t632 = 2.0f * (kmu * t631);
-  sink(10, 14, t632);
-  const float t633 = (t284 - tn1 * (t286));
-  const float t634 = 2.0f * (kmu * t633);
-  sink(11, 14, t634);
-  const float t635 = (t269 - tn1 * (t263 + t271));
-  const float t636 = 2.0f * (kmu * t635);
-  sink(12, 14, t636);
-  const float t637 = (t284 - tn1 * (t278 + t286));
-  const float t638 = 2.0f * (kmu * t637);
-  sink(13, 14, t638);
-  const float t639 = (t299 - tn1 * (t293 + t301));
-  const float t640 = 2.0f * (kmu * t639);
-  sink(14, 14, t640);
-  const float t641 = (t295);
-  const float t642 = (t291 - tn1 * (t293 + t293)) + (t295) + (t299 - tn1 * (t293 + t293));
-  const float t643 = 2.0f * (kmu * t641 + klam * t642);
-  sink(15, 14, t643);
-  const float t644 = (t478);
-  const float t645 = (t310 - tn1 * (t312 + t312)) + (t478) + (t480 - tn1 * (t312 + t312));
-  const float t646 = 2.0f * (kmu * t644 + klam * t645);
-  sink(16, 14, t646);
-  const float t647 = (t473);
-  const float t648 = (t269 - tn1 * (t271 + t271)) + (t473) + (t625 - tn1 * (t271 + t271));
-  const float t649 = 2.0f * (kmu * t647 + klam * t648);
-  sink(17, 14, t649);
-  const float t650 = (t284 - tn1 * (t278));
-  const float t651 = 2.0f * (kmu * t650);
-  sink(18, 14, t651);
-  const float t652 = (t473 - tn1 * (t267));
-  const float t653 = 2.0f * (kmu * t652);
-  sink(19, 14, t653);
-  const float t654 = (t480 - tn1 * (t312));
-  const float t655 = 2.0f * (kmu * t654);
-  sink(20, 14, t655);
-  const float t656 = (t299 - tn1 * (t293 + t293));
-  const float t657 = (t291 - tn1 * (t293 + t293)) + (t295) + (t299 - tn1 * (t293 + t293));
-  const float t658 = 2.0f * (kmu * t656 + klam * t657);
-  sink(21, 14, t658);
-  const float t659 = (t480 - tn1 * (t312 + t312));
-  const float t660 = (t310 - tn1 * (t312 + t312)) + (t478) + (t480 - tn1 * (t312 + t312));
-  const float t661 = 2.0f * (kmu * t659 + klam * t660);
-  sink(22, 14, t661);
-  const float t662 = (t625 - tn1 * (t271 + t271));
-  const float t663 = (t269 - tn1 * (t271 + t271)) + (t473) + (t625 - tn1 * (t271 + t271));
-  const float t664 = 2.0f * (kmu * t662 + klam * t663);
-  sink(23, 14, t664);
-  const float t665 = (t40 - tn2 * t29);
-  const float t666 = (t40 - tn2 * t29) + (t353 - tn2 * t44 - tn1 * (t44 + t44 + t44 + t44)) + (t359 - tn2 * t59);
-  const float t667 = 1.0f * (kmu * t665 + klam * t666);
-  sink(6, 15, t667);
-  const float t668 = t350 * x1;
-  const float t669 = t4 * t668 + 10.0f * t13 * t73 + 15.0f * t18 * x1;
-  const float t670 = x0 * t669;
-  const float t671 = a2 * t670;
-  const float t672 = t365 * x2;
-  const float t673 = t4 * t672 + t13 * t73 + 3.0f * t13 * t85 + 3.0f * t18 * x1;
-  const float t674 = x0 * t673;
-  const float t675 = a2 * t674;
-  const float t676 = (t78 - tn2 * t71);
-  const float t677 = (t78 - tn2 * t71) + (t671 - tn2 * t81 - tn1 * (t81 + t81 + t81 + t81)) + (t675 - tn2 * t94);
-  const float t678 = 1.0f * (kmu * t676 + klam * t677);
-  sink(7, 15, t678);
-  const float t679 = t350 * x2;
-  const float t680 = t4 * t679 + 6.0f * t13 * t108 + 3.0f * t18 * x2;
-  const float t681 = x0 * t680;
-  const float t682 = a2 * t681;
-  const float t683 = t356 * x2;
-  const float t684 = t4 * t683 + 3.0f * t13 * t108 + t13 * t118 + 3.0f * t18 * x2;
-  const float t685 = x0 * t684;
-  const float t686 = a2 * t685;
-  const float t687 = (t113 - tn2 * t106);
-  const float t688 = (t113 - tn2 * t106) + (t682 - tn2 * t116 - tn1 * (t116 + t116 + t116 + t116)) + (t686 - tn2 * t126);
-  const float t689 = 1.0f * (kmu * t687 + klam * t688);
-  sink(8, 15, t689);
-  const float t690 = (t78 - tn2 * t71 - tn1 * (t71 + t71));
-  const float t691 = 1.0f * (kmu * t690);
-  sink(9, 15, t691);
-  const float t692 = (t353 - tn2 * t44 - tn1 * (t44 + t44));
-  const float t693 = 1.0f * (kmu * t692);
-  sink(10, 15, t693);
-  const float t694 = (t368 - tn2 * t142 - tn1 * (t142 + t142));
-  const float t695 = 1.0f * (kmu * t694);
-  sink(11, 15, t695);
-  const float t696 = (t113 - tn2 * t106);
-  const float t697 = 1.0f * (kmu * t696);
-  sink(12, 15, t697);
-  const float t698 = (t368 - tn2 * t142);
-  const float t699 = 1.0f * (kmu * t698);
-  sink(13, 15, t699);
-  const float t700 = (t359 - tn2 * t59);
-  const float t701 = 1.0f * (kmu * t700);
-  sink(14, 15, t701);
-  const float t702 = (t353 - tn2 * t44 - tn1 * (t44 + t44 + t44 + t44));
-  const float t703 = (t40 - tn2 * t29) + (t353 - tn2 * t44 - tn1 * (t44 + t44 + t44 + t44)) + (t359 - tn2 * t59);
-  const float t704 = 1.0f * (kmu * t702 + klam * t703);
-  sink(15, 15, t704);
-  const float t705 = (t671 - tn2 * t81 - tn1 * (t81 + t81 + t81 + t81));
-  const float t706 = (t78 - tn2 * t71) + (t671 - tn2 * t81 - tn1 * (t81 + t81 + t81 + t81)) + (t675 - tn2 * t94);
-  const float t707 = 1.0f * (kmu * t705 + klam * t706);
-  sink(16, 15, t707);
-  const float t708 = (t682 - tn2 * t116 - tn1 * (t116 + t116 + t116 + t116));
-  const float t709 = (t113 - tn2 * t106) + (t682 - tn2 * t116 - tn1 * (t116 + t116 + t116 + t116)) + (t686 - tn2 * t126);
-  const float t710 = 1.0f * (kmu * t708 + klam * t709);
-  sink(17, 15, t710);
-  const float t711 = (t368 - tn2 * t142 - tn1 * (t142 + t142));
-  const float t712 = 1.0f * (kmu * t711);
-  sink(18, 15, t712);
-  const float t713 = (t682 - tn2 * t116 - tn1 * (t116 + t116));
-  const float t714 = 1.0f * (kmu * t713);
-  sink(19, 15, t714);
-  const float t715 = (t675 - tn2 * t94 - tn1 * (t94 + t94));
-  const float t716 = 1.0f * (kmu * t715);
-  sink(20, 15, t716);
-  const float t717 = (t359 - tn2 * t59);
-  const float t718 = (t40 - tn2 * t29) + (t353 - tn2 * t44 - tn1 * (t44 + t44 + t44 + t44)) + (t359 - tn2 * t59);
-  const float t719 = 1.0f * (kmu * t717 + klam * t718);
-  sink(21, 15, t719);
-  const float t720 = (t675 - tn2 * t94);
-  const float t721 = (t78 - tn2 * t71) + (t671 - tn2 * t81 - tn1 * (t81 + t81 + t81 + t81)) + (t675 - tn2 * t94);
-  const float t722 = 1.0f * (kmu * t720 + klam * t721);
-  sink(22, 15, t722);
-  const float t723 = (t686 - tn2 * t126);
-  const float t724 = (t113 - tn2 * t106) + (t682 - tn2 * t116 - tn1 * (t116 + t116 + t116 + t116)) + (t686 - tn2 * t126);
-  const float t725 = 1.0f * (kmu * t723 + klam * t724);
-  sink(23, 15, t725);
-  const float t726 = (t180 - tn2 * t178);
-  const float t727 = (t180 - tn2 * t178) + (t418 - tn2 * t182 - tn1 * (t182 + t182 + t182 + t182)) + (t420 - tn2 * t186);
-  const float t728 = 1.0f * (kmu * t726 + klam * t727);
-  sink(6, 16, t728);
-  const float t729 = x1 * t669 + 5.0f * t351;
-  const float t730 = a2 * t729;
-  const float t731 = x1 * t673 + 3.0f * t357;
-  const float t732 = a2 * t731;
-  const float t733 = (t195 - tn2 * t193);
-  const float t734 = (t195 - tn2 * t193) + (t730 - tn2 * t197 - tn1 * (t197 + t197 + t197 + t197)) + (t732 - tn2 * t201);
-  const float t735 = 1.0f * (kmu * t733 + klam * t734);
-  sink(7, 16, t735);
-  const float t736 = x1 * t680 + 4.0f * t366;
-  const float t737 = a2 * t736;
-  const float t738 = x1 * t684 + 2.0f * t372;
-  const float t739 = a2 * t738;
-  const float t740 = (t210 - tn2 * t208);
-  const float t741 = (t210 - tn2 * t208) + (t737 - tn2 * t212 - tn1 * (t212 + t212 + t212 + t212)) + (t739 - tn2 * t216);
-  const float t742 = 1.0f * (kmu * t740 + klam * t741);
-  sink(8, 16, t742);
-  const float t743 = (t195 - tn2 * t193 - tn1 * (t193 + t193));
-  const float t744 = 1.0f * (kmu * t743);
-  sink(9, 16, t744);
-  const float t745 = (t418 - tn2 * t182 - tn1 * (t182 + t182));
-  const float t746 = 1.0f * (kmu * t745);
-  sink(10, 16, t746);
-  const float t747 = (t425 - tn2 * t227 - tn1 * (t227 + t227));
-  const float t748 = 1.0f * (kmu * t747);
-  sink(11, 16, t748);
-  const float t749 = (t210 - tn2 * t208);
-  const float t750 = 1.0f * (kmu * t749);
-  sink(12, 16, t750);
-  const float t751 = (t425 - tn2 * t227);
-  const float t752 = 1.0f * (kmu * t751);
-  sink(13, 16, t752);
-  const float t753 = (t420 - tn2 * t186);
-  const float t754 = 1.0f * (kmu * t753);
-  sink(14, 16, t754);
-  const float t755 = (t418 - tn2 * t182 - tn1 * (t182 + t182 + t182 + t182));
-  const float t756 = (t180 - tn2 * t178) + (t418 - tn2 * t182 - tn1 * (t182 + t182 + t182 + t182)) + (t420 - tn2 * t186);
-  const float t757 = 1.0f * (kmu * t755 + klam * t756);
-  sink(15, 16, t757);
-  const float t758 = (t730 - tn2 * t197 - tn1 * (t197 + t197 + t197 + t197));
-  const float t759 = (t195 - tn2 * t193) + (t730 - tn2 * t197 - tn1 * (t197 + t197 + t197 + t197)) + (t732 - tn2 * t201);
-  const float t760 = 1.0f * (kmu * t758 + klam * t759);
-  sink(16, 16, t760);
-  const float t761 = (t737 - tn2 * t212 - tn1 * (t212 + t212 + t212 + t212));
-  const float t762 = (t210 - tn2 * t208) + (t737 - tn2 * t212 - tn1 * (t212 + t212 + t212 + t212)) + (t739 - tn2 * t216);
-  const float t763 = 1.0f * (kmu * t761 + klam * t762);
-  sink(17, 16, t763);
-  const float t764 = (t425 - tn2 * t227 - tn1 * (t227 + t227));
-  const float t765 = 1.0f * (kmu * t764);
-  sink(18, 16, t765);
-  const float t766 = (t737 - tn2 * t212 - tn1 * (t212 + t212));
-  const float t767 = 1.0f * (kmu * t766);
-  sink(19, 16, t767);
-  const float t768 = (t732 - tn2 * t201 - tn1 * (t201 + t201));
-  const float t769 = 1.0f * (kmu * t768);
-  sink(20, 16, t769);
-  const float t770 = (t420 - tn2 * t186);
-  const float t771 = (t180 - tn2 * t178) + (t418 - tn2 * t182 - tn1 * (t182 + t182 + t182 + t182)) + (t420 - tn2 * t186);
-  const float t772 = 1.0f * (kmu * t770 + klam * t771);
-  sink(21, 16, t772);
-  const float t773 = (t732 - tn2 * t201);
-  const float t774 = (t195 - tn2 * t193) + (t730 - tn2 * t197 - tn1 * (t197 + t197 + t197 + t197)) + (t732 - tn2 * t201);
-  const float t775 = 1.0f * (kmu * t773 + klam * t774);
-  sink(22, 16, t775);
-  const float t776 = (t739 - tn2 * t216);
-  const float t777 = (t210 - tn2 * t208) + (t737 - tn2 * t212 - tn1 * (t212 + t212 + t212 + t212)) + (t739 - tn2 * t216);
-  const float t778 = 1.0f * (kmu * t776 + klam * t777);
-  sink(23, 16, t778);
-  const float t779 = (t265 - tn2 * t263);
-  const float t780 = (t265 - tn2 * t263) + (t471 - tn2 * t267 - tn1 * (t267 + t267 + t267 + t267)) + (t473 - tn2 * t271);
-  const float t781 = 1.0f * (kmu * t779 + klam * t780);
-  sink(6, 17, t781);
-  const float t782 = x2 * t669;
-  const float t783 = a2 * t782;
-  const float t784 = x2 * t673 + 2.0f * t366;
-  const float t785 = a2 * t784;
-  const float t786 = (t280 - tn2 * t278);
-  const float t787 = (t280 - tn2 * t278) + (t783 - tn2 * t282 - tn1 * (t282 + t282 + t282 + t282)) + (t785 - tn2 * t286);
-  const float t788 = 1.0f * (kmu * t786 + klam * t787);
-  sink(7, 17, t788);
-  const float t789 = x2 * t680 + t351;
-  const float t790 = a2 * t789;
-  const float t791 = x2 * t684 + 3.0f * t357;
-  const float t792 = a2 * t791;
-  const float t793 = (t295 - tn2 * t293);
-  const float t794 = (t295 - tn2 * t293) + (t790 - tn2 * t297 - tn1 * (t297 + t297 + t297 + t297)) + (t792 - tn2 * t301);
-  const float t795 = 1.0f * (kmu * t793 + klam * t794);
-  sink(8, 17, t795);
-  const float t796 = (t280 - tn2 * t278 - tn1 * (t278 + t278));
-  const float t797 = 1.0f * (kmu * t796);
-  sink(9, 17, t797);
-  const float t798 = (t471 - tn2 * t267 - tn1 * (t267 + t267));
-  const float t799 = 1.0f * (kmu * t798);
-  sink(10, 17, t799);
-  const float t800 = (t478 - tn2 * t312 - tn1 * (t312 + t312));
-  const float t801 = 1.0f * (kmu * t800);
-  sink(11, 17, t801);
-  const float t802 = (t295 - tn2 * t293);
-  const float t803 = 1.0f * (kmu * t802);
-  sink(12, 17, t803);
-  const float t804 = (t478 - tn2 * t312);
-  const float t805 = 1.0f * (kmu * t804);
-  sink(13, 17, t805);
-  const float t806 = (t473 - tn2 * t271);
-  const float t807 = 1.0f * (kmu * t806);
-  sink(14, 17, t807);
-  const float t808 = (t471 - tn2 * t267 - tn1 * (t267 + t267 + t267 + t267));
-  const float t809 = (t265 - tn2 * t263) + (t471 - tn2 * t267 - tn1 * (t267 + t267 + t267 + t267)) + (t473 - tn2 * t271);
-  const float t810 = 1.0f * (kmu * t808 + klam * t809);
-  sink(15, 17, t810);
-  const float t811 = (t783 - tn2 * t282 - tn1 * (t282 + t282 + t282 + t282));
-  const float t812 = (t280 - tn2 * t278) + (t783 - tn2 * t282 - tn1 * (t282 + t282 + t282 + t282)) + (t785 - tn2 * t286);
-  const float t813 = 1.0f * (kmu * t811 + klam * t812);
-  sink(16, 17, t813);
-  const float t814 = (t790 - tn2 * t297 - tn1 * (t297 + t297 + t297 + t297));
-  const float t815 = (t295 - tn2 * t293) + (t790 - tn2 * t297 - tn1 * (t297 + t297 + t297 + t297)) + (t792 - tn2 * t301);
-  const float t816 = 1.0f * (kmu * t814 + klam * t815);
-  sink(17, 17, t816);
-  const float t817 = (t478 - tn2 * t312 - tn1 * (t312 + t312));
-  const float t818 = 1.0f * (kmu * t817);
-  sink(18, 17, t818);
-  const float t819 = (t790 - tn2 * t297 - tn1 * (t297 + t297));
-  const float t820 = 1.0f * (kmu * t819);
-  sink(19, 17, t820);
-  const float t821 = (t785 - tn2 * t286 - tn1 * (t286 + t286));
-  const float t822 = 1.0f * (kmu * t821);
-  sink(20, 17, t822);
-  const float t823 = (t473 - tn2 * t271);
-  const float t824 = (t265 - tn2 * t263) + (t471 - tn2 * t267 - tn1 * (t267 + t267 + t267 + t267)) + (t473 - tn2 * t271);
-  const float t825 = 1.0f * (kmu * t823 + klam * t824);
-  sink(21, 17, t825);
-  const float t826 = (t785 - tn2 * t286);
-  const float t827 = (t280 - tn2 * t278) + (t783 - tn2 * t282 - tn1 * (t282 + t282 + t282 + t282)) + (t785 - tn2 * t286);
-  const float t828 = 1.0f * (kmu * t826 + klam * t827);
-  sink(22, 17, t828);
-  const float t829 = (t792 - tn2 * t301);
-  const float t830 = (t295 - tn2 * t293) + (t790 - tn2 * t297 - tn1 * (t297 + t297 + t297 + t297)) + (t792 - tn2 * t301);
-  const float t831 = 1.0f * (kmu * t829 + klam * t830);
-  sink(23, 17, t831);
-  const float t832 = (t138);
-  const float t833 = (t138) + (t368 - tn1 * (t142 + t142)) + (t374 - tn1 * (t142 + t142));
-  const float t834 = 2.0f * (kmu * t832 + klam * t833);
-  sink(6, 18, t834);
-  const float t835 = (t113);
-  const float t836 = (t113) + (t682 - tn1 * (t116 + t116)) + (t686 - tn1 * (t116 + t116));
-  const float t837 = 2.0f * (kmu * t835 + klam * t836);
-  sink(7, 18, t837);
-  const float t838 = t371 * x2;
-  const float t839 = t4 * t838 + 6.0f * t13 * t85 + 3.0f * t18 * x1;
-  const float t840 = x0 * t839;
-  const float t841 = a2 * t840;
-  const float t842 = (t91);
-  const float t843 = (t91) + (t675 - tn1 * (t94 + t94)) + (t841 - tn1 * (t94 + t94));
-  const float t844 = 2.0f * (kmu * t842 + klam * t843);
-  sink(8, 18, t844);
-  const float t845 = (t113 - tn1 * (t106));
-  const float t846 = 2.0f * (kmu * t845);
-  sink(9, 18, t846);
-  const float t847 = (t368 - tn1 * (t142));
-  const float t848 = 2.0f * (kmu * t847);
-  sink(10, 18, t848);
-  const float t849 = (t359 - tn1 * (t59));
-  const float t850 = 2.0f * (kmu * t849);
-  sink(11, 18, t850);
-  const float t851 = (t91 - tn1 * (t71));
-  const float t852 = 2.0f * (kmu * t851);
-  sink(12, 18, t852);
-  const float t853 = (t359 - tn1 * (t44));
-  const float t854 = 2.0f * (kmu * t853);
-  sink(13, 18, t854);
-  const float t855 = (t374 - tn1 * (t142));
-  const float t856 = 2.0f * (kmu * t855);
-  sink(14, 18, t856);
-  const float t857 = (t368 - tn1 * (t142 + t142));
-  const float t858 = (t138) + (t368 - tn1 * (t142 + t142)) + (t374 - tn1 * (t142 + t142));
-  const float t859 = 2.0f * (kmu * t857 + klam * t858);
-  sink(15, 18, t859);
-  const float t860 = (t682 - tn1 * (t116 + t116));
-  const float t861 = (t113) + (t682 - tn1 * (t116 + t116)) + (t686 - tn1 * (t116 + t116));
-  const float t862 = 2.0f * (kmu * t860 + klam * t861);
-  sink(16, 18, t862);
-  const float t863 = (t675 - tn1 * (t94 + t94));
-  const float t864 = (t91) + (t675 - tn1 * (t94 + t94)) + (t841 - tn1 * (t94 + t94));
-  const float t865 = 2.0f * (kmu * t863 + klam * t864);
-  sink(17, 18, t865);
-  const float t866 = (t359 - tn1 * (t44 + t59));
-  const float t867 = 2.0f * (kmu * t866);
-  sink(18, 18, t867);
-  const float t868 = (t675 - tn1 * (t81 + t94));
-  const float t869 = 2.0f * (kmu * t868);
-  sink(19, 18, t869);
-  const float t870 = (t686 - tn1 * (t116 + t126));
-  const float t871 = 2.0f * (kmu * t870);
-  sink(20, 18, t871);
-  const float t872 = (t374 - tn1 * (t142 + t142));
-  const float t873 = (t138) + (t368 - tn1 * (t142 + t142)) + (t374 - tn1 * (t142 + t142));
-  const float t874 = 2.0f * (kmu * t872 + klam * t873);
-  sink(21, 18, t874);
-  const float t875 = (t686 - tn1 * (t116 + t116));
-  const float t876 = (t113) + (t682 - tn1 * (t116 + t116)) + (t686 - tn1 * (t116 + t116));
-  const float t877 = 2.0f * (kmu * t875 + klam * t876);
-  sink(22, 18, t877);
-  const float t878 = (t841 - tn1 * (t94 + t94));
-  const float t879 = (t91) + (t675 - tn1 * (t94 + t94)) + (t841 - tn1 * (t94 + t94));
-  const float t880 = 2.0f * (kmu * t878 + klam * t879);
-  sink(23, 18, t880);
-  const float t881 = (t225);
-  const float t882 = (t225) + (t425 - tn1 * (t227 + t227)) + (t427 - tn1 * (t227 + t227));
-  const float t883 = 2.0f * (kmu * t881 + klam * t882);
-  sink(6, 19, t883);
-  const float t884 = (t210);
-  const float t885 = (t210) + (t737 - tn1 * (t212 + t212)) + (t739 - tn1 * (t212 + t212));
-  const float t886 = 2.0f * (kmu * t884 + klam * t885);
-  sink(7, 19, t886);
-  const float t887 = x1 * t839 + t529;
-  const float t888 = a2 * t887;
-  const float t889 = (t199);
-  const float t890 = (t199) + (t732 - tn1 * (t201 + t201)) + (t888 - tn1 * (t201 + t201));
-  const float t891 = 2.0f * (kmu * t889 + klam * t890);
-  sink(8, 19, t891);
-  const float t892 = (t210 - tn1 * (t208));
-  const float t893 = 2.0f * (kmu * t892);
-  sink(9, 19, t893);
-  const float t894 = (t425 - tn1 * (t227));
-  const float t895 = 2.0f * (kmu * t894);
-  sink(10, 19, t895);
-  const float t896 = (t420 - tn1 * (t186));
-  const float t897 = 2.0f * (kmu * t896);
-  sink(11, 19, t897);
-  const float t898 = (t199 - tn1 * (t193));
-  const float t899 = 2.0f * (kmu * t898);
-  sink(12, 19, t899);
-  const float t900 = (t420 - tn1 * (t182));
-  const float t901 = 2.0f * (kmu * t900);
-  sink(13, 19, t901);
-  const float t902 = (t427 - tn1 * (t227));
-  const float t903 = 2.0f * (kmu * t902);
-  sink(14, 19, t903);
-  const float t904 = (t425 - tn1 * (t227 + t227));
-  const float t905 = (t225) + (t425 - tn1 * (t227 + t227)) + (t427 - tn1 * (t227 + t227));
-  const float t906 = 2.0f * (kmu * t904 + klam * t905);
-  sink(15, 19, t906);
-  const float t907 = (t737 - tn1 * (t212 + t212));
-  const float t908 = (t210) + (t737 - tn1 * (t212 + t212)) + (t739 - tn1 * (t212 + t212));
-  const float t909 = 2.0f * (kmu * t907 + klam * t908);
-  sink(16, 19, t909);
-  const float t910 = (t732 - tn1 * (t201 + t201));
-  const float t911 = (t199) + (t732 - tn1 * (t201 + t201)) + (t888 - tn1 * (t201 + t201));
-  const float t912 = 2.0f * (kmu * t910 + klam * t911);
-  sink(17, 19, t912);
-  const float t913 = (t420 - tn1 * (t182 + t186));
-  const float t914 = 2.0f * (kmu * t913);
-  sink(18, 19, t914);
-  const float t915 = (t732 - tn1 * (t197 + t201));
-  const float t916 = 2.0f * (kmu * t915);
-  sink(19, 19, t916);
-  const float t917 = (t739 - tn1 * (t212 + t216));
-  const float t918 = 2.0f * (kmu * t917);
-  sink(20, 19, t918);
-  const float t919 = (t427 - tn1 * (t227 + t227));
-  const float t920 = (t225) + (t425 - tn1 * (t227 + t227)) + (t427 - tn1 * (t227 + t227));
-  const float t921 = 2.0f * (kmu * t919 + klam * t920);
-  sink(21, 19, t921);
-  const float t922 = (t739 - tn1 * (t212 + t212));
-  const float t923 = (t210) + (t737 - tn1 * (t212 + t212)) + (t739 - tn1 * (t212 + t212));
-  const float t924 = 2.0f * (kmu * t922 + klam * t923);
-  sink(22, 19, t924);
-  const float t925 = (t888 - tn1 * (t201 + t201));
-  const float t926 = (t199) + (t732 - tn1 * (t201 + t201)) + (t888 - tn1 * (t201 + t201));
-  const float t927 = 2.0f * (kmu * t925 + klam * t926);
-  sink(23, 19, t927);
-  const float t928 = (t310);
-  const float t929 = (t310) + (t478 - tn1 * (t312 + t312)) + (t480 - tn1 * (t312 + t312));
-  const float t930 = 2.0f * (kmu * t928 + klam * t929);
-  sink(6, 20, t930);
-  const float t931 = (t295);
-  const float t932 = (t295) + (t790 - tn1 * (t297 + t297)) + (t792 - tn1 * (t297 + t297));
-  const float t933 = 2.0f * (kmu * t931 + klam * t932);
-  sink(7, 20, t933);
-  const float t934 = x2 * t839 + 4.0f * t372;
-  const float t935 = a2 * t934;
-  const float t936 = (t284);
-  const float t937 = (t284) + (t785 - tn1 * (t286 + t286)) + (t935 - tn1 * (t286 + t286));
-  const float t938 = 2.0f * (kmu * t936 + klam * t937);
-  sink(8, 20, t938);
-  const float t939 = (t295 - tn1 * (t293));
-  const float t940 = 2.0f * (kmu * t939);
-  sink(9, 20, t940);
-  const float t941 = (t478 - tn1 * (t312));
-  const float t942 = 2.0f * (kmu * t941);
-  sink(10, 20, t942);
-  const float t943 = (t473 - tn1 * (t271));
-  const float t944 = 2.0f * (kmu * t943);
-  sink(11, 20, t944);
-  const float t945 = (t284 - tn1 * (t278));
-  const float t946 = 2.0f * (kmu * t945);
-  sink(12, 20, t946);
-  const float t947 = (t473 - tn1 * (t267));
-  const float t948 = 2.0f * (kmu * t947);
-  sink(13, 20, t948);
-  const float t949 = (t480 - tn1 * (t312));
-  const float t950 = 2.0f * (kmu * t949);
-  sink(14, 20, t950);
-  const float t951 = (t478 - tn1 * (t312 + t312));
-  const float t952 = (t310) + (t478 - tn1 * (t312 + t312)) + (t480 - tn1 * (t312 + t312));
-  const float t953 = 2.0f * (kmu * t951 + klam * t952);
-  sink(15, 20, t953);
-  const float t954 = (t790 - tn1 * (t297 + t297));
-  const float t955 = (t295) + (t790 - tn1 * (t297 + t297)) + (t792 - tn1 * (t297 + t297));
-  const float t956 = 2.0f * (kmu * t954 + klam * t955);
-  sink(16, 20, t956);
-  const float t957 = (t785 - tn1 * (t286 + t286));
-  const float t958 = (t284) + (t785 - tn1 * (t286 + t286)) + (t935 - tn1 * (t286 + t286));
-  const float t959 = 2.0f * (kmu * t957 + klam * t958);
-  sink(17, 20, t959);
-  const float t960 = (t473 - tn1 * (t267 + t271));
-  const float t961 = 2.0f * (kmu * t960);
-  sink(18, 20, t961);
-  const float t962 = (t785 - tn1 * (t282 + t286));
-  const float t963 = 2.0f * (kmu * t962);
-  sink(19, 20, t963);
-  const float t964 = (t792 - tn1 * (t297 + t301));
-  const float t965 = 2.0f * (kmu * t964);
-  sink(20, 20, t965);
-  const float t966 = (t480 - tn1 * (t312 + t312));
-  const float t967 = (t310) + (t478 - tn1 * (t312 + t312)) + (t480 - tn1 * (t312 + t312));
-  const float t968 = 2.0f * (kmu * t966 + klam * t967);
-  sink(21, 20, t968);
-  const float t969 = (t792 - tn1 * (t297 + t297));
-  const float t970 = (t295) + (t790 - tn1 * (t297 + t297)) + (t792 - tn1 * (t297 + t297));
-  const float t971 = 2.0f * (kmu * t969 + klam * t970);
-  sink(22, 20, t971);
-  const float t972 = (t935 - tn1 * (t286 + t286));
-  const float t973 = (t284) + (t785 - tn1 * (t286 + t286)) + (t935 - tn1 * (t286 + t286));
-  const float t974 = 2.0f * (kmu * t972 + klam * t973);
-  sink(23, 20, t974);
-  const float t975 = (t55 - tn2 * t29);
-  const float t976 = (t55 - tn2 * t29) + (t359 - tn2 * t44) + (t531 - tn2 * t59 - tn1 * (t59 + t59 + t59 + t59));
-  const float t977 = 1.0f * (kmu * t975 + klam * t976);
-  sink(6, 21, t977);
-  const float t978 = (t91 - tn2 * t71);
-  const float t979 = (t91 - tn2 * t71) + (t675 - tn2 * t81) + (t841 - tn2 * t94 - tn1 * (t94 + t94 + t94 + t94));
-  const float t980 = 1.0f * (kmu * t978 + klam * t979);
-  sink(7, 21, t980);
-  const float t981 = t528 * x2;
-  const float t982 = t4 * t981 + 10.0f * t13 * t118 + 15.0f * t18 * x2;
-  const float t983 = x0 * t982;
-  const float t984 = a2 * t983;
-  const float t985 = (t123 - tn2 * t106);
-  const float t986 = (t123 - tn2 * t106) + (t686 - tn2 * t116) + (t984 - tn2 * t126 - tn1 * (t126 + t126 + t126 + t126));
-  const float t987 = 1.0f * (kmu * t985 + klam * t986);
-  sink(8, 21, t987);
-  const float t988 = (t91 - tn2 * t71);
-  const float t989 = 1.0f * (kmu * t988);
-  sink(9, 21, t989);
-  const float t990 = (t359 - tn2 * t44);
-  const float t991 = 1.0f * (kmu * t990);
-  sink(10, 21, t991);
-  const float t992 = (t374 - tn2 * t142);
-  const float t993 = 1.0f * (kmu * t992);
-  sink(11, 21, t993);
-  const float t994 = (t123 - tn2 * t106 - tn1 * (t106 + t106));
-  const float t995 = 1.0f * (kmu * t994);
-  sink(12, 21, t995);
-  const float t996 = (t374 - tn2 * t142 - tn1 * (t142 + t142));
-  const float t997 = 1.0f * (kmu * t996);
-  sink(13, 21, t997);
-  const float t998 = (t531 - tn2 * t59 - tn1 * (t59 + t59));
-  const float t999 = 1.0f * (kmu * t998);
-  sink(14, 21, t999);
-  const float t1000 = (t359 - tn2 * t44);
-  const float t1001 = (t55 - tn2 * t29) + (t359 - tn2 * t44) + (t531 - tn2 * t59 - tn1 * (t59 + t59 + t59 + t59));
-  const float t1002 = 1.0f * (kmu * t1000 + klam * t1001);
-  sink(15, 21, t1002);
-  const float t1003 = (t675 - tn2 * t81);
-  const float t1004 = (t91 - tn2 * t71) + (t675 - tn2 * t81) + (t841 - tn2 * t94 - tn1 * (t94 + t94 + t94 + t94));
-  const float t1005 = 1.0f * (kmu * t1003 + klam * t1004);
-  sink(16, 21, t1005);
-  const float t1006 = (t686 - tn2 * t116);
-  const float t1007 = (t123 - tn2 * t106) + (t686 - tn2 * t116) + (t984 - tn2 * t126 - tn1 * (t126 + t126 + t126 + t126));
-  const float t1008 = 1.0f * (kmu * t1006 + klam * t1007);
-  sink(17, 21, t1008);
-  const float t1009 = (t374 - tn2 * t142 - tn1 * (t142 + t142));
-  const float t1010 = 1.0f * (kmu * t1009);
-  sink(18, 21, t1010);
-  const float t1011 = (t686 - tn2 * t116 - tn1 * (t116 + t116));
-  const float t1012 = 1.0f * (kmu * t1011);
-  sink(19, 21, t1012);
-  const float t1013 = (t841 - tn2 * t94 - tn1 * (t94 + t94));
-  const float t1014 = 1.0f * (kmu * t1013);
-  sink(20, 21, t1014);
-  const float t1015 = (t531 - tn2 * t59 - tn1 * (t59 + t59 + t59 + t59));
-  const float t1016 = (t55 - tn2 * t29) + (t359 - tn2 * t44) + (t531 - tn2 * t59 - tn1 * (t59 + t59 + t59 + t59));
-  const float t1017 = 1.0f * (kmu * t1015 + klam * t1016);
-  sink(21, 21, t1017);
-  const float t1018 = (t841 - tn2 * t94 - tn1 * (t94 + t94 + t94 + t94));
-  const float t1019 = (t91 - tn2 * t71) + (t675 - tn2 * t81) + (t841 - tn2 * t94 - tn1 * (t94 + t94 + t94 + t94));
-  const float t1020 = 1.0f * (kmu * t1018 + klam * t1019);
-  sink(22, 21, t1020);
-  const float t1021 = (t984 - tn2 * t126 - tn1 * (t126 + t126 + t126 + t126));
-  const float t1022 = (t123 - tn2 * t106) + (t686 - tn2 * t116) + (t984 - tn2 * t126 - tn1 * (t126 + t126 + t126 + t126));
-  const float t1023 = 1.0f * (kmu * t1021 + klam * t1022);
-  sink(23, 21, t1023);
-  const float t1024 = (t184 - tn2 * t178);
-  const float t1025 = (t184 - tn2 * t178) + (t420 - tn2 * t182) + (t578 - tn2 * t186 - tn1 * (t186 + t186 + t186 + t186));
-  const float t1026 = 1.0f * (kmu * t1024 + klam * t1025);
-  sink(6, 22, t1026);
-  const float t1027 = (t199 - tn2 * t193);
-  const float t1028 = (t199 - tn2 * t193) + (t732 - tn2 * t197) + (t888 - tn2 * t201 - tn1 * (t201 + t201 + t201 + t201));
-  const float t1029 = 1.0f * (kmu * t1027 + klam * t1028);
-  sink(7, 22, t1029);
-  const float t1030 = x1 * t982;
-  const float t1031 = a2 * t1030;
-  const float t1032 = (t214 - tn2 * t208);
-  const float t1033 = (t214 - tn2 * t208) + (t739 - tn2 * t212) + (t1031 - tn2 * t216 - tn1 * (t216 + t216 + t216 + t216));
-  const float t1034 = 1.0f * (kmu * t1032 + klam * t1033);
-  sink(8, 22, t1034);
-  const float t1035 = (t199 - tn2 * t193);
-  const float t1036 = 1.0f * (kmu * t1035);
-  sink(9, 22, t1036);
-  const float t1037 = (t420 - tn2 * t182);
-  const float t1038 = 1.0f * (kmu * t1037);
-  sink(10, 22, t1038);
-  const float t1039 = (t427 - tn2 * t227);
-  const float t1040 = 1.0f * (kmu * t1039);
-  sink(11, 22, t1040);
-  const float t1041 = (t214 - tn2 * t208 - tn1 * (t208 + t208));
-  const float t1042 = 1.0f * (kmu * t1041);
-  sink(12, 22, t1042);
-  const float t1043 = (t427 - tn2 * t227 - tn1 * (t227 + t227));
-  const float t1044 = 1.0f * (kmu * t1043);
-  sink(13, 22, t1044);
-  const float t1045 = (t578 - tn2 * t186 - tn1 * (t186 + t186));
-  const float t1046 = 1.0f * (kmu * t1045);
-  sink(14, 22, t1046);
-  const float t1047 = (t420 - tn2 * t182);
-  const float t1048 = (t184 - tn2 * t178) + (t420 - tn2 * t182) + (t578 - tn2 * t186 - tn1 * (t186 + t186 + t186 + t186));
-  const float t1049 = 1.0f * (kmu * t1047 + klam * t1048);
-  sink(15, 22, t1049);
-  const float t1050 = (t732 - tn2 * t197);
-  const float t1051 = (t199 - tn2 * t193) + (t732 - tn2 * t197) + (t888 - tn2 * t201 - tn1 * (t201 + t201 + t201 + t201));
-  const float t1052 = 1.0f * (kmu * t1050 + klam * t1051);
-  sink(16, 22, t1052);
-  const float t1053 = (t739 - tn2 * t212);
-  const float t1054 = (t214 - tn2 * t208) + (t739 - tn2 * t212) + (t1031 - tn2 * t216 - tn1 * (t216 + t216 + t216 + t216));
-  const float t1055 = 1.0f * (kmu * t1053 + klam * t1054);
-  sink(17, 22, t1055);
-  const float t1056 = (t427 - tn2 * t227 - tn1 * (t227 + t227));
-  const float t1057 = 1.0f * (kmu * t1056);
-  sink(18, 22, t1057);
-  const float t1058 = (t739 - tn2 * t212 - tn1 * (t212 + t212));
-  const float t1059 = 1.0f * (kmu * t1058);
-  sink(19, 22, t1059);
-  const float t1060 = (t888 - tn2 * t201 - tn1 * (t201 + t201));
-  const float t1061 = 1.0f * (kmu * t1060);
-  sink(20, 22, t1061);
-  const float t1062 = (t578 - tn2 * t186 - tn1 * (t186 + t186 + t186 + t186));
-  const float t1063 = (t184 - tn2 * t178) + (t420 - tn2 * t182) + (t578 - tn2 * t186 - tn1 * (t186 + t186 + t186 + t186));
-  const float t1064 = 1.0f * (kmu * t1062 + klam * t1063);
-  sink(21, 22, t1064);
-  const float t1065 = (t888 - tn2 * t201 - tn1 * (t201 + t201 + t201 + t201));
-  const float t1066 = (t199 - tn2 * t193) + (t732 - tn2 * t197) + (t888 - tn2 * t201 - tn1 * (t201 + t201 + t201 + t201));
-  const float t1067 = 1.0f * (kmu * t1065 + klam * t1066);
-  sink(22, 22, t1067);
-  const float t1068 = (t1031 - tn2 * t216 - tn1 * (t216 + t216 + t216 + t216));
-  const float t1069 = (t214 - tn2 * t208) + (t739 - tn2 * t212) + (t1031 - tn2 * t216 - tn1 * (t216 + t216 + t216 + t216));
-  const float t1070 = 1.0f * (kmu * t1068 + klam * t1069);
-  sink(23, 22, t1070);
-  const float t1071 = (t269 - tn2 * t263);
-  const float t1072 = (t269 - tn2 * t263) + (t473 - tn2 * t267) + (t625 - tn2 * t271 - tn1 * (t271 + t271 + t271 + t271));
-  const float t1073 = 1.0f * (kmu * t1071 + klam * t1072);
-  sink(6, 23, t1073);
-  const float t1074 = (t284 - tn2 * t278);
-  const float t1075 = (t284 - tn2 * t278) + (t785 - tn2 * t282) + (t935 - tn2 * t286 - tn1 * (t286 + t286 + t286 + t286));
-  const float t1076 = 1.0f * (kmu * t1074 + klam * t1075);
-  sink(7, 23, t1076);
-  const float t1077 = x2 * t982 + 5.0f * t529;
-  const float t1078 = a2 * t1077;
-  const float t1079 = (t299 - tn2 * t293);
-  const float t1080 = (t299 - tn2 * t293) + (t792 - tn2 * t297) + (t1078 - tn2 * t301 - tn1 * (t301 + t301 + t301 + t301));
-  const float t1081 = 1.0f * (kmu * t1079 + klam * t1080);
-  sink(8, 23, t1081);
-  const float t1082 = (t284 - tn2 * t278);
-  const float t1083 = 1.0f * (kmu * t1082);
-  sink(9, 23, t1083);
-  const float t1084 = (t473 - tn2 * t267);
-  const float t1085 = 1.0f * (kmu * t1084);
-  sink(10, 23, t1085);
-  const float t1086 = (t480 - tn2 * t312);
-  const float t1087 = 1.0f * (kmu * t1086);
-  sink(11, 23, t1087);
-  const float t1088 = (t299 - tn2 * t293 - tn1 * (t293 + t293));
-  const float t1089 = 1.0f * (kmu * t1088);
-  sink(12, 23, t1089);
-  const float t1090 = (t480 - tn2 * t312 - tn1 * (t312 + t312));
-  const float t1091 = 1.0f * (kmu * t1090);
-  sink(13, 23, t1091);
-  const float t1092 = (t625 - tn2 * t271 - tn1 * (t271 + t271));
-  const float t1093 = 1.0f * (kmu * t1092);
-  sink(14, 23, t1093);
-  const float t1094 = (t473 - tn2 * t267);
-  const float t1095 = (t269 - tn2 * t263) + (t473 - tn2 * t267) + (t625 - tn2 * t271 - tn1 * (t271 + t271 + t271 + t271));
-  const float t1096 = 1.0f * (kmu * t1094 + klam * t1095);
-  sink(15, 23, t1096);
-  const float t1097 = (t785 - tn2 * t282);
-  const float t1098 = (t284 - tn2 * t278) + (t785 - tn2 * t282) + (t935 - tn2 * t286 - tn1 * (t286 + t286 + t286 + t286));
-  const float t1099 = 1.0f * (kmu * t1097 + klam * t1098);
-  sink(16, 23, t1099);
-  const float t1100 = (t792 - tn2 * t297);
-  const float t1101 = (t299 - tn2 * t293) + (t792 - tn2 * t297) + (t1078 - tn2 * t301 - tn1 * (t301 + t301 + t301 + t301));
-  const float t1102 = 1.0f * (kmu * t1100 + klam * t1101);
-  sink(17, 23, t1102);
-  const float t1103 = (t480 - tn2 * t312 - tn1 * (t312 + t312));
-  const float t1104 = 1.0f * (kmu * t1103);
-  sink(18, 23, t1104);
-  const float t1105 = (t792 - tn2 * t297 - tn1 * (t297 + t297));
-  const float t1106 = 1.0f * (kmu * t1105);
-  sink(19, 23, t1106);
-  const float t1107 = (t935 - tn2 * t286 - tn1 * (t286 + t286));
-  const float t1108 = 1.0f * (kmu * t1107);
-  sink(20, 23, t1108);
-  const float t1109 = (t625 - tn2 * t271 - tn1 * (t271 + t271 + t271 + t271));
-  const float t1110 = (t269 - tn2 * t263) + (t473 - tn2 * t267) + (t625 - tn2 * t271 - tn1 * (t271 + t271 + t271 + t271));
-  const float t1111 = 1.0f * (kmu * t1109 + klam * t1110);
-  sink(21, 23, t1111);
-  const float t1112 = (t935 - tn2 * t286 - tn1 * (t286 + t286 + t286 + t286));
-  const float t1113 = (t284 - tn2 * t278) + (t785 - tn2 * t282) + (t935 - tn2 * t286 - tn1 * (t286 + t286 + t286 + t286));
-  const float t1114 = 1.0f * (kmu * t1112 + klam * t1113);
-  sink(22, 23, t1114);
-  const float t1115 = (t1078 - tn2 * t301 - tn1 * (t301 + t301 + t301 + t301));
-  const float t1116 = (t299 - tn2 * t293) + (t792 - tn2 * t297) + (t1078 - tn2 * t301 - tn1 * (t301 + t301 + t301 + t301));
-  const float t1117 = 1.0f * (kmu * t1115 + klam * t1116);
-  sink(23, 23, t1117);
-}
 
 template <class Sink>
 IBEM_HD IBEM_INLINE void sph_self24f(const SphMatF& mc, Sink& sink) {

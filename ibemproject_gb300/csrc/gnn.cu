@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "mf.h"
+#include "mf_contract.cuh"
 #include "prof.h"
 
 namespace ibem {
@@ -195,42 +196,49 @@ __global__ void k_features(int num, const int* __restrict__ seg_of, const MatFea
 }
 
 // ---------------------------------------------------------------- edge corrections
-struct SmemSink {
-  float* M;
-  float scale;
-  __device__ __forceinline__ void operator()(int r, int c, float v) const { M[r * kMfNu + c] = v * scale; }
-};
-
-// C = sc * A B for 24 x 24 row-major matrices in shared memory; 64 threads, each a 3 x 3
-// register tile (rows 3 (t / 8) .., columns 3 (t % 8) ..): 6 shared loads per 9 FMAs
+// C = sc * A B for 24 x 24 row-major matrices in shared memory; threads 0 to 47, each a 3 x 4
+// register tile (rows 3 (t / 6) .., columns 4 (t % 6) ..): per 4 steps of k 3 + 4 wide loads
+// and 48 FMAs (with 3 x 3 tiles and one-word loads 24 and 36: bound by the shared loads)
 __device__ __forceinline__ void mm24(const float* A, const float* B, float* C, float sc) {
-  const int tr = 3 * (threadIdx.x >> 3), tc = 3 * (threadIdx.x & 7);
-  float acc[3][3] = {};
-#pragma unroll 4
-  for (int k = 0; k < kMfNu; ++k) {
-    float a[3], b[3];
+  if (threadIdx.x >= 48) return;
+  const int tr = 3 * (threadIdx.x / 6), tc = 4 * (threadIdx.x % 6);
+  float acc[3][4] = {};
 #pragma unroll
-    for (int i = 0; i < 3; ++i) a[i] = A[(tr + i) * kMfNu + k];
+  for (int k = 0; k < kMfNu; k += 4) {
+    float4 a[3], b[4];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) b[j] = B[k * kMfNu + tc + j];
+    for (int i = 0; i < 3; ++i) a[i] = *reinterpret_cast<const float4*>(A + (tr + i) * kMfNu + k);
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
+    for (int q = 0; q < 4; ++q) b[q] = *reinterpret_cast<const float4*>(B + (k + q) * kMfNu + tc);
 #pragma unroll
-      for (int j = 0; j < 3; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+    for (int i = 0; i < 3; ++i) {
+      const float av[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        acc[i][0] = fmaf(av[q], b[q].x, acc[i][0]);
+        acc[i][1] = fmaf(av[q], b[q].y, acc[i][1]);
+        acc[i][2] = fmaf(av[q], b[q].z, acc[i][2]);
+        acc[i][3] = fmaf(av[q], b[q].w, acc[i][3]);
+      }
+    }
   }
 #pragma unroll
   for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) C[(tr + i) * kMfNu + tc + j] = sc * acc[i][j];
+    *reinterpret_cast<float4*>(C + (tr + i) * kMfNu + tc) =
+        make_float4(sc * acc[i][0], sc * acc[i][1], sc * acc[i][2], sc * acc[i][3]);
 }
 
+// One CTA per edge: the two pair blocks, then four 24 x 24 products.  48 threads form a column
+// of a block each by the pair contraction of a unit vector (~570 FP32 instructions on two
+// warps; eight threads generating the sub-blocks, four code paths of ~8,000 instructions in one
+// warp: 1.02 ms for 67,000 edges, 0.40 ms now).
 __global__ void __launch_bounds__(64)
     k_edge_corr(int num, const int* __restrict__ nbr, const int* __restrict__ seg_of, const SphMatF* __restrict__ mats,
                 const double* __restrict__ cen, const double* __restrict__ rad, const float* __restrict__ B,
                 const float* __restrict__ wa, float* __restrict__ D, float* __restrict__ Q, int nrhs,
                 const float* __restrict__ rq, int64_t N, float* __restrict__ u) {
-  __shared__ float Aij[kMfNu * kMfNu], Aji[kMfNu * kMfNu], Bi[kMfNu * kMfNu], Bj[kMfNu * kMfNu];
-  __shared__ float T1[kMfNu * kMfNu], T2[kMfNu * kMfNu];
+  __shared__ __align__(16) float Aij[kMfNu * kMfNu], Aji[kMfNu * kMfNu], Bi[kMfNu * kMfNu], Bj[kMfNu * kMfNu];
+  __shared__ __align__(16) float T1[kMfNu * kMfNu], T2[kMfNu * kMfNu];
   const int64_t e = blockIdx.x;
   const int64_t E = (int64_t)num * kKnn;
   const int i = (int)(e / kKnn);
@@ -247,21 +255,23 @@ __global__ void __launch_bounds__(64)
     Bi[k] = bi[k];
     Bj[k] = bj[k];
   }
-  if (threadIdx.x < 8) {  // 8 generators: 4 sub-blocks (column order x row order) of each block
+  if (threadIdx.x < 2 * kMfNu) {
     const SphMatF mc = mats[seg_of[i]];
-    const bool ij = threadIdx.x < 4;  // As_ij: target i, source j; As_ji: target j, source i
-    const int fn = threadIdx.x & 3;
+    const bool ij = threadIdx.x < kMfNu;  // As_ij: target i, source j; As_ji: target j, source i
+    const int col = ij ? threadIdx.x : threadIdx.x - kMfNu;
     const int tgt = ij ? i : j, src = ij ? j : i;
     const double ia = 1.0 / rad[src];
     const float x0 = (float)((cen[3 * (int64_t)tgt] - cen[3 * (int64_t)src]) * ia);
     const float x1 = (float)((cen[3 * (int64_t)tgt + 1] - cen[3 * (int64_t)src + 1]) * ia);
     const float x2 = (float)((cen[3 * (int64_t)tgt + 2] - cen[3 * (int64_t)src + 2]) * ia);
-    float* M = ij ? Aij : Aji;
-    SmemSink sk{M, fn >= 2 ? (float)(rad[tgt] * ia) : 1.f};   // rows of order 1 carry a_tgt / a_src
-    if (fn == 0) sph_block24f_c0_r0(x0, x1, x2, 1.f, mc, sk);
-    else if (fn == 1) sph_block24f_c1_r0(x0, x1, x2, 1.f, mc, sk);
-    else if (fn == 2) sph_block24f_c0_r1(x0, x1, x2, 1.f, mc, sk);
-    else sph_block24f_c1_r1(x0, x1, x2, 1.f, mc, sk);
+    float x[kMfNu], y[kMfNu] = {};
+#pragma unroll
+    for (int r = 0; r < kMfNu; ++r) x[r] = r == col ? 1.f : 0.f;
+    // rows of order 1 carry a_tgt / a_src
+    sph_pair_apply24<float>(x0, x1, x2, 1.f, mc.kmu, mc.klam, mc.tn1, mc.tn2, x, (float)(rad[tgt] * ia), y);
+    float* M = (ij ? Aij : Aji) + col;
+#pragma unroll
+    for (int r = 0; r < kMfNu; ++r) M[r * kMfNu] = y[r];
   }
   __syncthreads();
   mm24(Aji, Bi, T1, 1.f);    // As_ji B_i

@@ -400,49 +400,63 @@ __global__ void k_mf_prep(int nu, int num, const double* __restrict__ cen, const
 }
 
 // Scaled diagonal block (FP64, x = 0, unit sphere, moduli / mu0) inverted by Gauss-Jordan
-// with partial pivoting; one CTA of 32 threads per realisation: in the scaled system a
-// sphere's own block depends on the materials only, so every sphere of a realisation shares
-// it (k_bcast_blocks copies it to each).
-__global__ void __launch_bounds__(32) k_block_jacobi(const SphMat* __restrict__ mats, float* __restrict__ P) {
+// with partial pivoting; one CTA per realisation: in the scaled system a sphere's own block
+// depends on the materials only, so every sphere of a realisation shares it (k_bcast_blocks
+// copies it to each).  One CTA's latency bounds it: 64 clocks per dependent-free FP64
+// multiply-add and warp.  24 threads form a column each by the pair contraction (~750
+// operations; one thread generating the block, ~6,000, and 32 threads eliminating: 133 us),
+// four warps eliminate: 56 us.
+constexpr int kBjThreads24 = 128;
+__global__ void __launch_bounds__(kBjThreads24) k_block_jacobi(const SphMat* __restrict__ mats, float* __restrict__ P) {
   __shared__ double M[kMfNu][2 * kMfNu + 1];
   const int p = blockIdx.x;   // realisation
   const int t = threadIdx.x;
-  for (int i = t; i < kMfNu * 2 * kMfNu; i += 32) {
-    const int r = i / (2 * kMfNu), c = i % (2 * kMfNu);
-    M[r][c] = (c >= kMfNu && c - kMfNu == r) ? 1.0 : 0.0;
+  SphMat mc = mats[p];
+  const double sc = 1.0 / mc.mu0;
+  mc.kmu *= sc;
+  mc.klam *= sc;
+  mc.lam0 *= sc;
+  mc.mu0 = 1.0;
+  if (t < kMfNu) {
+    double e[kMfNu], y[kMfNu] = {};
+#pragma unroll
+    for (int r = 0; r < kMfNu; ++r) {
+      e[r] = r == t ? 1.0 : 0.0;
+      M[r][kMfNu + t] = e[r];
+    }
+    sph_pair_apply24<double>(0.0, 0.0, 0.0, 1.0, mc.kmu, mc.klam, mc.tn1, mc.tn2, e, 1.0, y);
+#pragma unroll
+    for (int r = 0; r < kMfNu; ++r) M[r][t] = y[r];
   }
   __syncthreads();
   if (t == 0) {
-    SphMat mc = mats[p];
-    const double s = 1.0 / mc.mu0;
-    mc.kmu *= s;
-    mc.klam *= s;
-    mc.lam0 *= s;
-    mc.mu0 = 1.0;
     struct Put {
       double (*M)[2 * kMfNu + 1];
       __device__ void operator()(int r, int c, double v) const { M[r][c] += v; }
     } put{M};
-    sph_block24_c0_r0(0.0, 0.0, 0.0, 1.0, mc, put);
-    sph_block24_c1_r0(0.0, 0.0, 0.0, 1.0, mc, put);
-    sph_block24_c0_r1(0.0, 0.0, 0.0, 1.0, mc, put);
-    sph_block24_c1_r1(0.0, 0.0, 0.0, 1.0, mc, put);
     sph_self24(mc, put);
   }
   __syncthreads();
   __shared__ int piv;
   __shared__ double f[kMfNu];
   for (int k = 0; k < kMfNu; ++k) {
-    if (t == 0) {
-      int best = k;
-      for (int r = k + 1; r < kMfNu; ++r)
-        if (fabs(M[r][k]) > fabs(M[best][k])) best = r;
-      piv = best;
+    if (t < 32) {   // the first of the largest entries
+      double v = t >= k && t < kMfNu ? fabs(M[t][k]) : -1.0;
+      int r = t;
+      for (int o = 16; o; o >>= 1) {
+        const double vo = __shfl_xor_sync(0xffffffffu, v, o);
+        const int ro = __shfl_xor_sync(0xffffffffu, r, o);
+        if (vo > v || (vo == v && ro < r)) {
+          v = vo;
+          r = ro;
+        }
+      }
+      if (t == 0) piv = min(r, kMfNu - 1);
     }
     __syncthreads();
     const int pr = piv;
     if (pr != k)
-      for (int c = t; c < 2 * kMfNu; c += 32) {
+      for (int c = t; c < 2 * kMfNu; c += kBjThreads24) {
         const double v = M[k][c];
         M[k][c] = M[pr][c];
         M[pr][c] = v;
@@ -451,17 +465,17 @@ __global__ void __launch_bounds__(32) k_block_jacobi(const SphMat* __restrict__ 
     const double d = M[k][k];
     const double id = d != 0.0 ? 1.0 / d : 0.0;
     __syncthreads();
-    for (int c = t; c < 2 * kMfNu; c += 32) M[k][c] *= id;
+    for (int c = t; c < 2 * kMfNu; c += kBjThreads24) M[k][c] *= id;
     if (t < kMfNu) f[t] = M[t][k];  // column k of the other rows (row k is being scaled, unused)
     __syncthreads();
-    for (int i = t; i < kMfNu * 2 * kMfNu; i += 32) {
+    for (int i = t; i < kMfNu * 2 * kMfNu; i += kBjThreads24) {
       const int r = i / (2 * kMfNu), c = i % (2 * kMfNu);
       if (r != k) M[r][c] -= f[r] * M[k][c];
     }
     __syncthreads();
   }
   float* o = P + (int64_t)kMfNu * kMfNu * p;
-  for (int i = t; i < kMfNu * kMfNu; i += 32) o[i] = (float)M[i / kMfNu][kMfNu + i % kMfNu];
+  for (int i = t; i < kMfNu * kMfNu; i += kBjThreads24) o[i] = (float)M[i / kMfNu][kMfNu + i % kMfNu];
 }
 
 // P[p] = Pseg[seg_of[p]] (24 x 24 blocks, float4 copies)
@@ -1191,7 +1205,7 @@ ibem_status mf_apply_df(const MfBatch& b, const double* x, double* y, cudaStream
 ibem_status mf_block_jacobi(const MfBatch& b, float* P, cudaStream_t st) {
   float* Pseg = nullptr;
   IBEM_CUDA(alloc_async((void**)&Pseg, sizeof(float) * kMfNu * kMfNu * (size_t)b.nseg, st));
-  ::ibem::count_launch(), k_block_jacobi<<<b.nseg, 32, 0, st>>>(b.matd, Pseg);
+  ::ibem::count_launch(), k_block_jacobi<<<b.nseg, kBjThreads24, 0, st>>>(b.matd, Pseg);
   ::ibem::count_launch(), k_bcast_blocks<<<nblk((int64_t)b.num * kMfNu * kMfNu / 4), 256, 0, st>>>(b.num, b.seg_of, Pseg, P);
   free_async(Pseg, st);
   IBEM_LAUNCH_CHECK("block jacobi");
