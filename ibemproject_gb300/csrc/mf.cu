@@ -124,8 +124,8 @@ __global__ void __launch_bounds__(TT)
                    const SphMatF* __restrict__ mats, const float* __restrict__ x, float* __restrict__ y) {
   __shared__ float4 sgh[kMfChunk], sgl[kMfChunk];
   __shared__ float sx[kMfChunk * kMfNu];
-  mf_f32_item<TT>(tiles[blockIdx.x], blockIdx.y, gridDim.y, seg_begin, mask, mask_on, gh, gl, mats, x, y, sgh, sgl,
-                  sx);
+  mf_f32_item<TT>(tiles[blockIdx.x], blockIdx.y * gridDim.z + blockIdx.z, gridDim.y * gridDim.z,
+                  seg_begin, mask, mask_on, gh, gl, mats, x, y, sgh, sgl, sx);
 }
 
 // persistent form: as many CTAs as fit on the GPU at once walk a work list of (tile,
@@ -190,11 +190,11 @@ __device__ __forceinline__ bool source_is_far(const double* wlo, const double* w
   const double lim = __dmul_rn(kMfFarRadii, r);
   return d2 > __dmul_rn(lim, lim);
 }
-// The sources of one CTA (blockIdx.y of gridDim.y slices), in chunks of kMfChunk: chunk j
+// The sources of one CTA (piece blockIdx.z of slice blockIdx.y), in chunks of kMfChunk: chunk j
 // starts at first + j * step and ends at end at the latest.  The full product (mode 0) takes
-// a contiguous range of the realisation; the split ones take every gridDim.y-th chunk from
-// blockIdx.y.  In Morton order the near sources of a tile sit in a few neighbouring chunks:
-// dealt out in turn, every CTA gets about the average share of them.
+// a contiguous range of the realisation; the split ones deal the chunks
+// out to the CTAs in turn.  In Morton order the near sources of a tile sit in a few neighbouring chunks:
+// this way every CTA gets about the average share of them.
 struct MfSlice {
   int first, step, end;
   __device__ __forceinline__ bool holds(int p) const {
@@ -202,7 +202,7 @@ struct MfSlice {
   }
 };
 __device__ __forceinline__ MfSlice mf_slice(int hb0, int he0, int mode) {
-  const int k = blockIdx.y, ns = gridDim.y;
+  const int k = blockIdx.y * gridDim.z + blockIdx.z, ns = gridDim.y * gridDim.z;
   if (mode) return {hb0 + kMfChunk * k, kMfChunk * ns, he0};
   const int per = (he0 - hb0 + ns - 1) / ns;
   const int hb = hb0 + k * per;
@@ -789,12 +789,18 @@ inline unsigned nblk(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t
 
 }  // namespace
 
-// Most source slices of a product: 8 sources each.  A thread takes a slice's sources one after
-// the other (64 clocks per FP64 multiply-add and warp), so in a small realisation the slice is
-// the product's latency: 64 spheres with slices of 32 and of 8 sources, FP64 product 570 us
-// and 156 us, FP32 product 25 and 13 us.
-static int slice_cap(int max_seg) { return std::max(1, (max_seg + 7) / 8); }
+// Source slices of a product hold at least 32 sources.  Where that leaves too few CTAs, a slice
+// is cut into up to kMfPieces pieces (gridDim.z): a thread takes its sources one after the other
+// (64 clocks per FP64 multiply-add and warp), so in a small realisation the slice is the
+// product's latency: 64 spheres with one and with four pieces a slice (32 and 8 sources), FP64
+// product 570 us and 156 us, FP32 product 25 and 13 us.
+static int slice_cap(int max_seg) { return std::max(1, (max_seg + 31) / 32); }
 
+static MfSplit mf_split(int ctas, int max_seg) {
+  const int cap = slice_cap(max_seg);
+  const int pieces = std::max(1, std::min(kMfPieces, (ctas + cap - 1) / cap));
+  return {std::max(1, std::min(cap, (ctas + pieces - 1) / pieces)), pieces};
+}
 
 // ------------------------------------------------------------------ batch set-up
 ibem_status mf_batch_init(MfBatch& b, const ibem_e3d_batch& in, cudaStream_t st, int layout) {
@@ -839,8 +845,7 @@ ibem_status mf_batch_init(MfBatch& b, const ibem_e3d_batch& in, cudaStream_t st,
   IBEM_CUDA(cudaGetDevice(&dev));
   IBEM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const int want = std::max(1, nsm) * 4;
-  b.hsplit = std::max(1, std::min((want + b.ntiles - 1) / b.ntiles, slice_cap(b.max_seg)));
-  b.hsplit_wide = b.hsplit;
+  b.split = b.split_wide = mf_split((want + b.ntiles - 1) / b.ntiles, b.max_seg);
   std::vector<SphMat> md(in.nseg), ms(in.nseg);
   std::vector<SphMatF> mf(in.nseg);
   for (int s = 0; s < in.nseg; ++s) {
@@ -945,9 +950,10 @@ void mf_batch_free(MfBatch& b) {
   b = MfBatch();
 }
 
-ibem_status mf_set_f32_shape(MfBatch& b, int tshape, int hsplit, int persist, cudaStream_t st) {
+ibem_status mf_set_f32_shape(MfBatch& b, int tshape, MfSplit split, int persist, cudaStream_t st) {
+  const int hsplit = split.slices;
   b.tshape = tshape;
-  b.hsplit = hsplit;
+  b.split = split;
   b.persist = persist;
   if (!persist) return IBEM_OK;
   // work list: every (tile, slice) with sources, by decreasing targets x sources
@@ -1009,7 +1015,8 @@ struct TuneKey {
   }
 };
 struct TuneVal {
-  int hsplit, hsplit_wide, tshape, persist;
+  MfSplit split, split_wide;
+  int tshape, persist;
 };
 std::mutex g_tune_mu;
 std::map<TuneKey, TuneVal> g_tune;
@@ -1019,12 +1026,11 @@ int log2_bucket(int v) {
   while ((1 << b) < v) ++b;
   return b;
 }
-// slice counts that give 1, 2, 4 and 8 CTAs per SM in total
-std::vector<int> slice_candidates(int ntiles, int max_seg, int sms) {
-  const int cap = slice_cap(max_seg);
-  std::vector<int> cand;
+// splits of the source range that give 1, 2, 4 and 8 CTAs per SM in total
+std::vector<MfSplit> split_candidates(int ntiles, int max_seg, int sms) {
+  std::vector<MfSplit> cand;
   for (int per_sm : {1, 2, 4, 8}) {
-    const int h = std::max(1, std::min(cap, (sms * per_sm + ntiles - 1) / ntiles));
+    const MfSplit h = mf_split((sms * per_sm + ntiles - 1) / ntiles, max_seg);
     if (std::find(cand.begin(), cand.end(), h) == cand.end()) cand.push_back(h);
   }
   return cand;
@@ -1042,7 +1048,7 @@ ibem_status mf_tune(MfBatch& b, cudaStream_t st) {
   if (const char* f = b.nu == 24 ? std::getenv("IBEM_MF_F32_SHAPE") : nullptr) {
     int ts = 1, pers = 0, h = 1;
     if (std::sscanf(f, "%d,%d,%d", &ts, &pers, &h) == 3 && ts >= 0 && ts < 3 && (pers == 0 || pers == 1) && h >= 1)
-      return mf_set_f32_shape(b, ts, std::min(h, cap), pers, st);
+      return mf_set_f32_shape(b, ts, {std::min(h, cap), 1}, pers, st);
     return fail(IBEM_ERR_ARG, "IBEM_MF_F32_SHAPE: expected shape (0-2),persistent (0/1),slices (>= 1)");
   }
   {
@@ -1057,8 +1063,8 @@ ibem_status mf_tune(MfBatch& b, cudaStream_t st) {
       }
     }
     if (hit) {
-      b.hsplit_wide = std::min(v.hsplit_wide, cap);
-      return mf_set_f32_shape(b, v.tshape, std::min(v.hsplit, cap), v.persist, st);
+      b.split_wide = {std::min(v.split_wide.slices, cap), v.split_wide.pieces};
+      return mf_set_f32_shape(b, v.tshape, {std::min(v.split.slices, cap), v.split.pieces}, v.persist, st);
     }
   }
   float* xf = nullptr;
@@ -1091,33 +1097,34 @@ ibem_status mf_tune(MfBatch& b, cudaStream_t st) {
     cudaEventElapsedTime(&ms, e0, e1);
     return IBEM_OK;
   };
-  TuneVal best{b.hsplit, b.hsplit_wide, b.tshape, 0};
+  TuneVal best{b.split, b.split_wide, b.tshape, 0};
   float best_ms = 1e30f;
   for (int ts = 0; ts < 3 && !s; ++ts)
-    for (int h : slice_candidates(b.ntiles_s[ts], b.max_seg, sms)) {
+    for (MfSplit h : split_candidates(b.ntiles_s[ts], b.max_seg, sms)) {
       if (b.nu == 60 && ts != 0) break;   // the layout-60 products have 64-target tiles only
       for (int pers = 0; pers < (b.nu == 60 ? 1 : 2) && !s; ++pers) {
+        if (pers && h.pieces > 1) continue;   // the work list is of whole slices
         if ((s = mf_set_f32_shape(b, ts, h, pers, st))) break;
         float ms = 0.f;
         if ((s = time_it(false, ms))) break;
         if (ms < best_ms) {
           best_ms = ms;
           best.tshape = ts;
-          best.hsplit = h;
+          best.split = h;
           best.persist = pers;
         }
       }
       if (s) break;
     }
   best_ms = 1e30f;
-  for (int h : slice_candidates(b.nu == 60 ? b.ntiles_s[0] : b.ntiles, b.max_seg, sms)) {
+  for (MfSplit h : split_candidates(b.nu == 60 ? b.ntiles_s[0] : b.ntiles, b.max_seg, sms)) {
     if (s) break;
-    b.hsplit_wide = h;
+    b.split_wide = h;
     float ms = 0.f;
     if ((s = time_it(true, ms))) break;
     if (ms < best_ms) {
       best_ms = ms;
-      best.hsplit_wide = h;
+      best.split_wide = h;
     }
   }
   if (e0) cudaEventDestroy(e0);
@@ -1127,8 +1134,8 @@ ibem_status mf_tune(MfBatch& b, cudaStream_t st) {
   free_async(xd, st);
   free_async(yd, st);
   if (s) return s;
-  b.hsplit_wide = best.hsplit_wide;
-  if ((s = mf_set_f32_shape(b, best.tshape, best.hsplit, best.persist, st))) return s;
+  b.split_wide = best.split_wide;
+  if ((s = mf_set_f32_shape(b, best.tshape, best.split, best.persist, st))) return s;
   std::lock_guard<std::mutex> lk(g_tune_mu);
   g_tune[key] = best;
   return IBEM_OK;
@@ -1139,10 +1146,11 @@ void launch_f32(const MfBatch& b, const float* x, float* y, cudaStream_t st, con
   const MfTile* tiles = b.tiles_s[TT == 64 ? 0 : (TT == 128 ? 1 : 2)];
   if (b.persist)
     ::ibem::count_launch(), k_mf_apply_f32_persist<TT><<<b.persist_ctas, TT, 0, st>>>(
-        tiles, b.work, b.nwork, b.hsplit, b.seg_begin, mask, mask_on, b.gh, b.gl, b.matf, x, y);
+        tiles, b.work, b.nwork, b.split.slices, b.seg_begin, mask, mask_on, b.gh, b.gl, b.matf, x, y);
   else
-    ::ibem::count_launch(), k_mf_apply_f32<TT><<<dim3(b.ntiles_s[TT == 64 ? 0 : (TT == 128 ? 1 : 2)], b.hsplit), TT, 0,
-                                                 st>>>(tiles, b.seg_begin, mask, mask_on, b.gh, b.gl, b.matf, x, y);
+    ::ibem::count_launch(), k_mf_apply_f32<TT><<<dim3(b.ntiles_s[TT == 64 ? 0 : (TT == 128 ? 1 : 2)], b.split.slices,
+                                                      b.split.pieces), TT, 0, st>>>(
+        tiles, b.seg_begin, mask, mask_on, b.gh, b.gl, b.matf, x, y);
 }
 
 ibem_status mf_apply_f32(const MfBatch& b, const float* x, float* y, cudaStream_t st, const int* mask, int mask_on) {
@@ -1168,14 +1176,14 @@ ibem_status mf_apply_f64(const MfBatch& b, const double* x, double* y, cudaStrea
   // double-float everywhere).  In realisations below kMfSplitMin particles most (warp,
   // source) pairs are near, and one FP64 launch over every pair is faster than the two passes
   const bool split = b.max_seg >= kMfSplitMin;
-  ::ibem::count_launch(), k_mf_apply_f64<<<dim3(b.ntiles, b.hsplit_wide), kMfThreads, 0, st>>>(
+  ::ibem::count_launch(), k_mf_apply_f64<<<dim3(b.ntiles, b.split_wide.slices, b.split_wide.pieces), kMfThreads, 0, st>>>(
       b.tiles, b.seg_begin, mask, mask_on, b.cen, b.rad, b.mats, x, y, b.perm, split ? 1 : 0);
   if (split && b.max_seg < kMfSkipMin)
-    ::ibem::count_launch(), k_mf_apply_df<kMfThreads><<<dim3(b.ntiles, b.hsplit_wide), kMfThreads, 0, st>>>(
+    ::ibem::count_launch(), k_mf_apply_df<kMfThreads><<<dim3(b.ntiles, b.split_wide.slices, b.split_wide.pieces), kMfThreads, 0, st>>>(
         b.tiles, b.seg_begin, mask, mask_on, b.cen, b.rad, b.mats, x, y, b.perm, 2);
   else if (split)   // the same number of warps per SM, one CTA of 256 targets (tiles_s[2])
     ::ibem::count_launch(),
-        k_mf_apply_df<2 * kMfThreads><<<dim3(b.ntiles_s[2], std::min((b.max_seg + 31) / 32, 2 * b.hsplit_wide)),
+        k_mf_apply_df<2 * kMfThreads><<<dim3(b.ntiles_s[2], std::min((b.max_seg + 31) / 32, 2 * b.split_wide.slices)),
                                          2 * kMfThreads, 0, st>>>(b.tiles_s[2], b.seg_begin, mask, mask_on, b.cen,
                                                                   b.rad, b.mats, x, y, b.perm, 3);
   IBEM_LAUNCH_CHECK("mf apply f64");
@@ -1186,7 +1194,7 @@ ibem_status mf_apply_f64_all(const MfBatch& b, const double* x, double* y, cudaS
   ProfScope ps(PROF_MF_F64, st, 0.0);
   if (b.nu == 60) return mf60_apply_f64(b, x, y, st, nullptr, 1);
   IBEM_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * b.N, st));
-  ::ibem::count_launch(), k_mf_apply_f64<<<dim3(b.ntiles, b.hsplit_wide), kMfThreads, 0, st>>>(
+  ::ibem::count_launch(), k_mf_apply_f64<<<dim3(b.ntiles, b.split_wide.slices, b.split_wide.pieces), kMfThreads, 0, st>>>(
       b.tiles, b.seg_begin, nullptr, 1, b.cen, b.rad, b.mats, x, y, b.perm, 0);
   IBEM_LAUNCH_CHECK("mf apply f64 (all pairs)");
   return IBEM_OK;
@@ -1196,7 +1204,7 @@ ibem_status mf_apply_df(const MfBatch& b, const double* x, double* y, cudaStream
   ProfScope ps(PROF_MF_DF, st, 0.0);
   if (b.nu == 60) return mf60_apply_f64(b, x, y, st, mask, mask_on);   // no double-float form of layout 60
   IBEM_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * b.N, st));
-  ::ibem::count_launch(), k_mf_apply_df<kMfThreads><<<dim3(b.ntiles, b.hsplit_wide), kMfThreads, 0, st>>>(
+  ::ibem::count_launch(), k_mf_apply_df<kMfThreads><<<dim3(b.ntiles, b.split_wide.slices, b.split_wide.pieces), kMfThreads, 0, st>>>(
       b.tiles, b.seg_begin, mask, mask_on, b.cen, b.rad, b.mats, x, y, b.perm, 0);
   IBEM_LAUNCH_CHECK("mf apply df");
   return IBEM_OK;
@@ -1958,8 +1966,8 @@ extern "C" ibem_status ibem_e3d_mf_tuning(const ibem_e3d_batch* batch, int* slic
   ibem_status s = mf_batch_init(b, *batch, st);
   if (!s) s = mf_tune(b, st);
   if (!s) {
-    *slices_fp32 = b.hsplit;
-    *slices_wide = b.hsplit_wide;
+    *slices_fp32 = b.split.slices;
+    *slices_wide = b.split_wide.slices;
     const cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) s = cuda_fail(e, "mf_tuning");
   }
@@ -1978,7 +1986,7 @@ extern "C" ibem_status ibem_e3d_mf_tile_shape(const ibem_e3d_batch* batch, int* 
   if (!s) {
     *targets_per_cta = 64 << b.tshape;
     *persistent = b.persist;
-    *slices = b.hsplit;
+    *slices = b.split.slices;
     const cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) s = cuda_fail(e, "mf_tile_shape");
   }

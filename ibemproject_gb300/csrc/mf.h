@@ -39,6 +39,14 @@ struct MfTile {
 inline cudaError_t alloc_async(void** p, size_t bytes, cudaStream_t st) { return pool_alloc(p, bytes, st); }
 inline void free_async(void* p, cudaStream_t st) { pool_free(p, st); }
 
+// Split of a tile's sources over CTAs: slices of at least 32 sources (gridDim.y), each cut into
+// up to kMfPieces pieces (gridDim.z) where the slices alone leave too few CTAs
+constexpr int kMfPieces = 4;
+struct MfSplit {
+  int slices = 1, pieces = 1;
+  bool operator==(const MfSplit& o) const { return slices == o.slices && pieces == o.pieces; }
+};
+
 struct MfBatch {
   cudaStream_t st = nullptr;   // stream of the call that owns the batch's buffers
   int nu = 24;                 // unknowns per particle: 24 or 60
@@ -63,8 +71,8 @@ struct MfBatch {
   int ntiles = 0;
   int* perm = nullptr;        // num: particles of each realisation in the Morton order of their
                               // centres (position -> particle), used by the split FP64 product
-  int hsplit = 1;      // source slices per target tile, FP32 product (autotuned)
-  int hsplit_wide = 1; // the same for the double-float and FP64 products (~255 registers)
+  MfSplit split;       // of the sources of a target tile, FP32 product (autotuned)
+  MfSplit split_wide;  // the same for the double-float and FP64 products (~255 registers)
   // FP32 product (the GMRES operator): tile shape and launch form, picked by the autotuner
   MfTile* tiles_s[3] = {nullptr, nullptr, nullptr};   // tiles of 64, 128 and 256 targets
   int ntiles_s[3] = {0, 0, 0};
@@ -85,9 +93,9 @@ ibem_status mf60_block_jacobi(const MfBatch& b, float* Pseg, cudaStream_t st);
 ibem_status mf60_precond_apply(const MfBatch& b, const float* Pseg, const float* v, float* z, const int* kdev,
                                int64_t vstride, cudaStream_t st);
 
-// Sets the FP32 product's tile shape (0, 1, 2: 64, 128, 256 targets per CTA), source slices
-// and launch form; builds the persistent form's work list.
-ibem_status mf_set_f32_shape(MfBatch& b, int tshape, int hsplit, int persist, cudaStream_t st);
+// Sets the FP32 product's tile shape (0, 1, 2: 64, 128, 256 targets per CTA), source split
+// and launch form; builds the persistent form's work list (of whole slices: one piece each).
+ibem_status mf_set_f32_shape(MfBatch& b, int tshape, MfSplit split, int persist, cudaStream_t st);
 
 // layout 24 (orders 0 and 1) or 60 (orders 0 to 2: block-Jacobi preconditioner only)
 ibem_status mf_batch_init(MfBatch& b, const ibem_e3d_batch& in, cudaStream_t st, int layout = 24);

@@ -11,7 +11,7 @@
 // source's powers of 1/r by a_h^-(row order) and the sums by a_s^(row order) once.
 //
 // One thread per target particle, 64 consecutive targets of one realisation per CTA, source
-// slices over gridDim.y, partial sums added atomically to the target's own block times its
+// slices over gridDim.y (and their pieces over gridDim.z), partial sums added atomically to the target's own block times its
 // coefficients (k_self_apply60, which also clears the sums).  A target whose centre lies
 // inside a source (overlapping spheres) takes that pair from the generated dense block.
 //
@@ -143,8 +143,8 @@ __global__ void __launch_bounds__(kT)
   const MfTile t = tiles[blockIdx.x];
   if (mask && mask[t.seg] != mask_on) return;
   const int hb0 = seg_begin[t.seg], he0 = seg_begin[t.seg + 1];
-  const int per = (he0 - hb0 + gridDim.y - 1) / gridDim.y;
-  const int hb = hb0 + blockIdx.y * per, he = min(he0, hb + per);
+  const int ns = gridDim.y * gridDim.z, per = (he0 - hb0 + ns - 1) / ns;
+  const int hb = hb0 + (blockIdx.y * gridDim.z + blockIdx.z) * per, he = min(he0, hb + per);
   if (hb >= he) return;
   const int s = t.s0 + threadIdx.x;
   const bool act = threadIdx.x < t.ns;
@@ -206,8 +206,8 @@ __global__ void __launch_bounds__(kT)
   const MfTile t = tiles[blockIdx.x];
   if (mask && mask[t.seg] != mask_on) return;
   const int hb0 = seg_begin[t.seg], he0 = seg_begin[t.seg + 1];
-  const int per = (he0 - hb0 + gridDim.y - 1) / gridDim.y;
-  const int hb = hb0 + blockIdx.y * per, he = min(he0, hb + per);
+  const int ns = gridDim.y * gridDim.z, per = (he0 - hb0 + ns - 1) / ns;
+  const int hb = hb0 + (blockIdx.y * gridDim.z + blockIdx.z) * per, he = min(he0, hb + per);
   if (hb >= he) return;
   const int s = t.s0 + threadIdx.x;
   const bool act = threadIdx.x < t.ns;
@@ -338,15 +338,15 @@ ibem_status mf60_apply_f32(const MfBatch& b, const float* x, float* y, cudaStrea
                            int mask_on) {
   ::ibem::count_launch(), k_self_apply60<float><<<(unsigned)((b.N + 239) / 240), 240, 0, st>>>(b.N, b.seg_of, mask, mask_on,
                                                                                                b.self60, x, y);
-  ::ibem::count_launch(), k_mf60_f32<<<dim3(b.ntiles_s[0], b.hsplit), kT, 0, st>>>(b.tiles_s[0], b.seg_begin, mask, mask_on,
-                                                                                   b.gh, b.gl, b.matf, x, y);
+  ::ibem::count_launch(), k_mf60_f32<<<dim3(b.ntiles_s[0], b.split.slices, b.split.pieces), kT, 0, st>>>(
+      b.tiles_s[0], b.seg_begin, mask, mask_on, b.gh, b.gl, b.matf, x, y);
   IBEM_LAUNCH_CHECK("mf60 apply f32");
   return IBEM_OK;
 }
 
 ibem_status mf60_apply_f64(const MfBatch& b, const double* x, double* y, cudaStream_t st, const int* mask,
                            int mask_on) {
-  const dim3 grid(b.ntiles_s[0], b.hsplit_wide);
+  const dim3 grid(b.ntiles_s[0], b.split_wide.slices, b.split_wide.pieces);
   ::ibem::count_launch(), k_self_apply60<double><<<(unsigned)((b.N + 239) / 240), 240, 0, st>>>(b.N, b.seg_of, mask, mask_on,
                                                                                                 b.self60, x, y);
 #define IBEM_MF60_F64(RO)                                                                                         \
