@@ -61,6 +61,30 @@ struct MvSink {
   __device__ __forceinline__ void operator()(int r, int c, T v) const { acc[r] = fma_t(v, xs[c], acc[r]); }
 };
 
+// Source records (mf_contract.cuh) of a chunk: the coefficients are staged with a zero behind each
+// source's 24, the records summed from them, TT threads over the entries.
+__device__ const MfRecTab g_rec_tab = mf_rec_tab();
+template <class T>
+struct MfStage {
+  __align__(16) T rec[kMfChunk * kRecLen];
+  T raw[kMfChunk * (kMfNu + 1)];
+  unsigned tab[kRecLen];
+  __device__ __forceinline__ void init() {
+    for (int i = threadIdx.x; i < kRecLen; i += blockDim.x) tab[i] = g_rec_tab.v[i];
+  }
+  template <class F>
+  __device__ __forceinline__ void load(int nh, F value) {   // value(source of the chunk, coefficient)
+    for (int i = threadIdx.x; i < nh * (kMfNu + 1); i += blockDim.x) {
+      const int h = i / (kMfNu + 1), c = i % (kMfNu + 1);
+      raw[i] = c < kMfNu ? value(h, c) : T(0);
+    }
+  }
+  __device__ __forceinline__ void build(int nh) {
+    for (int i = threadIdx.x; i < nh * kRecLen; i += blockDim.x)
+      rec[i] = mf_rec_entry(tab[i % kRecLen], raw + (kMfNu + 1) * (i / kRecLen));
+  }
+};
+
 // One work item of the FP32 product: the TT targets of a tile against source slice `slice`
 // of `nslice` of its realisation (TT = blockDim.x, the tile shape the autotuner picks).
 template <int TT>
@@ -68,7 +92,7 @@ __device__ __forceinline__ void mf_f32_item(const MfTile t, int slice, int nslic
                                             const int* __restrict__ mask, int mask_on,
                                             const float4* __restrict__ gh, const float4* __restrict__ gl,
                                             const SphMatF* __restrict__ mats, const float* __restrict__ x,
-                                            float* __restrict__ y, float4* sgh, float4* sgl, float* sx) {
+                                            float* __restrict__ y, float4* sgh, float4* sgl, MfStage<float>& sx) {
   if (mask && mask[t.seg] != mask_on) return;  // realisation left out of this product
   const int hb0 = seg_begin[t.seg], he0 = seg_begin[t.seg + 1];
   const int per = (he0 - hb0 + nslice - 1) / nslice;
@@ -89,7 +113,9 @@ __device__ __forceinline__ void mf_f32_item(const MfTile t, int slice, int nslic
       sgh[i] = gh[h0 + i];
       sgl[i] = gl[h0 + i];
     }
-    for (int i = threadIdx.x; i < nh * kMfNu; i += TT) sx[i] = x[(int64_t)kMfNu * h0 + i];
+    sx.load(nh, [&](int h, int c) { return x[(int64_t)kMfNu * (h0 + h) + c]; });
+    __syncthreads();
+    sx.build(nh);
     __syncthreads();
     if (!act) continue;
 #pragma unroll 1
@@ -100,7 +126,7 @@ __device__ __forceinline__ void mf_f32_item(const MfTile t, int slice, int nslic
       const float x0 = ((ph.x - qh.x) + (pl.x - ql.x)) * ia;
       const float x1 = ((ph.y - qh.y) + (pl.y - ql.y)) * ia;
       const float x2 = ((ph.z - qh.z) + (pl.z - ql.z)) * ia;
-      sph_pair_apply24<float, true>(x0, x1, x2, 1.f, 0.f, 0.f, mc.tn1, mc.tn2, sx + kMfNu * hh, ph.w * ia, acc);
+      sph_pair_raw24<float>(x0, x1, x2, 2.f - mc.tn2, sx.rec + kRecLen * hh, ph.w * ia, acc);
     }
   }
   if (!act) return;
@@ -123,7 +149,8 @@ __global__ void __launch_bounds__(TT)
                    const float4* __restrict__ gh, const float4* __restrict__ gl,
                    const SphMatF* __restrict__ mats, const float* __restrict__ x, float* __restrict__ y) {
   __shared__ float4 sgh[kMfChunk], sgl[kMfChunk];
-  __shared__ float sx[kMfChunk * kMfNu];
+  __shared__ MfStage<float> sx;
+  sx.init();
   mf_f32_item<TT>(tiles[blockIdx.x], blockIdx.y * gridDim.z + blockIdx.z, gridDim.y * gridDim.z,
                   seg_begin, mask, mask_on, gh, gl, mats, x, y, sgh, sgl, sx);
 }
@@ -139,7 +166,8 @@ __global__ void __launch_bounds__(TT)
                            const float4* __restrict__ gh, const float4* __restrict__ gl,
                            const SphMatF* __restrict__ mats, const float* __restrict__ x, float* __restrict__ y) {
   __shared__ float4 sgh[kMfChunk], sgl[kMfChunk];
-  __shared__ float sx[kMfChunk * kMfNu];
+  __shared__ MfStage<float> sx;
+  sx.init();
   for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
     const int2 it = work[w];
     mf_f32_item<TT>(tiles[it.x], it.y, nslice, seg_begin, mask, mask_on, gh, gl, mats, x, y, sgh, sgl, sx);
@@ -235,7 +263,8 @@ __global__ void __launch_bounds__(kMfThreads)
                    const SphMat* __restrict__ mats, const double* __restrict__ x, double* __restrict__ y,
                    const int* __restrict__ perm, int mode) {
   __shared__ double sc[kMfChunk * 4];
-  __shared__ double sx[kMfChunk * kMfNu];
+  __shared__ MfStage<double> sx;
+  sx.init();
   const MfTile t = tiles[blockIdx.x];
   if (mask && mask[t.seg] != mask_on) return;  // realisation left out of this product
   const MfSlice sl = mf_slice(seg_begin[t.seg], seg_begin[t.seg + 1], mode);
@@ -269,8 +298,9 @@ __global__ void __launch_bounds__(kMfThreads)
       sc[4 * i + 2] = cen[3 * (int64_t)h + 2];
       sc[4 * i + 3] = 1.0 / rad[h];
     }
-    for (int i = threadIdx.x; i < nh * kMfNu; i += blockDim.x)
-      sx[i] = x[(int64_t)kMfNu * perm[h0 + i / kMfNu] + i % kMfNu];
+    sx.load(nh, [&](int h, int c) { return x[(int64_t)kMfNu * perm[h0 + h] + c]; });
+    __syncthreads();
+    sx.build(nh);
     __syncthreads();
     if (!act) continue;
 #pragma unroll 1
@@ -278,7 +308,7 @@ __global__ void __launch_bounds__(kMfThreads)
       const int hh = __ffs(m) - 1;
       const double ia = sc[4 * hh + 3];
       const double x0 = (p0 - sc[4 * hh]) * ia, x1 = (p1 - sc[4 * hh + 1]) * ia, x2 = (p2 - sc[4 * hh + 2]) * ia;
-      sph_pair_apply24<double, true>(x0, x1, x2, 1.0, 0.0, 0.0, mc.tn1, mc.tn2, sx + kMfNu * hh, as * ia, acc);
+      sph_pair_raw24<double>(x0, x1, x2, 2.0 - mc.tn2, sx.rec + kRecLen * hh, as * ia, acc);
     }
   }
   if (!act) return;
@@ -310,9 +340,10 @@ __global__ void __launch_bounds__(TT)
                   const SphMat* __restrict__ mats, const double* __restrict__ x, double* __restrict__ y,
                   const int* __restrict__ perm, int mode) {
   __shared__ DF sc[kMfChunk * 4];
-  __shared__ DF sx[kMfChunk * kMfNu];
-  __shared__ DF szero[kMfNu];   // the coefficients of a skipped source in mode 2
-  if (threadIdx.x < kMfNu) szero[threadIdx.x] = DF();
+  __shared__ MfStage<DF> sx;
+  __shared__ __align__(16) DF szero[kRecLen];   // the record of a skipped source in mode 2
+  sx.init();
+  for (int i = threadIdx.x; i < kRecLen; i += TT) szero[i] = DF();
   const MfTile t = tiles[blockIdx.x];
   if (mask && mask[t.seg] != mask_on) return;  // realisation left out of this product
   const MfSlice sl = mf_slice(seg_begin[t.seg], seg_begin[t.seg + 1], mode);
@@ -334,7 +365,7 @@ __global__ void __launch_bounds__(TT)
   }
   double wlo[3], whi[3];
   warp_box(act, q0, q1, q2, wlo, whi);
-  const DF tn1(mc.tn1), tn2(mc.tn2);
+  const DF tf(2.0 - mc.tn2);
   DF acc[kMfNu];
   const bool warp_on = __any_sync(0xffffffffu, act);
   for (int h0 = sl.first; h0 < sl.end; h0 += sl.step) {
@@ -348,18 +379,19 @@ __global__ void __launch_bounds__(TT)
       sc[4 * i + 2] = DF(cen[3 * (int64_t)h + 2]);
       sc[4 * i + 3] = DF(1.0 / rad[h]);
     }
-    for (int i = threadIdx.x; i < nh * kMfNu; i += blockDim.x)
-      sx[i] = DF(x[(int64_t)kMfNu * perm[h0 + i / kMfNu] + i % kMfNu]);
+    sx.load(nh, [&](int h, int c) { return DF(x[(int64_t)kMfNu * perm[h0 + h] + c]); });
+    __syncthreads();
+    sx.build(nh);
     __syncthreads();
     if (!act) continue;
     const unsigned all = nh >= 32 ? 0xffffffffu : (1u << nh) - 1u;
 #pragma unroll 1
     for (unsigned k = mode == 2 ? all : m; k; k &= k - 1u) {
       const int hh = __ffs(k) - 1;
-      const DF* xs = (m >> hh) & 1u ? sx + kMfNu * hh : szero;
+      const DF* xs = (m >> hh) & 1u ? sx.rec + kRecLen * hh : szero;
       const DF ia = sc[4 * hh + 3];
       const DF x0 = (p0 - sc[4 * hh]) * ia, x1 = (p1 - sc[4 * hh + 1]) * ia, x2 = (p2 - sc[4 * hh + 2]) * ia;
-      sph_pair_apply24<DF, true>(x0, x1, x2, DF(1.0), DF(), DF(), tn1, tn2, xs, as * ia, acc);
+      sph_pair_raw24<DF>(x0, x1, x2, tf, xs, as * ia, acc);
     }
   }
   if (!act) return;

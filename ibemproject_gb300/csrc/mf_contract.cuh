@@ -10,16 +10,31 @@
 // with e the strain that the source's eigenstrain x_h produces at the target centre (the
 // post-processor's sum, postProcessorElastic3D.cpp:407-470, contracted with the eigenstrain
 // before any tensor is formed: field_contract.cuh), and the order-1 rows are the same
-// combination of the gradient d r_ij / d x_r.  Every coefficient of the contraction is a
-// radial function F(u), u = |x|^2 / 2, times a polynomial in x; its gradient is F'(u) x
-// plus F times the polynomial's gradient, and F' is the next rung of the same u-derivative
-// ladder (V_n^(k) = -J_{n+1}^(k-1), J_m' = -(2m+3) J_{m+1} outside, 0 inside), so
-//   d_k r_ij = Ru_ij x_k + P_ijk,
-// Ru the contraction with every radial coefficient replaced by its u-derivative and P the
-// polynomial part (written out below).  About 750 operations per pair, against ~6,000 for
-// the generated block and its 576 multiply-adds.
+// combination of the gradient g_ijk = d r_ij / d x_k.
+//
+// In units of the source's radius (a = 1), with E the order-0 and F the order-1 coefficients as
+// tensors symmetric in their first two indices, V_n and J_m the sphere's radial potentials,
+// Ps = V_0 - V_1 and Q = V_1 - V_2 and a number the rung of their ladder of derivatives in
+// u = |x|^2 / 2 (V_n^(k) = -J_{n+1}^(k-1), J_m' = -(2m+3) J_{m+1} outside, 0 inside), t = 1 - nu0:
+//   L_ikl = F_ikl + F_ilk,  M_ijk = L_ijk + L_jik,  w_n = F_mmn,  v_n = F_mnm         (source only)
+//   Ep_ij = F_ijl x_l,  N_ik = L_ikl x_l,  n = N x,  k = N x / 2 + N' x
+//   Z  = 2 t (Ph2 E x + V1_2 n / 2 + V1_1 v),            Zu the same one rung up
+//   dB = 2 Ps3 E x + Q3 k + 2 Q2 v + b2 w,  W = dB - Z   (b_k = Q_k - 2 nu V1_{k-1})
+//   dA = 2 Ps4 E x + Q4 k + 2 Q3 v + b3 w,  Wu = dA - Zu
+//   A, Au, B: scalars of x.E.x, tr E, x.n, w.x and v.x
+//   r_ij  = p_i x_j + p_j x_i + C0 E_ij - 2 Q2 Ep_ij + C2 (N_ij + N_ji) + d_ij B,   p = A x / 2 + W
+//   R_ij  = C0u E_ij - 2 Q3 Ep_ij + C2u (N_ij + N_ji) + d_ij A
+//   Y_ik  = cE E_ik - 2 Q3 Ep_ik + 2 Q3 N_ki + C2u N_ik + dA_k x_i / 2 + (Au x_i / 2 + Wu_i) x_k + d_ik A
+//   g_ijk = R_ij x_k + Y_ik x_j + Y_jk x_i - 2 Q2 F_ijk + C2 M_ijk + d_ij dB_k + d_ik W_j + d_jk W_i
+// About 430 multiply-adds per pair (1,140 additions and multiplications, most of them not
+// fusable, when r and the tensors of g were expanded term by term from E and F; ~6,000 for the
+// generated block and its 576 multiply-adds).  The products that use it are bound by the
+// arithmetic pipe of their type (FP64, double-float and FP32), so their time is this count.
 #pragma once
-#include "gen_sphere_common.cuh"
+#include "gen_sphere_common.cuh"   // first: IBEM_HD and IBEM_INLINE
+
+#include "dfnum.cuh"
+#include "fp64_math.cuh"
 
 namespace ibem {
 
@@ -30,149 +45,346 @@ IBEM_HD IBEM_INLINE float rsqrt_t(float x) {
   return 1.0f / sqrtf(x);
 #endif
 }
-IBEM_HD IBEM_INLINE double rsqrt_t(double x) {
+IBEM_HD IBEM_INLINE double rsqrt_t(double x) { return rsqrt_h3(x); }
+
+// A sum of products: plain for float and double, compensated (dfloat.cuh: 12 instead of 18
+// FP32 instructions a term) for double-float numbers.
+template <class R>
+struct Sum {
+  R s;
+  IBEM_HD IBEM_INLINE explicit Sum(R a) : s(a) {}
+  IBEM_HD IBEM_INLINE Sum(R a, R b) : s(a * b) {}
+  IBEM_HD IBEM_INLINE void add(R a, R b) { s = s + a * b; }
+  IBEM_HD IBEM_INLINE R val() const { return s; }
+};
+template <>
+struct Sum<DF> {
+  dacc s;
+  IBEM_HD IBEM_INLINE explicit Sum(DF a) : s(dacc_of(a.v)) {}
+  IBEM_HD IBEM_INLINE Sum(DF a, DF b) : s(dacc_prod(a.v, b.v)) {}
+  IBEM_HD IBEM_INLINE void add(DF a, DF b) { dacc_fma(s, a.v, b.v); }
+  IBEM_HD IBEM_INLINE DF val() const { return DF(dacc_val(s)); }
+};
+// times a power of two (exact) or another FP32 constant
+IBEM_HD IBEM_INLINE float pow2_t(float c, float x) { return c * x; }
+IBEM_HD IBEM_INLINE double pow2_t(float c, double x) { return (double)c * x; }
+IBEM_HD IBEM_INLINE DF pow2_t(float c, DF x) { return DF(dfloat{c * x.v.hi, c * x.v.lo}); }
+IBEM_HD IBEM_INLINE float mulc_t(float c, float x) { return c * x; }
+IBEM_HD IBEM_INLINE double mulc_t(float c, double x) { return (double)c * x; }
+IBEM_HD IBEM_INLINE DF mulc_t(float c, DF x) { return DF(x.v * c); }
+template <class R>
+IBEM_HD IBEM_INLINE R dot3_t(R a0, R b0, R a1, R b1, R a2, R b2) {
+  Sum<R> s(a0, b0);
+  s.add(a1, b1);
+  s.add(a2, b2);
+  return s.val();
+}
+
+// ---- record of a source: [E (6), tr E, -] [w (3), v (3), -, -] [F (18), -, -] [L (18), -, -] [M (18), -, -]
+// F, M: 3 (ij) + k, L: 6 i + (kl), pairs in the order 00 01 02 11 12 22.
+constexpr int kRecE = 0, kRecW = 8, kRecF = 16, kRecL = 36, kRecM = 56, kRecLen = 76;
+// Every entry of the record is a sum of at most four coefficients: their indices, a byte each
+// (24: none).
+struct MfRecTab {
+  unsigned v[kRecLen];
+};
+constexpr MfRecTab mf_rec_tab() {
+  MfRecTab t{};
+  const int pi[6] = {0, 0, 0, 1, 1, 2}, pj[6] = {0, 1, 2, 1, 2, 2};
+  const int at[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
+  struct F {
+    static constexpr unsigned pack(int a, int b = 24, int c = 24, int d = 24) {
+      return (unsigned)a | (unsigned)b << 8 | (unsigned)c << 16 | (unsigned)d << 24;
+    }
+  };
+  for (int e = 0; e < kRecLen; ++e) t.v[e] = F::pack(24);
+  for (int i = 0; i < 6; ++i) t.v[kRecE + i] = F::pack(i);
+  t.v[kRecE + 6] = F::pack(0, 3, 5);
+  for (int n = 0; n < 3; ++n) {
+    t.v[kRecW + n] = F::pack(6 + n, 6 + 9 + n, 6 + 15 + n);
+    t.v[kRecW + 3 + n] = F::pack(6 + 3 * at[0][n], 6 + 3 * at[1][n] + 1, 6 + 3 * at[2][n] + 2);
+  }
+  for (int i = 0; i < 18; ++i) t.v[kRecF + i] = F::pack(6 + i);
+  for (int i = 0; i < 3; ++i)
+    for (int q = 0; q < 6; ++q) {
+      const int k = pi[q], l = pj[q];
+      t.v[kRecL + 6 * i + q] = F::pack(6 + 3 * at[i][k] + l, 6 + 3 * at[i][l] + k);
+    }
+  for (int q = 0; q < 6; ++q)
+    for (int k = 0; k < 3; ++k) {
+      const int i = pi[q], j = pj[q];
+      t.v[kRecM + 3 * q + k] = F::pack(6 + 3 * q + k, 6 + 3 * at[i][k] + j, 6 + 3 * q + k, 6 + 3 * at[j][k] + i);
+    }
+  return t;
+}
+// entry of a record from its packed indices and the coefficients (c[24] = 0)
+template <class R>
+IBEM_HD IBEM_INLINE R mf_rec_entry(unsigned q, const R* c) {
+  return (c[q & 31u] + c[(q >> 8) & 31u]) + (c[(q >> 16) & 31u] + c[q >> 24]);
+}
+
+// loads of N consecutive numbers from a 16-byte boundary
+template <int N>
+IBEM_HD IBEM_INLINE void mf_ld(const float* p, float (&o)[N]) {
 #ifdef __CUDA_ARCH__
-  return rsqrt(x);
+#pragma unroll
+  for (int i = 0; i < N; i += 4) {
+    const float4 q = *reinterpret_cast<const float4*>(p + i);
+    o[i] = q.x;
+    o[i + 1] = q.y;
+    o[i + 2] = q.z;
+    o[i + 3] = q.w;
+  }
 #else
-  return 1.0 / sqrt(x);
+  for (int i = 0; i < N; ++i) o[i] = p[i];
+#endif
+}
+template <int N>
+IBEM_HD IBEM_INLINE void mf_ld(const double* p, double (&o)[N]) {
+#ifdef __CUDA_ARCH__
+#pragma unroll
+  for (int i = 0; i < N; i += 2) {
+    const double2 q = *reinterpret_cast<const double2*>(p + i);
+    o[i] = q.x;
+    o[i + 1] = q.y;
+  }
+#else
+  for (int i = 0; i < N; ++i) o[i] = p[i];
+#endif
+}
+template <int N>
+IBEM_HD IBEM_INLINE void mf_ld(const DF* p, DF (&o)[N]) {
+#ifdef __CUDA_ARCH__
+#pragma unroll
+  for (int i = 0; i < N; i += 2) {
+    const float4 q = *reinterpret_cast<const float4*>(p + i);
+    o[i].v = dfloat{q.x, q.y};
+    o[i + 1].v = dfloat{q.z, q.w};
+  }
+#else
+  for (int i = 0; i < N; ++i) o[i] = p[i];
 #endif
 }
 
-// y[24] += the pair block (target at offset x from a source of radius a) times Eu[24];
-// kmu, klam, tn1 = 1 - nu0, tn2 = 2 nu0 as in SphMat; row_scale multiplies the order-1 rows.
-// With RAW, y instead accumulates the contraction itself (r_t in y[t], row_scale * d_k r_t in
-// y[6 + 3t + k]) and the caller applies the same kmu / klam map once after the sum over
-// sources (sph_pair_map24): the map is linear and the same for every source of a target.
-template <class R, bool RAW = false>
-IBEM_HD IBEM_INLINE void sph_pair_apply24(R x0, R x1, R x2, R a, R kmu, R klam, R tn1, R tn2,
-                                          const R* __restrict__ Eu, R row_scale, R (&y)[24]) {
+// y += a b, rounded as an addition to y (for double-float numbers the sum is normalised)
+template <class R>
+IBEM_HD IBEM_INLINE void mf_acc(R& y, R a, R b) {
+  Sum<R> s(y);
+  s.add(a, b);
+  y = s.val();
+}
+
+// The raw contraction for the target at offset x in units of the source's radius: r_t is added to
+// y[t], row_scale * g_tk to y[6 + 3 t + k] (t over the pairs above).  The caller applies the
+// kmu / klam map once after the sum over sources (sph_pair_map24: the map is linear and the
+// same for every source of a target).  f = 2 (1 - nu0), rec the source's record (16-byte
+// aligned on the device).
+template <class R>
+IBEM_HD IBEM_INLINE void sph_pair_raw24(R x0, R x1, R x2, R f, const R* __restrict__ rec, R row_scale, R (&y)[24]) {
+  constexpr int pi[6] = {0, 0, 0, 1, 1, 2}, pj[6] = {0, 1, 2, 1, 2, 2};
+  constexpr int at[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
   const R x[3] = {x0, x1, x2};
-  const R a2 = a * a;
-  const R r2 = x0 * x0 + x1 * x1 + x2 * x2;
-  const bool outside = r2 - a2 > R(0);
-  const R ext = outside ? R(1) : R(0);
-  // rho^2 = a^2 + lambda: |x|^2 outside, a^2 inside (lambda = 0, integratorElastic3DHelper.cpp:51-54)
-  const R ir = rsqrt_t(outside ? r2 : a2);
-  const R irho2 = ir * ir;
-  const R p1 = R(4.0 * IBEM_PI) * a * a2 * ir * irho2;
-  const R p2 = p1 * irho2, p3 = p2 * irho2, p4 = p3 * irho2, p5 = p4 * irho2, p6 = p5 * irho2;
-  const R J1 = p1 * R(1.0 / 3.0), J2 = p2 * R(1.0 / 5.0), J3 = p3 * R(1.0 / 7.0), J4 = p4 * R(1.0 / 9.0),
-          J5 = p5 * R(1.0 / 11.0), J6 = p6 * R(1.0 / 13.0);
-  // u-derivative ladders of V_0, V_1, V_2 (first to fourth derivative)
-  const R V0_1 = -J1, V0_2 = R(5) * ext * J2, V0_3 = R(-35) * ext * J3, V0_4 = R(315) * ext * J4;
-  const R V1_1 = -J2, V1_2 = R(7) * ext * J3, V1_3 = R(-63) * ext * J4, V1_4 = R(693) * ext * J5;
-  const R V2_1 = -J3, V2_2 = R(9) * ext * J4, V2_3 = R(-99) * ext * J5, V2_4 = R(1287) * ext * J6;
-  const R Ps2 = V0_1 - a2 * V1_1, Ps3 = V0_2 - a2 * V1_2, Ps4 = V0_3 - a2 * V1_3, Ps5 = V0_4 - a2 * V1_4;
-  const R Q2 = V1_1 - a2 * V2_1, Q3 = V1_2 - a2 * V2_2, Q4 = V1_3 - a2 * V2_3, Q5 = V1_4 - a2 * V2_4;
-  const R Ph1 = V0_1, Ph2 = V0_2, Ph3 = V0_3;
-  // coefficients as full tensors symmetric in the first two indices (absorbs map[m][n])
-  R E[3][3], F[3][3][3];
+  const R r2 = dot3_t(x0, x0, x1, x1, x2, x2);
+  const bool outside = r2 > R(1);
+  // rho^2 = 1 + lambda: |x|^2 outside, 1 inside (lambda = 0, integratorElastic3DHelper.cpp:51-54)
+  const R ir = rsqrt_t(outside ? r2 : R(1));
+  const R i2 = ir * ir;
+  const R p1 = R(4.0 * IBEM_PI) * (ir * i2), p2 = p1 * i2, p3 = p2 * i2;
+  // rungs above the first vanish inside
+  const R e2 = outside ? p2 : R(0), e3 = outside ? p3 : R(0);
+  const R e4 = e3 * i2, e5 = e4 * i2, e6 = e5 * i2;
+  const R q1 = R(1.0 / 3.0) * p1, q2 = R(1.0 / 5.0) * p2, q3 = R(1.0 / 7.0) * p3;   // J_1, J_2, J_3
+  const R f1 = f * q1, f2 = f * q2, fe2 = f * e2, fe3 = f * e3, fe4 = f * e4;
+  const R e3x5 = mulc_t(5.f, e3), e4x7 = mulc_t(7.f, e4);
+  const R Q2 = q3 - q2, Q3 = e3 - e4, Q4 = mulc_t(9.f, e5) - e4x7;
+  const R Ps3 = e2 - e3, Ps4 = e4x7 - e3x5, Q3x2 = pow2_t(2.f, Q3), Q2x2 = pow2_t(2.f, Q2);
+  const R a3 = fe2 - (e2 + e3);
+  const R b2 = (q2 + q3) - f2, b3 = fe3 - (e3 + e4);
+  const R C2 = Q2x2 + f2, C2u = Q3x2 - fe3;
+  const R Ps3x2 = pow2_t(2.f, Ps3), cE = Ps3x2 - fe2;
+
+  R Ex[3], n[3], k[3], v[3], w[3], Ep[6], N[3][3];
+  R q, tE;
+  R Z[3];
   {
-    const int pi[6] = {0, 0, 0, 1, 1, 2}, pj[6] = {0, 1, 2, 1, 2, 2};
+    R L[20];
+    mf_ld(rec + kRecL, L);
 #pragma unroll
-    for (int t = 0; t < 6; ++t) {
-      E[pi[t]][pj[t]] = E[pj[t]][pi[t]] = Eu[t];
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-      for (int p = 0; p < 3; ++p) F[pi[t]][pj[t]][p] = F[pj[t]][pi[t]][p] = Eu[6 + 3 * t + p];
+      for (int j = 0; j < 3; ++j)
+        N[i][j] = dot3_t(L[6 * i + at[j][0]], x0, L[6 * i + at[j][1]], x1, L[6 * i + at[j][2]], x2);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      n[i] = dot3_t(N[i][0], x0, N[i][1], x1, N[i][2], x2);
+      Sum<R> s(pow2_t(0.5f, n[i]));
+      s.add(N[0][i], x0);
+      s.add(N[1][i], x1);
+      s.add(N[2][i], x2);
+      k[i] = s.val();
     }
   }
-  // polynomial quantities: Ex = E x, Ep = F.x, Epx = Ep x, Gx[i][j] = (G^i x)_j = F_jli x_l,
-  // s_i = x.G^i.x, v_n = F_mnm, w_n = F_mmn (= g_n = tr G^n)
-  R Ex[3], Ep[3][3], Epx[3], Gx[3][3], s[3], v[3], w[3];
+  R E[8];
+  mf_ld(rec + kRecE, E);
+  tE = E[6];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) Ex[i] = E[i][0] * x0 + E[i][1] * x1 + E[i][2] * x2;
+  for (int i = 0; i < 3; ++i) Ex[i] = dot3_t(E[at[i][0]], x0, E[at[i][1]], x1, E[at[i][2]], x2);
+  q = dot3_t(Ex[0], x0, Ex[1], x1, Ex[2], x2);
+  {
+    R wv[8];
+    mf_ld(rec + kRecW, wv);
 #pragma unroll
-  for (int m = 0; m < 3; ++m)
-#pragma unroll
-    for (int n = m; n < 3; ++n) Ep[m][n] = Ep[n][m] = F[m][n][0] * x0 + F[m][n][1] * x1 + F[m][n][2] * x2;
-#pragma unroll
-  for (int n = 0; n < 3; ++n) {
-    v[n] = F[0][n][0] + F[1][n][1] + F[2][n][2];
-    w[n] = F[0][0][n] + F[1][1][n] + F[2][2][n];
-    Epx[n] = Ep[n][0] * x0 + Ep[n][1] * x1 + Ep[n][2] * x2;
+    for (int i = 0; i < 3; ++i) {
+      w[i] = wv[i];
+      v[i] = wv[3 + i];
+    }
   }
+  R A, Au, B, W[3], dB[3], hA[3], m[3];
+  {
+    const R nx = pow2_t(0.5f, dot3_t(n[0], x0, n[1], x1, n[2], x2));
+    const R wx = dot3_t(w[0], x0, w[1], x1, w[2], x2);
+    const R vx = dot3_t(v[0], x0, v[1], x1, v[2], x2);
+    const R Q4x2 = pow2_t(2.f, Q4);
+    Sum<R> s(Ps4, q);
+    s.add(a3, tE);
+    s.add(Q4, nx);
+    s.add(b3, wx);
+    s.add(Q3x2, vx);
+    A = s.val();
+    Sum<R> su(mulc_t(35.f, e4) - mulc_t(63.f, e5), q);
+    su.add((e3x5 + e4x7) - mulc_t(5.f, fe3), tE);
+    su.add(mulc_t(63.f, e5) - mulc_t(99.f, e6), nx);
+    su.add((e4x7 + mulc_t(9.f, e5)) - mulc_t(7.f, fe4), wx);
+    su.add(Q4x2, vx);
+    Au = pow2_t(0.5f, su.val());
+    Sum<R> sb(Ps3, q);
+    sb.add((q1 + q2) - f1, tE);
+    sb.add(Q3, nx);
+    sb.add(b2, wx);
+    sb.add(Q2x2, vx);
+    B = sb.val();
+    const R Ps4x2 = pow2_t(2.f, Ps4);
+    const R z1 = pow2_t(0.5f, fe3), z1u = mulc_t(-3.5f, fe4), z0u = mulc_t(-5.f, fe3);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-#pragma unroll
-    for (int j = 0; j < 3; ++j) Gx[i][j] = F[j][0][i] * x0 + F[j][1][i] * x1 + F[j][2][i] * x2;
-    s[i] = Gx[i][0] * x0 + Gx[i][1] * x1 + Gx[i][2] * x2;
+    for (int i = 0; i < 3; ++i) {
+      Sum<R> z(fe2, Ex[i]);
+      z.add(z1, n[i]);
+      z.add(-f2, v[i]);
+      Sum<R> zu(z0u, Ex[i]);
+      zu.add(z1u, n[i]);
+      zu.add(fe3, v[i]);
+      Sum<R> b(Ps3x2, Ex[i]);
+      b.add(Q3, k[i]);
+      b.add(Q2x2, v[i]);
+      b.add(b2, w[i]);
+      dB[i] = b.val();
+      W[i] = dB[i] - z.val();
+      Sum<R> a(Ps4x2, Ex[i]);
+      a.add(Q4, k[i]);
+      a.add(Q3x2, v[i]);
+      a.add(b3, w[i]);
+      const R dA = a.val();
+      hA[i] = pow2_t(0.5f, dA);
+      Sum<R> mm(dA - zu.val());
+      mm.add(Au, x[i]);
+      m[i] = mm.val();
+    }
   }
-  const R q = Ex[0] * x0 + Ex[1] * x1 + Ex[2] * x2;
-  const R tE = E[0][0] + E[1][1] + E[2][2];
-  const R qp = Epx[0] * x0 + Epx[1] * x1 + Epx[2] * x2;
-  const R tEp = Ep[0][0] + Ep[1][1] + Ep[2][2];
-  const R vx = v[0] * x0 + v[1] * x1 + v[2] * x2;
-  const R wx = w[0] * x0 + w[1] * x1 + w[2] * x2;
-  const R t2v = tEp + R(2) * vx;
-  // scalar coefficients and their u-derivatives (B_u = A)
-  const R A = Ps4 * q + Ps3 * tE - tn2 * tE * Ph2 + a2 * (Q4 * qp + Q3 * t2v - tn2 * wx * V1_2);
-  const R Au = Ps5 * q + Ps4 * tE - tn2 * tE * Ph3 + a2 * (Q5 * qp + Q4 * t2v - tn2 * wx * V1_3);
-  const R B = Ps3 * q + Ps2 * tE - tn2 * tE * Ph1 + a2 * (Q3 * qp + Q2 * t2v - tn2 * wx * V1_1);
-  const R cE = R(2) * Ps3 - R(2) * tn1 * Ph2, cEu = R(2) * Ps4 - R(2) * tn1 * Ph3;
-  const R cEp = a2 * (R(2) * Q3 - R(2) * tn1 * V1_2), cEpu = a2 * (R(2) * Q4 - R(2) * tn1 * V1_3);
-  const R cv = a2 * (R(2) * Q2 - R(2) * tn1 * V1_1), cvu = cEp;
-  const R cs = a2 * Q3, csu = a2 * Q4;
-  const R cg = a2 * Q2, cgu = cs;
-  const R cw = -a2 * tn2 * V1_1, cwu = -a2 * tn2 * V1_2;
-  const R C0 = R(2) * Ps2 - R(4) * tn1 * Ph1, C0u = R(2) * Ps3 - R(4) * tn1 * Ph2;
-  const R C1 = a2 * (R(2) * Q2 - R(4) * tn1 * V1_1), C1u = a2 * (R(2) * Q3 - R(4) * tn1 * V1_2);
-  const R C2 = cv, C2u = cEp;
-  R W[3], Wu[3], dA[3], dB[3];
+  R F[20];
+  mf_ld(rec + kRecF, F);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    W[i] = cE * Ex[i] + cEp * Epx[i] + cv * v[i] + cs * s[i] + (cg + cw) * w[i];
-    Wu[i] = cEu * Ex[i] + cEpu * Epx[i] + cvu * v[i] + csu * s[i] + (cgu + cwu) * w[i];
-    // polynomial parts of d_k A and d_k B: dq = 2 Ex, dqp = 2 Epx + s, dtEp = w, dvx = v, dwx = w
-    const R dqp = R(2) * Epx[i] + s[i], dt2v = w[i] + R(2) * v[i];
-    dA[i] = R(2) * Ps4 * Ex[i] + a2 * (Q4 * dqp + Q3 * dt2v - tn2 * V1_2 * w[i]);
-    dB[i] = R(2) * Ps3 * Ex[i] + a2 * (Q3 * dqp + Q2 * dt2v - tn2 * V1_1 * w[i]);
+  for (int t = 0; t < 6; ++t) Ep[t] = dot3_t(F[3 * t], x0, F[3 * t + 1], x1, F[3 * t + 2], x2);
+  // order 0
+  const R Q2m = -Q2x2;
+  {
+    const R hAs = pow2_t(0.5f, A);
+    const R C0 = pow2_t(2.f, (q2 - q1) + f1), C2x2 = pow2_t(2.f, C2);
+    R p[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      Sum<R> s(W[i]);
+      s.add(hAs, x[i]);
+      p[i] = s.val();
+    }
+#pragma unroll
+    for (int t = 0; t < 6; ++t) {
+      const int i = pi[t], j = pj[t];
+      Sum<R> s(i == j ? B : p[j] * x[i]);
+      s.add(i == j ? pow2_t(2.f, p[i]) : p[i], x[j]);
+      s.add(C0, E[t]);
+      s.add(Q2m, Ep[t]);
+      if (i == j) s.add(C2x2, N[i][i]);
+      else s.add(C2, N[i][j] + N[j][i]);
+      y[t] += s.val();
+    }
   }
-  const int pi[6] = {0, 0, 0, 1, 1, 2}, pj[6] = {0, 1, 2, 1, 2, 2};
-  R r[6], g[6][3];
+  // order 1
+  R Rr[6], Y[3][3];
+  {
+    const R C0u = pow2_t(2.f, Ps3 - fe2), C2ux2 = pow2_t(2.f, C2u), Q3m = -Q3x2;
+#pragma unroll
+    for (int t = 0; t < 6; ++t) {
+      const int i = pi[t], j = pj[t];
+      R X;
+      if (i == j) {
+        Sum<R> s(A);
+        s.add(Q3m, Ep[t]);
+        X = s.val();
+      } else {
+        X = Q3m * Ep[t];
+      }
+      Sum<R> s(X);
+      s.add(C0u, E[t]);
+      if (i == j) s.add(C2ux2, N[i][i]);
+      else s.add(C2u, N[i][j] + N[j][i]);
+      Rr[t] = s.val();
+      Sum<R> d(X);
+      d.add(cE, E[t]);
+      Y[i][j] = Y[j][i] = d.val();
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        Sum<R> s(Y[i][j]);
+        s.add(Q3x2, N[j][i]);
+        s.add(C2u, N[i][j]);
+        s.add(hA[j], x[i]);
+        s.add(m[i], x[j]);
+        Y[i][j] = s.val();
+      }
+  }
+  R M[20];
+  mf_ld(rec + kRecM, M);
+  const R xx[3] = {pow2_t(2.f, x0), pow2_t(2.f, x1), pow2_t(2.f, x2)};
 #pragma unroll
   for (int t = 0; t < 6; ++t) {
     const int i = pi[t], j = pj[t];
-    const R H = Gx[i][j] + Gx[j][i];
-    const R xij = x[i] * x[j];
-    r[t] = A * xij + W[i] * x[j] + W[j] * x[i] + C0 * E[i][j] + C1 * Ep[i][j] + C2 * H;
-    R Ru = Au * xij + Wu[i] * x[j] + Wu[j] * x[i] + C0u * E[i][j] + C1u * Ep[i][j] + C2u * H;
-    if (i == j) {
-      r[t] += B;
-      Ru += A;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      R g;
+      if (i == j) {
+        Sum<R> s(i == c ? dB[c] + pow2_t(2.f, W[c]) : dB[c]);
+        s.add(Y[i][c], xx[i]);
+        s.add(Rr[t], x[c]);
+        s.add(Q2m, F[3 * t + c]);
+        s.add(C2, M[3 * t + c]);
+        g = s.val();
+      } else {
+        Sum<R> s(i == c ? W[j] : (j == c ? W[i] : Rr[t] * x[c]));
+        if (i == c || j == c) s.add(Rr[t], x[c]);
+        s.add(Y[i][c], x[j]);
+        s.add(Y[j][c], x[i]);
+        s.add(Q2m, F[3 * t + c]);
+        s.add(C2, M[3 * t + c]);
+        g = s.val();
+      }
+      mf_acc(y[6 + 3 * t + c], row_scale, g);
     }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      // d_k W_i = Wu_i x_k + cE E_ik + cEp (Ep_ik + Gx_ki) + 2 cs Gx_ik
-      const R dWi = cE * E[i][k] + cEp * (Ep[i][k] + Gx[k][i]) + R(2) * cs * Gx[i][k];
-      const R dWj = cE * E[j][k] + cEp * (Ep[j][k] + Gx[k][j]) + R(2) * cs * Gx[j][k];
-      R P = dA[k] * xij + dWi * x[j] + dWj * x[i] + C1 * F[i][j][k] + C2 * (F[j][k][i] + F[i][k][j]);
-      if (i == j) P += dB[k];
-      if (i == k) P += A * x[j] + W[j];
-      if (j == k) P += A * x[i] + W[i];
-      g[t][k] = Ru * x[k] + P;
-    }
-  }
-  if (RAW) {
-#pragma unroll
-    for (int t = 0; t < 6; ++t) {
-      y[t] += r[t];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) y[6 + 3 * t + k] += row_scale * g[t][k];
-    }
-    return;
-  }
-  const R tr = r[0] + r[3] + r[5];
-  const R dtr[3] = {g[0][0] + g[3][0] + g[5][0], g[0][1] + g[3][1] + g[5][1], g[0][2] + g[3][2] + g[5][2]};
-#pragma unroll
-  for (int t = 0; t < 6; ++t) {
-    const bool d = (t == 0 || t == 3 || t == 5);
-    y[t] += d ? kmu * r[t] + klam * tr : kmu * r[t];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) y[6 + 3 * t + k] += row_scale * (d ? kmu * g[t][k] + klam * dtr[k] : kmu * g[t][k]);
   }
 }
 
-// y = the kmu / klam map of a raw accumulation (sph_pair_apply24<R, true>)
+// y = the kmu / klam map of a raw accumulation
 template <class R>
 IBEM_HD IBEM_INLINE void sph_pair_map24(const R (&acc)[24], R kmu, R klam, R (&y)[24]) {
   const R tr = acc[0] + acc[3] + acc[5];
@@ -186,6 +398,31 @@ IBEM_HD IBEM_INLINE void sph_pair_map24(const R (&acc)[24], R kmu, R klam, R (&y
 #pragma unroll
     for (int k = 0; k < 3; ++k) y[6 + 3 * t + k] = d ? kmu * acc[6 + 3 * t + k] + klam * dtr[k] : kmu * acc[6 + 3 * t + k];
   }
+}
+
+// y[24] += the pair block (target at offset x from a source of radius a) times Eu[24];
+// kmu, klam, tn1 = 1 - nu0, tn2 = 2 nu0 as in SphMat; row_scale multiplies the order-1 rows.  For single
+// pairs: the contraction in units of the radius, where the order-1 coefficients take a factor a
+// and the gradient 1 / a.
+template <class R>
+IBEM_HD IBEM_INLINE void sph_pair_apply24(R x0, R x1, R x2, R a, R kmu, R klam, R /*tn1*/, R tn2,
+                                          const R* __restrict__ Eu, R row_scale, R (&y)[24]) {
+  const R ia = R(1) / a;
+  constexpr MfRecTab tab = mf_rec_tab();
+  R c[25];
+#pragma unroll
+  for (int i = 0; i < 24; ++i) c[i] = i < 6 ? Eu[i] : a * Eu[i];
+  c[24] = R(0);
+  alignas(16) R rec[kRecLen];
+#pragma unroll
+  for (int e = 0; e < kRecLen; ++e) rec[e] = mf_rec_entry(tab.v[e], c);
+  R raw[24], b[24];
+#pragma unroll
+  for (int i = 0; i < 24; ++i) raw[i] = R(0);
+  sph_pair_raw24<R>(x0 * ia, x1 * ia, x2 * ia, R(2) - tn2, rec, row_scale * ia, raw);
+  sph_pair_map24<R>(raw, kmu, klam, b);
+#pragma unroll
+  for (int i = 0; i < 24; ++i) y[i] += b[i];
 }
 
 }  // namespace ibem
