@@ -144,8 +144,8 @@ def solve(batch: DeviceBatch, b, precond: int = PRECOND_BLOCK_JACOBI, params=Non
           inner_tol: float = 1e-5, restart: int = 50, max_outer: int = 8, max_cycles: int = 20, x=None,
           stepwise: bool = False):
     """Matrix-free solve of every realisation (the batch's layout: 24, or 60 with the
-    block-Jacobi preconditioner): returns (x, list of MfReport).  stepwise: launch each Arnoldi
-    step from the host instead of one captured CUDA graph per GMRES cycle."""
+    block-Jacobi preconditioner): returns (x, list of MfReport).  stepwise: wait for each
+    Arnoldi step instead of launching ahead of it."""
     _linear(batch, (NU, 60))
     import torch
     if x is None:

@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(TT)
                    const int* __restrict__ mask, int mask_on,
                    const float4* __restrict__ gh, const float4* __restrict__ gl,
                    const SphMatF* __restrict__ mats, const float* __restrict__ x, float* __restrict__ y) {
+  chain_wait();
   __shared__ float4 sgh[kMfChunk], sgl[kMfChunk];
   __shared__ MfStage<float> sx;
   sx.init();
@@ -165,6 +166,7 @@ __global__ void __launch_bounds__(TT)
                            const int* __restrict__ seg_begin, const int* __restrict__ mask, int mask_on,
                            const float4* __restrict__ gh, const float4* __restrict__ gl,
                            const SphMatF* __restrict__ mats, const float* __restrict__ x, float* __restrict__ y) {
+  chain_wait();
   __shared__ float4 sgh[kMfChunk], sgl[kMfChunk];
   __shared__ MfStage<float> sx;
   sx.init();
@@ -521,6 +523,20 @@ __global__ void k_bcast_blocks(int num, const int* __restrict__ seg_of, const fl
   reinterpret_cast<float4*>(P)[t] = reinterpret_cast<const float4*>(Pseg)[(int64_t)seg_of[p] * kQ + q];
 }
 
+// Control of the Arnoldi steps of a cycle, on the device: the kernels of a step read the step's
+// index and return at once when the cycle has stopped, so that steps can be launched ahead of
+// the host's knowing how many there will be.
+struct StepCtl {
+  int k;         // steps taken
+  int stop;      // the cycle is over
+  int nactive, arrived;   // of the update's CTAs
+};
+// what the host reads, in pinned memory
+struct HostCtl {
+  volatile int steps;   // steps finished (taken or skipped)
+  volatile int stop;
+};
+
 // z = P v for the block-sparse preconditioner: z_p = D_p v_p + sum_slot Q_(p,slot) v_nbr;
 // one thread per row (24 x 24 row-major blocks, float4 loads)
 __device__ __forceinline__ float dot24(const float* __restrict__ a, const float* __restrict__ b) {
@@ -534,33 +550,59 @@ __device__ __forceinline__ float dot24(const float* __restrict__ a, const float*
   }
   return s;
 }
-// kdev (graph-captured Arnoldi steps): v is column *kdev of a basis with column stride vstride
-__global__ void k_precond_apply(int num, const float* __restrict__ D, const float* __restrict__ Q,
-                                const int* __restrict__ nbr, const float* __restrict__ v, float* __restrict__ z,
-                                const int* __restrict__ kdev = nullptr, int64_t vstride = 0) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= (int64_t)num * kMfNu) return;
-  if (kdev) v += (int64_t)(*kdev) * vstride;
-  const int64_t p = t / kMfNu;
-  const int r = (int)(t % kMfNu);
-  float s = dot24(D + t * kMfNu, v + p * kMfNu);
-  if (Q) {
-    for (int k = 0; k < kKnn; ++k) {
-      const int j = nbr[p * kKnn + k];
-      if (j >= 0) s += dot24(Q + ((p * kKnn + k) * kMfNu + r) * kMfNu, v + (int64_t)j * kMfNu);
+// Four lanes share a row, each taking every fourth of its 16 neighbour slots (and one the
+// diagonal block), so that a small realisation's rows have four times the loads in flight.
+// zero: cleared (the step's product adds to it).  ctl (Arnoldi steps): v is column ctl->k of a basis with column stride vstride; nothing to
+// do once ctl->stop.
+constexpr int kPreLanes = 4;
+__global__ void __launch_bounds__(256) k_precond_apply(int num, const float* __restrict__ D, const float* __restrict__ Q,
+                                                       const int* __restrict__ nbr, const float* __restrict__ v,
+                                                       float* __restrict__ z, float* __restrict__ zero,
+                                                       const StepCtl* __restrict__ ctl, int64_t vstride) {
+  chain_wait();
+  const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kPreLanes;
+  const int q = threadIdx.x % kPreLanes;
+  if (ctl) {
+    if (ctl->stop) return;
+    v += (int64_t)ctl->k * vstride;
+  }
+  const bool in = t < (int64_t)num * kMfNu;
+  float s = 0.f;
+  if (in) {
+    const int64_t p = t / kMfNu;
+    const int r = (int)(t % kMfNu);
+    if (q == 0) s = dot24(D + t * kMfNu, v + p * kMfNu);
+    if (Q) {
+#pragma unroll
+      for (int k = q; k < kKnn; k += kPreLanes) {
+        const int j = nbr[p * kKnn + k];
+        if (j >= 0) s += dot24(Q + ((p * kKnn + k) * kMfNu + r) * kMfNu, v + (int64_t)j * kMfNu);
+      }
     }
   }
-  z[t] = s;
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  if (in && q == 0) z[t] = s;
+  if (in && q == 1 && zero) zero[t] = 0.f;
 }
 
-// out[seg * ldo + j] += sum over the segment's rows of V_j[row] * w[row], j < nv (+ *kdev).
-// grid (nseg, splits); a CTA of 256 threads holds up to 8 rows per thread in registers.
-constexpr int kDotRows = 8, kDotThreads = 256;
+// out[seg * ldo + j] += sum over the segment's rows of V_j[row] * w[row], j < nv (Arnoldi steps:
+// j <= ctl->k).  grid (nseg, splits, column groups); a CTA of 256 threads holds up to 8 rows per
+// thread in registers and takes kDotCols columns, whose sums it reduces together (one column at
+// a time, with a CTA reduction each, took 1.5 us a column).
+constexpr int kDotRows = 8, kDotThreads = 256, kDotCols = 8;
 template <class TV>
 __global__ void __launch_bounds__(kDotThreads)
     k_seg_dots(int nu, const int* __restrict__ seg_begin, int nv, const TV* __restrict__ V, int64_t ldv,
-               const TV* __restrict__ w, double* __restrict__ out, int ldo, const int* __restrict__ kdev = nullptr) {
-  if (kdev) nv += *kdev;
+               const TV* __restrict__ w, double* __restrict__ out, int ldo, const StepCtl* __restrict__ ctl = nullptr) {
+  chain_wait();
+  if (ctl) {
+    if (ctl->stop) return;
+    nv = ctl->k + 1;
+  }
+  const int j0 = blockIdx.z * kDotCols;
+  if (j0 >= nv) return;
+  const int nj = min(kDotCols, nv - j0);
   const int seg = blockIdx.x;
   const int64_t r0 = (int64_t)nu * seg_begin[seg], r1 = (int64_t)nu * seg_begin[seg + 1];
   const int64_t base = r0 + (int64_t)blockIdx.y * kDotThreads * kDotRows;
@@ -571,9 +613,10 @@ __global__ void __launch_bounds__(kDotThreads)
     const int64_t r = base + threadIdx.x + (int64_t)i * kDotThreads;
     wr[i] = r < r1 ? w[r] : TV(0);
   }
-  __shared__ double red[kDotThreads / 32];
-  for (int j = 0; j < nv; ++j) {
-    const TV* vj = V + (int64_t)j * ldv;
+  __shared__ double red[kDotThreads / 32][kDotCols];
+#pragma unroll 2
+  for (int j = 0; j < nj; ++j) {
+    const TV* vj = V + (int64_t)(j0 + j) * ldv;
     double s = 0;
 #pragma unroll
     for (int i = 0; i < kDotRows; ++i) {
@@ -581,39 +624,59 @@ __global__ void __launch_bounds__(kDotThreads)
       if (r < r1) s += (double)vj[r] * (double)wr[i];
     }
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double tot = 0;
-      for (int k = 0; k < kDotThreads / 32; ++k) tot += red[k];
-      atomicAdd(out + (int64_t)seg * ldo + j, tot);
-    }
-    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][j] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x < nj) {
+    double tot = 0;
+    for (int k = 0; k < kDotThreads / 32; ++k) tot += red[k][threadIdx.x];
+    atomicAdd(out + (int64_t)seg * ldo + j0 + threadIdx.x, tot);
   }
 }
 
-// w[row] -= sum_j h[seg(row) * ldh + j] V_j[row], j < nv (+ *kdev)
-__global__ void k_seg_sub(int nu, int64_t N, const int* __restrict__ seg_of, int nv, const float* __restrict__ V, int64_t ldv,
-                          const double* __restrict__ h, int ldh, float* __restrict__ w,
-                          const int* __restrict__ kdev = nullptr) {
+// w[row] -= sum_j h[seg(row) * ldh + j] V_j[row], j <= ctl->k; with n2, n2[seg] += w[row]^2
+__global__ void __launch_bounds__(256) k_seg_sub(int nu, int64_t N, const int* __restrict__ seg_of,
+                                                 const float* __restrict__ V, int64_t ldv, const double* __restrict__ h,
+                                                 int ldh, float* __restrict__ w, double* __restrict__ n2,
+                                                 const StepCtl* __restrict__ ctl) {
+  chain_wait();
+  if (ctl->stop) return;
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r >= N) return;
-  if (kdev) nv += *kdev;
-  const double* hs = h + (int64_t)seg_of[r / nu] * ldh;
-  float s = w[r];
-  for (int j = 0; j < nv; ++j) s -= (float)hs[j] * V[(int64_t)j * ldv + r];
-  w[r] = s;
+  const int nv = ctl->k + 1;
+  const bool in = r < N;
+  const int seg = in ? seg_of[r / nu] : -1;
+  float s = 0.f;
+  if (in) {
+    const double* hs = h + (int64_t)seg * ldh;
+    s = w[r];
+#pragma unroll 4
+    for (int j = 0; j < nv; ++j) s -= (float)hs[j] * V[(int64_t)j * ldv + r];
+    w[r] = s;
+  }
+  if (!n2) return;
+  // a warp's rows belong to one realisation, but for its borders
+  double q = (double)s * (double)s;
+  if (__all_sync(0xffffffffu, seg == __shfl_sync(0xffffffffu, seg, 0))) {
+    for (int o = 16; o; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+    if ((threadIdx.x & 31) == 0 && in) atomicAdd(n2 + seg, q);
+  } else if (in) {
+    atomicAdd(n2 + seg, q);
+  }
 }
 
-// y[row] (+)= scale[seg(row)] * x[row] (FP32 <- FP64 / FP32); with kdev, y is column
-// *kdev + 1 of a basis with column stride ystride
+// y[row] (+)= scale[seg(row)] * x[row] (FP32 <- FP64 / FP32); with ctl (after the step's update,
+// which has counted it), y is column ctl->k of a basis with column stride ystride
 template <class TX, class TY>
 __global__ void k_seg_scale(int nu, int64_t N, const int* __restrict__ seg_of, const double* __restrict__ scale,
-                            const TX* __restrict__ x, TY* __restrict__ y, int add, const int* __restrict__ kdev = nullptr,
-                            int64_t ystride = 0) {
+                            const TX* __restrict__ x, TY* __restrict__ y, int add,
+                            const StepCtl* __restrict__ ctl = nullptr, int64_t ystride = 0) {
+  chain_wait();
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= N) return;
-  if (kdev) y += (int64_t)(*kdev + 1) * ystride;
+  if (ctl) {
+    if (ctl->stop) return;
+    y += (int64_t)ctl->k * ystride;
+  }
   const double v = scale[seg_of[r / nu]] * (double)x[r];
   y[r] = add ? (TY)((double)y[r] + v) : (TY)v;
 }
@@ -640,44 +703,68 @@ struct Krylov {
   int* nactive;   // 1
 };
 
-__global__ void k_arnoldi_update(int nseg, int m, int k, Krylov K, const int* __restrict__ kdev = nullptr) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nseg) return;
-  if (kdev) k = *kdev;
-  if (!K.active[s]) {
-    K.inv[s] = 0.0;
+// The last CTA then counts the step: ctl->k += 1, and stop once k == m or no realisation is
+// active; `host` (pinned) is told.  d1, d2 and n2 are left zero for the next step.
+__global__ void k_arnoldi_update(int nseg, int m, Krylov K, StepCtl* __restrict__ ctl, HostCtl* __restrict__ host) {
+  chain_wait();
+  if (ctl->stop) {
+    if (host && blockIdx.x == 0 && threadIdx.x == 0) host->steps = host->steps + 1;
     return;
   }
-  double* H = K.H + (int64_t)s * (m + 1) * m;
-  double* g = K.g + (int64_t)s * (m + 1);
-  double* cs = K.cs + (int64_t)s * m;
-  double* sn = K.sn + (int64_t)s * m;
-  for (int i = 0; i <= k; ++i) H[i * m + k] = K.d1[(int64_t)s * (m + 1) + i] + K.d2[(int64_t)s * (m + 1) + i];
-  // ||w|| after the two Gram-Schmidt passes
-  const double hn = sqrt(fmax(K.n2[s], 0.0));
-  H[(k + 1) * m + k] = hn;
-  for (int i = 0; i < k; ++i) {
-    const double a = H[i * m + k], b = H[(i + 1) * m + k];
-    H[i * m + k] = cs[i] * a + sn[i] * b;
-    H[(i + 1) * m + k] = -sn[i] * a + cs[i] * b;
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  const int k = ctl->k;
+  int still = 0;
+  if (s < nseg) {
+    double* d1 = K.d1 + (int64_t)s * (m + 1);
+    double* d2 = K.d2 + (int64_t)s * (m + 1);
+    if (K.active[s]) {
+      double* H = K.H + (int64_t)s * (m + 1) * m;
+      double* g = K.g + (int64_t)s * (m + 1);
+      double* cs = K.cs + (int64_t)s * m;
+      double* sn = K.sn + (int64_t)s * m;
+      // ||w|| after the two Gram-Schmidt passes
+      const double hn = sqrt(fmax(K.n2[s], 0.0));
+      double a = d1[0] + d2[0];
+      for (int i = 0; i < k; ++i) {   // column k through the previous Givens rotations
+        const double b = d1[i + 1] + d2[i + 1];
+        H[i * m + k] = cs[i] * a + sn[i] * b;
+        a = -sn[i] * a + cs[i] * b;
+      }
+      const double den = hypot(a, hn);
+      cs[k] = den > 0 ? a / den : 1.0;
+      sn[k] = den > 0 ? hn / den : 0.0;
+      H[k * m + k] = den;
+      H[(k + 1) * m + k] = 0.0;
+      const double gk = g[k], gn = -sn[k] * gk;
+      g[k + 1] = gn;
+      g[k] = cs[k] * gk;
+      K.kc[s] = k + 1;
+      K.nsteps[s] += 1;
+      K.est[s] = fabs(gn);
+      still = !(fabs(gn) <= K.thr[s] || hn == 0.0 || k + 1 == m);
+      K.inv[s] = still ? 1.0 / hn : 0.0;
+      if (!still) K.active[s] = 0;
+    } else {
+      K.inv[s] = 0.0;
+    }
+    for (int i = 0; i <= k; ++i) d1[i] = d2[i] = 0.0;
+    K.n2[s] = 0.0;
   }
-  const double a = H[k * m + k], b = H[(k + 1) * m + k];
-  const double den = hypot(a, b);
-  cs[k] = den > 0 ? a / den : 1.0;
-  sn[k] = den > 0 ? b / den : 0.0;
-  H[k * m + k] = den;
-  H[(k + 1) * m + k] = 0.0;
-  g[k + 1] = -sn[k] * g[k];
-  g[k] = cs[k] * g[k];
-  K.kc[s] = k + 1;
-  K.nsteps[s] += 1;
-  K.est[s] = fabs(g[k + 1]);
-  K.inv[s] = hn > 0 ? 1.0 / hn : 0.0;
-  if (fabs(g[k + 1]) <= K.thr[s] || hn == 0.0 || k + 1 == m) {
-    K.active[s] = 0;
-    K.inv[s] = 0.0;
-  } else {
-    atomicAdd(K.nactive, 1);
+  const int n = __syncthreads_count(still);
+  if (threadIdx.x != 0) return;
+  if (n) atomicAdd(&ctl->nactive, n);
+  __threadfence();
+  if (atomicAdd(&ctl->arrived, 1) + 1 < (int)gridDim.x) return;
+  __threadfence();
+  const int na = *reinterpret_cast<volatile int*>(&ctl->nactive);
+  ctl->nactive = 0;
+  ctl->arrived = 0;
+  ctl->k = k + 1;
+  ctl->stop = !(k + 1 < m && na > 0);
+  if (host) {
+    if (ctl->stop) host->stop = 1;
+    __threadfence_system();
+    host->steps = host->steps + 1;
   }
 }
 
@@ -705,6 +792,7 @@ __global__ void k_cycle_start(int nseg, int m, Krylov K, const int* __restrict__
   if (s >= nseg) return;
   const double b = sqrt(fmax(K.n2[s], 0.0));
   K.beta[s] = b;
+  K.n2[s] = 0.0;
   if (first) K.thr[s] = inner_tol[s] * b;
   K.est[s] = b;
   double* g = K.g + (int64_t)s * (m + 1);
@@ -717,30 +805,18 @@ __global__ void k_cycle_start(int nseg, int m, Krylov K, const int* __restrict__
   if (a) atomicAdd(K.nactive, 1);
 }
 
-// x[row] += sum_j y[seg][j] V_j[row], j < nv (+ *kdev)
-__global__ void k_seg_combine(int nu, int64_t N, const int* __restrict__ seg_of, int nv, const float* __restrict__ V,
+// x[row] = sum_j y[seg][j] V_j[row], j < ctl->k
+__global__ void k_seg_combine(int nu, int64_t N, const int* __restrict__ seg_of, const float* __restrict__ V,
                               int64_t ldv, const double* __restrict__ y, int ldy, float* __restrict__ x,
-                              const int* __restrict__ kdev = nullptr) {
+                              const StepCtl* __restrict__ ctl) {
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= N) return;
-  if (kdev) nv += *kdev;
+  const int nv = ctl->k;
   const double* ys = y + (int64_t)seg_of[r / nu] * ldy;
   double s = 0;
   for (int j = 0; j < nv; ++j) s += ys[j] * (double)V[(int64_t)j * ldv + r];
-  x[r] += (float)s;
+  x[r] = (float)s;
 }
-
-// end of a graph-captured Arnoldi step: k += 1; the cycle's while loop goes on while
-// k < m and some realisation is still active
-__global__ void k_step_ctl(int* __restrict__ kdev, const int* __restrict__ nactive, int m,
-                           cudaGraphConditionalHandle h) {
-  const int k = *kdev + 1;
-  *kdev = k;
-  cudaGraphSetConditional(h, (k < m && *nactive > 0) ? 1u : 0u);
-}
-
-// steps taken by a captured cycle, added up for the launch count
-__global__ void k_add_steps(const int* __restrict__ kdev, int* __restrict__ total) { *total += *kdev; }
 
 template <class T>
 __global__ void k_fill(T* p, int64_t n, T v) {
@@ -1177,18 +1253,18 @@ template <int TT>
 void launch_f32(const MfBatch& b, const float* x, float* y, cudaStream_t st, const int* mask, int mask_on) {
   const MfTile* tiles = b.tiles_s[TT == 64 ? 0 : (TT == 128 ? 1 : 2)];
   if (b.persist)
-    ::ibem::count_launch(), k_mf_apply_f32_persist<TT><<<b.persist_ctas, TT, 0, st>>>(
-        tiles, b.work, b.nwork, b.split.slices, b.seg_begin, mask, mask_on, b.gh, b.gl, b.matf, x, y);
+    launch_chained(k_mf_apply_f32_persist<TT>, b.persist_ctas, TT, st, tiles, b.work, b.nwork, b.split.slices, b.seg_begin,
+                   mask, mask_on, b.gh, b.gl, b.matf, x, y);
   else
-    ::ibem::count_launch(), k_mf_apply_f32<TT><<<dim3(b.ntiles_s[TT == 64 ? 0 : (TT == 128 ? 1 : 2)], b.split.slices,
-                                                      b.split.pieces), TT, 0, st>>>(
-        tiles, b.seg_begin, mask, mask_on, b.gh, b.gl, b.matf, x, y);
+    launch_chained(k_mf_apply_f32<TT>, dim3(b.ntiles_s[TT == 64 ? 0 : (TT == 128 ? 1 : 2)], b.split.slices, b.split.pieces),
+                   TT, st, tiles, b.seg_begin, mask, mask_on, b.gh, b.gl, b.matf, x, y);
 }
 
-ibem_status mf_apply_f32(const MfBatch& b, const float* x, float* y, cudaStream_t st, const int* mask, int mask_on) {
+ibem_status mf_apply_f32(const MfBatch& b, const float* x, float* y, cudaStream_t st, const int* mask, int mask_on,
+                         bool clear) {
   ProfScope ps(PROF_MF_F32, st, 0.0);
   if (b.nu == 60) return mf60_apply_f32(b, x, y, st, mask, mask_on);
-  IBEM_CUDA(cudaMemsetAsync(y, 0, sizeof(float) * b.N, st));
+  if (clear) IBEM_CUDA(cudaMemsetAsync(y, 0, sizeof(float) * b.N, st));
   if (b.tshape == 0) launch_f32<64>(b, x, y, st, mask, mask_on);
   else if (b.tshape == 2) launch_f32<256>(b, x, y, st, mask, mask_on);
   else launch_f32<128>(b, x, y, st, mask, mask_on);
@@ -1256,6 +1332,54 @@ ibem_status mf_block_jacobi(const MfBatch& b, float* P, cudaStream_t st) {
 // ------------------------------------------------------------------ solver
 namespace {
 
+// A HostCtl in pinned memory for the life of one solve.  The slots are a page per process,
+// allocated on first use; a solve that finds none free (or is told not to) runs step by step.
+struct HostSlot {
+  static constexpr int kSlots = 64;
+  HostCtl* ctl = nullptr;
+  explicit HostSlot(bool wanted) {
+    if (!wanted) return;
+    std::lock_guard<std::mutex> l(mu());
+    Slots& p = slots();
+    if (!p.mem && !p.tried) {
+      p.tried = true;
+      void* m = nullptr;
+      if (cudaHostAlloc(&m, kSlots * kStride, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess)
+        p.mem = static_cast<char*>(m);
+      else
+        cudaGetLastError();
+    }
+    for (int i = 0; p.mem && i < kSlots; ++i)
+      if (!p.used[i]) {
+        p.used[i] = true;
+        ctl = reinterpret_cast<HostCtl*>(p.mem + i * kStride);
+        break;
+      }
+  }
+  ~HostSlot() {
+    if (!ctl) return;
+    std::lock_guard<std::mutex> l(mu());
+    slots().used[(reinterpret_cast<char*>(ctl) - slots().mem) / kStride] = false;
+  }
+  HostSlot(const HostSlot&) = delete;
+  HostSlot& operator=(const HostSlot&) = delete;
+
+ private:
+  static constexpr size_t kStride = 64;   // a cache line each
+  struct Slots {
+    char* mem = nullptr;
+    bool tried = false, used[kSlots] = {};
+  };
+  static std::mutex& mu() {
+    static std::mutex m;
+    return m;
+  }
+  static Slots& slots() {
+    static Slots s;
+    return s;
+  }
+};
+
 struct MfSolver {
   const MfBatch& b;
   cudaStream_t st;
@@ -1269,24 +1393,16 @@ struct MfSolver {
   float* r32 = nullptr;  // N   residual of a restarted cycle
   int* done = nullptr;   // nseg
   double* tolv = nullptr;  // nseg: residual reduction asked of this GMRES solve
-  int* kdev = nullptr;     // Arnoldi step index of the graph-captured cycle
-  int* steps_dev = nullptr;  // Arnoldi steps run by the captured cycles (launch count)
+  StepCtl* ctl = nullptr;  // control of the cycle's steps
+  HostSlot host;           // the host's view of it (none: the host reads ctl after every step)
   Krylov K{};
   void* kmem = nullptr;
   int splits = 1;
-  // one GMRES cycle's Arnoldi steps as a CUDA graph: a while node whose body is one step
-  // (captured once per solver; the buffers it uses live as long as the solver)
-  bool use_graph = false;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  long long step_kernels = 0;   // kernels in one captured step
-  const MfPrecond* graph_pc = nullptr;
-  MfSolver(const MfBatch& bb, cudaStream_t s, int mm, bool graphs) : b(bb), st(s), m(mm), N(bb.N), use_graph(graphs) {
+  MfSolver(const MfBatch& bb, cudaStream_t s, int mm, bool ahead) : b(bb), st(s), m(mm), N(bb.N), host(ahead) {
     splits = (int)((b.nu * (int64_t)b.max_seg + kDotThreads * kDotRows - 1) / (kDotThreads * kDotRows));
   }
   ~MfSolver() {
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
+    if (host.ctl) cudaStreamSynchronize(st);   // after an error steps may still report to the slot
     free_async(V, st);
     free_async(z, st);
     free_async(w, st);
@@ -1308,7 +1424,7 @@ struct MfSolver {
     IBEM_CUDA(alloc_async((void**)&tolv, sizeof(double) * b.nseg, st));
     const size_t S = b.nseg;
     const size_t nd = S * ((size_t)(m + 1) * m + (m + 1) + 2 * (size_t)m + 5 + 2 * (size_t)(m + 1) + m);
-    const size_t ni = 3 * S + 3;
+    const size_t ni = 3 * S + 1 + 4;
     IBEM_CUDA(alloc_async((void**)&kmem, nd * sizeof(double) + sizeof(int) * ni, st));
     double* p = (double*)kmem;
     K.H = p; p += S * (m + 1) * m;
@@ -1328,8 +1444,7 @@ struct MfSolver {
     K.active = ip; ip += S;
     K.nsteps = ip; ip += S;
     K.nactive = ip; ip += 1;
-    kdev = ip; ip += 1;
-    steps_dev = ip;
+    ctl = reinterpret_cast<StepCtl*>(ip);
     IBEM_CUDA(cudaMemsetAsync(kmem, 0, nd * sizeof(double) + sizeof(int) * ni, st));
     return IBEM_OK;
   }
@@ -1342,83 +1457,69 @@ struct MfSolver {
   }
   template <class T>
   ibem_status seg_norm2(const T* v, double* n2) { return seg_norm2(v, n2, st); }
-  int read_nactive(ibem_status& s) {
+  int read_int(const int* p, ibem_status& s) {
     int h = 0;
-    cudaError_t e = cudaMemcpyAsync(&h, K.nactive, sizeof(int), cudaMemcpyDeviceToHost, st);
+    cudaError_t e = cudaMemcpyAsync(&h, p, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) s = cuda_fail(e, "gmres: read active count");
     return h;
   }
   // z = P v (layout 24: the block-sparse preconditioner; layout 60: the realisation's
   // block-Jacobi block, P.D holding one 60 x 60 block per realisation)
-  ibem_status precond(const MfPrecond& P, const float* v, float* z, const int* kd, int64_t vstride, cudaStream_t s) {
-    if (b.nu == 60) return mf60_precond_apply(b, P.D, v, z, kd, vstride, s);
-    ::ibem::count_launch(), k_precond_apply<<<nblk(N), 256, 0, s>>>(b.num, P.D, P.Q, P.nbr, v, z, kd, vstride);
+  ibem_status precond(const MfPrecond& P, const float* v, float* z, float* zero, const StepCtl* c, int64_t vstride) {
+    if (b.nu == 60) return mf60_precond_apply(b, P.D, v, z, c ? &c->k : nullptr, vstride, st);
+    launch_chained(k_precond_apply, nblk(N * kPreLanes), 256, st, b.num, P.D, P.Q, P.nbr, v, z, zero, c, vstride);
     IBEM_LAUNCH_CHECK("preconditioner");
     return IBEM_OK;
   }
-  // Arnoldi step k on stream s: w = As P v_k, two Gram-Schmidt passes against v_0..v_k,
-  // the per-realisation Hessenberg update, v_(k+1) = w / ||w||.  With kd (graph capture) the
-  // kernels read k from *kd instead.
-  ibem_status arnoldi_step(const MfPrecond& P, int k, const int* kd, cudaStream_t s) {
+  // The next Arnoldi step: w = As P v_k, two Gram-Schmidt passes against v_0..v_k, the
+  // per-realisation Hessenberg update, v_(k+1) = w / ||w||, k = ctl->k read by the kernels.
+  ibem_status arnoldi_step(const MfPrecond& P) {
     const int S = b.nseg;
-    const float* vk = kd ? V : V + (int64_t)k * N;
-    const int nv = kd ? 1 : k + 1;   // k_seg_dots / k_seg_sub add *kd
-    ibem_status r = precond(P, vk, z, kd, kd ? N : 0, s);
+    const dim3 dots(S, splits, (m + kDotCols - 1) / kDotCols);
+    ibem_status r = precond(P, V, z, w, ctl, N);
     if (r) return r;
-    r = mf_apply_f32(b, z, w, s, K.active, 1);   // converged realisations sit out
+    r = mf_apply_f32(b, z, w, st, K.active, 1, false);   // converged realisations sit out
     if (r) return r;
-    ProfScope pg(PROF_GMRES_OTHER, s);
-    IBEM_CUDA(cudaMemsetAsync(K.d1, 0, sizeof(double) * 2 * (size_t)S * (m + 1), s));
-    ::ibem::count_launch(), k_seg_dots<float><<<dim3(S, splits), kDotThreads, 0, s>>>(b.nu, b.seg_begin, nv, V, N, w, K.d1, m + 1, kd);
-    ::ibem::count_launch(), k_seg_sub<<<nblk(N), 256, 0, s>>>(b.nu, N, b.seg_of, nv, V, N, K.d1, m + 1, w, kd);
-    ::ibem::count_launch(), k_seg_dots<float><<<dim3(S, splits), kDotThreads, 0, s>>>(b.nu, b.seg_begin, nv, V, N, w, K.d2, m + 1, kd);
-    ::ibem::count_launch(), k_seg_sub<<<nblk(N), 256, 0, s>>>(b.nu, N, b.seg_of, nv, V, N, K.d2, m + 1, w, kd);
-    if ((r = seg_norm2(w, K.n2, s))) return r;
-    IBEM_CUDA(cudaMemsetAsync(K.nactive, 0, sizeof(int), s));
-    ::ibem::count_launch(), k_arnoldi_update<<<nblk(S, 128), 128, 0, s>>>(S, m, k, K, kd);
-    float* vnext = kd ? V : V + (int64_t)(k + 1) * N;
-    ::ibem::count_launch(), k_seg_scale<float, float><<<nblk(N), 256, 0, s>>>(b.nu, N, b.seg_of, K.inv, w, vnext, 0, kd,
-                                                                               kd ? N : 0);
+    ProfScope pg(PROF_GMRES_OTHER, st);
+    launch_chained(k_seg_dots<float>, dots, kDotThreads, st, b.nu, b.seg_begin, 0, V, N, w, K.d1, m + 1, ctl);
+    launch_chained(k_seg_sub, nblk(N), 256, st, b.nu, N, b.seg_of, V, N, K.d1, m + 1, w, nullptr, ctl);
+    launch_chained(k_seg_dots<float>, dots, kDotThreads, st, b.nu, b.seg_begin, 0, V, N, w, K.d2, m + 1, ctl);
+    launch_chained(k_seg_sub, nblk(N), 256, st, b.nu, N, b.seg_of, V, N, K.d2, m + 1, w, K.n2, ctl);
+    launch_chained(k_arnoldi_update, nblk(S, 128), 128, st, S, m, K, ctl, host.ctl);
+    launch_chained(k_seg_scale<float, float>, nblk(N), 256, st, b.nu, N, b.seg_of, K.inv, w, V, 0, ctl, N);
     IBEM_LAUNCH_CHECK("arnoldi step");
     return IBEM_OK;
   }
-  // The cycle graph: while (k < m and a realisation is active) { Arnoldi step *kdev; k += 1 }.
-  // Captured on a private stream (capture only records; the graph runs on st).
-  ibem_status build_graph(const MfPrecond& P) {
-    cudaStream_t cs = nullptr;
-    cudaGraphConditionalHandle h;
-    cudaGraphNodeParams cp{};
-    cudaGraphNode_t node;
-    IBEM_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-    cudaError_t e = cudaGraphCreate(&graph, 0);
-    if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault);
-    if (e == cudaSuccess) {
-      cp.type = cudaGraphNodeTypeConditional;
-      cp.conditional.handle = h;
-      cp.conditional.type = cudaGraphCondTypeWhile;
-      cp.conditional.size = 1;
-      e = cudaGraphAddNode(&node, graph, nullptr, nullptr, 0, &cp);
+  // The steps of a cycle, launched while the one before is still running: the update kernel reports through pinned memory, so the stream never runs dry
+  // between steps, and the kernels of steps past the end return at once.  (A while node of a
+  // CUDA graph around one captured step left the GPU idle for 37 us between steps, and its
+  // capture and instantiation cost 120 us a solve.)
+  ibem_status run_steps(const MfPrecond& P) {
+    constexpr int kAhead = 1;
+    ibem_status s = IBEM_OK;
+    if (!host.ctl) {   // step by step
+      do {
+        if ((s = arnoldi_step(P))) return s;
+      } while (!read_int(&ctl->stop, s) && !s);
+      return s;
     }
-    ibem_status r = IBEM_OK;
-    if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(cs, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                                            cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-      const long long before = launches_so_far();
-      r = arnoldi_step(P, 0, kdev, cs);
-      if (!r) ::ibem::count_launch(), k_step_ctl<<<1, 1, 0, cs>>>(kdev, K.nactive, m, h);
-      step_kernels = launches_so_far() - before;
-      add_launches(-step_kernels);   // captured, not run
-      cudaGraph_t body = nullptr;
-      const cudaError_t e2 = cudaStreamEndCapture(cs, &body);
-      if (e2 != cudaSuccess && !r) e = e2;
+    host.ctl->steps = 0;
+    host.ctl->stop = 0;
+    for (int launched = 0; launched < m; ++launched) {
+      long long spins = 0;
+      while (launched - __atomic_load_n(const_cast<int*>(&host.ctl->steps), __ATOMIC_ACQUIRE) > kAhead) {
+        // the flag can only stay behind when the stream failed; look at it now and then
+        if (++spins % 65536 == 0) {
+          const cudaError_t e = cudaStreamQuery(st);
+          if (e != cudaSuccess && e != cudaErrorNotReady) return cuda_fail(e, "gmres: Arnoldi steps");
+          if (e == cudaSuccess && launched - host.ctl->steps > kAhead) return fail(IBEM_ERR_CUDA, "gmres: lost an Arnoldi step");
+        }
+      }
+      if (host.ctl->stop) break;
+      if ((s = arnoldi_step(P))) return s;
     }
-    if (e == cudaSuccess && !r) e = cudaGraphInstantiate(&exec, graph, 0);
-    cudaStreamDestroy(cs);
-    if (r) return r;
-    if (e != cudaSuccess) return cuda_fail(e, "gmres: cycle graph");
-    graph_pc = &P;
-    return IBEM_OK;
+    return s;
   }
   // FP32 GMRES(m) with restarts on As d = rin, right-preconditioned by P; d overwritten.
   // Realisations flagged in `done` take no step.  Stops each realisation once
@@ -1426,9 +1527,6 @@ struct MfSolver {
   ibem_status gmres(const MfPrecond& P, int max_cycles) {
     const int S = b.nseg;
     ibem_status s = IBEM_OK;
-    // the phase profiler records events, which a graph's while loop cannot hold
-    const bool graphed = use_graph && !prof_on();
-    if (graphed && (!exec || graph_pc != &P) && (s = build_graph(P))) return s;
     IBEM_CUDA(cudaMemsetAsync(d, 0, sizeof(float) * N, st));
     for (int cyc = 0; cyc < max_cycles && !s; ++cyc) {
       const float* r = rin;
@@ -1438,43 +1536,21 @@ struct MfSolver {
         r = r32;
       }
       if ((s = seg_norm2(r, K.n2))) break;
-      IBEM_CUDA(cudaMemsetAsync(K.nactive, 0, sizeof(int), st));
+      IBEM_CUDA(cudaMemsetAsync(K.nactive, 0, sizeof(int) + sizeof(StepCtl), st));   // and ctl behind it
       ::ibem::count_launch(), k_cycle_start<<<nblk(S, 128), 128, 0, st>>>(S, m, K, done, cyc == 0, tolv);
       ::ibem::count_launch(), k_seg_scale<float, float><<<nblk(N), 256, 0, st>>>(b.nu, N, b.seg_of, K.inv, r, V, 0);
       IBEM_LAUNCH_CHECK("gmres cycle start");
-      const int na = read_nactive(s);
+      const int na = read_int(K.nactive, s);
       if (s || na == 0) break;
-      int k = 0;
-      if (graphed) {
-        IBEM_CUDA(cudaMemsetAsync(kdev, 0, sizeof(int), st));
-        IBEM_CUDA(cudaGraphLaunch(exec, st));
-        ::ibem::count_launch(), k_add_steps<<<1, 1, 0, st>>>(kdev, steps_dev);
-        IBEM_LAUNCH_CHECK("gmres cycle graph");
-      } else {
-        while (k < m) {
-          if ((s = arnoldi_step(P, k, nullptr, st))) break;
-          ++k;
-          if (read_nactive(s) == 0 || s) break;
-        }
-      }
-      if (s) break;
+      if ((s = run_steps(P))) break;
       // d += P V y
       ::ibem::count_launch(), k_hess_solve<<<nblk(S, 128), 128, 0, st>>>(S, m, K);
-      IBEM_CUDA(cudaMemsetAsync(w, 0, sizeof(float) * N, st));
-      ::ibem::count_launch(), k_seg_combine<<<nblk(N), 256, 0, st>>>(b.nu, N, b.seg_of, graphed ? 0 : k, V, N, K.yv, m, w,
-                                                                    graphed ? kdev : nullptr);
-      if ((s = precond(P, w, z, nullptr, 0, st))) break;
+      ::ibem::count_launch(), k_seg_combine<<<nblk(N), 256, 0, st>>>(b.nu, N, b.seg_of, V, N, K.yv, m, w, ctl);
+      if ((s = precond(P, w, z, nullptr, nullptr, 0))) break;
       ::ibem::count_launch(), k_add_f32<<<nblk(N), 256, 0, st>>>(N, z, d);
       IBEM_LAUNCH_CHECK("gmres update");
     }
     return s;
-  }
-  // kernels the captured cycles ran (read once, when the solve has synchronised)
-  long long graph_launches() {
-    if (!exec) return 0;
-    int h = 0;
-    if (cudaMemcpy(&h, steps_dev, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return 0;
-    return (long long)h * step_kernels;
   }
 };
 
@@ -1595,7 +1671,6 @@ ibem_status mf_solve(const MfBatch& b, const double* bvec, double* x, const MfPr
       rep[i].outer = outer_of[i];
       rep[i].inner = steps[i];
     }
-    if (!s) add_launches(g.graph_launches());
     for (int i = 0; i < S && !s; ++i)
       if (!(rep[i].rel_residual <= o.tol)) s = fail(IBEM_ERR_NOCONV, "mf solve: a realisation missed the tolerance");
   }

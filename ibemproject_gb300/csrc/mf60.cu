@@ -120,6 +120,7 @@ __global__ void __launch_bounds__(240) k_self_apply60(int64_t n, const int* __re
                                                       const int* __restrict__ mask, int mask_on,
                                                       const double* __restrict__ S, const T* __restrict__ x,
                                                       T* __restrict__ y) {
+  chain_wait();
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= n) return;
   const int64_t p = t / kNu;
@@ -138,6 +139,7 @@ __global__ void __launch_bounds__(kT)
     k_mf60_f32(const MfTile* __restrict__ tiles, const int* __restrict__ seg_begin, const int* __restrict__ mask,
                int mask_on, const float4* __restrict__ gh, const float4* __restrict__ gl,
                const SphMatF* __restrict__ mats, const float* __restrict__ x, float* __restrict__ y) {
+  chain_wait();
   __shared__ float4 sgh[kChunk], sgl[kChunk];
   __shared__ __align__(16) float sx[kChunk * kNu];
   const MfTile t = tiles[blockIdx.x];
@@ -309,10 +311,11 @@ __global__ void __launch_bounds__(kBjThreads) k_block_jacobi60(const double* __r
 }
 
 // z = P v with the realisation's block (Pseg[seg], 60 x 60 row-major); kdev: v is column
-// *kdev of a basis with column stride vstride (graph-captured Arnoldi steps)
+// *kdev of a basis with column stride vstride (Arnoldi steps)
 __global__ void k_precond_apply60(int num, const int* __restrict__ seg_of, const float* __restrict__ Pseg,
                                   const float* __restrict__ v, float* __restrict__ z, const int* __restrict__ kdev,
                                   int64_t vstride) {
+  chain_wait();
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= (int64_t)num * kNu) return;
   if (kdev) v += (int64_t)(*kdev) * vstride;
@@ -336,10 +339,9 @@ ibem_status mf60_self(const MfBatch& b, double* S, cudaStream_t st) {
 
 ibem_status mf60_apply_f32(const MfBatch& b, const float* x, float* y, cudaStream_t st, const int* mask,
                            int mask_on) {
-  ::ibem::count_launch(), k_self_apply60<float><<<(unsigned)((b.N + 239) / 240), 240, 0, st>>>(b.N, b.seg_of, mask, mask_on,
-                                                                                               b.self60, x, y);
-  ::ibem::count_launch(), k_mf60_f32<<<dim3(b.ntiles_s[0], b.split.slices, b.split.pieces), kT, 0, st>>>(
-      b.tiles_s[0], b.seg_begin, mask, mask_on, b.gh, b.gl, b.matf, x, y);
+  launch_chained(k_self_apply60<float>, (unsigned)((b.N + 239) / 240), 240, st, b.N, b.seg_of, mask, mask_on, b.self60, x, y);
+  launch_chained(k_mf60_f32, dim3(b.ntiles_s[0], b.split.slices, b.split.pieces), kT, st, b.tiles_s[0], b.seg_begin, mask,
+                 mask_on, b.gh, b.gl, b.matf, x, y);
   IBEM_LAUNCH_CHECK("mf60 apply f32");
   return IBEM_OK;
 }
@@ -370,8 +372,7 @@ ibem_status mf60_block_jacobi(const MfBatch& b, float* Pseg, cudaStream_t st) {
 ibem_status mf60_precond_apply(const MfBatch& b, const float* Pseg, const float* v, float* z, const int* kdev,
                                int64_t vstride, cudaStream_t st) {
   const int64_t n = (int64_t)b.num * kNu;
-  ::ibem::count_launch(), k_precond_apply60<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(b.num, b.seg_of, Pseg, v, z,
-                                                                                       kdev, vstride);
+  launch_chained(k_precond_apply60, (unsigned)((n + 255) / 256), 256, st, b.num, b.seg_of, Pseg, v, z, kdev, vstride);
   IBEM_LAUNCH_CHECK("mf60 preconditioner");
   return IBEM_OK;
 }

@@ -234,10 +234,10 @@ typedef struct {
   int max_outer;      /* FP64 refinement steps (0 = 8) */
   double tol;         /* target rel_residual (0 = 1e-10) */
   double inner_tol;   /* residual reduction asked of each FP32 GMRES solve (0 = 1e-5) */
-  int stepwise;       /* 0: the Arnoldi steps of each GMRES cycle run as one launch of a
-                       * captured CUDA graph (a device-side while loop: no host round trip
-                       * per step); 1: each step launched from the host, which reads the
-                       * count of still-active realisations after it */
+  int stepwise;       /* 0: the Arnoldi steps of a GMRES cycle are launched ahead of their
+                       * completion (a finished step reports through pinned memory, steps past
+                       * the cycle's end return at once); 1: the host reads after every step
+                       * whether a realisation is still active */
 } ibem_mf_options;
 
 typedef struct {
