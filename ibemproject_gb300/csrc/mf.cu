@@ -537,53 +537,54 @@ struct HostCtl {
   volatile int stop;
 };
 
-// z = P v for the block-sparse preconditioner: z_p = D_p v_p + sum_slot Q_(p,slot) v_nbr;
-// one thread per row (24 x 24 row-major blocks, float4 loads)
-__device__ __forceinline__ float dot24(const float* __restrict__ a, const float* __restrict__ b) {
-  const float4* x = reinterpret_cast<const float4*>(a);
-  const float4* y = reinterpret_cast<const float4*>(b);
-  float s = 0.f;
-#pragma unroll
-  for (int c = 0; c < kMfNu / 4; ++c) {
-    const float4 u = x[c], v = y[c];
-    s = fmaf(u.x, v.x, fmaf(u.y, v.y, fmaf(u.z, v.z, fmaf(u.w, v.w, s))));
-  }
-  return s;
-}
-// Four lanes share a row, each taking every fourth of its 16 neighbour slots (and one the
-// diagonal block), so that a small realisation's rows have four times the loads in flight.
-// zero: cleared (the step's product adds to it).  ctl (Arnoldi steps): v is column ctl->k of a basis with column stride vstride; nothing to
-// do once ctl->stop.
-constexpr int kPreLanes = 4;
-__global__ void __launch_bounds__(256) k_precond_apply(int num, const float* __restrict__ D, const float* __restrict__ Q,
-                                                       const int* __restrict__ nbr, const float* __restrict__ v,
-                                                       float* __restrict__ z, float* __restrict__ zero,
-                                                       const StepCtl* __restrict__ ctl, int64_t vstride) {
+// z = P v for the block-sparse preconditioner: z_p = D_p v_p + sum_slot Q_(p,slot) v_nbr
+// (24 x 24 row-major blocks).  zero: cleared (the step's product adds to it).  ctl (Arnoldi
+// steps): v is column ctl->k of a basis with column stride vstride; nothing to do once ctl->stop.
+//
+// Bound by reading Q once (37 KB a particle).  144 threads take a particle, each the same four
+// columns of the same row of all 17 blocks, so that a block is read in one piece and a thread
+// has 16 independent loads.  With a row per thread (and four lanes to a row) every cache line was
+// asked for by eight loads: 45 -> 25 us for 4,200 particles (154 MB).
+constexpr int kPreQ = kMfNu * kMfNu / 4;         // float4 of a block, threads of a particle
+constexpr int kPrePart = 2;                      // particles of a CTA
+constexpr int kPreThreads = kPreQ * kPrePart;
+__global__ void __launch_bounds__(kPreThreads) k_precond_apply(int num, const float* __restrict__ D,
+                                                               const float* __restrict__ Q, const int* __restrict__ nbr,
+                                                               const float* __restrict__ v, float* __restrict__ z,
+                                                               float* __restrict__ zero, const StepCtl* __restrict__ ctl,
+                                                               int64_t vstride) {
   chain_wait();
-  const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kPreLanes;
-  const int q = threadIdx.x % kPreLanes;
+  __shared__ float red[kPreThreads];
   if (ctl) {
     if (ctl->stop) return;
     v += (int64_t)ctl->k * vstride;
   }
-  const bool in = t < (int64_t)num * kMfNu;
+  const int64_t p = (int64_t)blockIdx.x * kPrePart + threadIdx.x / kPreQ;
+  const int e = threadIdx.x % kPreQ, c = e % (kMfNu / 4);
+  const float4* v4 = reinterpret_cast<const float4*>(v) + c;
+  auto dot = [](const float4& a, const float4& b, float s) {
+    return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, s))));
+  };
   float s = 0.f;
-  if (in) {
-    const int64_t p = t / kMfNu;
-    const int r = (int)(t % kMfNu);
-    if (q == 0) s = dot24(D + t * kMfNu, v + p * kMfNu);
+  if (p < num) {
+    s = dot(reinterpret_cast<const float4*>(D)[p * kPreQ + e], v4[p * (kMfNu / 4)], 0.f);
     if (Q) {
+      const float4* q = reinterpret_cast<const float4*>(Q) + p * kKnn * kPreQ + e;
+      const int* nb = nbr + p * kKnn;
 #pragma unroll
-      for (int k = q; k < kKnn; k += kPreLanes) {
-        const int j = nbr[p * kKnn + k];
-        if (j >= 0) s += dot24(Q + ((p * kKnn + k) * kMfNu + r) * kMfNu, v + (int64_t)j * kMfNu);
+      for (int k = 0; k < kKnn; ++k) {
+        const int j = nb[k];
+        if (j >= 0) s = dot(q[k * kPreQ], v4[(int64_t)j * (kMfNu / 4)], s);
       }
     }
   }
-  s += __shfl_xor_sync(0xffffffffu, s, 1);
-  s += __shfl_xor_sync(0xffffffffu, s, 2);
-  if (in && q == 0) z[t] = s;
-  if (in && q == 1 && zero) zero[t] = 0.f;
+  red[threadIdx.x] = s;
+  __syncthreads();
+  const int64_t row = (int64_t)blockIdx.x * kPrePart * kMfNu + threadIdx.x;
+  if (threadIdx.x >= kPrePart * kMfNu || row >= (int64_t)num * kMfNu) return;
+  const float* r = red + threadIdx.x * (kMfNu / 4);
+  z[row] = ((r[0] + r[1]) + (r[2] + r[3])) + (r[4] + r[5]);
+  if (zero) zero[row] = 0.f;
 }
 
 // out[seg * ldo + j] += sum over the segment's rows of V_j[row] * w[row], j < nv (Arnoldi steps:
@@ -1032,7 +1033,8 @@ ibem_status mf_batch_init(MfBatch& b, const ibem_e3d_batch& in, cudaStream_t st,
   IBEM_LAUNCH_CHECK("mf prep");
   if (b.nu == 60) {
     IBEM_CUDA(alloc_async((void**)&b.self60, sizeof(double) * 3600 * in.nseg, st));
-    if (ibem_status q = mf60_self(b, b.self60, st)) return q;
+    IBEM_CUDA(alloc_async((void**)&b.self60f, sizeof(float) * 3600 * in.nseg, st));
+    if (ibem_status q = mf60_self(b, st)) return q;
   }
   // the host vectors above must outlive the copies
   IBEM_CUDA(cudaStreamSynchronize(st));
@@ -1049,6 +1051,7 @@ void mf_batch_free(MfBatch& b) {
   free_async(b.matf, st);
   free_async(b.mats, st);
   free_async(b.self60, st);
+  free_async(b.self60f, st);
   free_async(b.dr, st);
   free_async(b.dc, st);
   free_async(b.tiles, st);
@@ -1468,7 +1471,7 @@ struct MfSolver {
   // block-Jacobi block, P.D holding one 60 x 60 block per realisation)
   ibem_status precond(const MfPrecond& P, const float* v, float* z, float* zero, const StepCtl* c, int64_t vstride) {
     if (b.nu == 60) return mf60_precond_apply(b, P.D, v, z, c ? &c->k : nullptr, vstride, st);
-    launch_chained(k_precond_apply, nblk(N * kPreLanes), 256, st, b.num, P.D, P.Q, P.nbr, v, z, zero, c, vstride);
+    launch_chained(k_precond_apply, nblk(b.num, kPrePart), kPreThreads, st, b.num, P.D, P.Q, P.nbr, v, z, zero, c, vstride);
     IBEM_LAUNCH_CHECK("preconditioner");
     return IBEM_OK;
   }

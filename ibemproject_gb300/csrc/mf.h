@@ -93,6 +93,7 @@ struct MfBatch {
   SphMatF* matf = nullptr;    // per segment, divided by mu0
   SphMat* mats = nullptr;     // per segment, FP64, divided by mu0 (scaled system)
   double* self60 = nullptr;   // layout 60: own block of each realisation's particles, column-major (scaled system)
+  float* self60f = nullptr;   // the same in FP32
   double* dr = nullptr;       // N: row scaling
   double* dc = nullptr;       // N: column scaling
   MfTile* tiles = nullptr;
@@ -111,12 +112,12 @@ struct MfBatch {
 };
 
 // layout-60 products (mf60.cu; y is overwritten): FP32 and FP64 (the double-float entry points
-// fall back to FP64 there), the realisations' block-Jacobi inverses (Pseg: nseg x 60 x 60) and their
+// fall back to FP64 there), the realisations' block-Jacobi inverses (Pseg: nseg x 60 x 60, by columns) and their
 // application
 ibem_status mf60_apply_f32(const MfBatch& b, const float* x, float* y, cudaStream_t st, const int* mask, int mask_on);
 ibem_status mf60_apply_f64(const MfBatch& b, const double* x, double* y, cudaStream_t st, const int* mask,
                            int mask_on);
-ibem_status mf60_self(const MfBatch& b, double* S, cudaStream_t st);   // fills b.self60 (nseg x 60 x 60)
+ibem_status mf60_self(const MfBatch& b, cudaStream_t st);   // fills b.self60 and b.self60f (nseg x 60 x 60)
 ibem_status mf60_block_jacobi(const MfBatch& b, float* Pseg, cudaStream_t st);
 ibem_status mf60_precond_apply(const MfBatch& b, const float* Pseg, const float* v, float* z, const int* kdev,
                                int64_t vstride, cudaStream_t st);

@@ -98,7 +98,8 @@ __device__ __noinline__ void pair_inside(double x0, double x1, double x2, double
 // Own block of a realisation's particles (unit sphere at x = 0 plus C0, moduli / mu0; the same
 // for all of them in the scaled system): S[seg][column][row].  One CTA per realisation, the
 // nine sub-blocks by one thread of a warp each.
-__global__ void __launch_bounds__(288) k_self60(const SphMat* __restrict__ mats, double* __restrict__ S) {
+__global__ void __launch_bounds__(288) k_self60(const SphMat* __restrict__ mats, double* __restrict__ S,
+                                                float* __restrict__ Sf) {
   __shared__ double M[kNu * kNu];
   for (int i = threadIdx.x; i < kNu * kNu; i += blockDim.x) M[i] = 0.0;
   __syncthreads();
@@ -111,26 +112,50 @@ __global__ void __launch_bounds__(288) k_self60(const SphMat* __restrict__ mats,
   __syncthreads();
   if (threadIdx.x == 0) sph_self60(mc, put);
   __syncthreads();
-  for (int i = threadIdx.x; i < kNu * kNu; i += blockDim.x) S[(int64_t)blockIdx.x * kNu * kNu + i] = M[i];
+  for (int i = threadIdx.x; i < kNu * kNu; i += blockDim.x) {
+    S[(int64_t)blockIdx.x * kNu * kNu + i] = M[i];
+    Sf[(int64_t)blockIdx.x * kNu * kNu + i] = (float)M[i];
+  }
 }
 
-// y = own block times the particle's coefficients, or 0 for a realisation masked out
+// Row of M x with a realisation's 60 x 60 block stored by columns: a warp's rows are neighbours.
+__device__ __forceinline__ float block60_row(const float* __restrict__ m, const float* __restrict__ x) {
+  const float4* x4 = reinterpret_cast<const float4*>(x);
+  float s = 0.f;
+#pragma unroll
+  for (int c = 0; c < kNu / 4; ++c) {
+    const float4 v = x4[c];
+    s = fmaf(m[(4 * c) * kNu], v.x, s);
+    s = fmaf(m[(4 * c + 1) * kNu], v.y, s);
+    s = fmaf(m[(4 * c + 2) * kNu], v.z, s);
+    s = fmaf(m[(4 * c + 3) * kNu], v.w, s);
+  }
+  return s;
+}
+
+// y = own block times the particle's coefficients, or 0 for a realisation masked out.  The FP32
+// form reads an FP32 copy of the blocks: converting their entries took the FP64 pipe 13 of
+// 17 us for 2,100 particles.
 template <class T>
 __global__ void __launch_bounds__(240) k_self_apply60(int64_t n, const int* __restrict__ seg_of,
                                                       const int* __restrict__ mask, int mask_on,
-                                                      const double* __restrict__ S, const T* __restrict__ x,
+                                                      const T* __restrict__ S, const T* __restrict__ x,
                                                       T* __restrict__ y) {
   chain_wait();
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= n) return;
   const int64_t p = t / kNu;
-  const int r = (int)(t % kNu), seg = seg_of[p];
+  const int seg = seg_of[p];
   T s = T(0);
   if (!mask || mask[seg] == mask_on) {
-    const double* m = S + (int64_t)seg * kNu * kNu + r;
+    const T* m = S + (int64_t)seg * kNu * kNu + t % kNu;
     const T* v = x + p * kNu;
+    if constexpr (sizeof(T) == 4) {
+      s = block60_row(m, v);
+    } else {
 #pragma unroll 10
-    for (int c = 0; c < kNu; ++c) s += (T)m[c * kNu] * v[c];
+      for (int c = 0; c < kNu; ++c) s += m[c * kNu] * v[c];
+    }
   }
   y[t] = s;
 }
@@ -261,85 +286,99 @@ __global__ void __launch_bounds__(kT)
   for (int r = 0; r < NR; ++r) atomicAdd(o + r, acc[r] * (RO == 0 ? 1.0 : RO == 1 ? as : as * as));
 }
 
-// The own block of a realisation's particles inverted by Gauss-Jordan with partial pivoting in
-// FP64: one CTA of 64 threads per realisation, the 60 x 120 augmented matrix in dynamic shared
-// memory (57.6 KB).
-constexpr int kBjThreads = 64;
-constexpr size_t kBjSmem = sizeof(double) * kNu * (2 * kNu + 1);
+// The own block of a realisation's particles inverted by Gauss-Jordan elimination in place, with
+// partial pivoting, in FP64; one CTA per realisation.  P is stored by columns, as its product
+// reads it.  Bound by the FP64 pipe (3,600 multiply-adds a step at 2 per clock) and three
+// barriers and a pivot search a step: 154 us; on the augmented matrix with 64 threads and a
+// serial search 711 us.
+constexpr int kBjThreads = 512;
 __global__ void __launch_bounds__(kBjThreads) k_block_jacobi60(const double* __restrict__ S, float* __restrict__ P) {
-  extern __shared__ double smem[];
-  double (*M)[2 * kNu + 1] = reinterpret_cast<double (*)[2 * kNu + 1]>(smem);
-  __shared__ int piv;
-  __shared__ double f[kNu];
+  __shared__ double M[kNu][kNu + 1];
+  __shared__ double f[kNu], ipiv;
+  __shared__ int piv[kNu], from[kNu];
   const int p = blockIdx.x;
   const int t = threadIdx.x;
-  for (int i = t; i < kNu * 2 * kNu; i += kBjThreads) {
-    const int r = i / (2 * kNu), c = i % (2 * kNu);
-    M[r][c] = c < kNu ? S[(int64_t)p * kNu * kNu + c * kNu + r] : (c - kNu == r ? 1.0 : 0.0);
-  }
+  for (int i = t; i < kNu * kNu; i += kBjThreads) M[i % kNu][i / kNu] = S[(int64_t)p * kNu * kNu + i];
   __syncthreads();
   for (int k = 0; k < kNu; ++k) {
-    if (t == 0) {
-      int best = k;
-      for (int r = k + 1; r < kNu; ++r)
-        if (fabs(M[r][k]) > fabs(M[best][k])) best = r;
-      piv = best;
+    if (t < 32) {   // the first of the largest entries of column k
+      double v = t >= k ? fabs(M[t][k]) : -1.0;
+      int r = t;
+      if (t + 32 < kNu && t + 32 >= k && fabs(M[t + 32][k]) > v) {
+        v = fabs(M[t + 32][k]);
+        r = t + 32;
+      }
+      for (int o = 16; o; o >>= 1) {
+        const double vo = __shfl_xor_sync(0xffffffffu, v, o);
+        const int ro = __shfl_xor_sync(0xffffffffu, r, o);
+        if (vo > v || (vo == v && ro < r)) {
+          v = vo;
+          r = ro;
+        }
+      }
+      if (t == 0) {
+        r = r >= k ? r : k;   // no number in the column
+        const double d = M[r][k];
+        piv[k] = r;
+        ipiv = d != 0.0 ? 1.0 / d : 0.0;
+      }
+    } else if (t >= 64 && t < 64 + kNu) {
+      f[t - 64] = M[t - 64][k];
     }
     __syncthreads();
-    const int pr = piv;
-    if (pr != k)
-      for (int c = t; c < 2 * kNu; c += kBjThreads) {
-        const double v = M[k][c];
-        M[k][c] = M[pr][c];
-        M[pr][c] = v;
-      }
+    const int pr = piv[k];
+    if (t < kNu) {   // swap rows k and pr, scale row k
+      const double a = M[k][t], b = M[pr][t];
+      M[pr][t] = a;
+      M[k][t] = t == k ? ipiv : b * ipiv;
+    }
     __syncthreads();
-    const double d = M[k][k];
-    const double id = d != 0.0 ? 1.0 / d : 0.0;
-    __syncthreads();
-    for (int c = t; c < 2 * kNu; c += kBjThreads) M[k][c] *= id;
-    for (int r = t; r < kNu; r += kBjThreads) f[r] = M[r][k];
-    __syncthreads();
-    for (int i = t; i < kNu * 2 * kNu; i += kBjThreads) {
-      const int r = i / (2 * kNu), c = i % (2 * kNu);
-      if (r != k) M[r][c] -= f[r] * M[k][c];
+    for (int i = t; i < kNu * kNu; i += kBjThreads) {
+      const int r = i / kNu, c = i % kNu;
+      if (r != k) M[r][c] = (c == k ? 0.0 : M[r][c]) - f[r == pr ? k : r] * M[k][c];
     }
     __syncthreads();
   }
+  if (t == 0) {   // the row swaps, undone on the columns of the inverse
+    for (int c = 0; c < kNu; ++c) from[c] = c;
+    for (int k = kNu - 1; k >= 0; --k) {
+      const int c = from[k];
+      from[k] = from[piv[k]];
+      from[piv[k]] = c;
+    }
+  }
+  __syncthreads();
   float* o = P + (int64_t)kNu * kNu * p;
-  for (int i = t; i < kNu * kNu; i += kBjThreads) o[i] = (float)M[i / kNu][kNu + i % kNu];
+  for (int i = t; i < kNu * kNu; i += kBjThreads) o[i] = (float)M[i % kNu][from[i / kNu]];
 }
 
-// z = P v with the realisation's block (Pseg[seg], 60 x 60 row-major); kdev: v is column
-// *kdev of a basis with column stride vstride (Arnoldi steps)
-__global__ void k_precond_apply60(int num, const int* __restrict__ seg_of, const float* __restrict__ Pseg,
-                                  const float* __restrict__ v, float* __restrict__ z, const int* __restrict__ kdev,
-                                  int64_t vstride) {
+// z = P v with the realisation's block (Pseg[seg], 60 x 60 by columns); kdev: v is column
+// *kdev of a basis with column stride vstride (Arnoldi steps).  With the block by rows a warp's
+// loads touched 32 lines each: 13.0 -> 4.3 us for 2,100 particles.
+__global__ void __launch_bounds__(240) k_precond_apply60(int num, const int* __restrict__ seg_of,
+                                                         const float* __restrict__ Pseg, const float* __restrict__ v,
+                                                         float* __restrict__ z, const int* __restrict__ kdev,
+                                                         int64_t vstride) {
   chain_wait();
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= (int64_t)num * kNu) return;
   if (kdev) v += (int64_t)(*kdev) * vstride;
   const int64_t p = t / kNu;
-  const int r = (int)(t % kNu);
-  const float* row = Pseg + (int64_t)seg_of[p] * kNu * kNu + (int64_t)r * kNu;
-  const float* vp = v + p * kNu;
-  float s = 0.f;
-#pragma unroll 4
-  for (int c = 0; c < kNu; ++c) s = fmaf(row[c], vp[c], s);
-  z[t] = s;
+  z[t] = block60_row(Pseg + (int64_t)seg_of[p] * kNu * kNu + t % kNu, v + p * kNu);
 }
 
 }  // namespace
 
-ibem_status mf60_self(const MfBatch& b, double* S, cudaStream_t st) {
-  ::ibem::count_launch(), k_self60<<<b.nseg, 288, 0, st>>>(b.mats, S);
+ibem_status mf60_self(const MfBatch& b, cudaStream_t st) {
+  ::ibem::count_launch(), k_self60<<<b.nseg, 288, 0, st>>>(b.mats, b.self60, b.self60f);
   IBEM_LAUNCH_CHECK("mf60 own blocks");
   return IBEM_OK;
 }
 
 ibem_status mf60_apply_f32(const MfBatch& b, const float* x, float* y, cudaStream_t st, const int* mask,
                            int mask_on) {
-  launch_chained(k_self_apply60<float>, (unsigned)((b.N + 239) / 240), 240, st, b.N, b.seg_of, mask, mask_on, b.self60, x, y);
+  launch_chained(k_self_apply60<float>, (unsigned)((b.N + 239) / 240), 240, st, b.N, b.seg_of, mask, mask_on,
+                 b.self60f, x, y);
   launch_chained(k_mf60_f32, dim3(b.ntiles_s[0], b.split.slices, b.split.pieces), kT, st, b.tiles_s[0], b.seg_begin, mask,
                  mask_on, b.gh, b.gl, b.matf, x, y);
   IBEM_LAUNCH_CHECK("mf60 apply f32");
@@ -363,8 +402,7 @@ ibem_status mf60_apply_f64(const MfBatch& b, const double* x, double* y, cudaStr
 }
 
 ibem_status mf60_block_jacobi(const MfBatch& b, float* Pseg, cudaStream_t st) {
-  IBEM_CUDA(cudaFuncSetAttribute(k_block_jacobi60, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBjSmem));
-  ::ibem::count_launch(), k_block_jacobi60<<<b.nseg, kBjThreads, kBjSmem, st>>>(b.self60, Pseg);
+  ::ibem::count_launch(), k_block_jacobi60<<<b.nseg, kBjThreads, 0, st>>>(b.self60, Pseg);
   IBEM_LAUNCH_CHECK("mf60 block jacobi");
   return IBEM_OK;
 }
@@ -372,7 +410,7 @@ ibem_status mf60_block_jacobi(const MfBatch& b, float* Pseg, cudaStream_t st) {
 ibem_status mf60_precond_apply(const MfBatch& b, const float* Pseg, const float* v, float* z, const int* kdev,
                                int64_t vstride, cudaStream_t st) {
   const int64_t n = (int64_t)b.num * kNu;
-  launch_chained(k_precond_apply60, (unsigned)((n + 255) / 256), 256, st, b.num, b.seg_of, Pseg, v, z, kdev, vstride);
+  launch_chained(k_precond_apply60, (unsigned)((n + 239) / 240), 240, st, b.num, b.seg_of, Pseg, v, z, kdev, vstride);
   IBEM_LAUNCH_CHECK("mf60 preconditioner");
   return IBEM_OK;
 }

@@ -79,3 +79,21 @@ def test_products_against_matrix(sizes, overlap):
                 sel = order[rows] == o
                 scale = np.abs(dr[rows][:, None] * A * dc[rows])[sel].sum(axis=1).max()
                 assert np.abs(y[rows] - want)[sel].max() <= tol * scale, (precision, s, o)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nu0", [0.0, 0.3, 0.49])
+def test_block_jacobi_inverts_the_own_block(nu0):
+    """A realisation of one particle is its own block: the FP32 inverse leaves 1e-4 of a residual at
+    most (rounding times the block's condition, about 100), so refinement to 1e-11 takes at most
+    three GMRES calls of at most two steps."""
+    import torch
+
+    from ibemproject_gb300 import batch as B, cases
+    cs = [cases.generated_case(1, 0.01, 0.2, seed=k, E1=70e9 * (0.2 + 4 * k), nu0=nu0) for k in range(5)]
+    bt = B.DeviceBatch(cs, layout=60)
+    dr, _ = bt.scalings()
+    b = torch.from_numpy(np.random.default_rng(4).standard_normal(bt.N) / dr).cuda()
+    _, reps = B.solve(bt, b, B.PRECOND_BLOCK_JACOBI, tol=1e-11)
+    for r in reps:
+        assert r.rel_residual <= 1e-11 and r.outer <= 3 and r.inner <= 6, (r.outer, r.inner)
