@@ -16,7 +16,7 @@
 // tensors symmetric in their first two indices, V_n and J_m the sphere's radial potentials,
 // Ps = V_0 - V_1 and Q = V_1 - V_2 and a number the rung of their ladder of derivatives in
 // u = |x|^2 / 2 (V_n^(k) = -J_{n+1}^(k-1), J_m' = -(2m+3) J_{m+1} outside, 0 inside), t = 1 - nu0:
-//   L_ikl = F_ikl + F_ilk,  M_ijk = L_ijk + L_jik,  w_n = F_mmn,  v_n = F_mnm         (source only)
+//   L, S, w, v: sums of F, formed once per source (contract_num.cuh)
 //   Ep_ij = F_ijl x_l,  N_ik = L_ikl x_l,  n = N x,  k = N x / 2 + N' x
 //   Z  = 2 t (Ph2 E x + V1_2 n / 2 + V1_1 v),            Zu the same one rung up
 //   dB = 2 Ps3 E x + Q3 k + 2 Q2 v + b2 w,  W = dB - Z   (b_k = Q_k - 2 nu V1_{k-1})
@@ -25,146 +25,15 @@
 //   r_ij  = p_i x_j + p_j x_i + C0 E_ij - 2 Q2 Ep_ij + C2 (N_ij + N_ji) + d_ij B,   p = A x / 2 + W
 //   R_ij  = C0u E_ij - 2 Q3 Ep_ij + C2u (N_ij + N_ji) + d_ij A
 //   Y_ik  = cE E_ik - 2 Q3 Ep_ik + 2 Q3 N_ki + C2u N_ik + dA_k x_i / 2 + (Au x_i / 2 + Wu_i) x_k + d_ik A
-//   g_ijk = R_ij x_k + Y_ik x_j + Y_jk x_i - 2 Q2 F_ijk + C2 M_ijk + d_ij dB_k + d_ik W_j + d_jk W_i
+//   g_ijk = R_ij x_k + Y_ik x_j + Y_jk x_i + C1 F_ijk + C2 S_ijk + d_ij dB_k + d_ik W_j + d_jk W_i
 // About 430 multiply-adds per pair (1,140 additions and multiplications, most of them not
 // fusable, when r and the tensors of g were expanded term by term from E and F; ~6,000 for the
 // generated block and its 576 multiply-adds).  The products that use it are bound by the
 // arithmetic pipe of their type (FP64, double-float and FP32), so their time is this count.
 #pragma once
-#include "gen_sphere_common.cuh"   // first: IBEM_HD and IBEM_INLINE
-
-#include "dfnum.cuh"
-#include "fp64_math.cuh"
+#include "contract_num.cuh"
 
 namespace ibem {
-
-IBEM_HD IBEM_INLINE float rsqrt_t(float x) {
-#ifdef __CUDA_ARCH__
-  return rsqrtf(x);
-#else
-  return 1.0f / sqrtf(x);
-#endif
-}
-IBEM_HD IBEM_INLINE double rsqrt_t(double x) { return rsqrt_h3(x); }
-
-// A sum of products: plain for float and double, compensated (dfloat.cuh: 12 instead of 18
-// FP32 instructions a term) for double-float numbers.
-template <class R>
-struct Sum {
-  R s;
-  IBEM_HD IBEM_INLINE explicit Sum(R a) : s(a) {}
-  IBEM_HD IBEM_INLINE Sum(R a, R b) : s(a * b) {}
-  IBEM_HD IBEM_INLINE void add(R a, R b) { s = s + a * b; }
-  IBEM_HD IBEM_INLINE R val() const { return s; }
-};
-template <>
-struct Sum<DF> {
-  dacc s;
-  IBEM_HD IBEM_INLINE explicit Sum(DF a) : s(dacc_of(a.v)) {}
-  IBEM_HD IBEM_INLINE Sum(DF a, DF b) : s(dacc_prod(a.v, b.v)) {}
-  IBEM_HD IBEM_INLINE void add(DF a, DF b) { dacc_fma(s, a.v, b.v); }
-  IBEM_HD IBEM_INLINE DF val() const { return DF(dacc_val(s)); }
-};
-// times a power of two (exact) or another FP32 constant
-IBEM_HD IBEM_INLINE float pow2_t(float c, float x) { return c * x; }
-IBEM_HD IBEM_INLINE double pow2_t(float c, double x) { return (double)c * x; }
-IBEM_HD IBEM_INLINE DF pow2_t(float c, DF x) { return DF(dfloat{c * x.v.hi, c * x.v.lo}); }
-IBEM_HD IBEM_INLINE float mulc_t(float c, float x) { return c * x; }
-IBEM_HD IBEM_INLINE double mulc_t(float c, double x) { return (double)c * x; }
-IBEM_HD IBEM_INLINE DF mulc_t(float c, DF x) { return DF(x.v * c); }
-template <class R>
-IBEM_HD IBEM_INLINE R dot3_t(R a0, R b0, R a1, R b1, R a2, R b2) {
-  Sum<R> s(a0, b0);
-  s.add(a1, b1);
-  s.add(a2, b2);
-  return s.val();
-}
-
-// ---- record of a source: [E (6), tr E, -] [w (3), v (3), -, -] [F (18), -, -] [L (18), -, -] [M (18), -, -]
-// F, M: 3 (ij) + k, L: 6 i + (kl), pairs in the order 00 01 02 11 12 22.
-constexpr int kRecE = 0, kRecW = 8, kRecF = 16, kRecL = 36, kRecM = 56, kRecLen = 76;
-// Every entry of the record is a sum of at most four coefficients: their indices, a byte each
-// (24: none).
-struct MfRecTab {
-  unsigned v[kRecLen];
-};
-constexpr MfRecTab mf_rec_tab() {
-  MfRecTab t{};
-  const int pi[6] = {0, 0, 0, 1, 1, 2}, pj[6] = {0, 1, 2, 1, 2, 2};
-  const int at[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
-  struct F {
-    static constexpr unsigned pack(int a, int b = 24, int c = 24, int d = 24) {
-      return (unsigned)a | (unsigned)b << 8 | (unsigned)c << 16 | (unsigned)d << 24;
-    }
-  };
-  for (int e = 0; e < kRecLen; ++e) t.v[e] = F::pack(24);
-  for (int i = 0; i < 6; ++i) t.v[kRecE + i] = F::pack(i);
-  t.v[kRecE + 6] = F::pack(0, 3, 5);
-  for (int n = 0; n < 3; ++n) {
-    t.v[kRecW + n] = F::pack(6 + n, 6 + 9 + n, 6 + 15 + n);
-    t.v[kRecW + 3 + n] = F::pack(6 + 3 * at[0][n], 6 + 3 * at[1][n] + 1, 6 + 3 * at[2][n] + 2);
-  }
-  for (int i = 0; i < 18; ++i) t.v[kRecF + i] = F::pack(6 + i);
-  for (int i = 0; i < 3; ++i)
-    for (int q = 0; q < 6; ++q) {
-      const int k = pi[q], l = pj[q];
-      t.v[kRecL + 6 * i + q] = F::pack(6 + 3 * at[i][k] + l, 6 + 3 * at[i][l] + k);
-    }
-  for (int q = 0; q < 6; ++q)
-    for (int k = 0; k < 3; ++k) {
-      const int i = pi[q], j = pj[q];
-      t.v[kRecM + 3 * q + k] = F::pack(6 + 3 * q + k, 6 + 3 * at[i][k] + j, 6 + 3 * q + k, 6 + 3 * at[j][k] + i);
-    }
-  return t;
-}
-// entry of a record from its packed indices and the coefficients (c[24] = 0)
-template <class R>
-IBEM_HD IBEM_INLINE R mf_rec_entry(unsigned q, const R* c) {
-  return (c[q & 31u] + c[(q >> 8) & 31u]) + (c[(q >> 16) & 31u] + c[q >> 24]);
-}
-
-// loads of N consecutive numbers from a 16-byte boundary
-template <int N>
-IBEM_HD IBEM_INLINE void mf_ld(const float* p, float (&o)[N]) {
-#ifdef __CUDA_ARCH__
-#pragma unroll
-  for (int i = 0; i < N; i += 4) {
-    const float4 q = *reinterpret_cast<const float4*>(p + i);
-    o[i] = q.x;
-    o[i + 1] = q.y;
-    o[i + 2] = q.z;
-    o[i + 3] = q.w;
-  }
-#else
-  for (int i = 0; i < N; ++i) o[i] = p[i];
-#endif
-}
-template <int N>
-IBEM_HD IBEM_INLINE void mf_ld(const double* p, double (&o)[N]) {
-#ifdef __CUDA_ARCH__
-#pragma unroll
-  for (int i = 0; i < N; i += 2) {
-    const double2 q = *reinterpret_cast<const double2*>(p + i);
-    o[i] = q.x;
-    o[i + 1] = q.y;
-  }
-#else
-  for (int i = 0; i < N; ++i) o[i] = p[i];
-#endif
-}
-template <int N>
-IBEM_HD IBEM_INLINE void mf_ld(const DF* p, DF (&o)[N]) {
-#ifdef __CUDA_ARCH__
-#pragma unroll
-  for (int i = 0; i < N; i += 2) {
-    const float4 q = *reinterpret_cast<const float4*>(p + i);
-    o[i].v = dfloat{q.x, q.y};
-    o[i + 1].v = dfloat{q.z, q.w};
-  }
-#else
-  for (int i = 0; i < N; ++i) o[i] = p[i];
-#endif
-}
 
 // y += a b, rounded as an addition to y (for double-float numbers the sum is normalised)
 template <class R>
@@ -354,8 +223,9 @@ IBEM_HD IBEM_INLINE void sph_pair_raw24(R x0, R x1, R x2, R f, const R* __restri
         Y[i][j] = s.val();
       }
   }
-  R M[20];
-  mf_ld(rec + kRecM, M);
+  R S[20];
+  mf_ld(rec + kRecS, S);
+  const R C1 = C2 + f2;
   const R xx[3] = {pow2_t(2.f, x0), pow2_t(2.f, x1), pow2_t(2.f, x2)};
 #pragma unroll
   for (int t = 0; t < 6; ++t) {
@@ -367,16 +237,16 @@ IBEM_HD IBEM_INLINE void sph_pair_raw24(R x0, R x1, R x2, R f, const R* __restri
         Sum<R> s(i == c ? dB[c] + pow2_t(2.f, W[c]) : dB[c]);
         s.add(Y[i][c], xx[i]);
         s.add(Rr[t], x[c]);
-        s.add(Q2m, F[3 * t + c]);
-        s.add(C2, M[3 * t + c]);
+        s.add(C1, F[3 * t + c]);
+        s.add(C2, S[3 * t + c]);
         g = s.val();
       } else {
         Sum<R> s(i == c ? W[j] : (j == c ? W[i] : Rr[t] * x[c]));
         if (i == c || j == c) s.add(Rr[t], x[c]);
         s.add(Y[i][c], x[j]);
         s.add(Y[j][c], x[i]);
-        s.add(Q2m, F[3 * t + c]);
-        s.add(C2, M[3 * t + c]);
+        s.add(C1, F[3 * t + c]);
+        s.add(C2, S[3 * t + c]);
         g = s.val();
       }
       mf_acc(y[6 + 3 * t + c], row_scale, g);
