@@ -122,6 +122,7 @@ struct GridSync {
 //     original values of the (up to nb) rows it picked as pivots: cand[cta], flag f0[cta].
 //  2. The leader of every group of F consecutive CTAs waits for its members, runs the same
 //     elimination on their candidates and publishes its nb winners: lcand[g], flag f1[g].
+//     (One group, F = all CTAs: step 3 takes their candidates and this step is left out.)
 //  3. CTA 0 waits for every group, eliminates their winners and so fixes the nb pivot rows
 //     and the factored top block (L11 below the diagonal, U11 on and above it).  It turns
 //     the pivot order into LAPACK row exchanges (ipiv) and a short list of the rows >= nb
@@ -206,7 +207,7 @@ __device__ __forceinline__ unsigned calu_key(float av, int q) {
 }
 
 template <typename T, int R>
-__device__ __forceinline__ void calu_elim(T (&a)[R][kLeaf], bool (&live)[R], int k, T* s_top, T* s_pr, int* s_sel,
+__device__ __forceinline__ std::enable_if_t<sizeof(T) == 4> calu_elim(T (&a)[R][kLeaf], bool (&live)[R], int k, T* s_top, T* s_pr, int* s_sel,
                                           unsigned* s_key) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int nw = kPanelThreads / 32;
@@ -227,24 +228,31 @@ __device__ __forceinline__ void calu_elim(T (&a)[R][kLeaf], bool (&live)[R], int
       break;
     }
     const int bq = 1023 - (int)(key & 1023u);
-    // the owner thread alone publishes the pivot row: un-rotated into s_top[j] (the
-    // factored block) and rotated into s_pr (the update's operand, static offsets, zero
-    // where a[] holds multipliers)
+    // the owner thread alone publishes the pivot row, rotated as it holds it: into s_pr[kLeaf..]
+    // as it is and into s_pr[0..] with zeros where a[] holds multipliers (the update's operand).
+    // Wide stores at fixed offsets: one thread's instructions are the step's latency.
     if (tid == bq % kPanelThreads) {
       const int oi = bq / kPanelThreads;
 #pragma unroll
-      for (int c = 0; c < kLeaf; ++c) {
-        T v = a[0][c];
+      for (int c0 = 0; c0 < kLeaf; c0 += 4) {
+        float v[4], z[4];
 #pragma unroll
-        for (int i = 1; i < R; ++i) v = oi == i ? a[i][c] : v;  // selects, not an indexed read
-        s_top[j * kLdS + ((c + j) & (kLeaf - 1))] = v;
-        s_pr[c] = (c + j < kLeaf) ? v : (T)0;
+        for (int u = 0; u < 4; ++u) {
+          v[u] = a[0][c0 + u];
+#pragma unroll
+          for (int i = 1; i < R; ++i) v[u] = oi == i ? a[i][c0 + u] : v[u];  // selects, not an indexed read
+          z[u] = c0 + u + j < kLeaf ? v[u] : 0.f;
+        }
+        *reinterpret_cast<float4*>(s_pr + c0) = make_float4(z[0], z[1], z[2], z[3]);
+        *reinterpret_cast<float4*>(s_pr + kLeaf + c0) = make_float4(v[0], v[1], v[2], v[3]);
       }
 #pragma unroll
       for (int i = 0; i < R; ++i) live[i] = live[i] && oi != i;
       s_sel[j] = bq;
     }
     __syncthreads();
+    // un-rotated into the factored block
+    if (warp == nw - 1) s_top[j * kLdS + ((lane + j) & (kLeaf - 1))] = s_pr[kLeaf + lane];
     T pr[kLeaf];
 #pragma unroll
     for (int c = 0; c < kLeaf; ++c) pr[c] = s_pr[c];
@@ -362,6 +370,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_panel(T* __restrict__ P, i
   __shared__ int s_fail;
   const int cta = blockIdx.x, ncta = gridDim.x, tid = threadIdx.x;
   const int G = (ncta + F - 1) / F;
+  const bool flat = G == 1;   // the root takes the CTAs' candidates themselves
   const int r0 = cta * rows_per;
   const int nr = max(0, min(rows_per, m - r0));
   int* f0 = cb.flags;
@@ -397,7 +406,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_panel(T* __restrict__ P, i
     if (tid == 0) st_release_s32(f0 + cta, tag);
   }
   // ---- 2. group leaders: nb winners among the members' candidates
-  if (cta % F == 0) {
+  if (cta % F == 0 && !flat) {
     const int g = cta / F, gsz = min(F, ncta - cta);
     calu_wait(f0 + cta, gsz, tag, gs, &s_fail);
     if (s_fail) return;
@@ -431,16 +440,19 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_panel(T* __restrict__ P, i
   }
   // ---- 3. root: the nb pivots, the factored top block and the row exchanges
   if (cta == 0) {
-    calu_wait(f1, G, tag, gs, &s_fail);
+    const T* rv = flat ? cb.cand : cb.lcand;
+    const int* ri = flat ? cb.cidx : cb.lidx;
+    const int nroot = flat ? ncta : G;
+    calu_wait(flat ? f0 : f1, nroot, tag, gs, &s_fail);
     if (s_fail) return;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
       const int q = slot + SL * i;
-      live[i] = q < G * kLeaf && __ldcg(cb.lidx + q) >= 0;
+      live[i] = q < nroot * kLeaf && __ldcg(ri + q) >= 0;
 #pragma unroll
       for (int cc = 0; cc < NC; ++cc) {
         const int c = Q * cc + lq;
-        a[i][cc] = (live[i] && c < nb) ? __ldcg(cb.lcand + (size_t)q * kLeaf + c) : (T)0;
+        a[i][cc] = (live[i] && c < nb) ? __ldcg(rv + (size_t)q * kLeaf + c) : (T)0;
       }
     }
     calu_elim(a, live, nb, s_top, s_pr, s_sel, s_key);
@@ -449,7 +461,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_panel(T* __restrict__ P, i
       cb.top[j * kLeaf + c] = s_top[j * kLdS + c];
       cb.orig[j * kLeaf + c] = P[(int64_t)c * lda + j];
     }
-    if (tid < nb) s_meta[3 * kLeaf + 1 + tid] = __ldcg(cb.lidx + s_sel[tid]);
+    if (tid < nb) s_meta[3 * kLeaf + 1 + tid] = __ldcg(ri + s_sel[tid]);
     __syncthreads();
     if (tid == 0) {
       // pivot order -> sequential row exchanges; track where the original top rows go
@@ -1239,9 +1251,16 @@ static ibem_status panel(T* A, int64_t lda, int64_t k0, int64_t m, int nb, LuWor
   ncta = (int)((m + rows_per - 1) / rows_per);
   int F = 1;
   while (F * F < ncta) ++F;
+  if constexpr (sizeof(T) == 4) {
+    // FP32: one level of the tree (the root takes every CTA's candidates, F = ncta) up to 16 CTAs.
+    // An elimination is 32 dependent steps of two barriers each, a level costs one and an
+    // exchange through memory: 61 us a panel of 1,400 rows with two levels, 41 us with one.  With
+    // 32 CTAs the root's four rows a thread cost as much as the level saves.
+    if (ncta <= 2 * kPanelThreads / kLeaf) F = ncta;
+  }
   const int G = (ncta + F - 1) / F;
   // rows of the largest elimination (own rows, a group's or the root's candidates)
-  const int rows = std::max(rows_per, std::max(F, G) * kLeaf);
+  const int rows = std::max(rows_per, std::max(F, G) * kLeaf);   // (F = ncta: the root's)
   if (rows > 1024 || ncta > kCaluMaxCta) return fail(IBEM_ERR_ARG, "panel too tall for the panel kernel");
   const int sets = (rows + kPanelRows<T> - 1) / kPanelRows<T>;   // register sets of rows
   const void* fn = nullptr;
