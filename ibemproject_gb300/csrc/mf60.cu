@@ -27,6 +27,7 @@
 #include "gen_sphere60.cuh"
 #include "gen_sphere60_f32.cuh"
 #include "mf.h"
+#include "fp64_math.cuh"
 #include "mf60_contract.cuh"
 #include "prof.h"
 
@@ -36,21 +37,6 @@ namespace {
 constexpr int kNu = 60;
 constexpr int kT = kMf60Targets;   // targets per CTA
 constexpr int kChunk = 16;         // sources staged per chunk
-
-template <int RO>
-struct Rows;
-template <>
-struct Rows<0> {
-  static constexpr int off = 0, n = 6;
-};
-template <>
-struct Rows<1> {
-  static constexpr int off = 6, n = 18;
-};
-template <>
-struct Rows<2> {
-  static constexpr int off = 24, n = 36;
-};
 
 // acc[r] += v * xs[c]
 template <class T>
@@ -222,12 +208,41 @@ __global__ void __launch_bounds__(kT)
   for (int r = 0; r < kNu; ++r) atomicAdd(o + r, acc[r] * (r < 6 ? 1.f : r < 24 ? ph.w : ph.w * ph.w));
 }
 
-template <int RO>
+// The pairs of the FP64 product whose target centre lies inside the source sphere (overlapping
+// spheres; usually none), by the generated block: a few operations a pair to look for them.  In the
+// product's own loop the call cost its kernel 87 registers.
+__global__ void __launch_bounds__(kT)
+    k_mf60_inside(const MfTile* __restrict__ tiles, const int* __restrict__ seg_begin, const int* __restrict__ mask,
+                  int mask_on, const double* __restrict__ cen, const double* __restrict__ rad,
+                  const SphMat* __restrict__ mats, const double* __restrict__ x, double* __restrict__ y) {
+  const MfTile t = tiles[blockIdx.x];
+  if (mask && mask[t.seg] != mask_on) return;
+  const int hb0 = seg_begin[t.seg], he0 = seg_begin[t.seg + 1];
+  const int ns = gridDim.y * gridDim.z, per = (he0 - hb0 + ns - 1) / ns;
+  const int hb = hb0 + (blockIdx.y * gridDim.z + blockIdx.z) * per, he = min(he0, hb + per);
+  if (threadIdx.x >= t.ns) return;
+  const int s = t.s0 + threadIdx.x;
+  const double p0 = cen[3 * (int64_t)s], p1 = cen[3 * (int64_t)s + 1], p2 = cen[3 * (int64_t)s + 2];
+#pragma unroll 4
+  for (int h = hb; h < he; ++h) {
+    const double ia = 1.0 / rad[h];
+    const double x0 = (p0 - cen[3 * (int64_t)h]) * ia, x1 = (p1 - cen[3 * (int64_t)h + 1]) * ia,
+                 x2 = (p2 - cen[3 * (int64_t)h + 2]) * ia;
+    const double r2 = x0 * x0 + x1 * x1 + x2 * x2;
+    if (!(r2 > 1.0) && h != s)
+      pair_inside(x0, x1, x2, rad[s], ia, mats[t.seg], x + (int64_t)kNu * h, y + (int64_t)kNu * s);
+  }
+}
+
+// FP64 product, bound by the FP64 pipe: HI false, the rows of orders 0 and 1, and true, of order 2.
+// One kernel for all 60 rows spills; one per order turned each source's coefficients into the
+// frame of the offset three times (12 realisations of U[50, 300]: 4.3 ms a product, now 3.5).
+template <bool HI>
 __global__ void __launch_bounds__(kT)
     k_mf60_f64(const MfTile* __restrict__ tiles, const int* __restrict__ seg_begin, const int* __restrict__ mask,
                int mask_on, const double* __restrict__ cen, const double* __restrict__ rad,
                const SphMat* __restrict__ mats, const double* __restrict__ x, double* __restrict__ y) {
-  constexpr int NR = Rows<RO>::n;
+  constexpr int NR = HI ? 36 : 24;
   __shared__ double sc[kChunk * 4];
   __shared__ __align__(16) double sx[kChunk * kNu];
   const MfTile t = tiles[blockIdx.x];
@@ -266,24 +281,30 @@ __global__ void __launch_bounds__(kT)
       const double ia = sc[4 * hh + 3];
       const double x0 = (p0 - sc[4 * hh]) * ia, x1 = (p1 - sc[4 * hh + 1]) * ia, x2 = (p2 - sc[4 * hh + 2]) * ia;
       const double r2 = x0 * x0 + x1 * x1 + x2 * x2;
-      if (!(r2 > 1.0)) {
-        if (RO == 0 && h0 + hh != s)
-          pair_inside(x0, x1, x2, as, ia, mats[t.seg], x + (int64_t)kNu * (h0 + hh), y + (int64_t)kNu * s);
-        continue;
-      }
-      const double ir = rsqrt(r2);
+      if (!(r2 > 1.0)) continue;   // k_mf60_inside
+      const double ir = rsqrt_h3(r2);
       Mf60Frame<double> f;
       mf60_frame(x0 * ir, x1 * ir, x2 * ir, f);
       double A0[6], A1[6][3], A2[6][6];
       mf60_source(f, sx + kNu * hh, A0, A1, A2);
-      mf60_rows<RO>(f, A0, A1, A2, ir, RO == 0 ? 1.0 : RO == 1 ? ia : ia * ia, nu, acc);
+      if constexpr (HI) {
+        mf60_rows<2>(f, A0, A1, A2, ir, ia * ia, nu, acc);
+      } else {
+        mf60_rows<0>(f, A0, A1, A2, ir, 1.0, nu, acc);
+        mf60_rows<1>(f, A0, A1, A2, ir, ia, nu, acc + 6);
+      }
     }
   }
   if (!act) return;
-  mf60_map<RO>(kmu, klam, acc);
-  double* o = y + (int64_t)kNu * s + Rows<RO>::off;
+  if constexpr (HI) {
+    mf60_map<2>(kmu, klam, acc);
+  } else {
+    mf60_map<0>(kmu, klam, acc);
+    mf60_map<1>(kmu, klam, acc + 6);
+  }
+  double* o = y + (int64_t)kNu * s + (HI ? 24 : 0);
 #pragma unroll
-  for (int r = 0; r < NR; ++r) atomicAdd(o + r, acc[r] * (RO == 0 ? 1.0 : RO == 1 ? as : as * as));
+  for (int r = 0; r < NR; ++r) atomicAdd(o + r, acc[r] * (HI ? as * as : r < 6 ? 1.0 : as));
 }
 
 // The own block of a realisation's particles inverted by Gauss-Jordan elimination in place, with
@@ -390,12 +411,13 @@ ibem_status mf60_apply_f64(const MfBatch& b, const double* x, double* y, cudaStr
   const dim3 grid(b.ntiles_s[0], b.split_wide.slices, b.split_wide.pieces);
   ::ibem::count_launch(), k_self_apply60<double><<<(unsigned)((b.N + 239) / 240), 240, 0, st>>>(b.N, b.seg_of, mask, mask_on,
                                                                                                 b.self60, x, y);
-#define IBEM_MF60_F64(RO)                                                                                         \
-  ::ibem::count_launch(), k_mf60_f64<RO><<<grid, kT, 0, st>>>(b.tiles_s[0], b.seg_begin, mask, mask_on, b.cen, b.rad, \
+#define IBEM_MF60_F64(HI)                                                                                         \
+  ::ibem::count_launch(), k_mf60_f64<HI><<<grid, kT, 0, st>>>(b.tiles_s[0], b.seg_begin, mask, mask_on, b.cen, b.rad, \
                                                               b.mats, x, y)
-  IBEM_MF60_F64(2);
-  IBEM_MF60_F64(1);
-  IBEM_MF60_F64(0);
+  IBEM_MF60_F64(true);
+  IBEM_MF60_F64(false);
+  ::ibem::count_launch(), k_mf60_inside<<<grid, kT, 0, st>>>(b.tiles_s[0], b.seg_begin, mask, mask_on, b.cen, b.rad, b.mats,
+                                                             x, y);
 #undef IBEM_MF60_F64
   IBEM_LAUNCH_CHECK("mf60 apply f64");
   return IBEM_OK;
