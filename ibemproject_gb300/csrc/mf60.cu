@@ -11,15 +11,17 @@
 // source's powers of 1/r by a_h^-(row order) and the sums by a_s^(row order) once.
 //
 // One thread per target particle, 64 consecutive targets of one realisation per CTA, source
-// slices over gridDim.y (and their pieces over gridDim.z), partial sums added atomically to the target's own block times its
-// coefficients (k_self_apply60, which also clears the sums).  A target whose centre lies
-// inside a source (overlapping spheres) takes that pair from the generated dense block.
+// slices over gridDim.y (and their pieces over gridDim.z), partial sums added atomically to the
+// target's own block times its coefficients (k_self_apply60, which also clears the sums).  A
+// target whose centre lies inside a source (overlapping spheres) takes that pair from the
+// generated dense block (FP64: k_mf60_inside).
 //
 // Bound by the FP32 (FP64) multiply-adds.  FP32: one kernel for all 60 rows, which rotates a
-// source's coefficients once.  FP64: one kernel per row order, because 60 sums and 60 rotated
-// coefficients do not fit 255 registers; the rotation of the coefficients is repeated.
-// Measured, 12 realisations of 50 to 300 spheres (437,000 pairs): FP32 product 1.13 -> 0.14 ms,
-// FP64 product 45.2 -> 5.0 ms, against the generated blocks in 18 and 7 kernels.
+// source's coefficients once.  FP64: the rows of orders 0 and 1 in one kernel and those of order
+// 2 in another, because 60 sums and 60 rotated coefficients do not fit 255 registers; the
+// rotation of the coefficients is repeated.  Measured, 12 realisations of 50 to 300 spheres
+// (437,000 pairs): FP32 product 1.13 -> 0.09 ms, FP64 product 45.2 -> 3.5 ms, against the
+// generated blocks in 18 and 7 kernels.
 #include <cuda_runtime.h>
 
 #include <type_traits>
