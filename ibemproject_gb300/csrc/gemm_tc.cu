@@ -29,6 +29,7 @@
 
 #include "prof.h"
 #include "solver.h"
+#include "chain.cuh"
 #include "umma.cuh"
 
 namespace ibem {
@@ -47,6 +48,7 @@ constexpr int64_t kMaxKChunk = 8192;  // K is processed in chunks to bound the s
 // A (m x k, column-major, lda) -> hi/lo, K-major rows of length kp: out[i * kp + kk]
 __global__ void k_split_a(int64_t m, int64_t k, const float* __restrict__ A, int64_t lda, int64_t kp,
                           __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
+  ::ibem::chain_wait();
   __shared__ float t[32][33];
   const int64_t i0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
   for (int j = threadIdx.y; j < 32; j += blockDim.y) {
@@ -68,6 +70,7 @@ __global__ void k_split_a(int64_t m, int64_t k, const float* __restrict__ A, int
 // B (k x n, column-major, ldb) -> hi/lo, K-major rows of length kp: out[j * kp + kk]
 __global__ void k_split_b(int64_t k, int64_t n, const float* __restrict__ B, int64_t ldb, int64_t kp,
                           __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
+  ::ibem::chain_wait();
   const int64_t kk = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (kk >= kp) return;
   for (int64_t j = blockIdx.y; j < n; j += gridDim.y) {
@@ -316,10 +319,10 @@ ibem_status gemm_sub_f32_tc(int64_t m, int64_t n, int64_t k, const float* A, int
     __nv_bfloat16* blo = bhi + (size_t)n * kp;
     {
       ProfScope psplit(PROF_GEMM_SPLIT, st);
-    ::ibem::count_launch(), k_split_a<<<dim3((unsigned)((m + 31) / 32), (unsigned)(kp / 32)), dim3(32, 8), 0, st>>>(
-        m, kc, A + k0 * lda, lda, kp, ahi, alo);
-    ::ibem::count_launch(), k_split_b<<<dim3((unsigned)((kp + 255) / 256), (unsigned)std::min<int64_t>(n, 65535)), 256, 0, st>>>(
-        kc, n, B + k0, ldb, kp, bhi, blo);
+      launch_chained(k_split_a, dim3((unsigned)((m + 31) / 32), (unsigned)(kp / 32)), dim3(32, 8), st, m, kc, A + k0 * lda, lda,
+                     kp, ahi, alo);
+      launch_chained(k_split_b, dim3((unsigned)((kp + 255) / 256), (unsigned)std::min<int64_t>(n, 65535)), 256, st, kc, n,
+                     B + k0, ldb, kp, bhi, blo);
       IBEM_LAUNCH_CHECK("gemm_tc split");
     }
     alignas(64) CUtensorMap maps[4];

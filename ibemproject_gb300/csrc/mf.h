@@ -20,40 +20,13 @@
 
 #include "gen_sphere_common.cuh"
 #include "gen_sphere24_f32.cuh"
+#include "chain.cuh"
 #include "ibem_internal.h"
 
 namespace ibem {
 
 constexpr int kMfNu = 24;   // unknowns per particle of the matrix-free path
 constexpr int kKnn = 16;    // neighbours per particle of the learned preconditioner
-
-// Kernels of an Arnoldi step depend on each other and take a few microseconds each in a small
-// batch, as long as a launch.  They are launched so that the successor's launch overlaps the end
-// of its predecessor, and begin with chain_wait(): nothing is read or written before the
-// predecessor has finished and its writes are visible.  A kernel of few CTAs (kChainCtas, two
-// per SM) lets its successor's CTAs be set up as soon as its own have all started; one of many
-// leaves that to their end, because CTAs set up early crowd onto the SMs that are free first.
-constexpr unsigned kChainCtas = 304;
-__device__ __forceinline__ void chain_wait() {
-#ifdef __CUDA_ARCH__
-  if (gridDim.x * gridDim.y * gridDim.z <= kChainCtas) cudaTriggerProgrammaticLaunchCompletion();
-  cudaGridDependencySynchronize();
-#endif
-}
-template <class... P, class... A>
-inline void launch_chained(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t st, A... a) {
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t c{};
-  c.gridDim = grid;
-  c.blockDim = block;
-  c.stream = st;
-  c.attrs = &at;
-  c.numAttrs = 1;
-  count_launch();
-  (void)cudaLaunchKernelEx(&c, k, P(a)...);   // its error is the thread's last error
-}
 
 constexpr int kMf60Targets = 64;   // targets per CTA of the layout-60 products (tiles_s[0])
 

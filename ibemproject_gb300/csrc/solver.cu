@@ -37,6 +37,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "chain.cuh"
 #include "ibem_internal.h"
 #include "prof.h"
 #include "solver.h"
@@ -625,6 +626,7 @@ constexpr int kSwapCols = 4, kSwapThreads = 256, kSwapPerCta = kSwapThreads / 32
 template <typename T>
 __global__ void __launch_bounds__(kSwapThreads) k_laswp(T* __restrict__ A, int64_t lda, int64_t k0,
                                                         const int* __restrict__ meta, int nb, int64_t ncols) {
+  ::ibem::chain_wait();
   const int lane = threadIdx.x & 31;
   const int nd = meta[3 * kLeaf];
   const int w = lane < nb ? meta[3 * kLeaf + 1 + lane] : lane;
@@ -692,6 +694,7 @@ constexpr int kTrsmCols = 128;
 template <typename T, int NB>
 __global__ void __launch_bounds__(kTrsmCols) k_trsm_small_fixed(const T* __restrict__ L, int64_t ldl,
                                                                 T* __restrict__ B, int64_t ldb, int64_t n2) {
+  ::ibem::chain_wait();
   extern __shared__ __align__(16) unsigned char trsm_smem[];
   T* sL = reinterpret_cast<T*>(trsm_smem);   // [i][k] = L(k, i) for k > i
   T* sB = sL + NB * NB;                      // [r][cc], stride kTrsmCols + 1
@@ -847,6 +850,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_gemm_sub_smallk(int64_t m, int64_t n, int k, const T* __restrict__ A,
                                                          int64_t lda, const T* __restrict__ B, int64_t ldb,
                                                          T* __restrict__ C, int64_t ldc) {
+  ::ibem::chain_wait();
   extern __shared__ __align__(16) unsigned char gs_smem[];
   T* sA = reinterpret_cast<T*>(gs_smem);  // [kk][r], stride 65
   T* sB = sA + kSmallK * 65;              // [kk][c], stride 65
@@ -1332,8 +1336,7 @@ ibem_status gemm_sub<float>(int64_t m, int64_t n, int64_t k, const float* A, int
   ProfScope ps(PROF_GEMM_SIMT, st, 2.0 * m * n * k);
   dim3 grid((unsigned)((m + 63) / 64), (unsigned)((n + 63) / 64));
   if (k <= kSmallK)
-    ::ibem::count_launch(), k_gemm_sub_smallk<float><<<grid, 256, gemm_smallk_smem<float>(), st>>>(m, n, (int)k, A, lda, B,
-                                                                                         ldb, C, ldc);
+    launch_chained_smem(k_gemm_sub_smallk<float>, grid, 256, gemm_smallk_smem<float>(), st, m, n, (int)k, A, lda, B, ldb, C, ldc);
   else
     ::ibem::count_launch(), k_gemm_sub<float><<<grid, 256, 0, st>>>(m, n, k, A, lda, B, ldb, C, ldc);
   IBEM_LAUNCH_CHECK("gemm f32");
@@ -1352,11 +1355,11 @@ static ibem_status trsm(const T* L, int64_t ldl, int64_t n1, T* B, int64_t ldb, 
       if (n1 <= 32) ::ibem::count_launch(), k_trsm_f64<32><<<grid, 8 * kTrsm64Cols, 0, st>>>(L, ldl, (int)n1, B, ldb, n2);
       else ::ibem::count_launch(), k_trsm_f64<64><<<grid, 8 * kTrsm64Cols, 0, st>>>(L, ldl, (int)n1, B, ldb, n2);
     } else if (n1 == 32)
-      ::ibem::count_launch(), k_trsm_small_fixed<T, 32><<<(unsigned)((n2 + kTrsmCols - 1) / kTrsmCols), kTrsmCols,
-                                                          trsm_fixed_smem<T, 32>(), st>>>(L, ldl, B, ldb, n2);
+      launch_chained_smem(k_trsm_small_fixed<T, 32>, (unsigned)((n2 + kTrsmCols - 1) / kTrsmCols), kTrsmCols,
+                          trsm_fixed_smem<T, 32>(), st, L, ldl, B, ldb, n2);
     else if (n1 == 64)
-      ::ibem::count_launch(), k_trsm_small_fixed<T, 64><<<(unsigned)((n2 + kTrsmCols - 1) / kTrsmCols), kTrsmCols,
-                                                          trsm_fixed_smem<T, 64>(), st>>>(L, ldl, B, ldb, n2);
+      launch_chained_smem(k_trsm_small_fixed<T, 64>, (unsigned)((n2 + kTrsmCols - 1) / kTrsmCols), kTrsmCols,
+                          trsm_fixed_smem<T, 64>(), st, L, ldl, B, ldb, n2);
     else
       ::ibem::count_launch(), k_trsm_small<T><<<(unsigned)((n2 + 63) / 64), 64, 2 * 64 * 65 * sizeof(T), st>>>(
           L, ldl, (int)n1, B, ldb, n2);
@@ -1381,9 +1384,13 @@ static ibem_status lu_rec(T* A, int64_t lda, int64_t N, int64_t k0, int64_t n, L
     // exchanges of this panel on the columns to its left and right (within [0, N))
     ProfScope ps(PROF_LASWP, st);
     const int64_t ncols = N - n;  // every column outside the panel
-    if (ncols > 0)
-      ::ibem::count_launch(), k_laswp<T><<<(unsigned)((ncols + kSwapPerCta - 1) / kSwapPerCta), kSwapThreads, 0, st>>>(
-          A, lda, k0, w.cb.meta, (int)n, ncols);
+    if (ncols > 0) {
+      const unsigned grid = (unsigned)((ncols + kSwapPerCta - 1) / kSwapPerCta);
+      if constexpr (sizeof(T) == 4)
+        launch_chained(k_laswp<T>, grid, kSwapThreads, st, A, lda, k0, w.cb.meta, (int)n, ncols);
+      else
+        ::ibem::count_launch(), k_laswp<T><<<grid, kSwapThreads, 0, st>>>(A, lda, k0, w.cb.meta, (int)n, ncols);
+    }
     IBEM_LAUNCH_CHECK("laswp");
     return IBEM_OK;
   }
