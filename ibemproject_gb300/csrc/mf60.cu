@@ -48,6 +48,17 @@ struct RowSink {
   __device__ __forceinline__ void operator()(int r, int c, T v) const { acc[r] += v * xs[c]; }
 };
 
+// Offset of a target (centre p) from a source (centre c, ia = 1 / radius) in units of the source's
+// radius.  True: outside the source.  The FP64 product decides this for a pair in three kernels,
+// which have to agree on a centre within a rounding of the surface: hence rounded operations,
+// which the compiler does not fuse into multiply-adds of its own choice.
+__device__ __forceinline__ bool offset60(const double* p, const double* c, double ia, double (&x)[3], double& r2) {
+#pragma unroll
+  for (int d = 0; d < 3; ++d) x[d] = __dmul_rn(__dsub_rn(p[d], c[d]), ia);
+  r2 = __dadd_rn(__dadd_rn(__dmul_rn(x[0], x[0]), __dmul_rn(x[1], x[1])), __dmul_rn(x[2], x[2]));
+  return r2 > 1.0;
+}
+
 // A pair whose target centre lies inside the source, from the generated blocks (dense): rare
 // (overlapping spheres), so out of line and straight into y.  as, ia: radius of the target,
 // 1 / radius of the source; xs: the source's coefficients.
@@ -79,6 +90,9 @@ __device__ __noinline__ void pair_inside(double x0, double x1, double x2, double
   double acc[kNu];
   for (int r = 0; r < kNu; ++r) acc[r] = 0.0;
   RowSink<double> sk{acc, xs};
+  // the sub-blocks compare |x|^2 with 1 themselves, by operations of their own: a centre within a few
+  // roundings of the surface is moved 2^-50 of its distance inwards, so that all of them see it inside
+  if (x0 * x0 + x1 * x1 + x2 * x2 > 1.0 - 0x1p-48) x0 -= 0x1p-50 * x0, x1 -= 0x1p-50 * x1, x2 -= 0x1p-50 * x2;
   for (int i = 0; i < 9; ++i) blocks60(i, x0, x1, x2, mc, sk);
   for (int r = 0; r < kNu; ++r) atomicAdd(y + r, acc[r] * (r < 6 ? 1.0 : r < 24 ? as * ia : as * ia * as * ia));
 }
@@ -224,15 +238,13 @@ __global__ void __launch_bounds__(kT)
   const int hb = hb0 + (blockIdx.y * gridDim.z + blockIdx.z) * per, he = min(he0, hb + per);
   if (threadIdx.x >= t.ns) return;
   const int s = t.s0 + threadIdx.x;
-  const double p0 = cen[3 * (int64_t)s], p1 = cen[3 * (int64_t)s + 1], p2 = cen[3 * (int64_t)s + 2];
+  const double p[3] = {cen[3 * (int64_t)s], cen[3 * (int64_t)s + 1], cen[3 * (int64_t)s + 2]};
 #pragma unroll 4
   for (int h = hb; h < he; ++h) {
     const double ia = 1.0 / rad[h];
-    const double x0 = (p0 - cen[3 * (int64_t)h]) * ia, x1 = (p1 - cen[3 * (int64_t)h + 1]) * ia,
-                 x2 = (p2 - cen[3 * (int64_t)h + 2]) * ia;
-    const double r2 = x0 * x0 + x1 * x1 + x2 * x2;
-    if (!(r2 > 1.0) && h != s)
-      pair_inside(x0, x1, x2, rad[s], ia, mats[t.seg], x + (int64_t)kNu * h, y + (int64_t)kNu * s);
+    double u[3], r2;
+    if (!offset60(p, cen + 3 * (int64_t)h, ia, u, r2) && h != s)
+      pair_inside(u[0], u[1], u[2], rad[s], ia, mats[t.seg], x + (int64_t)kNu * h, y + (int64_t)kNu * s);
   }
 }
 
@@ -256,11 +268,10 @@ __global__ void __launch_bounds__(kT)
   const int s = t.s0 + threadIdx.x;
   const bool act = threadIdx.x < t.ns;
   const double kmu = mats[t.seg].kmu, klam = mats[t.seg].klam, nu = 0.5 * mats[t.seg].tn2;
-  double p0 = 0.0, p1 = 0.0, p2 = 0.0, as = 1.0;
+  double p[3] = {0.0, 0.0, 0.0}, as = 1.0;
   if (act) {
-    p0 = cen[3 * (int64_t)s];
-    p1 = cen[3 * (int64_t)s + 1];
-    p2 = cen[3 * (int64_t)s + 2];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) p[d] = cen[3 * (int64_t)s + d];
     as = rad[s];
   }
   double acc[NR];
@@ -281,12 +292,11 @@ __global__ void __launch_bounds__(kT)
 #pragma unroll 1
     for (int hh = 0; hh < nh; ++hh) {
       const double ia = sc[4 * hh + 3];
-      const double x0 = (p0 - sc[4 * hh]) * ia, x1 = (p1 - sc[4 * hh + 1]) * ia, x2 = (p2 - sc[4 * hh + 2]) * ia;
-      const double r2 = x0 * x0 + x1 * x1 + x2 * x2;
-      if (!(r2 > 1.0)) continue;   // k_mf60_inside
+      double u[3], r2;
+      if (!offset60(p, sc + 4 * hh, ia, u, r2)) continue;   // k_mf60_inside
       const double ir = rsqrt_h3(r2);
       Mf60Frame<double> f;
-      mf60_frame(x0 * ir, x1 * ir, x2 * ir, f);
+      mf60_frame(u[0] * ir, u[1] * ir, u[2] * ir, f);
       double A0[6], A1[6][3], A2[6][6];
       mf60_source(f, sx + kNu * hh, A0, A1, A2);
       if constexpr (HI) {
