@@ -72,8 +72,9 @@ struct Layout {
 // the FP64 distance and inserts only the few candidates (about 22) within it.  Without that
 // bound some lane of the warp inserts at almost every step, 16 compare-and-swaps each.  The
 // FP32 offset from the centres' hi / lo parts is off by at most 2^-22 of itself per axis, its
-// square by less than 2e-6, and the lo parts leave out less than `slack`.  20,000 particles:
-// 16.0 -> 2.0 ms.
+// square by less than 2e-6, and the lo parts leave out less than `slack`; squares below 2^-126 lose
+// digits to underflow, 2^-149 at a time, so distances up to 2^-63 are all left to FP64.  20,000
+// particles: 16.0 -> 2.0 ms.
 __global__ void k_knn(int num, const int* __restrict__ seg_of, const int* __restrict__ seg_begin,
                       const double* __restrict__ cen, const float4* __restrict__ gh, const float4* __restrict__ gl,
                       int* __restrict__ nbr) {
@@ -109,7 +110,7 @@ __global__ void k_knn(int num, const int* __restrict__ seg_of, const int* __rest
   }
   const unsigned at = __ballot_sync(0xffffffffu, rank == kKnn - 1);
   const float bound = at ? __shfl_sync(0xffffffffu, near, __ffs(at) - 1) : INFINITY;
-  const float far = sqrtf(bound) + 2.f * slack, limit = far * far * 1.00001f;
+  const float far = sqrtf(bound) + 2.f * slack, limit = far * far * 1.00001f + 0x1p-126f;
 #pragma unroll 4
   for (int q = b0 + lane; q < b1; q += 32) {
     if (q == p || d2f(q) > limit) continue;   // (false for NaN: the FP64 test decides)
