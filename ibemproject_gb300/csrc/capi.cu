@@ -327,6 +327,31 @@ ibem_status ibem_gemm_sub_f32(int64_t m, int64_t n, int64_t k, const float* A_de
   return s;
 }
 
+ibem_status ibem_gemm_sub_f64(int64_t m, int64_t n, int64_t k, const double* A_dev, int64_t lda,
+                              const double* B_dev, int64_t ldb, double* C_dev, int64_t ldc, void* stream) {
+  if (m < 0 || n < 0 || k < 0 || lda < m || ldb < k || ldc < m) return fail(IBEM_ERR_ARG, "gemm_sub_f64: bad sizes");
+  if (m == 0 || n == 0 || k == 0) return IBEM_OK;
+  cudaStream_t st = as_stream(stream);
+  const size_t ws_bytes = gemm_tc64_workspace_bytes(m, n);
+  void* ws = nullptr;
+  int* err = nullptr;
+  IBEM_CUDA(pool_alloc(&ws, ws_bytes, st));
+  cudaError_t ce = pool_alloc(&err, sizeof(int), st);
+  if (ce == cudaSuccess) ce = cudaMemsetAsync(err, 0, sizeof(int), st);
+  ibem_status s = ce == cudaSuccess ? IBEM_OK : cuda_fail(ce, "gemm_sub_f64");
+  if (!s) s = gemm_sub_f64_tc(m, n, k, A_dev, lda, B_dev, ldb, C_dev, ldc, ws, ws_bytes, err, st);
+  int herr = 0;
+  if (!s) {
+    ce = cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+    if (ce != cudaSuccess) s = cuda_fail(ce, "gemm_sub_f64");
+    else if (herr) s = fail(IBEM_ERR_TIMEOUT, "gemm_sub_f64: a device-side wait gave up");
+  }
+  pool_free(ws, st);
+  pool_free(err, st);
+  return s;
+}
+
 ibem_status ibem_selftest_bounded_wait(int which, long long limit, void* stream) {
   if (which == 0) return selftest_flag_wait(limit, as_stream(stream));
   if (which == 1) return selftest_mbar_wait(limit, as_stream(stream));

@@ -1,22 +1,29 @@
 // FP64 trailing updates of the dense factorisation on the tensor cores:  C -= A * B with FP64
-// storage, accuracy and range, on sm_103a's BF16 tcgen05 pipe (Ozaki's error-free splitting).
+// storage on sm_103a's BF16 tcgen05 pipe (Ozaki's error-free splitting).
 //
 // Why: GB300's FP64 pipe does 2 multiply-adds per clock and SM (0.60 T/s measured), so a SIMT
 // FP64 update is bound by it whatever its tiling; the BF16 tensor pipe does 3,200 times as
 // many, and 28 BF16 products carry one FP64 product.
 //
-// Scheme.  Row i of A is written as 2^ea_i times 56-bit fixed-point numbers, column j of B
-// likewise, and each number as seven signed 8-bit digits (|d| <= 128, exact in BF16).  The
-// digit products of equal weight, g = p + q, are summed in one FP32 accumulator of TMEM:
-// over a chunk of 256 columns |sum| <= (g + 1) 256 128^2 = (g + 1) 2^22, which FP32 holds
-// exactly for g <= 3; g = 4..6 (weights 2^-32 and below of the leading one) may round once
-// past 2^24, for data whose digits are all of one sign and size, at 2^-53 of the leading sum
-// or less.  After every chunk the accumulators are added to two 64-bit integers per entry
-// (g <= 3 and g >= 4, exact), which are converted to FP64 once at the end.  Digits below
-// weight 2^-56 of a row's (column's) largest entry and products below 2^-56 (g >= 7) are
-// dropped: an entry of the product is off by at most k 2^-53 max|a_i.| max|b_.j|, typically
-// far less than the rounding of an FP64 sum of k products (tests/test_gpu_gemm64.py).
-// A row or column that holds an infinity or NaN gives NaN in its whole row or column of C.
+// Scheme.  Row i of A is written as 2^ea_i times fixed-point numbers of 55 bits and a sign (the
+// largest one between 2^54 and 2^55), column j of B likewise, and each number as seven signed
+// 8-bit digits (|d| <= 128, exact in BF16).  The digit products of equal weight, g = p + q, are
+// summed in one FP32 accumulator of TMEM: over a chunk of 192 columns |sum| <= (g + 1) 192 128^2
+// = (g + 1) 3 2^20, which FP32 holds exactly for g <= 4.  g = 5 and 6 (weights 2^-40 and below of
+// the leading one) lose the units of a few additions past 2^24, for data whose digits are all
+// of one sign and near the largest: below 0.1 k 2^-53 of what the bound below counts in.
+// (Chunks of 256 columns let g = 4 past 2^24 too; the additions truncate, and such data came
+// out off by 7 k 2^-53.)  After every chunk the accumulators are added to two 64-bit integers
+// per entry (g <= 3 and g >= 4, exact), which are converted to FP64 once at the end.
+//
+// Accuracy is to the largest entry of a row and column, not to each entry.  In units where the
+// largest products are 2^108 to 2^110, the products left out (g >= 7) are worth at most 6.03
+// 2^54 a term and the rounding of the two operands 2 2^54: an entry of the product is off by at
+// most 4.1 k 2^-53 max|a_i.| max|b_.j|, typically far less than the rounding of an FP64 sum of k
+// products (tests/test_gemm64_product.py).  Entries that are small beside their row keep fewer
+// than 53 bits: the solve gives the digits that this costs back by a step of refinement
+// (solver.cu).  A row or column that holds an infinity or NaN gives NaN in its whole row or
+// column of C.
 //
 // Measured (random normal entries): 3600^3 29 TFLOP/s, 8192 x 8192 x 2048 32 TFLOP/s (the FP64
 // pipe gives 1.2), rms error 7e-18 and 9e-18 of sum |a||b| where FP64 multiply-adds give 5e-17.
@@ -26,7 +33,7 @@
 // tile: a TMA producer warp (two 86 KB stages of 32 columns x 7 digit planes of A and B), an
 // MMA warp (56 tcgen05.mma of 128 x 64 x 16 per stage into seven accumulators of 64 TMEM
 // columns), eight epilogue warps.  The tile is as wide as seven accumulators allow (448 of
-// 512 TMEM columns).  The accumulators are read back once per 256 columns, about a tenth of
+// 512 TMEM columns).  The accumulators are read back once per 192 columns, about an eighth of
 // the chunk's MMA time, so they are not double-buffered.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -45,7 +52,7 @@ namespace {
 
 constexpr int NS = 7;                               // digits of an operand, accumulators
 constexpr int BM = 128, BN = 64, BK = 32, STAGES = 2;
-constexpr int CHUNK = 8;                            // K blocks between two readings of the accumulators
+constexpr int CHUNK = 6;                            // K blocks between two readings of the accumulators (192 columns)
 constexpr int A_PLANE = BM * BK * 2, B_PLANE = BN * BK * 2;   // 8 and 4 KB
 constexpr int STAGE_BYTES = NS * (A_PLANE + B_PLANE);         // 86,016
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;

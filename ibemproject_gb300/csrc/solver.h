@@ -17,8 +17,9 @@ ibem_status gemm_sub_f32_tc(int64_t m, int64_t n, int64_t k, const float* A, int
                             cudaStream_t st);
 size_t gemm_tc_workspace_bytes(int64_t max_m, int64_t max_n);
 
-// The same with FP64 storage and at least FP64 accuracy (gemm_tc64.cu), any sizes; `ws` of at
-// least gemm_tc64_workspace_bytes(max m, max n) bytes.
+// The same with FP64 storage and FP64 accuracy relative to the largest entries of a row of A and
+// column of B (gemm_tc64.cu), any sizes; `ws` of at least gemm_tc64_workspace_bytes(max m, max n)
+// bytes.
 ibem_status gemm_sub_f64_tc(int64_t m, int64_t n, int64_t k, const double* A, int64_t lda, const double* B,
                             int64_t ldb, double* C, int64_t ldc, void* ws, size_t ws_bytes, int* err,
                             cudaStream_t st);

@@ -176,6 +176,17 @@ ibem_status ibem_e3d_solve_bj(int64_t N, int block, const double* A_dev, int64_t
 ibem_status ibem_gemm_sub_f32(int64_t m, int64_t n, int64_t k, const float* A_dev, int64_t lda,
                               const float* B_dev, int64_t ldb, float* C_dev, int64_t ldc, void* stream);
 
+/* The trailing-update primitive of the FP64 factorisation, exposed for testing and reuse: the same
+ * with FP64 storage, on the tensor cores by seven 8-bit digits of each operand (exact sums of the
+ * digits' products).  Operands are rounded to 55 to 56 bits below the largest entry of their row
+ * (A) or column (B): an entry of the product is off by at most 4.1 k 2^-53 max|a_i.| max|b_.j|
+ * and its own rounding, for random entries by a sixth of what FP64 multiply-adds leave.  A
+ * non-finite entry makes its whole row or column of C NaN.  Allocates its scratch;
+ * synchronous.  No reference counterpart. */
+ibem_status ibem_gemm_sub_f64(int64_t m, int64_t n, int64_t k, const double* A_dev, int64_t lda,
+                              const double* B_dev, int64_t ldb, double* C_dev, int64_t ldc,
+                              void* stream);
+
 /* The plain FP64 solve of ibem_e3d_solve for callers that may not allocate device
  * memory; it has no counterpart in the reference.  Meant for code whose device memory
  * belongs to a host framework (a caching allocator or a budget reserved up front, where a
