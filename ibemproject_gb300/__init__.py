@@ -85,6 +85,8 @@ SIGNATURES = {
     "ibem_last_error": (ctypes.c_char_p, []),
     "ibem_layout_size": (_int, [_int]),
     "ibem_kernel_launches": (ctypes.c_longlong, []),
+    "ibem_memory_kept": (ctypes.c_longlong, []),
+    "ibem_memory_trim": (_int, []),
     "ibem_prof_enable": (None, [_int]),
     "ibem_prof_report": (_int, [ctypes.c_char_p, _int]),
     "ibem_e3d_pair_blocks": (_int, [_vp, _vp, _int, ctypes.POINTER(Material), _int, _vp, _i64, _i64, _i64, _vp]),
@@ -177,6 +179,16 @@ def lib():
 def check(status: int) -> None:
     if status != IBEM_OK:
         raise IbemError(status, lib().ibem_last_error().decode(errors="replace"))
+
+
+def memory_kept() -> int:
+    """Bytes of device memory that the library holds unused on the current device."""
+    return int(lib().ibem_memory_kept())
+
+
+def memory_trim() -> None:
+    """Give that memory back to the device (ibem_memory_trim)."""
+    check(lib().ibem_memory_trim())
 
 
 def material(E0, nu0, E1, nu1) -> Material:

@@ -300,6 +300,13 @@ ibem_status ibem_e3d_solve_bj(int64_t N, int block, const double* A_dev, int64_t
                      as_stream(stream), block);
 }
 
+long long ibem_memory_kept(void) { return (long long)pool_kept(); }
+
+ibem_status ibem_memory_trim(void) {
+  const cudaError_t e = pool_trim();
+  return e == cudaSuccess ? IBEM_OK : cuda_fail(e, "memory_trim");
+}
+
 ibem_status ibem_gemm_sub_f32(int64_t m, int64_t n, int64_t k, const float* A_dev, int64_t lda,
                               const float* B_dev, int64_t ldb, float* C_dev, int64_t ldc, void* stream) {
   if (m < 0 || n < 0 || k < 0 || lda < m || ldb < k || ldc < m) return fail(IBEM_ERR_ARG, "gemm_sub_f32: bad sizes");

@@ -32,10 +32,13 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 // beyond goes back at the next synchronisation), because mapping and unmapping memory on
 // every call cost more than the small solves themselves (a training step: 0.4 of 1.3 ms; six
 // ellipsoid realisations on four threads: 19 of 34 ms in cudaMalloc alone); an allocation that
-// fails gives everything kept back and tries once more.
+// fails gives everything kept back and tries again.  pool_kept: bytes that the current device's
+// pool holds unused; pool_trim gives them back.
 constexpr size_t kPoolKeep = (size_t)1 << 30;
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st);
 void pool_free(void* p, cudaStream_t st);
+size_t pool_kept();
+cudaError_t pool_trim();
 template <class T>
 cudaError_t pool_alloc(T** p, size_t bytes, cudaStream_t st) {
   return pool_alloc(reinterpret_cast<void**>(p), bytes, st);

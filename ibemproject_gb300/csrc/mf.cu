@@ -1858,7 +1858,8 @@ extern "C" ibem_status ibem_e3d_batch_dense_solve(const ibem_e3d_batch* batch, i
   // block-Jacobi form runs several workers at once, so that one realisation's
   // latency-bound steps (host-driven GMRES, small kernels) overlap another's products; the
   // factorising forms run one worker (their panel kernel needs every SM to itself).  As many
-  // workers as fit in a quarter of the free device memory, at most kDenseWorkers.
+  // workers as fit in a quarter of the free device memory (what the library keeps unused is
+  // free to it), at most kDenseWorkers.
   constexpr int kDenseWorkers = 4;
   const size_t per_worker = sizeof(double) * nmax * nmax +
                             (form == IBEM_SOLVE_GMRES_BJ ? sizeof(float) * ((nmax + 3) / 4 * 4) * nmax : 0);
@@ -1867,7 +1868,7 @@ extern "C" ibem_status ibem_e3d_batch_dense_solve(const ibem_e3d_batch* batch, i
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess)
       nwork = (int)std::max<size_t>(1, std::min<size_t>({(size_t)kDenseWorkers, (size_t)batch->nseg,
-                                                         free_b / 4 / per_worker}));
+                                                         (free_b + pool_kept()) / 4 / per_worker}));
   }
   // b_dev is written on the caller's stream: let it land before the workers read it
   cudaError_t e0 = cudaStreamSynchronize(st);

@@ -64,13 +64,32 @@ cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st) {
   if (bytes == 0) bytes = 1;
   const cudaMemPool_t pool = device_pool(dev);
   e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMallocAsync(p, bytes, st);
-  if (e == cudaErrorMemoryAllocation && pool) {
+  // out of memory: what this stream, then what any stream has released goes back first
+  for (int all = 0; all < 2 && e == cudaErrorMemoryAllocation && pool; ++all) {
     cudaGetLastError();
-    cudaStreamSynchronize(st);   // what this stream released goes back too
+    if (all) cudaDeviceSynchronize();
+    else cudaStreamSynchronize(st);
     cudaMemPoolTrimTo(pool, 0);
     e = cudaMallocFromPoolAsync(p, bytes, pool, st);
   }
   return e;
+}
+size_t pool_kept() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  uint64_t reserved = 0, used = 0;
+  const cudaMemPool_t pool = device_pool(dev);
+  if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+    return 0;
+  return reserved > used ? (size_t)(reserved - used) : 0;
+}
+cudaError_t pool_trim() {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const cudaMemPool_t pool = device_pool(dev);
+  return pool ? cudaMemPoolTrimTo(pool, 0) : cudaSuccess;
 }
 void pool_free(void* p, cudaStream_t st) {
   if (p) cudaFreeAsync(p, st);

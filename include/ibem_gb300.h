@@ -50,6 +50,14 @@ const char* ibem_last_error(void);
 /* Number of kernels this library has launched since it was loaded (all threads). */
 long long ibem_kernel_launches(void);
 
+/* Device memory.  The library's buffers come from a stream-ordered pool of its own, one per device,
+ * which keeps up to 1 GiB unused between calls.  ibem_memory_kept: bytes that the current
+ * device's pool holds unused; ibem_memory_trim gives them back to the device, as an allocation
+ * of the library that fails does by itself (memory released on a stream goes back once the
+ * stream has come to that point).  Any thread, any time. */
+long long ibem_memory_kept(void);
+ibem_status ibem_memory_trim(void);
+
 /* Phase profiler: with profiling on, CUDA events are recorded on the launching stream around
  * each phase (pair blocks, field sums, panels, row exchanges, tensor-core GEMMs, ...);
  * ibem_prof_enable(1) also clears what was recorded.  ibem_prof_report writes a JSON object
