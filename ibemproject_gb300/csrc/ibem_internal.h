@@ -26,6 +26,16 @@ ibem_status cuda_fail(cudaError_t e, const char* where);
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// What the library sets up once, on first use, must not end a stream capture that this or another
+// thread has under way: calls that the runtime counts as unsafe there are made inside one of these.
+struct CaptureSafe {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  CaptureSafe() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~CaptureSafe() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  CaptureSafe(const CaptureSafe&) = delete;
+  CaptureSafe& operator=(const CaptureSafe&) = delete;
+};
+
 // Stream-ordered device memory for the library's buffers and workspaces, from a pool of its own
 // (one per device, made on first use): allocation and release are queued on the stream, safe
 // from any thread and stream.  Between calls the pool keeps at most kPoolKeep bytes (what is

@@ -1347,6 +1347,7 @@ struct HostSlot {
     if (!p.mem && !p.tried) {
       p.tried = true;
       void* m = nullptr;
+      CaptureSafe safe;
       if (cudaHostAlloc(&m, kSlots * kStride, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess)
         p.mem = static_cast<char*>(m);
       else

@@ -46,6 +46,7 @@ cudaMemPool_t device_pool(int dev) {
     props.location.id = dev;
     cudaMemPool_t pool = nullptr;
     uint64_t keep = kPoolKeep;
+    CaptureSafe safe;
     if (cudaMemPoolCreate(&pool, &props) == cudaSuccess &&
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
       g_mem[dev] = pool;
