@@ -167,6 +167,15 @@ def tuning(batch: DeviceBatch):
     return a.value, b.value
 
 
+def pieces(batch: DeviceBatch):
+    """(pieces that each source slice is cut into, FP32 product, double-float / FP64 products)
+    of the same choice: slices x pieces CTAs per target tile."""
+    _linear(batch)
+    a, b = ctypes.c_int(0), ctypes.c_int(0)
+    check(lib().ibem_e3d_mf_pieces(batch.ref(), ctypes.byref(a), ctypes.byref(b), None))
+    return a.value, b.value
+
+
 def tile_shape(batch: DeviceBatch):
     """(targets per CTA, persistent launch 0/1, source slices) of the FP32 product chosen by
     the library's autotuner for this batch's shape."""
@@ -323,7 +332,7 @@ def train(batch: DeviceBatch, r_hat, e_hat, params, steps: int, lr: float = 2e-3
     return hist
 
 
-__all__ = ["DeviceBatch", "farfield_rhs", "dense_batch_solve", "matvec", "solve", "tuning", "effective_modulus",
+__all__ = ["DeviceBatch", "farfield_rhs", "dense_batch_solve", "matvec", "solve", "tuning", "pieces", "effective_modulus",
            "dense_system", "dense_solve",
            "training_pairs", "training_pairs_mf", "param_count", "init_params", "prepare", "loss_grad", "edge_weights", "adamw", "train",
            "PRECOND_BLOCK_JACOBI", "PRECOND_LEARNED", "PRECOND_NEUMANN", "IbemError"]

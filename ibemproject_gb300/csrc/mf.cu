@@ -1154,13 +1154,14 @@ ibem_status mf_tune(MfBatch& b, cudaStream_t st) {
   IBEM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const TuneKey key{log2_bucket(b.ntiles), log2_bucket(b.max_seg), sms * 100 + b.nu};
   const int cap = slice_cap(b.max_seg);
-  // IBEM_MF_F32_SHAPE="shape,persistent,slices" fixes the FP32 product's launch (tests and
-  // measurements of every shape); the wide products keep the batch's initial slice count
+  // IBEM_MF_F32_SHAPE="shape,persistent,slices[,pieces]" fixes the FP32 product's launch (tests and
+  // measurements of every shape); the wide products keep the batch's initial split
   if (const char* f = b.nu == 24 ? std::getenv("IBEM_MF_F32_SHAPE") : nullptr) {
-    int ts = 1, pers = 0, h = 1;
-    if (std::sscanf(f, "%d,%d,%d", &ts, &pers, &h) == 3 && ts >= 0 && ts < 3 && (pers == 0 || pers == 1) && h >= 1)
-      return mf_set_f32_shape(b, ts, {std::min(h, cap), 1}, pers, st);
-    return fail(IBEM_ERR_ARG, "IBEM_MF_F32_SHAPE: expected shape (0-2),persistent (0/1),slices (>= 1)");
+    int ts = 1, pers = 0, h = 1, pc = 1;
+    if (std::sscanf(f, "%d,%d,%d,%d", &ts, &pers, &h, &pc) >= 3 && ts >= 0 && ts < 3 && (pers == 0 || pers == 1) && h >= 1 &&
+        pc >= 1 && pc <= (pers ? 1 : kMfPieces))
+      return mf_set_f32_shape(b, ts, {std::min(h, cap), pc}, pers, st);
+    return fail(IBEM_ERR_ARG, "IBEM_MF_F32_SHAPE: expected shape (0-2),persistent (0/1),slices (>= 1)[,pieces (1-4, persistent 1)]");
   }
   {
     bool hit = false;
@@ -2083,6 +2084,24 @@ extern "C" ibem_status ibem_e3d_mf_tuning(const ibem_e3d_batch* batch, int* slic
     *slices_wide = b.split_wide.slices;
     const cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) s = cuda_fail(e, "mf_tuning");
+  }
+  mf_batch_free(b);
+  return s;
+}
+
+extern "C" ibem_status ibem_e3d_mf_pieces(const ibem_e3d_batch* batch, int* pieces_fp32, int* pieces_wide,
+                                         void* stream) {
+  if (batch && batch->axes_dev) return fail(IBEM_ERR_ARG, "matrix-free products and the learned preconditioner take spheres; solve ellipsoid batches with ibem_e3d_batch_dense_solve");
+  if (!batch || !pieces_fp32 || !pieces_wide) return fail(IBEM_ERR_ARG, "mf_pieces: bad arguments");
+  cudaStream_t st = as_stream(stream);
+  MfBatch b;
+  ibem_status s = mf_batch_init(b, *batch, st);
+  if (!s) s = mf_tune(b, st);
+  if (!s) {
+    *pieces_fp32 = b.split.pieces;
+    *pieces_wide = b.split_wide.pieces;
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) s = cuda_fail(e, "mf_pieces");
   }
   mf_batch_free(b);
   return s;

@@ -315,9 +315,15 @@ ibem_status ibem_e3d_mf_matvec_layout(const ibem_e3d_batch* batch, int layout, i
 ibem_status ibem_e3d_mf_tuning(const ibem_e3d_batch* batch, int* slices_fp32, int* slices_wide,
                                void* stream);
 
+/* The rest of that choice: in small batches each slice (at least 32 sources) is cut into up to 4
+ * pieces, a CTA each, so a product runs slices x pieces CTAs per target tile (the persistent form:
+ * whole slices, 1).  No reference counterpart.  Synchronous. */
+ibem_status ibem_e3d_mf_pieces(const ibem_e3d_batch* batch, int* pieces_fp32, int* pieces_wide,
+                               void* stream);
+
 /* The FP32 product's tile shape the same autotuner picks (it times every candidate of the
  * shape class once): targets per CTA (64, 128 or 256), launch form (0: one CTA per (tile,
- * source slice); 1: persistent CTAs, as many as fit on the GPU, over the (tile, slice)
+ * piece of a source slice: ibem_e3d_mf_pieces); 1: persistent CTAs, as many as fit on the GPU, over the (tile, slice)
  * items sorted by decreasing cost) and source slices.  No reference counterpart.
  * Synchronous. */
 ibem_status ibem_e3d_mf_tile_shape(const ibem_e3d_batch* batch, int* targets_per_cta, int* persistent,
