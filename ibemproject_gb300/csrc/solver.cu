@@ -4,7 +4,8 @@
 // Both forms first equilibrate A (row, then column max scaling): the raw iBEM matrix
 // spans ~47 decades, which partial pivoting alone cannot handle (full pivoting can).
 //
-//   IBEM_SOLVE_FP64      LU with partial pivoting of the scaled matrix in FP64.
+//   IBEM_SOLVE_FP64      LU with partial pivoting of the scaled matrix in FP64 (trailing updates
+//                        on the tensor cores, gemm_tc64.cu) and one step of refinement.
 //   IBEM_SOLVE_MIXED_IR  LU with partial pivoting in FP32 (trailing updates on the tensor
 //                        cores with the split-BF16 "x3" scheme, FP32 accumulation), then
 //                        FP64 GMRES iterative refinement preconditioned by the FP32 factors;
@@ -2045,12 +2046,13 @@ ibem_status solve_dense(ibem_solver_form form, int64_t N, double* A, int64_t lda
     }
     if (!s) s = finish_norm();
     if (!s) s = scaled_backward_error(cx, A, lda, ys, bs, rvec, tmp, as_norm, R.backward_error);
-    if (!s && w.gemm_ws && std::isfinite(R.backward_error)) {
+    if (!s && std::isfinite(R.backward_error)) {
       // One step of refinement.  The tensor-core updates round normwise (to the largest entry
       // of a row and column), which costs the small entries of the solution digits that an
       // FP64 residual gives back: 300 spheres (N = 7,200) against a 64-bit solution 9.3e-15
       // with FP64 updates, 4.9e-14 with the tensor-core updates alone, 2.0e-15 with this step
-      // (1.2 ms of 86).
+      // (1.2 ms of 82).  Also taken where there was no room for the digits and the updates ran
+      // in FP64: a solve's accuracy does not depend on the memory that is free.
       s = lu_apply<double>(W, N, N, w, rvec, st);
       if (!s) s = sticky_err(w, st);
       if (!s) ::ibem::count_launch(), k_axpby<<<nb, 256, 0, st>>>(N, 1.0, rvec, 1.0, ys);

@@ -141,7 +141,11 @@ ibem_status ibem_e3d_farfield_rhs(int num, const ibem_material* mat, int layout,
 /* ---- systemSolver (systemSolverElastic3D.h) ------------------------------- */
 
 typedef enum {
-  IBEM_SOLVE_FP64 = 0,     /* equilibrated partial-pivot LU in FP64 (plain path) */
+  IBEM_SOLVE_FP64 = 0,     /* equilibrated partial-pivot LU in FP64 (plain path), one step of
+                            * refinement.  The trailing updates run on the tensor cores, exact to
+                            * 55 bits below the largest entry of a row and column
+                            * (ibem_gemm_sub_f64), or, where there is no room for their scratch
+                            * (28 KB a row), in FP64; the refinement makes up for either */
   IBEM_SOLVE_MIXED_IR = 1, /* FP32 LU, split-BF16 tensor-core updates, FP64 GMRES-IR */
   IBEM_SOLVE_GMRES_BJ = 2  /* no factorisation: FP64 refinement of FP32-product GMRES,
                             * block-Jacobi preconditioned (ibem_e3d_solve_bj) */
