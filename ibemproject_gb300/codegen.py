@@ -735,8 +735,8 @@ def generate(out_dir: str | None = None) -> dict:
         parts.append(gen_self_function(f"sph_self{lay}", lay))
         files[f"gen_sphere{lay}.cuh"] = "\n\n".join(parts) + "\n"
         if lay == 60:
-            # FP32 blocks of the layout-60 matrix-free products (scaled coordinates, a = 1): the
-            # large sub-blocks split into groups of 6 columns (one symmetric pair (m, n) each),
+            # FP32 blocks of the layout-60 matrix-free products (scaled coordinates, a = 1) for pairs
+            # whose target centre lies inside the source: the large sub-blocks split into groups of 6 columns (one symmetric pair (m, n) each),
             # so that each kernel's straight-line code keeps its values in registers: the
             # order-1 columns of the order-2 rows in 3 groups, the order-2 columns of the
             # order-1 and order-2 rows in 6
@@ -756,10 +756,10 @@ def generate(out_dir: str | None = None) -> dict:
                             add(f"sph_block60_c1g{g}_r2", ro, [c for c in cols if (U[c][1], U[c][2]) in prs])
                     else:
                         add(f"sph_block60m_c{co}_r{ro}", ro, cols)
-            fparts.append(to_f32(gen_self_function("sph_self60", 60), "sph_self60", "sph_self60f"))
             files["gen_sphere60_f32.cuh"] = "\n\n".join(fparts) + "\n"
     # boundary stress kernels: one function per (order, W tuple, dof) and the
-    # post-processing variant (order 0, all dofs)
+    # post-processing variant (order 0, all dofs); the library's kernels take moments and
+    # contractions of them instead (bem_moments.cuh, bem_contract.cuh), which the tests compare
     parts = [FILE_HEAD]
     for o in range(3):
         Ws = [()] if o == 0 else ([(w,) for w in range(3)] if o == 1 else
@@ -769,10 +769,11 @@ def generate(out_dir: str | None = None) -> dict:
                 wn = "".join(str(v) for v in W)
                 parts.append(gen_bem_stress_function(f"bem_stress_o{o}_w{wn}_n{n}", o, W, [n]))
     parts.append(gen_bem_stress_function("bem_stress_post", 0, (), [0, 1, 2]))
-    files["gen_bem.cuh"] = "\n\n".join(parts) + "\n"
+    test_files = {"gen_bem.cuh": "\n\n".join(parts) + "\n"}
     files["gen_mf60.cuh"] = codegen_mf60.generate_source()
-    for fn, src in files.items():
-        path = os.path.join(out_dir, fn)
+    tests = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "tests", "hostgen")
+    for fn, src in (files | test_files if os.path.isdir(tests) else files).items():
+        path = os.path.join(tests if fn in test_files else out_dir, fn)
         old = open(path).read() if os.path.exists(path) else None
         if old != src:
             with open(path, "w") as f:

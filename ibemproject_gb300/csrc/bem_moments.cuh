@@ -2,7 +2,7 @@
 // of R over an element, for one (particle, element) pair.
 //
 // Every entry of the stress kernels and their first two gradients (get_for_stress_BEM*,
-// restated per entry by gen_bem.cuh) is a combination of derivatives of R = |y - P|: with
+// restated per entry by codegen.gen_bem_stress_function) is a combination of derivatives of R = |y - P|: with
 // G_ij = A d_ij / R - B R_,ij, p = 1/R (p_,a = 1/2 R_,aii) and R biharmonic,
 //   Dst[kl][n] =  dlam d_kl (A - 2B) p_,nW + dmu [A (d_nk p_,lW + d_nl p_,kW) - 2B R_,nklW]
 //   Dsu[kl][n] =  n_m { dlam d_kl 2 mu0 (A - 2B) p_,mnW + dmu [2 lam0 (A - 2B) d_mn p_,klW
