@@ -43,8 +43,10 @@ struct DeviceArray {   // memory of the library's pool, allocated on the configu
   ~DeviceArray() { reset(); }
   void reset() {
     if (p) {
-      cudaDeviceSynchronize();   // cudaFree waits for nothing when it gives pool memory back
-      cudaFree(p);
+      // its own stream may be gone: once nothing runs, any stream will do (cudaFree would leave the
+      // pool counting it as in use)
+      cudaDeviceSynchronize();
+      cudaFreeAsync(p, nullptr);
     }
     p = nullptr;
     n = 0;
