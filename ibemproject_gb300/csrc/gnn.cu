@@ -671,6 +671,7 @@ struct Net {
   int64_t E;
   cudaStream_t st;
   Layout L;
+  int sms = 0;                                       // of the device
   void* mem = nullptr;                               // all buffers, one stream-ordered allocation
   std::vector<std::pair<float**, int64_t>> want;     // the buffers asked for, in order
   float *H[kGnnLayers + 1], *Ein[kGnnLayers], *Mm[kGnnLayers], *Uin[kGnnLayers], *Upd[kGnnLayers];
@@ -680,6 +681,9 @@ struct Net {
   ~Net() { free_async(mem, st); }
   void buf(float*& p, int64_t n) { want.push_back({&p, (std::max<int64_t>(n, 1) + 63) / 64 * 64}); }
   ibem_status alloc(bool backward) {
+    int dev = 0;
+    IBEM_CUDA(cudaGetDevice(&dev));
+    IBEM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     for (int l = 0; l <= kGnnLayers; ++l) buf(H[l], (int64_t)num * kH);
     for (int l = 0; l < kGnnLayers; ++l) {
       buf(Ein[l], E * kEin);
@@ -725,7 +729,7 @@ struct Net {
     // slices of M: about two CTAs per SM in total, at least 64 rows each (with 512 rows each a
     // gradient of 1,500 particles ran on 2 to 6 CTAs; the nine of a step 1.28 -> 0.18 ms)
     const int tiles = ((N + kGT - 1) / kGT) * ((K + kGT - 1) / kGT);
-    const int splits = std::max(1, std::min((2 * 152 + tiles - 1) / tiles, M / 64));
+    const int splits = std::max(1, std::min((2 * sms + tiles - 1) / tiles, M / 64));
     dim3 g((N + kGT - 1) / kGT, (K + kGT - 1) / kGT, splits);
     ::ibem::count_launch(), k_gemm<true, false><<<g, 256, 0, st>>>(K, N, M, X, K, dZ, N, gW, N, nullptr, 0, 1);
     ::ibem::count_launch(), k_colsum<<<dim3(std::max(1, std::min(512, M / 64)), (N + 63) / 64), 256, 0, st>>>(M, N, dZ, gb);

@@ -347,8 +347,8 @@ ibem_status launch_field24(const SphLaunch& p, const double* pts, int nump, cons
   SphMat mc = sph_mat_init(p.E0, p.nu0, p.E1, p.nu1);
   ProfScope ps(PROF_FIELD, st);
   // slices of the spheres: about 16 CTAs per SM in total, so that the SMs with one more than the
-  // others cost little, and at least two chunks a slice.  The sums of the slices take at most
-  // 17 x 152 x 128 x 52 bytes; without room for them one slice does.
+  // others cost little, and at least two chunks a slice.  The sums of the slices take less than
+  // 32 x SMs x 128 x 52 bytes (32 MB at 152 SMs); without room for them one slice does.
   int dev = 0, sms = 0;
   IBEM_CUDA(cudaGetDevice(&dev));
   IBEM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
