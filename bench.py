@@ -251,11 +251,11 @@ def roofline_chosen(prof, case):
 # whose points are far from every sphere, 2.431e10 flops / 6.554e7 pairs).
 FIELD_ALG_FLOPS_PER_PAIR = 370.9
 # Executed FP32 flops per pair on this workload (the same count over both kernels of one
-# full-size call, double-float within 12 radii: 1.731e11 far + 1.592e11 near = 3.323e11 /
+# full-size call, double-float within 12 radii: 1.731e11 far + 1.419e11 near = 3.150e11 /
 # 5.243e8 pairs) and the call's DRAM bytes (read + write of both kernels) from the same capture.
-FIELD_DF_FLOPS_PER_PAIR = 633.8
-FIELD_DF_TRAFFIC_PER_LAUNCH = 43.59e6
-FIELD_DF_SOURCE = "profiles/field24_far_near_bench2000.md"
+FIELD_DF_FLOPS_PER_PAIR = 600.8
+FIELD_DF_TRAFFIC_PER_LAUNCH = 43.97e6
+FIELD_DF_SOURCE = "profiles/kernels_small_cases.md"
 
 
 # ------------------------------------------------------------------ clocks

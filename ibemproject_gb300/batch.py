@@ -244,7 +244,7 @@ def training_pairs(batch: DeviceBatch, nrhs: int, seed: int = 0):
 
 def training_pairs_mf(batch: DeviceBatch, nrhs: int, seed: int = 0, tol: float = 1e-10):
     """The pairs of training_pairs for microstructures too large for the dense LU (a
-    2,000-sphere system is 60 s in FP64): e_hat = As^-1 r_hat from the matrix-free solver
+    2,000-sphere system takes 3.5 s and 37 GB in FP64): e_hat = As^-1 r_hat from the matrix-free solver
     with block-Jacobi preconditioning and FP64 refinement to relative residual tol, i.e.
     ||r_hat - As e_hat|| <= tol ||r_hat|| per realisation."""
     import torch

@@ -25,7 +25,7 @@
 // (solver.cu).  A row or column that holds an infinity or NaN gives NaN in its whole row or
 // column of C.
 //
-// Measured (random normal entries): 3600^3 29 TFLOP/s, 8192 x 8192 x 2048 32 TFLOP/s (the FP64
+// Measured (random normal entries): 3600^3 28 TFLOP/s, 8192 x 8192 x 2048 31 TFLOP/s (the FP64
 // pipe gives 1.2), rms error 7e-18 and 9e-18 of sum |a||b| where FP64 multiply-adds give 5e-17.
 //
 // Kernels: k_split64 makes the digit planes (one pass for the exponents, one for the digits,

@@ -1286,7 +1286,10 @@ ibem_status mf_apply_f64(const MfBatch& b, const double* x, double* y, cudaStrea
   // of the largest term, the level of the FP64 rounding of the near pairs (measured: split
   // against all pairs in FP64 6.6e-16 relative, 5.2e-16 with 8 radii, 1.7e-14 for
   // double-float everywhere).  In realisations below kMfSplitMin particles most (warp,
-  // source) pairs are near, and one FP64 launch over every pair is faster than the two passes
+  // source) pairs are near, and one FP64 launch over every pair is faster than the two passes:
+  // 900 spheres 0.73 and 0.90 ms, 1,280 1.55 and 1.16 ms, 20,000 395 and 94 ms.  Skipping near
+  // sources in the far pass against evaluating them with zero coefficients: 2,000 spheres 1.76 and
+  // 1.69 ms, 5,000 7.3 and 8.1 ms
   const bool split = b.max_seg >= kMfSplitMin;
   ::ibem::count_launch(), k_mf_apply_f64<<<dim3(b.ntiles, b.split_wide.slices, b.split_wide.pieces), kMfThreads, 0, st>>>(
       b.tiles, b.seg_begin, mask, mask_on, b.cen, b.rad, b.mats, x, y, b.perm, split ? 1 : 0);

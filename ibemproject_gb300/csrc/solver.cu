@@ -1317,7 +1317,7 @@ ibem_status gemm_sub<double>(int64_t m, int64_t n, int64_t k, const double* A, i
   if (m <= 0 || n <= 0 || k <= 0) return IBEM_OK;
   // tensor cores from 32 in every dimension: a 64 x 64 SIMT tile takes 1.08 us per unit of k on
   // the FP64 pipe (34 us at k = 32), a whole tensor-core call of that size 25 us (300 spheres,
-  // N = 7,200: all updates 246 ms on the FP64 pipe, 29 ms on the tensor cores)
+  // N = 7,200: all updates 246 ms on the FP64 pipe, 30 ms on the tensor cores)
   if (w.gemm_ws && m >= 32 && n >= 32 && k >= 32)
     return gemm_sub_f64_tc(m, n, k, A, lda, B, ldb, C, ldc, w.gemm_ws, w.gemm_ws_bytes, w.gemm_err, st);
   ProfScope ps(PROF_GEMM_SIMT, st, 2.0 * m * n * k);

@@ -297,10 +297,10 @@ ibem_status ibem_e3d_mf_solve(const ibem_e3d_batch* batch, const double* b_dev, 
                               const ibem_mf_options* opt, ibem_mf_report* reports, void* stream);
 
 /* The same for quadratic eigenstrain (layout 60: orders 0, 1 and 2, 60 unknowns per sphere,
- * integratorElastic3D.cpp:341-682) or layout 24: every 60 x 60 pair block is evaluated
- * inside the products from the same generated code as ibem_e3d_pair_blocks(layout 60), in
- * FP32 for the GMRES products and in FP64 for the refinement residuals (both of them; there
- * is no double-float form of layout 60).  Layout 60 takes IBEM_PRECOND_BLOCK_JACOBI only (the
+ * integratorElastic3D.cpp:341-682) or layout 24: every 60 x 60 pair product is taken in the
+ * frame of the pair's offset (for a centre inside another sphere from the generated code of
+ * ibem_e3d_pair_blocks(layout 60)), in FP32 for the GMRES products and in FP64 for the
+ * refinement residuals (both of them; there is no double-float form of layout 60).  Layout 60 takes IBEM_PRECOND_BLOCK_JACOBI only (the
  * realisation's own 60 x 60 block, the same for all its spheres in the scaled system).
  * b_dev, x_dev: layout * seg_begin[nseg] doubles. */
 ibem_status ibem_e3d_mf_solve_layout(const ibem_e3d_batch* batch, int layout, const double* b_dev,
