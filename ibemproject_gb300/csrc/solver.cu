@@ -5,7 +5,8 @@
 // spans ~47 decades, which partial pivoting alone cannot handle (full pivoting can).
 //
 //   IBEM_SOLVE_FP64      LU with partial pivoting of the scaled matrix in FP64 (trailing updates
-//                        on the tensor cores, gemm_tc64.cu) and one step of refinement.
+//                        on the tensor cores, gemm_tc64.cu; a nearly singular matrix once more
+//                        with FP64 updates) and one step of refinement.
 //   IBEM_SOLVE_MIXED_IR  LU with partial pivoting in FP32 (trailing updates on the tensor
 //                        cores with the split-BF16 "x3" scheme, FP32 accumulation), then
 //                        FP64 GMRES iterative refinement preconditioned by the FP32 factors;
@@ -1414,8 +1415,9 @@ static ibem_status lu_rec(T* A, int64_t lda, int64_t N, int64_t k0, int64_t n, L
   return lu_rec(A, lda, N, k0 + n1, n2, w, st);
 }
 
+// tc: with the workspace of the tensor-core updates
 template <typename T>
-static ibem_status lu_alloc(LuWork<T>& w, int64_t N) {
+static ibem_status lu_alloc(LuWork<T>& w, int64_t N, bool tc = true) {
   int dev = 0, nsm = 0;
   IBEM_CUDA(cudaGetDevice(&dev));
   IBEM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -1451,7 +1453,7 @@ static ibem_status lu_alloc(LuWork<T>& w, int64_t N) {
     IBEM_CUDA(pool_alloc(&w.gemm_ws, w.gemm_ws_bytes, w.st));
     IBEM_CUDA(pool_alloc(&w.gemm_err, sizeof(int), w.st));
     IBEM_CUDA(cudaMemsetAsync(w.gemm_err, 0, sizeof(int), w.st));
-  } else {
+  } else if (tc) {
     w.gemm_ws_bytes = gemm_tc64_workspace_bytes(N, N / 2 + 2 * kLeaf);
     if (pool_alloc(&w.gemm_ws, w.gemm_ws_bytes, w.st) != cudaSuccess) {   // no room: the updates stay on the FP64 pipe
       cudaGetLastError();
@@ -1872,19 +1874,54 @@ static ibem_status equilibrate(SolveCtx& cx, const double* A, int64_t lda) {
   return IBEM_OK;
 }
 
+// out[0], out[1] = smallest and largest |u_ii| (one CTA)
+__global__ void __launch_bounds__(256) k_pivot_range(int64_t n, const double* __restrict__ F, double* __restrict__ out) {
+  __shared__ double lo[256], hi[256];
+  double a = INFINITY, b = 0.0;
+  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+    const double v = fabs(F[i * (n + 1)]);
+    a = fmin(a, v);
+    b = fmax(b, v);
+  }
+  lo[threadIdx.x] = a;
+  hi[threadIdx.x] = b;
+  __syncthreads();
+  for (int t = blockDim.x / 2; t > 0; t >>= 1) {
+    if (threadIdx.x < t) {
+      lo[threadIdx.x] = fmin(lo[threadIdx.x], lo[threadIdx.x + t]);
+      hi[threadIdx.x] = fmax(hi[threadIdx.x], hi[threadIdx.x + t]);
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[0] = lo[0], out[1] = hi[0];
+}
+// Whether a pivot is as small as what the tensor-core updates round away (N 2^-53 of the largest)
+static ibem_status pivot_in_noise(const double* W, int64_t N, LuWork<double>& w, bool& yes, cudaStream_t st) {
+  double h[2];
+  ::ibem::count_launch(), k_pivot_range<<<1, 256, 0, st>>>(N, W, w.tmp);
+  IBEM_LAUNCH_CHECK("pivot range");
+  IBEM_CUDA(cudaMemcpyAsync(h, w.tmp, sizeof h, cudaMemcpyDeviceToHost, st));
+  IBEM_CUDA(cudaStreamSynchronize(st));
+  yes = h[0] <= (double)N * 0x1p-53 * h[1];
+  return IBEM_OK;
+}
+
+// W set on entry: A is factorised once more, from the same scalings
 template <typename T>
-static ibem_status factor(SolveCtx& cx, const double* A, int64_t lda, T*& W, LuWork<T>& w, int& info) {
+static ibem_status factor(SolveCtx& cx, const double* A, int64_t lda, T*& W, LuWork<T>& w, int& info, bool tc = true) {
   const int64_t N = cx.N;
-  IBEM_CUDA(pool_alloc(&W, sizeof(T) * (size_t)N * N, cx.st));
+  const bool again = W != nullptr;
+  if (!again) IBEM_CUDA(pool_alloc(&W, sizeof(T) * (size_t)N * N, cx.st));
   w.st = cx.st;
   {
     ProfScope ps(PROF_EQUIL, cx.st);
-    if (ibem_status q = equilibrate(cx, A, lda)) return q;
+    if (!again)
+      if (ibem_status q = equilibrate(cx, A, lda)) return q;
     dim3 g((unsigned)((N + 255) / 256), (unsigned)std::min<int64_t>(N, 65535));
     ::ibem::count_launch(), k_scale_copy<T><<<g, 256, 0, cx.st>>>(N, A, lda, cx.r, cx.c, W, N);
     IBEM_LAUNCH_CHECK("equilibrate");
   }
-  ibem_status s = lu_alloc(w, N);
+  ibem_status s = lu_alloc(w, N, tc);
   if (s) return s;
   s = lu_rec<T>(W, N, N, 0, N, w, cx.st);
   if (!s) s = trsv_prepare<T>(W, N, N, w, cx.st);
@@ -2036,6 +2073,18 @@ ibem_status solve_dense(ibem_solver_form form, int64_t N, double* A, int64_t lda
     LuWork<double> w;
     int info = 0;
     s = factor<double>(cx, A, lda, W, w, info);
+    // A system with equations that are multiples of one another ends in a zero pivot when row minus
+    // multiple cancels operation by operation, as FP64 updates do; the tensor-core updates round
+    // the sum of the products instead, and leave a pivot of that size.  Such a factorisation is
+    // done over with FP64 updates, which then decide whether the system is refused.
+    if (!s && !info && w.gemm_ws && N >= kLeaf) {
+      bool noise = false;
+      s = pivot_in_noise(W, N, w, noise, st);
+      if (!s && noise) {
+        lu_free(w);
+        s = factor<double>(cx, A, lda, W, w, info, false);
+      }
+    }
     cudaEventRecord(e1, st);
     if (!s && info) { R.info = info; s = fail(IBEM_ERR_SINGULAR, "zero pivot in the FP64 factorisation"); }
     if (!s) {
